@@ -21,9 +21,9 @@ vp = C.c_void_p
 
 
 def reference_tree(tree: str | None = None) -> str | None:
-    """The reference's source tree: the argument, else $ISC_REFERENCE_TREE; None when neither names a directory."""
+    """The reference's source tree: the argument, else $ISC_REFERENCE_TREE; None when neither holds its sources."""
     tree = tree or os.environ.get("ISC_REFERENCE_TREE")
-    return tree if tree and os.path.isdir(tree) else None
+    return tree if tree and os.path.isdir(os.path.join(tree, "adapter")) else None
 
 
 def build(reference: bool = True, tree: str | None = None) -> None:
