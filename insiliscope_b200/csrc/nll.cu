@@ -12,8 +12,8 @@
 // then the chain through phi (x, y, z, Zernike), dNLL/dN = sum w PSF, dNLL/db = sum w.
 //
 // One CTA per emitter at a time (a persistent grid): the pupil phase in float64, reduced mod 2 pi, then float32
-// sincos; the four complex matmuls (forward 32x32 -> 32x64 -> 64x64, adjoint back) in shared memory in float32; the
-// per-emitter sums in float64. The gradient pass recomputes the field instead of storing per-emitter PSFs. The
+// sincos; the four products (forward 32x32 -> 32x64 -> 64x64, adjoint back) folded about the ROI's centre, in float32;
+// the per-emitter sums in float64. The gradient pass recomputes the field instead of storing per-emitter PSFs. The
 // Zernike gradient accumulates per CTA in float64 across its emitters and is added once per CTA.
 
 #include "iscu_internal.h"
@@ -31,7 +31,7 @@ struct iscu_nll_model
    double kappa = 0.0;
    iscu::DevBuf samples;   // M*M x double4: (p kx, p ky, kz, a)
    iscu::DevBuf basis;     // J x M*M float64: 2 pi Z_j
-   iscu::DevBuf A;         // P x M float2
+   iscu::DevBuf cs;        // the folded transform's cosines and sines (NllTables)
    iscu::DevBuf zphase;    // M*M float64: 2 pi sum c_j Z_j of the current evaluation
    iscu::DevBuf zern;      // J float64
 };
@@ -40,61 +40,37 @@ namespace iscu {
 
 namespace {
 
-constexpr int kM = 32, kP = 64, kThreads = 256, kMaxJ = 32;
-constexpr int kPre = 4;   // observed counts a thread loads ahead (ROIs up to 32 x 32 pixels)
+constexpr int kM = 32, kP = 64, kThreads = 128, kMaxJ = 32;
+constexpr int kCtasPerSm = 4;
+// The aperture is the samples of |q| <= kQ, q = m - 16 on each axis (dk = 2 kMax / 28 puts its radius at 14 samples).
+constexpr int kQ = 14, kR = 2 * kQ + 1, kQuad = (kQ + 1) * (kQ + 1);
+constexpr int kT = kP / 2;          // sample pairs per axis
+constexpr int kTp = kT + 1;         // row pitch of T in float4 (a row's lanes 4 banks apart: conflict-free)
 
-__device__ __forceinline__ float2 Cmul(float2 a, float2 b)
+// Two-lane float32 arithmetic: each lane rounds as the one-lane instruction.
+__device__ __forceinline__ uint64_t Dup(float v)
 {
-   return make_float2(a.x * b.x - a.y * b.y, a.x * b.y + a.y * b.x);
+   uint64_t d;
+   asm("mov.b64 %0, {%1, %1};" : "=l"(d) : "r"(__float_as_uint(v)));
+   return d;
 }
 
-__device__ __forceinline__ void Cfma(float2& acc, float2 a, float2 b)
+__device__ __forceinline__ float2 Unpack(uint64_t v)
 {
-   acc.x = fmaf(a.x, b.x, acc.x);
-   acc.x = fmaf(-a.y, b.y, acc.x);
-   acc.y = fmaf(a.x, b.y, acc.y);
-   acc.y = fmaf(a.y, b.x, acc.y);
+   uint32_t lo, hi;
+   asm("mov.b64 {%0, %1}, %2;" : "=r"(lo), "=r"(hi) : "l"(v));
+   return make_float2(__uint_as_float(lo), __uint_as_float(hi));
 }
 
-// C[r][c] = sum_k L(r, k) R(k, c) over a ROWS x COLS output, a TR x TC tile per thread (rows ty + 16 i, columns
-// tx + 16 j); epi(r, c, value) stores.
-template <int ROWS, int COLS, int K, class LF, class RF, class EF>
-__device__ __forceinline__ void SmemGemm(LF L, RF R, EF epi)
+__device__ __forceinline__ uint64_t Fma2(uint64_t a, uint64_t b, uint64_t c)
 {
-   constexpr int TR = ROWS / 16, TC = COLS / 16;
-   static_assert(TR * 16 == ROWS && TC * 16 == COLS, "16 x 16 threads");
-   const int tx = threadIdx.x & 15, ty = threadIdx.x >> 4;
-   float2 acc[TR][TC];
-#pragma unroll
-   for (int i = 0; i < TR; ++i)
-#pragma unroll
-      for (int j = 0; j < TC; ++j)
-         acc[i][j] = make_float2(0.f, 0.f);
-#pragma unroll 4
-   for (int k = 0; k < K; ++k)
-   {
-      float2 l[TR], r[TC];
-#pragma unroll
-      for (int i = 0; i < TR; ++i)
-         l[i] = L(ty + 16 * i, k);
-#pragma unroll
-      for (int j = 0; j < TC; ++j)
-         r[j] = R(k, tx + 16 * j);
-#pragma unroll
-      for (int i = 0; i < TR; ++i)
-#pragma unroll
-         for (int j = 0; j < TC; ++j)
-            Cfma(acc[i][j], l[i], r[j]);
-   }
-#pragma unroll
-   for (int i = 0; i < TR; ++i)
-#pragma unroll
-      for (int j = 0; j < TC; ++j)
-         epi(ty + 16 * i, tx + 16 * j, acc[i][j]);
+   uint64_t d;
+   asm("fma.rn.f32x2 %0, %1, %2, %3;" : "=l"(d) : "l"(a), "l"(b), "l"(c));
+   return d;
 }
 
-// Sums of NV float64 values over the CTA in one exchange, each in BlockSum's order (every thread calls it; every
-// thread gets the sums). red: NV x (kThreads / 32) doubles.
+// Sums of NV float64 values over the CTA in one exchange (every thread calls it; every thread gets the sums). red:
+// NV x (kThreads / 32) doubles.
 template <int NV>
 __device__ __forceinline__ void BlockSums(double (&v)[NV], double* red)
 {
@@ -121,24 +97,6 @@ __device__ __forceinline__ void BlockSums(double (&v)[NV], double* red)
    }
 }
 
-// Sum over the CTA in float64 (every thread calls it; the result is returned to every thread).
-__device__ __forceinline__ double BlockSum(double v, double* red)
-{
-#pragma unroll
-   for (int d = 16; d > 0; d >>= 1)
-      v += __shfl_xor_sync(0xffffffffu, v, d);
-   const int lane = threadIdx.x & 31, warp = threadIdx.x >> 5;
-   __syncthreads();
-   if (lane == 0)
-      red[warp] = v;
-   __syncthreads();
-   double s = 0.0;
-#pragma unroll
-   for (int w = 0; w < kThreads / 32; ++w)
-      s += red[w];
-   return s;
-}
-
 __global__ void ZernPhaseKernel(const double* __restrict__ basis, const double* __restrict__ zern, int J, int MM,
                                 double* __restrict__ zphase)
 {
@@ -155,7 +113,7 @@ struct NllArgs
 {
    const double4* samples;
    const double* basis;
-   const float2* A;
+   const float* cs;          // the folded transform's cosines and sines (NllTables)
    const double* zphase;
    int J, R, os;
    double kappa;
@@ -173,37 +131,101 @@ struct NllArgs
    int* err;                 // 1: an emitter names a frame outside the batch
 };
 
-struct NllSmem
+// cos / sin of q theta (t + 1/2), theta = dk p / os, laid out as the products read them: fwd[q - 1][w] the cosines then
+// the sines of t = 8 w .. 8 w + 7 (q = 1 .. kQ), adj[t][w] those of q = 4 w .. 4 w + 3 (q beyond kQ: zeros).
+struct NllTables
 {
-   float2 A[kP][kM];
-   float2 At[kM][kP];     // A transposed: the first product reads it along rows (conflict-free) instead of down A's
-                          // columns (16 lanes 256 bytes apart, one bank)
-   float2 U[kM][kM];
-   float2 T[kM][kP];
-   float2 E[kP][kP];
-   float dphi[kM * kM];
-   double dphiSum[kM * kM];   // the CTA's emitters' dNLL/dphi, summed in float64, for the Zernike gradient
-   double red[3 * (kThreads / 32)];
+   float fwd[kQ][4][16];
+   float adj[kT][4][8];
 };
 
-template <bool kGrad>
-__global__ void __launch_bounds__(kThreads, 2) NllKernel(NllArgs a)
+struct NllSmem
+{
+   NllTables tab;
+   float4 T[kR][kTp];         // T, then its adjoint: row r, sample pair t
+   union
+   {
+      float4 U[kQ + 1][32];   // the folded pupil, then its adjoint: (P.re, P.im, N.re, N.im) of column pair q, row r
+      struct
+      {
+         float4 C[kT / 2][32], S[kT / 2][32];   // half of the weighted field's row sums and differences
+      } E;
+      double blk[64 + 64];    // ROIs of at most 4 x 4 pixels: the 8 x 8-sample blocks' sums, the pixels' weights
+   };
+   float4 Uraw[2][kQuad];     // the pupil: (+y +x, +y -x), (-y +x, -y -x) of each quadrant sample
+   double dphiSum[4][kQuad];  // the CTA's emitters' dNLL/dphi, summed in float64, for the Zernike gradient
+   double red[5 * (kThreads / 32)];
+};
+
+// One pixel's likelihood terms from its sample sum: the expected counts, the NLL's term and, for the gradient, the
+// sums' terms and the samples' weight.
+struct PixelSums
+{
+   double part = 0.0, gN = 0.0, gB = 0.0;
+};
+
+// NP pixels of a thread in stages, so that their float64 chains (the logarithm, the quotient) run side by side.
+template <bool kGrad, int NP>
+__device__ __forceinline__ void Pixels(const NllArgs& a, uint32_t e, const int (&p)[NP], const bool (&on)[NP],
+                                       const float (&sum)[NP], double N, double b, PixelSums& s, float (&G)[NP])
+{
+   const size_t base = static_cast<size_t>(e) * a.R * a.R;
+   float k[NP];
+   double mu[NP], lg[NP];
+#pragma unroll
+   for (int q = 0; q < NP; ++q)
+      k[q] = on[q] ? __ldg(a.counts + base + p[q]) : 0.f;
+#pragma unroll
+   for (int q = 0; q < NP; ++q)
+      mu[q] = on[q] ? N * (a.kappa * static_cast<double>(sum[q])) + b : 1.0;
+#pragma unroll
+   for (int q = 0; q < NP; ++q)
+      lg[q] = log(mu[q]);
+#pragma unroll
+   for (int q = 0; q < NP; ++q)
+   {
+      const double kk = static_cast<double>(k[q]);
+      if (on[q])
+      {
+         s.part += mu[q] - kk * lg[q];
+         if (a.mu)
+            a.mu[base + p[q]] = static_cast<float>(mu[q]);
+      }
+      if (kGrad)
+      {
+         const double w = on[q] ? 1.0 - kk / mu[q] : 0.0;
+         s.gN += w * (a.kappa * static_cast<double>(sum[q]));
+         s.gB += w;
+         G[q] = static_cast<float>(w * N * a.kappa);
+      }
+   }
+}
+
+// A CTA of four warps takes an emitter at a time; OS: the samples per pixel and axis (1, 2, 4, 8; 0: 16 and more).
+//
+// Both products are folded. The samples are symmetric about the ROI's centre (their common phase ramp goes into the
+// pupil as a shift by half the ROI), so exp(i q theta tau) of +-q and +-tau are one cosine and one sine: a row of U
+// is folded into P = U[q] + U[-q] and N = U[q] - U[-q], and C = sum cos P, S = sum sin N give the samples C + i S at
+// +tau and C - i S at -tau -- real by complex products of a quarter of the size. With the aperture's 29 of the 32
+// samples an emitter's four products take 334 K multiply-adds instead of 1.57 M, exactly the same sums.
+//
+// What bounds it: shared-memory reads and FP32 multiply-adds about equally (each product reads its constants by
+// broadcast -- a warp's t or q group is the same for its lanes -- and its data once per lane, 16 bytes at a time),
+// then the float64 logarithm of each pixel. 128 threads and 55 KB, four CTAs per SM, so that one CTA's products run
+// under another's logarithms and barriers.
+template <bool kGrad, int OS>
+__global__ void __launch_bounds__(kThreads, kCtasPerSm) NllKernel(NllArgs a)
 {
    extern __shared__ __align__(16) unsigned char smemRaw[];
    NllSmem& s = *reinterpret_cast<NllSmem*>(smemRaw);
-   const int tid = threadIdx.x;
-   for (int i = tid; i < kP * kM; i += kThreads)
-   {
-      s.A[i / kM][i % kM] = a.A[i];
-      s.At[i % kM][i / kM] = a.A[i];
-   }
-   // the Zernike gradient is linear in dNLL/dphi: the CTA sums dphi over its emitters (float64, each sample by one
-   // thread) and projects the sum onto the modes once, at the end
-   for (int m = tid; m < kM * kM; m += kThreads)
-      s.dphiSum[m] = 0.0;
+   const int tid = threadIdx.x, lane = tid & 31, warp = tid >> 5;
+   for (int i = tid; i < static_cast<int>(sizeof(NllTables) / sizeof(float)); i += kThreads)
+      reinterpret_cast<float*>(&s.tab)[i] = a.cs[i];
+   if (kGrad)
+      for (int m = tid; m < 4 * kQuad; m += kThreads)
+         s.dphiSum[m / kQuad][m % kQuad] = 0.0;
    double nllAcc = 0.0;
-   const int R = a.R, os = a.os, RR = R * R;
-   __syncthreads();
+   const int R = a.R, RR = R * R;
    for (uint32_t e = blockIdx.x; e < a.n; e += gridDim.x)
    {
       const float4 pr = a.params[e];
@@ -212,189 +234,419 @@ __global__ void __launch_bounds__(kThreads, 2) NllKernel(NllArgs a)
       if (!frameOk && tid == 0)
          atomicExch(a.err, 1);
       const double b = frameOk ? static_cast<double>(a.bg[f]) : 0.0;
-      const double x = pr.x, y = pr.y, z = pr.z, N = pr.w;
-      // the observed counts of this thread's pixels p = tid + 256 q, loaded now so that their latency passes under
-      // the pupil and the forward products (ROIs of up to 32 x 32 pixels: at most four a thread)
-      const float* k = a.counts + static_cast<size_t>(e) * RR;
-      const bool pre = RR <= kPre * kThreads;
-      float kpre[kPre];
-#pragma unroll
-      for (int q = 0; q < kPre; ++q)
-         kpre[q] = pre && tid + q * kThreads < RR ? k[tid + q * kThreads] : 0.f;
-      // 1. the pupil
-      for (int m = tid; m < kM * kM; m += kThreads)
+      // the position from the ROI's centre: the samples' common ramp
+      const double x = static_cast<double>(pr.x) - 0.5 * R, y = static_cast<double>(pr.y) - 0.5 * R, z = pr.z, N = pr.w;
+      // the next emitter's counts on their way to L2 while this one computes
+      if (e + gridDim.x < a.n && tid * 32 < RR)
+         asm volatile("prefetch.global.L2 [%0];" ::"l"(a.counts + static_cast<size_t>(e + gridDim.x) * RR + tid * 32));
+      // 1. the pupil, folded: a thread per quadrant sample and its mirrors
+      for (int qd = tid; qd < kQuad; qd += kThreads)
       {
-         const double4 sm = a.samples[m];
-         const double ph = ReduceTwoPi(z * sm.z + a.zphase[m] - (sm.x * x + sm.y * y));
-         float sn, cs;
-         __sincosf(static_cast<float>(ph), &sn, &cs);
+         const int qy = qd / (kQ + 1), qx = qd % (kQ + 1), m0 = kM / 2 * kM + kM / 2;
+         const double4 sm = a.samples[m0 + qy * kM + qx];
+         const double zk = z * sm.z, ax = sm.x * x, ay = sm.y * y;
          const float amp = static_cast<float>(sm.w);
-         s.U[m / kM][m % kM] = make_float2(amp * cs, amp * sn);
-      }
-      __syncthreads();
-      // 2. T = U A^T (32 x 64), 3. E = A T (64 x 64)
-      SmemGemm<kM, kP, kM>([&](int r, int k) { return s.U[r][k]; }, [&](int k, int c) { return s.At[k][c]; },
-                           [&](int r, int c, float2 v) { s.T[r][c] = v; });
-      __syncthreads();
-      SmemGemm<kP, kP, kM>([&](int r, int k) { return s.A[r][k]; }, [&](int k, int c) { return s.T[k][c]; },
-                           [&](int r, int c, float2 v) { s.E[r][c] = v; });
-      __syncthreads();
-      // 4. expected counts and the likelihood; the gradient weights into E
-      double part = 0.0, gN = 0.0, gB = 0.0;
-      auto pixel = [&](int p, float kf) {
-         const int i = p / R, j = p % R;
-         float sum = 0.f;
-         for (int ty = 0; ty < os; ++ty)
-            for (int tx = 0; tx < os; ++tx)
+         float2 u[2][2];
+#pragma unroll
+         for (int iy = 0; iy < 2; ++iy)
+#pragma unroll
+            for (int ix = 0; ix < 2; ++ix)
             {
-               const float2 v = s.E[i * os + ty][j * os + tx];
-               sum = fmaf(v.x, v.x, fmaf(v.y, v.y, sum));
+               const int m = m0 + (iy ? -qy : qy) * kM + (ix ? -qx : qx);
+               const double ph = ReduceTwoPi(zk + a.zphase[m] - ((ix ? -ax : ax) + (iy ? -ay : ay)));
+               float sn, cs;
+               __sincosf(static_cast<float>(ph), &sn, &cs);
+               const float am = (iy && qy == 0) || (ix && qx == 0) ? 0.f : amp;   // one sample on an axis, not two
+               u[iy][ix] = make_float2(am * cs, am * sn);
             }
-         const double psf = a.kappa * static_cast<double>(sum);
-         const double mu = N * psf + b;
-         const double kk = static_cast<double>(kf);
-         part += mu - kk * log(mu);
-         if (a.mu)
-            a.mu[static_cast<size_t>(e) * RR + p] = static_cast<float>(mu);
          if (kGrad)
          {
-            const double w = 1.0 - kk / mu;
-            gN += w * psf;
-            gB += w;
-            const float G = static_cast<float>(w * N * a.kappa);
-            for (int ty = 0; ty < os; ++ty)
-               for (int tx = 0; tx < os; ++tx)
-               {
-                  float2& v = s.E[i * os + ty][j * os + tx];
-                  v = make_float2(G * v.x, G * v.y);
-               }
+            s.Uraw[0][qd] = make_float4(u[0][0].x, u[0][0].y, u[0][1].x, u[0][1].y);
+            s.Uraw[1][qd] = make_float4(u[1][0].x, u[1][0].y, u[1][1].x, u[1][1].y);
          }
-      };
-      if (RR == kPre * kThreads)
+         const float2 p0 = make_float2(u[0][0].x + u[0][1].x, u[0][0].y + u[0][1].y);
+         const float2 n0 = make_float2(u[0][0].x - u[0][1].x, u[0][0].y - u[0][1].y);
+         const float2 p1 = make_float2(u[1][0].x + u[1][1].x, u[1][0].y + u[1][1].y);
+         const float2 n1 = make_float2(u[1][0].x - u[1][1].x, u[1][0].y - u[1][1].y);
+         s.U[qx][qy] = make_float4(p0.x + p1.x, p0.y + p1.y, n0.x + n1.x, n0.y + n1.y);
+         if (qy)
+            s.U[qx][kQ + qy] = make_float4(p0.x - p1.x, p0.y - p1.y, n0.x - n1.x, n0.y - n1.y);
+      }
+      __syncthreads();
+      // 2. T = U A^T over the folded rows: lane = row, a warp's eight t
       {
-         // Every thread has kPre pixels (32 x 32 ROIs): the same operations as `pixel`, in stages across its pixels so
-         // that their float64 chains (the logarithm, the quotient) run side by side; each sum takes its terms in the
-         // same order, so the results are the pixel-by-pixel form's.
-         double psf[kPre], mu[kPre], lg[kPre], w[kPre];
+         const int r = min(lane, kR - 1);
+         uint64_t cre[4], cim[4], sre[4], sim[4];
+         const float4 u0 = s.U[0][r];
 #pragma unroll
-         for (int q = 0; q < kPre; ++q)
+         for (int k = 0; k < 4; ++k)
          {
-            const int p = tid + q * kThreads, i = p / R, j = p % R;
-            float sum = 0.f;
-            for (int ty = 0; ty < os; ++ty)
-               for (int tx = 0; tx < os; ++tx)
+            cre[k] = Dup(u0.x);
+            cim[k] = Dup(u0.y);
+            sre[k] = sim[k] = 0;
+         }
+#pragma unroll 2
+         for (int q = 1; q <= kQ; ++q)
+         {
+            const float4 u = s.U[q][r];
+            const ulonglong2* t = reinterpret_cast<const ulonglong2*>(s.tab.fwd[q - 1][warp]);
+            const ulonglong2 c0 = t[0], c1 = t[1], s0 = t[2], s1 = t[3];
+            const uint64_t c[4] = {c0.x, c0.y, c1.x, c1.y}, sn[4] = {s0.x, s0.y, s1.x, s1.y};
+            const uint64_t pr2 = Dup(u.x), pi2 = Dup(u.y), nr2 = Dup(u.z), ni2 = Dup(u.w);
+#pragma unroll
+            for (int k = 0; k < 4; ++k)
+            {
+               cre[k] = Fma2(c[k], pr2, cre[k]);
+               cim[k] = Fma2(c[k], pi2, cim[k]);
+               sre[k] = Fma2(sn[k], nr2, sre[k]);
+               sim[k] = Fma2(sn[k], ni2, sim[k]);
+            }
+         }
+         if (lane < kR)
+#pragma unroll
+            for (int k = 0; k < 4; ++k)
+            {
+               const float2 cr = Unpack(cre[k]), ci = Unpack(cim[k]), sr = Unpack(sre[k]), si = Unpack(sim[k]);
+               s.T[r][8 * warp + 2 * k] = make_float4(cr.x - si.x, ci.x + sr.x, cr.x + si.x, ci.x - sr.x);
+               s.T[r][8 * warp + 2 * k + 1] = make_float4(cr.y - si.y, ci.y + sr.y, cr.y + si.y, ci.y - sr.y);
+            }
+      }
+      __syncthreads();
+      // 3. E = A T: lane = the column pair +-t, a warp's eight row pairs. E[row sign][column sign][row]
+      float2 E[2][2][8];
+      {
+         uint64_t cre[2][4], cim[2][4], sre[2][4], sim[2][4];
+         const float4 t0 = s.T[0][lane];
+#pragma unroll
+         for (int k = 0; k < 4; ++k)
+         {
+            cre[0][k] = Dup(t0.x);
+            cim[0][k] = Dup(t0.y);
+            cre[1][k] = Dup(t0.z);
+            cim[1][k] = Dup(t0.w);
+            sre[0][k] = sim[0][k] = sre[1][k] = sim[1][k] = 0;
+         }
+#pragma unroll 2
+         for (int q = 1; q <= kQ; ++q)
+         {
+            const float4 tp = s.T[q][lane], tn = s.T[kQ + q][lane];
+            const ulonglong2* t = reinterpret_cast<const ulonglong2*>(s.tab.fwd[q - 1][warp]);
+            const ulonglong2 c0 = t[0], c1 = t[1], s0 = t[2], s1 = t[3];
+            const uint64_t c[4] = {c0.x, c0.y, c1.x, c1.y}, sn[4] = {s0.x, s0.y, s1.x, s1.y};
+            {
+               const uint64_t d0 = Dup(tp.x), d1 = Dup(tp.y), d2 = Dup(tp.z), d3 = Dup(tp.w);
+#pragma unroll
+               for (int k = 0; k < 4; ++k)
                {
-                  const float2 v = s.E[i * os + ty][j * os + tx];
-                  sum = fmaf(v.x, v.x, fmaf(v.y, v.y, sum));
+                  cre[0][k] = Fma2(c[k], d0, cre[0][k]);
+                  cim[0][k] = Fma2(c[k], d1, cim[0][k]);
+                  cre[1][k] = Fma2(c[k], d2, cre[1][k]);
+                  cim[1][k] = Fma2(c[k], d3, cim[1][k]);
                }
-            psf[q] = a.kappa * static_cast<double>(sum);
-            mu[q] = N * psf[q] + b;
+            }
+            const uint64_t d0 = Dup(tn.x), d1 = Dup(tn.y), d2 = Dup(tn.z), d3 = Dup(tn.w);
+#pragma unroll
+            for (int k = 0; k < 4; ++k)
+            {
+               sre[0][k] = Fma2(sn[k], d0, sre[0][k]);
+               sim[0][k] = Fma2(sn[k], d1, sim[0][k]);
+               sre[1][k] = Fma2(sn[k], d2, sre[1][k]);
+               sim[1][k] = Fma2(sn[k], d3, sim[1][k]);
+            }
          }
 #pragma unroll
-         for (int q = 0; q < kPre; ++q)
-            lg[q] = log(mu[q]);
+         for (int c = 0; c < 2; ++c)
 #pragma unroll
-         for (int q = 0; q < kPre; ++q)
-            w[q] = 1.0 - static_cast<double>(kpre[q]) / mu[q];
-#pragma unroll
-         for (int q = 0; q < kPre; ++q)
-         {
-            const int p = tid + q * kThreads, i = p / R, j = p % R;
-            part += mu[q] - static_cast<double>(kpre[q]) * lg[q];
-            if (a.mu)
-               a.mu[static_cast<size_t>(e) * RR + p] = static_cast<float>(mu[q]);
-            if (kGrad)
+            for (int k = 0; k < 4; ++k)
             {
-               gN += w[q] * psf[q];
-               gB += w[q];
-               const float G = static_cast<float>(w[q] * N * a.kappa);
-               for (int ty = 0; ty < os; ++ty)
-                  for (int tx = 0; tx < os; ++tx)
+               const float2 cr = Unpack(cre[c][k]), ci = Unpack(cim[c][k]), sr = Unpack(sre[c][k]),
+                            si = Unpack(sim[c][k]);
+               E[0][c][2 * k] = make_float2(cr.x - si.x, ci.x + sr.x);
+               E[1][c][2 * k] = make_float2(cr.x + si.x, ci.x - sr.x);
+               E[0][c][2 * k + 1] = make_float2(cr.y - si.y, ci.y + sr.y);
+               E[1][c][2 * k + 1] = make_float2(cr.y + si.y, ci.y - sr.y);
+            }
+      }
+      // 4. expected counts and the likelihood. A pixel's samples: OS of a thread's rows by OS neighbouring lanes; the
+      // lanes exchange their row sums, each takes its share of the pixels and hands their weights back.
+      PixelSums ps;
+      constexpr int kOS = OS ? OS : 8, kG = 8 / kOS, kNp = 4 * kG;   // row groups of a thread; pixels of a lane group
+      float W[kNp];   // pixel n = (group, row sign, column sign)
+#pragma unroll
+      for (int n = 0; n < kNp; ++n)
+      {
+         float v = 0.f;
+#pragma unroll
+         for (int k = 0; k < kOS; ++k)
+         {
+            const float2 q = E[(n >> 1) & 1][n & 1][(n >> 2) * kOS + k];
+            v = fmaf(q.x, q.x, fmaf(q.y, q.y, v));
+         }
+#pragma unroll
+         for (int d = 1; d < kOS; d <<= 1)
+            v += __shfl_xor_sync(0xffffffffu, v, d);
+         W[n] = v;
+      }
+      if (OS)
+      {
+         constexpr int kBatch = kNp >= 4 * kOS ? 4 : (kNp + kOS - 1) / kOS;   // pixels of a lane per stage
+         const int sub = lane % kOS;
+         const int rc = R / 2 + lane / kOS, rr = R / 2 + warp * kG;   // the group's +column, the first +row
+#pragma unroll
+         for (int n0 = 0; n0 < kNp; n0 += kBatch * kOS)
+         {
+            int p[kBatch];
+            bool on[kBatch];
+            float sum[kBatch], G[kBatch];
+#pragma unroll
+            for (int i = 0; i < kBatch; ++i)
+            {
+               sum[i] = 0.f;
+               p[i] = 0;
+               on[i] = false;
+#pragma unroll
+               for (int o = 0; o < kOS; ++o)
+               {
+                  const int n = n0 + i * kOS + o;
+                  if (n < kNp && sub == o)
                   {
-                     float2& v = s.E[i * os + ty][j * os + tx];
-                     v = make_float2(G * v.x, G * v.y);
+                     const int row = (n >> 1) & 1 ? R - 1 - (rr + (n >> 2)) : rr + (n >> 2);
+                     const int col = n & 1 ? R - 1 - rc : rc;
+                     sum[i] = W[n];
+                     p[i] = row * R + col;
+                     on[i] = true;
                   }
+               }
+               G[i] = 0.f;
+            }
+            Pixels<kGrad, kBatch>(a, e, p, on, sum, N, b, ps, G);
+            if (kGrad)
+#pragma unroll
+               for (int i = 0; i < kBatch; ++i)
+#pragma unroll
+                  for (int o = 0; o < kOS; ++o)
+                     if (n0 + i * kOS + o < kNp)
+                        W[n0 + i * kOS + o] = kOS == 1 ? G[i]
+                                                       : __shfl_sync(0xffffffffu, G[i], (lane & ~(kOS - 1)) | o);
+         }
+      }
+      else
+      {
+         // 16 samples a pixel and more: the 8 x 8 grid of 8 x 8-sample blocks through shared memory
+         double* blk = s.blk;
+         const int bc = lane / 8;
+         if (lane % 8 == 0)
+#pragma unroll
+            for (int n = 0; n < 4; ++n)
+               blk[((n >> 1) & 1 ? 3 - warp : 4 + warp) * 8 + (n & 1 ? 3 - bc : 4 + bc)] = W[n];
+         __syncthreads();
+         const int per = 8 / R;   // blocks per pixel and axis
+         int p[1] = {tid};
+         bool on[1] = {tid < RR};
+         float sum[1] = {0.f}, G[1] = {0.f};
+         if (on[0])
+            for (int by = 0; by < per; ++by)
+               for (int bx = 0; bx < per; ++bx)
+                  sum[0] += static_cast<float>(blk[(tid / R * per + by) * 8 + tid % R * per + bx]);
+         Pixels<kGrad, 1>(a, e, p, on, sum, N, b, ps, G);
+         if (kGrad)
+         {
+            if (on[0])
+               blk[64 + tid] = G[0];
+            __syncthreads();
+#pragma unroll
+            for (int n = 0; n < 4; ++n)
+               W[n] = static_cast<float>(blk[64 + ((n >> 1) & 1 ? 3 - warp : 4 + warp) / per * R +
+                                             (n & 1 ? 3 - bc : 4 + bc) / per]);
+            __syncthreads();   // the adjoint's first writes share the memory
+         }
+      }
+      nllAcc += ps.part;
+      if (!kGrad)
+      {
+         if (!OS)
+            __syncthreads();   // the blocks share the next pupil's memory
+         continue;
+      }
+      // 5. T_bar = A^H (G o E): lane = the column pair, a warp's four q; the row pairs' sums and differences through
+      // shared memory in two halves of every warp's rows
+      uint64_t pre[2][2], pim[2][2], nre[2][2], nim[2][2];   // [column sign][q pair]
+#pragma unroll
+      for (int c = 0; c < 2; ++c)
+#pragma unroll
+         for (int k = 0; k < 2; ++k)
+            pre[c][k] = pim[c][k] = nre[c][k] = nim[c][k] = 0;
+#pragma unroll
+      for (int half = 0; half < 2; ++half)
+      {
+         if (half)
+            __syncthreads();
+#pragma unroll
+         for (int k = 0; k < 4; ++k)
+         {
+            const int row = 4 * half + k, g = 4 * (row / kOS);
+            float2 up[2], dn[2];
+#pragma unroll
+            for (int c = 0; c < 2; ++c)
+            {
+               const float2 ep = E[0][c][row], em = E[1][c][row];
+               const float gp = W[g + c], gm = W[g + 2 + c];
+               const float2 wp = make_float2(gp * ep.x, gp * ep.y), wm = make_float2(gm * em.x, gm * em.y);
+               up[c] = make_float2(wp.x + wm.x, wp.y + wm.y);
+               dn[c] = make_float2(wp.y - wm.y, wm.x - wp.x);   // -i (+ minus -)
+            }
+            s.E.C[4 * warp + k][lane] = make_float4(up[0].x, up[0].y, up[1].x, up[1].y);
+            s.E.S[4 * warp + k][lane] = make_float4(dn[0].x, dn[0].y, dn[1].x, dn[1].y);
+         }
+         __syncthreads();
+#pragma unroll 2
+         for (int i = 0; i < kT / 2; ++i)
+         {
+            const float4 ec = s.E.C[i][lane], es = s.E.S[i][lane];
+            const ulonglong2* t =
+               reinterpret_cast<const ulonglong2*>(s.tab.adj[8 * (i >> 2) + 4 * half + (i & 3)][warp]);
+            const ulonglong2 c2 = t[0], s2 = t[1];
+            const uint64_t c[2] = {c2.x, c2.y}, sn[2] = {s2.x, s2.y};
+            const uint64_t c0 = Dup(ec.x), c1 = Dup(ec.y), c3 = Dup(ec.z), c4 = Dup(ec.w);
+            const uint64_t d0 = Dup(es.x), d1 = Dup(es.y), d3 = Dup(es.z), d4 = Dup(es.w);
+#pragma unroll
+            for (int k = 0; k < 2; ++k)
+            {
+               pre[0][k] = Fma2(c[k], c0, pre[0][k]);
+               pim[0][k] = Fma2(c[k], c1, pim[0][k]);
+               pre[1][k] = Fma2(c[k], c3, pre[1][k]);
+               pim[1][k] = Fma2(c[k], c4, pim[1][k]);
+               nre[0][k] = Fma2(sn[k], d0, nre[0][k]);
+               nim[0][k] = Fma2(sn[k], d1, nim[0][k]);
+               nre[1][k] = Fma2(sn[k], d3, nre[1][k]);
+               nim[1][k] = Fma2(sn[k], d4, nim[1][k]);
             }
          }
       }
-      else if (pre)
-      {
+      // the columns folded: (+t plus -t, -i (+t minus -t)) of each row
 #pragma unroll
-         for (int q = 0; q < kPre; ++q)
-            if (tid + q * kThreads < RR)
-               pixel(tid + q * kThreads, kpre[q]);
-      }
-      else
-         for (int p = tid; p < RR; p += kThreads)
-            pixel(p, k[p]);
-      nllAcc += part;
-      if (!kGrad)
+      for (int k = 0; k < 2; ++k)
       {
-         __syncthreads();
-         continue;
+         const float2 a0 = Unpack(pre[0][k]), a1 = Unpack(pim[0][k]), b0 = Unpack(pre[1][k]), b1 = Unpack(pim[1][k]);
+         const float2 e0 = Unpack(nre[0][k]), e1 = Unpack(nim[0][k]), f0 = Unpack(nre[1][k]), f1 = Unpack(nim[1][k]);
+         const int q = 4 * warp + 2 * k;
+         if (q <= kQ)
+            s.T[q][lane] = make_float4(a0.x + b0.x, a1.x + b1.x, a1.x - b1.x, b0.x - a0.x);
+         if (q + 1 <= kQ)
+            s.T[q + 1][lane] = make_float4(a0.y + b0.y, a1.y + b1.y, a1.y - b1.y, b0.y - a0.y);
+         if (q >= 1 && q <= kQ)
+            s.T[kQ + q][lane] = make_float4(e0.x + f0.x, e1.x + f1.x, e1.x - f1.x, f0.x - e0.x);
+         if (q + 1 <= kQ)
+            s.T[kQ + q + 1][lane] = make_float4(e0.y + f0.y, e1.y + f1.y, e1.y - f1.y, f0.y - e0.y);
       }
-      double nb[2] = {gN, gB};   // one exchange for both sums
-      BlockSums<2>(nb, s.red);
-      gN = nb[0];
-      gB = nb[1];
-      if (tid == 0 && frameOk)
-         atomicAdd(&a.gBg[f], gB);
       __syncthreads();
-      // 5. T_bar = A^H (G o E) (32 x 64), 6. U_bar = T_bar conj(A) (32 x 32) and dNLL/dphi
-      SmemGemm<kM, kP, kP>([&](int r, int k) { const float2 v = s.A[k][r]; return make_float2(v.x, -v.y); },
-                           [&](int k, int c) { return s.E[k][c]; },
-                           [&](int r, int c, float2 v) { s.T[r][c] = v; });
-      __syncthreads();
-      SmemGemm<kM, kM, kP>([&](int r, int k) { return s.T[r][k]; },
-                           [&](int k, int c) { const float2 v = s.A[k][c]; return make_float2(v.x, -v.y); },
-                           [&](int r, int c, float2 v) {
-                              const float2 u = s.U[r][c];
-                              // -2 Im(conj(U_bar) U) = -2 (Ubar.x u.y - Ubar.y u.x)
-                              s.dphi[r * kM + c] = -2.f * (v.x * u.y - v.y * u.x);
-                           });
-      __syncthreads();
-      // 7. the chain through phi
-      double gx = 0.0, gy = 0.0, gzd = 0.0;
-      for (int m = tid; m < kM * kM; m += kThreads)
+      // 6. U_bar = T_bar conj(A), folded: lane = row, a warp's four q
       {
-         const double4 sm = a.samples[m];
-         const double d = s.dphi[m];
-         gx -= d * sm.x;
-         gy -= d * sm.y;
-         gzd += d * sm.z;
-         s.dphiSum[m] += d;
+         const int r = min(lane, kR - 1);
+         uint64_t upr[2] = {0, 0}, upi[2] = {0, 0}, unr[2] = {0, 0}, uni[2] = {0, 0};
+#pragma unroll 4
+         for (int i = 0; i < kT; ++i)
+         {
+            const float4 t = s.T[r][i];
+            const ulonglong2* tb = reinterpret_cast<const ulonglong2*>(s.tab.adj[i][warp]);
+            const ulonglong2 c2 = tb[0], s2 = tb[1];
+            const uint64_t c[2] = {c2.x, c2.y}, sn[2] = {s2.x, s2.y};
+            const uint64_t cr = Dup(t.x), ci = Dup(t.y), sr = Dup(t.z), si = Dup(t.w);
+#pragma unroll
+            for (int k = 0; k < 2; ++k)
+            {
+               upr[k] = Fma2(c[k], cr, upr[k]);
+               upi[k] = Fma2(c[k], ci, upi[k]);
+               unr[k] = Fma2(sn[k], sr, unr[k]);
+               uni[k] = Fma2(sn[k], si, uni[k]);
+            }
+         }
+#pragma unroll
+         for (int k = 0; k < 2; ++k)
+         {
+            const float2 pr2 = Unpack(upr[k]), pi2 = Unpack(upi[k]), nr2 = Unpack(unr[k]), ni2 = Unpack(uni[k]);
+            const int q = 4 * warp + 2 * k;
+            if (q <= kQ)
+               s.U[q][lane] = make_float4(pr2.x, pi2.x, nr2.x, ni2.x);
+            if (q + 1 <= kQ)
+               s.U[q + 1][lane] = make_float4(pr2.y, pi2.y, nr2.y, ni2.y);
+         }
       }
-      double xyz[3] = {gx, gy, gzd};
-      BlockSums<3>(xyz, s.red);
-      gx = xyz[0];
-      gy = xyz[1];
-      gzd = xyz[2];
+      __syncthreads();
+      // 7. dNLL/dphi of each quadrant sample and its mirrors, and the chain through phi
+      double sums[5] = {0.0, 0.0, 0.0, ps.gN, ps.gB};
+      for (int qd = tid; qd < kQuad; qd += kThreads)
+      {
+         const int qy = qd / (kQ + 1), qx = qd % (kQ + 1);
+         const double4 sm = a.samples[kM / 2 * kM + kM / 2 + qy * kM + qx];
+         const float4 p = s.U[qx][qy], u0 = s.Uraw[0][qd], u1 = s.Uraw[1][qd];
+         float4 n = make_float4(0.f, 0.f, 0.f, 0.f);
+         if (qy)
+            n = s.U[qx][kQ + qy];
+         // U_bar of (sy, sx) = PP + sy NP + sx (PN + sy NN); -2 Im(conj(U_bar) U) = -2 (Ubar.x u.y - Ubar.y u.x)
+         const float2 a0 = make_float2(p.x + n.x, p.y + n.y), a1 = make_float2(p.x - n.x, p.y - n.y);
+         const float2 b0 = make_float2(p.z + n.z, p.w + n.w), b1 = make_float2(p.z - n.z, p.w - n.w);
+         const float d0 = -2.f * ((a0.x + b0.x) * u0.y - (a0.y + b0.y) * u0.x);
+         const float d1 = -2.f * ((a0.x - b0.x) * u0.w - (a0.y - b0.y) * u0.z);
+         const float d2 = -2.f * ((a1.x + b1.x) * u1.y - (a1.y + b1.y) * u1.x);
+         const float d3 = -2.f * ((a1.x - b1.x) * u1.w - (a1.y - b1.y) * u1.z);
+         const double e0 = d0, e1 = d1, e2 = d2, e3 = d3;
+         sums[0] -= ((e0 - e1) + (e2 - e3)) * sm.x;
+         sums[1] -= ((e0 + e1) - (e2 + e3)) * sm.y;
+         sums[2] += ((e0 + e1) + (e2 + e3)) * sm.z;
+         s.dphiSum[0][qd] += e0;
+         s.dphiSum[1][qd] += e1;
+         s.dphiSum[2][qd] += e2;
+         s.dphiSum[3][qd] += e3;
+      }
+      BlockSums<5>(sums, s.red);
       if (tid == 0)
-         a.gParams[e] = make_float4(static_cast<float>(gx), static_cast<float>(gy), static_cast<float>(gzd),
-                                    static_cast<float>(gN));
-      __syncthreads();
+      {
+         a.gParams[e] = make_float4(static_cast<float>(sums[0]), static_cast<float>(sums[1]),
+                                    static_cast<float>(sums[2]), static_cast<float>(sums[3]));
+         if (frameOk)
+            atomicAdd(&a.gBg[f], sums[4]);
+      }
    }
    // the CTA's sums
-   const double nllCta = BlockSum(nllAcc, s.red);
+   double nllCta[1] = {nllAcc};
+   BlockSums<1>(nllCta, s.red);
    if (tid == 0)
-      atomicAdd(a.nll, nllCta);
+      atomicAdd(a.nll, nllCta[0]);
    if (kGrad)
    {
-      // warp w projects the summed dphi onto modes j = w, w + 8, ...
+      // warp w projects the summed dphi onto modes j = w, w + 4, ...
       __syncthreads();
-      const int lane = tid & 31, warp = tid >> 5;
       for (int j = warp; j < a.J; j += kThreads / 32)
       {
-         const double* Zj = a.basis + static_cast<size_t>(j) * kM * kM;
+         const double* Zj = a.basis + static_cast<size_t>(j) * kM * kM + kM / 2 * kM + kM / 2;
          double v = 0.0;
-         for (int m = lane; m < kM * kM; m += 32)
-            v += s.dphiSum[m] * Zj[m];
+         for (int qd = lane; qd < kQuad; qd += 32)
+         {
+            const int o = qd / (kQ + 1) * kM, qx = qd % (kQ + 1);
+            v += (s.dphiSum[0][qd] * Zj[o + qx] + s.dphiSum[1][qd] * Zj[o - qx]) +
+                 (s.dphiSum[2][qd] * Zj[-o + qx] + s.dphiSum[3][qd] * Zj[-o - qx]);
+         }
 #pragma unroll
          for (int d = 16; d > 0; d >>= 1)
             v += __shfl_xor_sync(0xffffffffu, v, d);
          if (lane == 0)
             atomicAdd(&a.gZern[j], v);
       }
+   }
+}
+
+using NllFn = void (*)(NllArgs);
+template <bool kGrad>
+NllFn NllOf(int os)
+{
+   switch (os)
+   {
+   case 1: return NllKernel<kGrad, 1>;
+   case 2: return NllKernel<kGrad, 2>;
+   case 4: return NllKernel<kGrad, 4>;
+   case 8: return NllKernel<kGrad, 8>;
+   default: return NllKernel<kGrad, 0>;
    }
 }
 
@@ -488,20 +740,25 @@ int iscu_nll_model_create(iscu_ctx* ctx, const iscu_nll_spec* spec, iscu_nll_mod
                basis[static_cast<size_t>(j) * MM + m] =
                   2.0 * pi * ZernikeNoll(spec->noll[j], std::sqrt(kr2) / kmax, std::atan2(ky, kx));
       }
-   std::vector<float2> A(static_cast<size_t>(P) * M);
-   for (int sIdx = 0; sIdx < P; ++sIdx)
-      for (int m = 0; m < M; ++m)
+   NllTables tab = {};
+   for (int t = 0; t < kT; ++t)
+      for (int q = 0; q <= kQ; ++q)
       {
-         const double u = (sIdx + 0.5) / spec->os;
-         const double ph = (m - M / 2) * dk * spec->pixel_nm * u;
-         A[static_cast<size_t>(sIdx) * M + m] = make_float2(static_cast<float>(std::cos(ph)),
-                                                            static_cast<float>(std::sin(ph)));
+         const double ph = q * dk * spec->pixel_nm * ((t + 0.5) / spec->os);
+         const float c = static_cast<float>(std::cos(ph)), sn = static_cast<float>(std::sin(ph));
+         if (q)
+         {
+            tab.fwd[q - 1][t / 8][t % 8] = c;
+            tab.fwd[q - 1][t / 8][8 + t % 8] = sn;
+         }
+         tab.adj[t][q / 4][q % 4] = c;
+         tab.adj[t][q / 4][4 + q % 4] = sn;
       }
    const double L = 2.0 * pi / dk, px = spec->pixel_nm / spec->os;
    mdl->kappa = px * px / (L * L * aSum);
    ISCU_CK(mdl->samples.Reserve(samp.size() * sizeof(double)));
    ISCU_CK(mdl->basis.Reserve(std::max<size_t>(basis.size(), 1) * sizeof(double)));
-   ISCU_CK(mdl->A.Reserve(A.size() * sizeof(float2)));
+   ISCU_CK(mdl->cs.Reserve(sizeof(NllTables)));
    ISCU_CK(mdl->zphase.Reserve(MM * sizeof(double)));
    ISCU_CK(mdl->zern.Reserve(kMaxJ * sizeof(double)));
    ISCU_CK(cudaMemcpyAsync(mdl->samples.p, samp.data(), samp.size() * sizeof(double), cudaMemcpyHostToDevice,
@@ -509,12 +766,10 @@ int iscu_nll_model_create(iscu_ctx* ctx, const iscu_nll_spec* spec, iscu_nll_mod
    if (!basis.empty())
       ISCU_CK(cudaMemcpyAsync(mdl->basis.p, basis.data(), basis.size() * sizeof(double), cudaMemcpyHostToDevice,
                               ctx->stream));
-   ISCU_CK(cudaMemcpyAsync(mdl->A.p, A.data(), A.size() * sizeof(float2), cudaMemcpyHostToDevice, ctx->stream));
+   ISCU_CK(cudaMemcpyAsync(mdl->cs.p, &tab, sizeof(tab), cudaMemcpyHostToDevice, ctx->stream));
    ISCU_CK(cudaStreamSynchronize(ctx->stream));
-   ISCU_CK(cudaFuncSetAttribute(NllKernel<false>, cudaFuncAttributeMaxDynamicSharedMemorySize,
-                                static_cast<int>(sizeof(NllSmem))));
-   ISCU_CK(cudaFuncSetAttribute(NllKernel<true>, cudaFuncAttributeMaxDynamicSharedMemorySize,
-                                static_cast<int>(sizeof(NllSmem))));
+   for (NllFn fn : {NllOf<false>(spec->os), NllOf<true>(spec->os)})
+      ISCU_CK(cudaFuncSetAttribute(fn, cudaFuncAttributeMaxDynamicSharedMemorySize, static_cast<int>(sizeof(NllSmem))));
    *out = mdl.release();
    return ISCU_OK;
 }
@@ -576,7 +831,7 @@ int iscu_nll_eval_dev(iscu_nll_model* model, uint32_t n_emitters, const float* p
    NllArgs a;
    a.samples = model->samples.as<double4>();
    a.basis = model->basis.as<double>();
-   a.A = model->A.as<float2>();
+   a.cs = model->cs.as<float>();
    a.zphase = model->zphase.as<double>();
    a.J = model->J;
    a.R = model->spec.roi;
@@ -596,15 +851,10 @@ int iscu_nll_eval_dev(iscu_nll_model* model, uint32_t n_emitters, const float* p
    a.err = err_dev;
    const size_t smem = sizeof(NllSmem);
    int perSm = 0;
-   if (grad)
-      ISCU_CK(cudaOccupancyMaxActiveBlocksPerMultiprocessor(&perSm, NllKernel<true>, kThreads, smem));
-   else
-      ISCU_CK(cudaOccupancyMaxActiveBlocksPerMultiprocessor(&perSm, NllKernel<false>, kThreads, smem));
+   const NllFn fn = grad ? NllOf<true>(model->spec.os) : NllOf<false>(model->spec.os);
+   ISCU_CK(cudaOccupancyMaxActiveBlocksPerMultiprocessor(&perSm, fn, kThreads, smem));
    const uint32_t grid = std::min<uint32_t>(n_emitters, static_cast<uint32_t>(std::max(1, perSm) * ctx->smCount));
-   if (grad)
-      NllKernel<true><<<grid, kThreads, smem, ctx->stream>>>(a);
-   else
-      NllKernel<false><<<grid, kThreads, smem, ctx->stream>>>(a);
+   fn<<<grid, kThreads, smem, ctx->stream>>>(a);
    ISCU_CK_LAUNCH(ctx, "NllKernel");
    return ISCU_OK;
 }

@@ -103,3 +103,36 @@ def test_bad_frame_reported(problem):
     fr[5] = 99
     with pytest.raises(IscuError):
         model.evaluate(p, fr, bg, prob.zern, k)
+
+
+@pytest.mark.parametrize("roi,n", [(64, 3), (32, 700), (16, 5), (8, 5), (4, 5), (2, 5), (1, 1)])
+def test_sample_groupings_match_oracle(engine, roi, n):
+    """Every grouping of the 64 x 64 samples into pixels (1 to 64 samples per pixel and axis) and more emitters than
+    CTAs: expected counts within 1e-5 of their maximum, each gradient within 1e-4 of its largest entry."""
+    kw = dict(roi=roi, os=64 // roi)
+    ospec = OSpec(**kw)
+    t = tables(ospec)
+    model = NllModel(engine, NllSpec(**kw))
+    rng = np.random.default_rng(roi)
+    c = roi / 2.0
+    params = np.column_stack([c + rng.uniform(-0.2, 0.2, (n, 2)) * min(roi, 8), rng.uniform(-400, 400, n),
+                              rng.uniform(800, 3000, n)]).astype(np.float32)
+    frame = rng.integers(0, 3, n).astype(np.int32)
+    bg = rng.uniform(5, 20, 3).astype(np.float32)
+    zern = rng.normal(0.0, 0.03, len(ospec.noll))
+    pd, bd = params.astype(np.float64), bg.astype(np.float64)
+    want_mu = expected(ospec, pd, frame, bd, zern, t)
+    counts = rng.poisson(want_mu * rng.uniform(0.8, 1.2, (n, 1, 1))).astype(np.float32)
+    value, wp, wb, wz = gradient(ospec, pd, frame, bd, zern, counts.astype(np.float64), t)
+    dev = [torch.from_numpy(a).cuda() for a in (params, frame, bg)]
+    k = torch.from_numpy(counts).cuda()
+    got, mu, g = model.evaluate(*dev, zern, k, grad=True, want_mu=True)
+    fwd, mu0, _ = model.evaluate(*dev, zern, k, want_mu=True)
+    assert np.max(np.abs(mu.cpu().numpy() - want_mu)) <= 1e-5 * np.max(want_mu)
+    assert torch.equal(mu, mu0) and abs(fwd - got) <= 1e-12 * abs(got)
+    assert abs(got - value) <= 1e-5 * abs(value)
+    for have, want in ((g[0].cpu().numpy(), wp), (g[1].cpu().numpy()[None].T, wb[:, None]),
+                       (g[2].cpu().numpy()[:, None], wz[:, None])):
+        for col in range(want.shape[1]):
+            assert np.max(np.abs(have[:, col] - want[:, col])) <= 1e-4 * np.max(np.abs(want[:, col])), col
+    model.close()
