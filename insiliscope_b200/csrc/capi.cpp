@@ -45,6 +45,16 @@ CameraView MakeCameraView(const iscu_camera& c)
    v.maxAdu = std::ldexp(1.0, std::min(16, std::max(1, static_cast<int>(c.bit_depth)))) - 1.0;
    v.emGain = std::max(1.0, c.em_gain);
    v.cic = c.cic_electrons;
+   // The fast form bounds its float32 error relative to the sums' terms, so these must not cancel: QE, dark and CIC
+   // at least 0, and every magnitude that is not 0 well inside float32's range.
+   const auto ok = [](double x) { return x == 0.0 || (std::fabs(x) > 1e-20 && std::fabs(x) < 1e20); };
+   v.fast = ok(v.qe) && ok(v.dark) && ok(v.gain) && ok(v.readNoise) && ok(v.emGain) && ok(v.cic) && v.qe >= 0.0 &&
+            v.dark >= 0.0 && v.cic >= 0.0;
+   v.qeF = static_cast<float>(v.qe);
+   v.addF = static_cast<float>(v.emccd ? v.dark + v.cic : v.dark);
+   v.gainF = static_cast<float>(v.gain);
+   v.readF = static_cast<float>(v.readNoise);
+   v.invEmF = static_cast<float>(1.0 / v.emGain);
    return v;
 }
 

@@ -160,6 +160,9 @@ struct CameraView
    double qe = 1.0, dark = 0.0, gain = 1.0, readNoise = 0.0;
    int emccd = 0;
    double maxAdu = 65535.0, emGain = 1.0, cic = 0.0;
+   // float32 forms for the noise chain's fast decisions (noise_chain.cuh); fast 0: settings outside their bounds
+   float qeF = 1.f, addF = 0.f, gainF = 1.f, readF = 0.f, invEmF = 1.f;   // addF: dark (+ CIC on an EMCCD)
+   int fast = 0;
 };
 CameraView MakeCameraView(const iscu_camera& c);
 

@@ -9,20 +9,26 @@
 
 namespace iscu {
 
-// Pixel i (of the frame; the sensor pixel is i + pixel_base) of a frame whose stream u is keyed by (seed, frame):
-// sCMOS or EMCCD, per-pixel maps where set, else the camera scalars (offset 0).
-__device__ __forceinline__ uint16_t NoisePixel(float photonValue, uint32_t i, const CameraView& cam,
-                                               const StaticView& st, CounterRng& u)
+// A pixel's camera values: its maps where set, else the camera scalars (offset 0).
+struct PixelCamera
 {
-   u.Pixel(i + st.pixelBase);
+   double qe, dark, cic, emGain, maxAdu, readNoise, gain, offset;
+   int emccd;
+};
+
+// The float64 chain of sensor pixel `pix` of the frame that `u` is keyed to, its roundings and decisions taken from
+// the float32 normal where that is sure. Out of line: NoisePixel comes here where its float32 decisions are in doubt.
+static __device__ __noinline__ uint32_t NoisePixelExact(float photonValue, uint32_t pix, uint32_t seed, uint32_t frame,
+                                                 PixelCamera cam)
+{
+   CounterRng u(seed, frame);
+   u.Pixel(pix);
    const double pv = static_cast<double>(photonValue);
    const double photons = pv > 0.0 ? pv : 0.0;   // std::max(0.0, v)
    if (cam.emccd)
    {
       const double ne = CounterPoisson(photons * cam.qe + cam.dark + cam.cic, u);
-      const double readE = (st.readNoise ? static_cast<double>(st.readNoise[i]) : cam.readNoise) / cam.emGain;
-      const double gain = st.gain ? static_cast<double>(st.gain[i]) : cam.gain;
-      const double offset = st.offset ? static_cast<double>(st.offset[i]) : 0.0;
+      const double readE = cam.readNoise / cam.emGain, gain = cam.gain, offset = cam.offset;
       // The register's Gamma with float32 decisions (GammaSure), else CounterGamma from the saved stream; then the
       // rounding (before the clamp) from the float32 read-noise normal when no boundary is within the bound of both
       // float32 errors, else the Gamma (if it was not exact) and the normal again in float64 from the saved stream.
@@ -56,9 +62,7 @@ __device__ __forceinline__ uint16_t NoisePixel(float photonValue, uint32_t i, co
       return static_cast<uint16_t>(adu < 0.0 ? 0.0 : (adu > cam.maxAdu ? cam.maxAdu : adu));
    }
    const double ne = CounterPoisson(photons * cam.qe + cam.dark, u);
-   const double readNoise = st.readNoise ? static_cast<double>(st.readNoise[i]) : cam.readNoise;
-   const double gain = st.gain ? static_cast<double>(st.gain[i]) : cam.gain;
-   const double offset = st.offset ? static_cast<double>(st.offset[i]) : 0.0;
+   const double readNoise = cam.readNoise, gain = cam.gain, offset = cam.offset;
    const GaussDraw d = DrawGauss(u);
    // The ADU from the float32 normal when it is sure: inside (0, 65535) and no rounding boundary within
    // |readNoise / gain| kGaussFastErr of it (the float64 operations' own rounding, ~1e-13, inside the 1e-9 term).
@@ -71,6 +75,294 @@ __device__ __forceinline__ uint16_t NoisePixel(float photonValue, uint32_t i, co
    double adu = offset + (ne + readNoise * g) / gain;
    adu = adu < 0.0 ? 0.0 : (adu > 65535.0 ? 65535.0 : adu);
    return static_cast<uint16_t>(floor(adu + 0.5));
+}
+
+// ------------------------------------------------------------------------------------------------ the fast chain
+// NoisePixel is the same chain with every decision taken in float32 where it is sure, so the ADU are the float64
+// chain's bits. What bounds the chain is the issue and integer rate of the Knuth loop's hashes (its trip count is the
+// reference's by definition), so the loop carries nothing in float64: 29 instructions a hash against 44, one word of
+// the stream selected instead of queued, no float64 exponential, logarithm, quotient or conversion (a conversion
+// issues at a quarter of the float64 rate). Error bounds, each stated where it is used, are at least 1.4 times what the
+// operations' documented bounds add up to; in doubt (about one pixel in 10^4) the float64 chain decides. Measured: the
+// sCMOS noise of 16 frames of 512 x 512 px 159 -> 97 us a call, the EMCCD noise of 64 such frames 0.66 -> 0.36 ms.
+
+__device__ __forceinline__ float Ex2Approx(float x)
+{
+   float r;
+   asm("ex2.approx.ftz.f32 %0, %1;" : "=f"(r) : "f"(x));
+   return r;
+}
+__device__ __forceinline__ float Lg2Approx(float x)
+{
+   float r;
+   asm("lg2.approx.ftz.f32 %0, %1;" : "=f"(r) : "f"(x));
+   return r;
+}
+__device__ __forceinline__ float RsqrtApprox(float x)
+{
+   float r;
+   asm("rsqrt.approx.ftz.f32 %0, %1;" : "=f"(r) : "f"(x));
+   return r;
+}
+__device__ __forceinline__ float RcpApprox(float x)
+{
+   float r;
+   asm("rcp.approx.ftz.f32 %0, %1;" : "=f"(r) : "f"(x));
+   return r;
+}
+
+// UniformOf's value in float32, exact: 1 + (x >> 9) 2^-23 from the bits, less 1 - 2^-24 (a 24-bit result).
+__device__ __forceinline__ float UniformF(uint32_t x)
+{
+   return __uint_as_float(__funnelshift_r(x, 0x7fu, 9)) - 0.999999940395355224609375f;
+}
+
+// A pixel's hashes by counter. Before its first exclusive-or the permutation's words d, a and b are linear in the
+// counter: a step adds a constant to each.
+struct PixelHashes
+{
+   uint32_t a0, b0, c0, sb;   // the words' constant parts, and b's step per counter
+
+   __device__ __forceinline__ PixelHashes(uint32_t seed, uint32_t frame, uint32_t pix)
+   {
+      const uint32_t mul = 1664525u, inc = 1013904223u;
+      const uint32_t bf = frame * mul + inc;
+      c0 = pix * mul + inc;
+      a0 = seed * mul + inc + bf * inc;   // a at counter 0, after a += b d
+      b0 = bf + c0 * a0;                  // b at counter 0, after b += c a
+      sb = c0 * (bf * mul);
+   }
+   // The counter's words from the linear state (d, a, b at that counter).
+   __device__ __forceinline__ void Finish(uint32_t d, uint32_t a, uint32_t b, uint32_t (&w)[4]) const
+   {
+      uint32_t c = c0 + a * b;
+      d += b * c;
+      a ^= a >> 16;
+      b ^= b >> 16;
+      c ^= c >> 16;
+      d ^= d >> 16;
+      a += b * d;
+      b += c * a;
+      c += a * b;
+      d += b * c;
+      w[0] = a;
+      w[1] = b;
+      w[2] = c;
+      w[3] = d;
+   }
+   __device__ __forceinline__ void At(uint32_t frame, uint32_t ctr, uint32_t (&w)[4]) const
+   {
+      const uint32_t mul = 1664525u, inc = 1013904223u;
+      Finish(inc + ctr * mul, a0 + ctr * ((frame * mul + inc) * mul), b0 + ctr * sb, w);
+   }
+   // Words pos .. pos + 2 of the stream.
+   __device__ __forceinline__ void Words3(uint32_t frame, uint32_t pos, uint32_t& w0, uint32_t& w1, uint32_t& w2) const
+   {
+      uint32_t lo[4], hi[4];
+      At(frame, pos >> 2, lo);
+      At(frame, (pos >> 2) + 1, hi);
+      const bool odd = pos & 1, two = pos & 2;
+      const uint32_t x0 = odd ? lo[1] : lo[0], x1 = odd ? lo[2] : lo[1], x2 = odd ? lo[3] : lo[2],
+                     x3 = odd ? hi[0] : lo[3], x4 = odd ? hi[1] : hi[0];
+      w0 = two ? x2 : x0;
+      w1 = two ? x3 : x1;
+      w2 = two ? x4 : x2;
+   }
+};
+
+// The stream's normal of the uniform words (radius first, angle second) and a bound of its distance from the float64
+// formula's value: lg2.approx is within 2^-22 of log2 on (0.5, 2) and 2^-22 relative elsewhere, so x = -2 ln u1 is
+// within 3.4e-7 near 1 and the radius within 3.4e-7 / r; elsewhere the radius and the cosine (__cosf: 2^-21.19 on
+// [-pi, pi], its argument rounded) add at most 1.3e-6 r, r <= 5.8. Near u1 = 1 the radius can be NaN; so are its sums.
+struct NormalF
+{
+   float g, e;
+};
+__device__ __forceinline__ NormalF DrawNormalF(uint32_t w1, uint32_t w2)
+{
+   const float x = -1.38629436f * Lg2Approx(UniformF(w1));
+   const float ir = RsqrtApprox(x), r = x * ir;
+   const float h = UniformF(w2) - 0.5f;   // exact; cos(2 pi u2) = -cos(2 pi (u2 - 1/2))
+   return {-(r * __cosf(6.28318531f * h)), fmaf(8e-7f, ir, 1.6e-5f)};
+}
+
+// floor(v + 0.5) of a v within m of vf (|vf| < 2^22): false when a rounding boundary is within m (or NaN).
+__device__ __forceinline__ bool RoundsSurelyF(float vf, float m, float& out)
+{
+   const float t = vf + 0.5f;
+   const float f = floorf(t);
+   out = f;
+   return fabsf((t - f) - 0.5f) < 0.5f - m;
+}
+
+// Pixel i (of the frame; the sensor pixel is i + pixel_base) of a frame whose stream u is keyed by (seed, frame):
+// sCMOS or EMCCD, per-pixel maps where set, else the camera scalars (offset 0).
+__device__ __forceinline__ uint16_t NoisePixel(float photonValue, uint32_t i, const CameraView& cam,
+                                               const StaticView& st, const CounterRng& u)
+{
+   const uint32_t seed = u.seed, frame = u.frame, pix = i + st.pixelBase;
+   const float readF = st.readNoise ? st.readNoise[i] : cam.readF, gainF = st.gain ? st.gain[i] : cam.gainF,
+               offF = st.offset ? st.offset[i] : 0.f;
+   // lambda within 3 roundings (1.8e-7 relative) of the float64 mean: its terms are not negative
+   const float lf = fmaxf(photonValue, 0.f) * cam.qeF + cam.addF;
+   bool ok = cam.fast != 0;
+   float ne = 0.f;
+   uint32_t pos = 0;          // words of the stream consumed
+   uint32_t g1 = 0, g2 = 0;   // sCMOS: the read noise's words
+   const PixelHashes H(seed, frame, pix);
+   if (lf <= 59.9999f && lf >= 1e-6f)
+   {
+      // Knuth. L within 1.2e-5 + 4e-6 (lambda's error, the argument's rounding, ex2.approx) of exp(-mean); the
+      // product within 2^-24 per factor of the float64 one, 256 factors at most here (1.6e-5): the margin is 6e-5.
+      const float L = Ex2Approx(lf * -1.44269504f), hi = L * 1.00006f, lo = L * 0.99994f;
+      const uint32_t mul = 1664525u, inc = 1013904223u, sa = (frame * mul + inc) * mul;
+      uint32_t d = inc, a = H.a0, b = H.b0, w[4];
+      float p = 1.f, u0, u2, p2, p4;
+      int blk = 0;
+      for (;; ++blk)
+      {
+         H.Finish(d, a, b, w);
+         u0 = UniformF(w[0]);
+         u2 = UniformF(w[2]);
+         p2 = u0 * UniformF(w[1]);
+         p4 = p * (p2 * (u2 * UniformF(w[3])));
+         d += mul;
+         a += sa;
+         b += H.sb;
+         if (!(p4 > hi) || blk == 63)
+            break;
+         p = p4;
+      }
+      // the block's first product at or below L: its factor ends the draw
+      const float q1 = p * u0, q2 = p * p2, q3 = q2 * u2;
+      const bool o1 = q1 > hi, o2 = o1 && q2 > hi, o3 = o2 && q3 > hi;
+      const float last = o3 ? p4 : (o2 ? q3 : (o1 ? q2 : q1));
+      ok = ok && last < lo;
+      const int n = o3 ? 3 : (o2 ? 2 : (o1 ? 1 : 0));
+      pos = 4 * blk + n;
+      ne = static_cast<float>(pos);
+      ++pos;
+      if (!cam.emccd)
+      {
+         uint32_t x[4];
+         H.Finish(d, a, b, x);
+         g1 = o3 ? x[0] : (o2 ? w[3] : (o1 ? w[2] : w[1]));
+         g2 = o3 ? x[1] : (o2 ? x[0] : (o1 ? w[3] : w[2]));
+      }
+   }
+   else
+   {
+      uint32_t w[4];
+      H.At(frame, 0, w);
+      // (beyond 2e4 an EMCCD's float32 bounds are mostly too wide: the exact chain straight away)
+      if (lf > 60.0001f && lf < (cam.emccd ? 2e4f : 1e6f))
+      {
+         // the rounded normal floor(l + sqrt(l) g + 0.5), at least 1 where it is taken here
+         pos = 2;
+         const NormalF z = DrawNormalF(w[0], w[1]);
+         const float s = lf * RsqrtApprox(lf);
+         if (!(RoundsSurelyF(fmaf(s, z.g, lf), fmaf(lf, 1.2e-6f, s * z.e), ne) && ne >= 1.f))
+         {
+            const double ld = static_cast<double>(fmaxf(photonValue, 0.f)) * cam.qe + cam.dark;
+            const double l = cam.emccd ? ld + cam.cic : ld, sd = sqrt(l);
+            double r;
+            if (!RoundsSurely(l + sd * static_cast<double>(z.g), sd * static_cast<double>(z.e) + 1e-9 * l, r) ||
+                !(r >= 1.0))
+               r = fmax(0.0, floor(l + sd * GaussExact({UniformOf(w[0]), UniformOf(w[1]), 0.f}) + 0.5));
+            ne = static_cast<float>(r);
+            ok = ok && r < 16777216.0;
+         }
+         g1 = w[2];
+         g2 = w[3];
+      }
+      else
+      {
+         // no photons and no dark current: nothing drawn, no electrons
+         ok = ok && !(photonValue > 0.f) && (cam.emccd ? cam.dark + cam.cic : cam.dark) == 0.0;
+         g1 = w[0];
+         g2 = w[1];
+      }
+   }
+   const float ig = RcpApprox(gainF), aig = fabsf(ig);
+   if (cam.emccd)
+   {
+      // The register's Gamma (CounterGamma's steps and draws): x within e; t = 1 + c x within dt; v = t^3 within dv;
+      // the squeeze and the logarithmic test each within a bound of their terms' errors.
+      float out = 0.f, outErr = 0.f;
+      if (ne > 0.f && ok)
+      {
+         const float d = ne - 0.333333333f, c = RsqrtApprox(9.f * d);
+         ok = false;
+         for (int it = 0; it < 16; ++it)
+         {
+            uint32_t w1, w2, w3;
+            H.Words3(frame, pos, w1, w2, w3);
+            const NormalF z = DrawNormalF(w1, w2);
+            const float x = z.g, cx = c * x, t = 1.f + cx, dt = fmaf(c, z.e, fmaf(5e-7f, fabsf(cx), 1.3e-7f));
+            const bool negative = t + dt <= 0.f;   // drawn again before its third uniform
+            pos += negative ? 2 : 3;
+            if (negative)
+               continue;
+            const float tt = t + dt, v = t * t * t, dv = fmaf(3.f * tt * tt, dt, 2.5e-7f * v);
+            const float w = UniformF(w3), x2 = x * x, ax = fabsf(x) + z.e;
+            const float s = fmaf(-0.0331f * x2, x2, 1.f);
+            const float ds = fmaf(0.14f * ax * ax * ax, z.e, fmaf(4e-8f * x2, x2, 4e-7f));
+            out = d * v;
+            outErr = fmaf(d, dv, 3.6e-7f * out);
+            ok = t > dt && w < s - ds;
+            if (ok || !(t > dt) || !(w >= s + ds))
+               break;
+            const float lw = 0.693147181f * Lg2Approx(w), lv = 0.693147181f * Lg2Approx(v);
+            const float rhs = fmaf(0.5f, x2, d * (1.f - v + lv));
+            const float iv = RcpApprox(v);
+            const float alw = fabsf(lw), alv = fabsf(lv);
+            const float m = fmaf(1e-6f, alw, 1e-6f) + fmaf(ax, z.e, 4e-7f * x2) +
+                            d * (fmaf(fabsf(iv - 1.f) + dv * iv, dv, fmaf(1e-6f, alv, 1e-6f) + 4e-7f * v));
+            ok = lw < rhs - m;
+            if (ok || !(lw > rhs + m))
+               break;
+         }
+      }
+      if (ok)
+      {
+         uint32_t w1, w2, w3;
+         H.Words3(frame, pos, w1, w2, w3);
+         const NormalF z = DrawNormalF(w1, w2);
+         const float rn = readF * cam.invEmF, rz = rn * z.g;
+         const float af = fmaf(out + rz, ig, offF);
+         const float m = aig * (outErr + fabsf(rn) * z.e) + 1.2e-6f * fmaf(out + fabsf(rz), aig, fabsf(offF));
+         float r;
+         if (RoundsSurelyF(af, m, r))   // (m passes 0.5 well before af leaves the float integers)
+         {
+            const float top = static_cast<float>(cam.maxAdu);
+            return static_cast<uint16_t>(fminf(fmaxf(r, 0.f), top));
+         }
+      }
+   }
+   else if (ok)
+   {
+      // the ADU inside (0, 65535): the float32 value within its terms' roundings (eight at most) and the normal's bound
+      const NormalF z = DrawNormalF(g1, g2);
+      const float rz = readF * z.g, af = fmaf(ne + rz, ig, offF);
+      const float m = fabsf(readF * ig) * z.e + 1.2e-6f * fmaf(ne + fabsf(rz), aig, fabsf(offF));
+      float r;
+      if (RoundsSurelyF(af, m, r) && af > m && af < 65535.f - m)
+         return static_cast<uint16_t>(r);
+      // in float64 from the same normal, then from the float64 one
+      const double rd = st.readNoise ? static_cast<double>(readF) : cam.readNoise,
+                   gd = st.gain ? static_cast<double>(gainF) : cam.gain, od = offF, nd = ne;
+      double adu = od + (nd + rd * static_cast<double>(z.g)) / gd, rr;
+      const double md = fabs(rd / gd) * static_cast<double>(z.e) + 1e-9 * (1.0 + fabs(adu));
+      if (adu > md && adu < 65535.0 - md && RoundsSurely(adu, md, rr))
+         return static_cast<uint16_t>(rr);
+      adu = od + (nd + rd * GaussExact({UniformOf(g1), UniformOf(g2), 0.f})) / gd;
+      adu = adu < 0.0 ? 0.0 : (adu > 65535.0 ? 65535.0 : adu);
+      return static_cast<uint16_t>(floor(adu + 0.5));
+   }
+   return static_cast<uint16_t>(NoisePixelExact(
+      photonValue, pix, seed, frame,
+      {cam.qe, cam.dark, cam.cic, cam.emGain, cam.maxAdu, st.readNoise ? static_cast<double>(readF) : cam.readNoise,
+       st.gain ? static_cast<double>(gainF) : cam.gain, static_cast<double>(offF), cam.emccd}));
 }
 
 } // namespace iscu

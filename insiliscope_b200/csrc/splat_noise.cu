@@ -131,8 +131,10 @@ __global__ void __launch_bounds__(kThreads) RenderGpuRecordsKernel(const iscu_gp
 }
 
 // ---------------------------------------------------------------------------------------------- noise only
-__global__ void NoiseFramesKernel(const float* __restrict__ photons, const uint32_t* __restrict__ frames,
-                                  StaticView st, CameraView cam, uint32_t seed, uint16_t* __restrict__ adu)
+__global__ void __launch_bounds__(256, 6) NoiseFramesKernel(const float* __restrict__ photons,
+                                                            const uint32_t* __restrict__ frames, StaticView st,
+                                                            CameraView cam, uint32_t seed,
+                                                            uint16_t* __restrict__ adu)
 {
    const size_t n = static_cast<size_t>(st.width) * st.height;
    const uint32_t i = blockIdx.x * blockDim.x + threadIdx.x;

@@ -915,9 +915,9 @@ __global__ void __launch_bounds__(kThreads, kMinCtas) XInverseKernel(const float
 
 // The noise chain of every pixel of the photon frames (frame frame0 + plane) -> ADU. A kernel of its own: the
 // float64 chain wants many resident warps, the transforms wants registers. grid (ceil(nx ny / 256), nz).
-__global__ void __launch_bounds__(256) WfNoiseKernel(const float* __restrict__ photons, uint32_t npix, StaticView st,
-                                                     CameraView cam, uint32_t seed, uint32_t frame0,
-                                                     uint16_t* __restrict__ adu)
+__global__ void __launch_bounds__(256, 6) WfNoiseKernel(const float* __restrict__ photons, uint32_t npix,
+                                                        StaticView st, CameraView cam, uint32_t seed, uint32_t frame0,
+                                                        uint16_t* __restrict__ adu)
 {
    const uint32_t i = blockIdx.x * blockDim.x + threadIdx.x;
    if (i >= npix)

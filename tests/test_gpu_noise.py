@@ -61,3 +61,54 @@ def test_noise_chain_bit_exact(engine, oracle, emccd):
                                   rn.reshape(H, W), 42 ^ 0x9E3779B9, frames[k], pixel_base=7 * W)
         mism += int((got[k] != want).sum())
     assert mism == 0
+
+
+CAMERAS = {
+    "scmos_maps": dict(gain=2.2, read_noise_e=1.5),
+    "scmos_scalars": dict(quantum_efficiency=0.82, dark_electrons=0.35, gain=0.46, read_noise_e=1.1),
+    "scmos_no_read_noise": dict(gain=1.0, read_noise_e=0.0),
+    "emccd_maps": dict(quantum_efficiency=0.95, gain=1.0, read_noise_e=50.0, emccd=True, em_gain=300.0,
+                       cic_electrons=0.002),
+    "emccd_scalars": dict(quantum_efficiency=0.9, dark_electrons=0.02, gain=0.05, read_noise_e=30.0, emccd=True,
+                          em_gain=4.0, cic_electrons=0.0, bit_depth=14),
+    "negative_dark": dict(dark_electrons=-0.5, gain=2.0, read_noise_e=1.5),   # outside the float32 form's bounds
+}
+
+
+@pytest.mark.parametrize("name", list(CAMERAS))
+def test_float_decisions_bit_exact(engine, oracle, name):
+    """The float32 decisions over every branch's edges: means spread over 1e-8 .. 1e9 by logarithm, dense around the
+    60-photon switch and among small counts, and zero, negative, NaN and infinite ones; every ADU the CPU chain's."""
+    import torch
+    kw = dict(CAMERAS[name])
+    rng = np.random.default_rng(len(name))
+    W, H, n = 211, 97, 12
+    ph = 10.0 ** rng.uniform(-8.0, 9.0, (n, H, W))
+    ph[1:4] = rng.uniform(0.0, 130.0, (3, H, W))
+    ph[4:7] = rng.uniform(0.0, 12.0, (3, H, W))
+    ph[7] = 60.0 / kw.get("quantum_efficiency", 1.0) + rng.normal(0.0, 2e-4, (H, W))
+    ph[8:10] = rng.uniform(100.0, 5000.0, (2, H, W))
+    ph = ph.astype(np.float32)
+    ph[0, 0, :8] = [0.0, -0.0, -3.0, np.nan, np.inf, -np.inf, 1e-45, 3e38]
+    ph[10, :, ::3] = 0.0
+    off = gain = rn = None
+    if name.endswith("maps"):
+        off, gain, rn = oracle.camera_maps(W, H, 5, 100.0, 2.0, 2.2, 0.1 / 2.2, 1.5, 0.2)
+        if kw.get("emccd"):
+            gain = rn = None
+        else:
+            gain[3], gain[4], gain[5] = 0.0, -2.0, 1e-38
+            rn[6], rn[7] = 0.0, 400.0
+            off[8], off[9] = -50.0, 65530.0
+    cam = CameraParams(**kw)
+    engine.set_static(W, H, pixel_base=3 * W, offset=off, gain=gain, read_noise=rn, flat_bg=0.0)
+    frames = [0, 1, 2, 199, 4096, 2**31 + 5, 7, 8, 9, 10, 11, 12]
+    got = engine.noise_frames_dev(torch.from_numpy(ph).cuda(), frames, cam, 977).cpu().numpy()
+    shaped = [None if a is None else a.reshape(H, W) for a in (off, gain, rn)]
+    finite = np.isfinite(ph) & (np.abs(ph) < 1e15)   # beyond, the float64 ADU's own conversion is undefined
+    for k in range(n):
+        want = oracle.noise_chain(ph[k], cam, *shaped, 977, frames[k], pixel_base=3 * W)
+        diff = (got[k] != want) & finite[k]
+        if gain is not None:
+            diff.reshape(-1)[3] = False              # a zero gain's ADU is not a number
+        assert not diff.any(), (k, int(diff.sum()), ph[k][diff][:4], got[k][diff][:4], want[diff][:4])
