@@ -29,7 +29,9 @@ struct iscu_binned
    iscu_ctx* ctx = nullptr;
    uint32_t W = 0, H = 0;
    int u = 1, R = 1, nz = 1;
+   bool dense = false;     // the dense kernel's shared memory and plane table hold this renderer
    iscu::DevBuf kernels;   // nz x (2R + 1)^2 floats
+   iscu::DevBuf denseKernels, oddPlane;   // the same with rows of a multiple of 16 bytes; planes to be added by test
 };
 
 namespace iscu {
@@ -189,6 +191,315 @@ __global__ void __launch_bounds__(kThreads) BinnedRenderKernel(const iscu_emitte
       alone[o] += static_cast<float>(sum);
 }
 
+// ------------------------------------------------------------------------------------------------ dense frames
+// The same sums for frames of several emitters per plane, with the plane's kernel in shared memory and a block of
+// cells in every thread's registers. A CTA takes 128 x 64 cells of a frame, a warp eight rows of them, a lane 4 x 8
+// cells (columns lane, lane + 32, ...). The tile's emitters are sorted by plane (stable: event order within a plane)
+// and each plane's kernel is staged once (while the plane before it is added, where two fit), with a margin of zeros
+// as wide as a warp's block, so that an emitter costs a block one shared load, two shifts and one float64 multiply-add
+// per cell and no test.
+//
+// The kernel stays float32 in shared memory (half the reads of float64, and a float -> double conversion issues at a
+// quarter of the float64 rate): the double with the float's exponent and mantissa bits, hi = b >> 3, lo = b << 29, is
+// K 2^-896 for every non-negative finite float, zero and subnormals included, and the photons carry 2^896, so the
+// multiply-add rounds as photons x K does. A plane with a negative or non-finite value, or an emitter whose photons
+// are not a normal float, is added cell by cell with the reach tested instead.
+//
+// What bounds it: issue and the latency of 16 warps per SM (the accumulators are half the registers), the shared loads
+// at 45 %, the float64 pipe at 15 %; 54 % of the multiply-adds lie in an emitter's reach at R = 32. 200 frames of
+// 128 x 128 px, 2,400 emitters a frame, u = 2, R = 32: 1.10 ms against 2.03 ms of the kernel above.
+constexpr int kTileX = 128, kTileY = 64, kRows = 8, kCap = 1024, kMaxPlanes = 512;
+constexpr size_t kDenseMaxBytes = 226 * 1024;
+
+struct DenseSmem
+{
+   uint2 kept[kCap];      // (cell x, y from the tile's corner as 16 + 16 bits, photons)
+   uint2 sorted[kCap];
+   uint16_t plane[kCap];
+   int start[kMaxPlanes + 1], cursor[kMaxPlanes];
+   int warpKept[kThreads / 32];
+};
+constexpr size_t kDenseHead = (sizeof(DenseSmem) + 15) / 16 * 16;
+
+// Shared-memory row pitch (32 zeros, the row, at least 31 zeros) and rows of a staged kernel.
+inline int DensePitch(int R) { return 2 * R + 1 + 63 <= 128 ? 128 : 192; }
+inline int DenseRows(int R) { return 2 * R + 1 + 2 * (kRows - 1); }
+inline size_t DenseKernelBytes(int R) { return sizeof(float) * DensePitch(R) * static_cast<size_t>(DenseRows(R)); }
+inline bool DenseFits(int R, int nz) { return 2 * R + 1 + 63 <= 192 && nz <= kMaxPlanes; }
+inline int DenseBuffers(int R) { return DensePitch(R) == 128 ? 2 : 1; }
+inline size_t DenseBytes(int R)
+{
+   return kDenseHead + std::max(DenseBuffers(R) * DenseKernelBytes(R), sizeof(float) * kTileX * kTileY);
+}
+
+// The kernels with rows of a multiple of 16 bytes (zeros behind them), and per plane whether it has a negative or
+// non-finite value. A CTA per plane.
+__global__ void DenseKernelsKernel(const float* __restrict__ K, int D, int rowPitch, float* __restrict__ out,
+                                   int* __restrict__ odd)
+{
+   const float* Kp = K + static_cast<size_t>(blockIdx.x) * D * D;
+   float* o = out + static_cast<size_t>(blockIdx.x) * D * rowPitch;
+   int any = 0;
+   for (int i = threadIdx.x; i < D * rowPitch; i += blockDim.x)
+   {
+      const int y = i / rowPitch, x = i % rowPitch;
+      const float v = x < D ? Kp[y * D + x] : 0.f;
+      any |= __float_as_uint(v) >= 0x7F800000u;
+      o[i] = v;
+   }
+   any = __syncthreads_or(any);
+   if (threadIdx.x == 0)
+      odd[blockIdx.x] = any;
+}
+
+// kPitch: the staged row pitch, a constant so that a block's rows are immediate offsets.
+template <int kPitch, int kBuffers>
+__global__ void __launch_bounds__(kThreads, kBuffers) BinnedDenseKernel(
+   const iscu_emitter* __restrict__ em, uint32_t nEm, const iscu_frame* __restrict__ frames,
+   const float* __restrict__ K, const int* __restrict__ oddPlane, int nz, int R, int U, uint32_t W, uint32_t H,
+   float* __restrict__ img, float* __restrict__ alone)
+{
+   extern __shared__ __align__(16) unsigned char smemRaw[];
+   DenseSmem& s = *reinterpret_cast<DenseSmem*>(smemRaw);
+   float* sK = reinterpret_cast<float*>(smemRaw + kDenseHead);
+   const int tid = threadIdx.x, lane = tid & 31, warp = tid >> 5;
+   const int D = 2 * R + 1, rows = D + 2 * (kRows - 1), quads = (D + 3) / 4;
+   const int pw = kTileX / U, phh = kTileY / U;   // the tile's pixels
+   const int gw = static_cast<int>(W) * U, gh = static_cast<int>(H) * U;
+   const int tx0 = blockIdx.x * pw * U, ty0 = blockIdx.y * phh * U;
+   const int tx1 = min(tx0 + pw * U, gw) - 1, ty1 = min(ty0 + phh * U, gh) - 1;
+   const int reachX0 = max(-R, tx0 - R), reachX1 = min(gw + R - 1, tx1 + R);
+   const int reachY0 = max(-R, ty0 - R), reachY1 = min(gh + R - 1, ty1 + R);
+   const iscu_frame fr = frames[blockIdx.z];
+   const uint32_t begin = min(fr.em_start, nEm), end = min(begin + fr.em_count, nEm);
+   for (int i = tid; i < kBuffers * kPitch * rows; i += kThreads)
+      sK[i] = 0.f;
+   double acc[kTileX / 32][kRows];
+#pragma unroll
+   for (int c = 0; c < kTileX / 32; ++c)
+#pragma unroll
+      for (int j = 0; j < kRows; ++j)
+         acc[c][j] = 0.0;
+   // plane p's rows into buffer `buf`, 16 bytes a copy
+   const int stepRow = kThreads / quads, stepCol = kThreads % quads;
+   auto stage = [&](int p, int buf) {
+      const float* src = K + static_cast<size_t>(p) * D * quads * 4;
+      float* dst = sK + buf * kPitch * rows + (kRows - 1) * kPitch + 32;
+      int y = tid / quads, x = tid % quads;
+      while (y < D)
+      {
+         const uint32_t to = static_cast<uint32_t>(__cvta_generic_to_shared(dst + y * kPitch + 4 * x));
+         asm volatile("cp.async.ca.shared.global [%0], [%1], 16;" ::"r"(to), "l"(src + (y * quads + x) * 4) : "memory");
+         y += stepRow;
+         x += stepCol;
+         if (x >= quads)
+         {
+            x -= quads;
+            ++y;
+         }
+      }
+      asm volatile("cp.async.commit_group;" ::: "memory");
+   };
+   for (uint32_t base = begin; base < end;)
+   {
+      // emitters that reach the tile, in event order, until the buffer could overflow
+      int kept = 0, general = 0;
+      for (; base < end && kept <= kCap - kThreads; base += kThreads)
+      {
+         uint2 e = make_uint2(0, 0);
+         int plane = 0;
+         bool keep = false;
+         if (base + tid < end)
+         {
+            const iscu_emitter m = em[base + tid];
+            if (m.photons > 0.0 && fabs(m.x_px) < 1e9 && fabs(m.y_px) < 1e9)
+            {
+               const int cx = static_cast<int>(floor((m.x_px + 0.5) * U));
+               const int cy = static_cast<int>(floor((m.y_px + 0.5) * U));
+               keep = cx >= reachX0 && cx <= reachX1 && cy >= reachY0 && cy <= reachY1;
+               const float ph = static_cast<float>(m.photons);
+               e = make_uint2((static_cast<uint32_t>(cy - ty0) << 16) | (static_cast<uint32_t>(cx - tx0) & 0xFFFFu),
+                              __float_as_uint(ph));
+               plane = min(nz - 1, max(0, m.plane & 0xFFFF));
+            }
+         }
+         const unsigned ballot = __ballot_sync(0xFFFFFFFFu, keep);
+         if (lane == 0)
+            s.warpKept[warp] = __popc(ballot);
+         general |= __syncthreads_or(keep && (e.y < 0x00800000u || e.y >= 0x7F800000u));
+         int offset = kept;
+#pragma unroll
+         for (int w = 0; w < kThreads / 32; ++w)
+         {
+            offset += w < warp ? s.warpKept[w] : 0;
+            kept += s.warpKept[w];
+         }
+         if (keep)
+         {
+            offset += __popc(ballot & ((1u << lane) - 1u));
+            s.kept[offset] = e;
+            s.plane[offset] = static_cast<uint16_t>(plane);
+         }
+         __syncthreads();
+      }
+      // a stable counting sort by plane
+      for (int p = tid; p < nz; p += kThreads)
+         s.cursor[p] = 0;
+      __syncthreads();
+      for (int k = tid; k < kept; k += kThreads)
+         atomicAdd(&s.cursor[s.plane[k]], 1);
+      __syncthreads();
+      if (warp == 0)
+      {
+         int carry = 0;
+         for (int p0 = 0; p0 < nz; p0 += 32)
+         {
+            const int v = p0 + lane < nz ? s.cursor[p0 + lane] : 0;
+            int x = v;
+#pragma unroll
+            for (int d = 1; d < 32; d <<= 1)
+            {
+               const int u = __shfl_up_sync(0xFFFFFFFFu, x, d);
+               x += lane >= d ? u : 0;
+            }
+            if (p0 + lane < nz)
+               s.start[p0 + lane] = s.cursor[p0 + lane] = carry + x - v;
+            carry += __shfl_sync(0xFFFFFFFFu, x, 31);
+         }
+         if (lane == 0)
+            s.start[nz] = carry;
+         __syncwarp();
+         for (int k0 = 0; k0 < kept; k0 += 32)
+         {
+            const bool on = k0 + lane < kept;
+            const int k = on ? k0 + lane : k0, plane = s.plane[k];
+            const unsigned peers = __match_any_sync(0xFFFFFFFFu, on ? plane : -1);
+            const int rank = __popc(peers & ((1u << lane) - 1u));
+            const int at = on ? s.cursor[plane] : 0;
+            __syncwarp();
+            if (on)
+            {
+               s.sorted[at + rank] = s.kept[k];
+               if (rank == 0)
+                  s.cursor[plane] = at + __popc(peers);
+            }
+            __syncwarp();
+         }
+      }
+      __syncthreads();
+      auto next = [&](int p) {
+         while (p < nz && s.start[p] == s.start[p + 1])
+            ++p;
+         return p;
+      };
+      int p = next(0), buf = 0;
+      if (kBuffers == 2 && p < nz)
+         stage(p, buf);
+      while (p < nz)
+      {
+         const int after = next(p + 1);
+         if (kBuffers == 1)
+            stage(p, 0);
+         asm volatile("cp.async.wait_group 0;" ::: "memory");
+         __syncthreads();   // the plane is staged, and the plane before it added by every warp
+         if (kBuffers == 2 && after < nz)
+            stage(after, buf ^ 1);
+         const int k0 = s.start[p], k1 = s.start[p + 1];
+         // the kernel's sample for (this warp's first row, this lane's first column) of an emitter in the tile's corner
+         const float* Kb = sK + buf * kPitch * rows + (kRows * warp + R + kRows - 1) * kPitch + R + 32 + lane;
+         if (general || oddPlane[p])
+         {
+            for (int k = k0; k < k1; ++k)
+            {
+               const uint2 e = s.sorted[k];
+               const int ex = static_cast<int16_t>(e.x & 0xFFFFu), ey = static_cast<int>(e.x) >> 16;
+               const double ph = __uint_as_float(e.y);
+               const int r0 = kRows * warp - ey, c0 = lane - ex;
+#pragma unroll
+               for (int c = 0; c < kTileX / 32; ++c)
+#pragma unroll
+                  for (int j = 0; j < kRows; ++j)
+                     if (r0 + j >= -R && r0 + j <= R && c0 + 32 * c >= -R && c0 + 32 * c <= R)
+                        acc[c][j] += ph * static_cast<double>(Kb[-ey * kPitch - ex + 32 * c + j * kPitch]);
+            }
+         }
+         else
+            for (int k = k0; k < k1; k += 32)
+            {
+               // 32 emitters at a time: which reach the warp's rows, and which of its column blocks
+               const bool on = k + lane < k1;
+               const uint2 e = s.sorted[on ? k + lane : k];
+               const int ex = static_cast<int16_t>(e.x & 0xFFFFu), ey = static_cast<int>(e.x) >> 16;
+               unsigned reach = __ballot_sync(0xFFFFFFFFu, on && static_cast<unsigned>(kRows * warp - ey + R + kRows - 1) <=
+                                                                    static_cast<unsigned>(2 * R + kRows - 1));
+               unsigned cols[kTileX / 32];
+#pragma unroll
+               for (int c = 0; c < kTileX / 32; ++c)
+                  cols[c] = __ballot_sync(0xFFFFFFFFu, static_cast<unsigned>(32 * c - ex + R + 31) <=
+                                                          static_cast<unsigned>(2 * R + 31));
+               const int offset = -ey * kPitch - ex;
+               while (reach)
+               {
+                  const int src = __ffs(reach) - 1;
+                  reach &= reach - 1;
+                  // photons x 2^896: a normal float's exponent, 896 up
+                  const unsigned pb = __shfl_sync(0xFFFFFFFFu, e.y, src);
+                  const double ph =
+                     __hiloint2double(static_cast<int>((pb >> 3) + 0x70000000u), static_cast<int>(pb << 29));
+                  const float* Ke = Kb + __shfl_sync(0xFFFFFFFFu, offset, src);
+#pragma unroll
+                  for (int c = 0; c < kTileX / 32; ++c)
+                     if ((cols[c] >> src) & 1u)
+                     {
+#pragma unroll
+                        for (int j = 0; j < kRows; ++j)
+                        {
+                           const unsigned b = __float_as_uint(Ke[32 * c + j * kPitch]);
+                           acc[c][j] = fma(ph, __hiloint2double(static_cast<int>(b >> 3), static_cast<int>(b << 29)),
+                                           acc[c][j]);
+                        }
+                     }
+               }
+            }
+         if (kBuffers == 1)
+            __syncthreads();   // the buffer is rewritten
+         p = after;
+         buf ^= kBuffers - 1;
+      }
+      __syncthreads();   // the sorted emitters are rewritten
+   }
+   // a cell is the float image's value, clamped at 0; the pixel sums its cells in float64, rows first
+   __syncthreads();
+#pragma unroll
+   for (int c = 0; c < kTileX / 32; ++c)
+#pragma unroll
+      for (int j = 0; j < kRows; ++j)
+      {
+         const float v = static_cast<float>(acc[c][j]);
+         sK[(kRows * warp + j) * kTileX + 32 * c + lane] = v > 0.f ? v : 0.f;
+      }
+   __syncthreads();
+   for (int i = tid; i < pw * phh; i += kThreads)
+   {
+      const int x = i % pw, y = i / pw;
+      const uint32_t px = blockIdx.x * pw + x, py = blockIdx.y * phh + y;
+      if (px >= W || py >= H)
+         continue;
+      double sum = 0.0;
+      for (int j = 0; j < U; ++j)
+         for (int k = 0; k < U; ++k)
+            sum += sK[(y * U + j) * kTileX + x * U + k];
+      const size_t o = (static_cast<size_t>(blockIdx.z) * H + py) * W + px;
+      img[o] += static_cast<float>(sum);
+      if (alone)
+         alone[o] += static_cast<float>(sum);
+   }
+}
+
+using DenseFn = void (*)(const iscu_emitter*, uint32_t, const iscu_frame*, const float*, const int*, int, int, int,
+                         uint32_t, uint32_t, float*, float*);
+DenseFn DenseOf(int R) { return DensePitch(R) == 128 ? BinnedDenseKernel<128, 2> : BinnedDenseKernel<192, 1>; }
+
 // KernelWidefieldPsf::ValidUpscale (WidefieldRender.cpp:262-269).
 int ValidUpscale(int oversampling, int requested)
 {
@@ -197,6 +508,21 @@ int ValidUpscale(int oversampling, int requested)
       if (os % u == 0)
          return u;
    return 1;
+}
+
+// Whether the dense kernel is the faster one. A CTA pays for each plane it has an emitter of (the kernel's 17-66 KB
+// staged, a barrier), the kernel above for every emitter and pixel: at two emitters of a plane within a tile's reach
+// the two take the same (200 frames of 128 x 128 px, 49 planes, u = 2: 200, 400 and 2,400 emitters a frame 0.40, 0.32
+// (100 frames) and 2.18 ms against 0.44, 0.32 and 1.19, the camera's noise included); with one buffer and one CTA per
+// SM (R > 32) at five (u = 4, R = 64, 20 frames of 2,400 emitters, 5.9 a plane: 0.80 against 0.73 ms; 50 frames of 400:
+// 0.37 against 0.73). Fewer tiles than two per SM leave it idle (100 frames of 64 x 64 px at u = 1: 88 against 108 us).
+bool DensePays(const iscu_binned* b, int smCount, uint32_t nEmitters, uint32_t nFrames, dim3 tiles)
+{
+   const double reach = 2.0 * b->R, gw = static_cast<double>(b->W) * b->u, gh = static_cast<double>(b->H) * b->u;
+   const double part = std::min(1.0, (kTileX + reach) / (gw + reach)) * std::min(1.0, (kTileY + reach) / (gh + reach));
+   const double perPlane = static_cast<double>(nEmitters) / nFrames * part / b->nz;
+   return perPlane >= (DenseBuffers(b->R) == 2 ? 2.0 : 5.0) &&
+          static_cast<uint64_t>(tiles.x) * tiles.y * tiles.z >= 2ull * static_cast<uint64_t>(smCount);
 }
 
 } // namespace
@@ -280,6 +606,18 @@ int iscu_binned_create(iscu_ctx* ctx, int32_t slot, double sigma_px, uint32_t wi
    }
    if (b->u > 8)
       return Fail(ISCU_ERR_LIMIT, "binned render: at most 8 cells per pixel");
+   if (DenseFits(b->R, b->nz))
+   {
+      const int D = 2 * b->R + 1, rowPitch = (D + 3) / 4 * 4;
+      ISCU_CK(b->denseKernels.Reserve(static_cast<size_t>(b->nz) * D * rowPitch * sizeof(float)));
+      ISCU_CK(b->oddPlane.Reserve(b->nz * sizeof(int)));
+      DenseKernelsKernel<<<b->nz, 256, 0, ctx->stream>>>(b->kernels.as<float>(), D, rowPitch,
+                                                         b->denseKernels.as<float>(), b->oddPlane.as<int>());
+      ISCU_CK_LAUNCH(ctx, "DenseKernelsKernel");
+      ISCU_CK(cudaFuncSetAttribute(DenseOf(b->R), cudaFuncAttributeMaxDynamicSharedMemorySize,
+                                   static_cast<int>(kDenseMaxBytes)));
+      b->dense = true;
+   }
    ISCU_CK(cudaStreamSynchronize(ctx->stream));
    *out = b.release();
    return ISCU_OK;
@@ -331,8 +669,18 @@ int iscu_binned_render_dev(iscu_binned* b, const iscu_emitter* emitters_dev, uin
    ClearError();
    if (!n_frames)
       return ISCU_OK;
-   const dim3 grid((b->W + kSide - 1) / kSide, (b->H + kSide - 1) / kSide, n_frames);
    const float* K = b->kernels.as<float>();
+   const uint32_t pw = kTileX / b->u, ph = kTileY / b->u;
+   const dim3 tiles((b->W + pw - 1) / pw, (b->H + ph - 1) / ph, n_frames);
+   if (b->dense && DensePays(b, ctx->smCount, n_emitters, n_frames, tiles))
+   {
+      DenseOf(b->R)<<<tiles, kThreads, DenseBytes(b->R), ctx->stream>>>(
+         emitters_dev, n_emitters, frames_dev, b->denseKernels.as<float>(), b->oddPlane.as<int>(), b->nz, b->R, b->u,
+         b->W, b->H, img_dev, alone_dev);
+      ISCU_CK_LAUNCH(ctx, "BinnedDenseKernel");
+      return ISCU_OK;
+   }
+   const dim3 grid((b->W + kSide - 1) / kSide, (b->H + kSide - 1) / kSide, n_frames);
 #define ISCU_BINNED_LAUNCH(UU)                                                                                          \
    BinnedRenderKernel<UU><<<grid, kThreads, 0, ctx->stream>>>(emitters_dev, n_emitters, frames_dev, K, b->nz, b->R,  \
                                                               b->W, b->H, img_dev, alone_dev)

@@ -5,7 +5,7 @@ oracle and 5e-6 of the reference's (its float FFT's rounding), added into the ca
 import numpy as np
 import pytest
 
-from insiliscope_b200 import BinnedRenderer, INTERP_CUBIC
+from insiliscope_b200 import BinnedRenderer, EMITTER_DTYPE, INTERP_CUBIC, frames_table
 from oracle.oracle import binned_cell_kernels_f64, binned_gauss_kernel_f64, binned_render_f64
 from test_binned_oracle import H, W, _req, binned_movie
 
@@ -81,4 +81,38 @@ def test_dense_frames_128(engine, reference):
     _, alone = _render(r, mv.emitters, mv.frames, np.zeros((len(mv.frames), mv.height, mv.width), np.float32))
     want = binned_render_f64(K, u, R, mv.emitters, mv.frames, mv.width, mv.height)
     assert _rel(alone, want) <= 1e-6
+    r.close()
+
+
+@pytest.mark.parametrize("half,os_,upscale,w,h,nz,signed", [
+    (5, 4, 2, 70, 45, 3, False), (5, 4, 4, 33, 17, 5, False), (8, 2, 1, 130, 66, 3, False), (3, 3, 3, 43, 22, 3, False),
+    (4, 4, 2, 64, 32, 3, True), (2, 1, 1, 5, 3, 3, False)])
+def test_dense_kernel(engine, half, os_, upscale, w, h, nz, signed):
+    """Frames of many emitters per plane (the kernel with the plane's samples in shared memory), tiles' edges and
+    remainders, planes with negative samples, more emitters than its buffer: the oracle within 1e-6 of the maximum, and
+    within a float's last place of the per-pixel kernel, which the same frames take among many empty ones."""
+    rng = np.random.default_rng(half * 7 + upscale)
+    n = 2 * half * os_ + 1
+    planes = rng.random((nz, n, n)).astype(np.float32) / (n * n)
+    planes[:, 0, :] = 0.0
+    if signed:
+        planes[1] -= 0.3 / (n * n)
+    engine.kernel_set_planes(0, planes, os_, 100.0, INTERP_CUBIC)
+    r = BinnedRenderer(engine, w, h, upscale, slot=0)
+    counts = np.tile([2300, 0, 37, 411], 75)      # 300 frames: tiles for every SM
+    total = int(counts.sum())
+    em = np.zeros(total, EMITTER_DTYPE)
+    em["x_px"] = rng.uniform(-half - 2.0, w + half + 2.0, total)
+    em["y_px"] = rng.uniform(-half - 2.0, h + half + 2.0, total)
+    em["photons"] = rng.uniform(-50.0, 2000.0, total)
+    em["plane"] = rng.integers(0, nz + 1, total)
+    fr = frames_table(counts)
+    want = binned_render_f64(*binned_cell_kernels_f64(planes, os_, upscale), em, fr[:4], w, h)
+    base = rng.random((len(fr), h, w)).astype(np.float32)
+    img, alone = _render(r, em, fr, base)
+    assert _rel(alone[:4], want) <= 1e-6
+    assert np.array_equal(img, base + alone)
+    pad = frames_table(np.concatenate([counts[:4], np.zeros(20000, np.int64)]))
+    _, sparse = _render(r, em[:int(counts[:4].sum())], pad, np.zeros((len(pad), h, w), np.float32))
+    assert np.all(np.abs(sparse[:4] - alone[:4]) <= 1.2e-7 * np.abs(alone[:4]))
     r.close()
