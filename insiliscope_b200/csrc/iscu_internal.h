@@ -206,6 +206,7 @@ struct iscu_ctx
    std::recursive_mutex mu;
    std::atomic<uint64_t> launches{0};
    int smCount = 0;
+   iscu::DevBuf psfScratch;        // a PSF library call's temporaries (psf.cu), kept up to 64 MB
    int renderConfig = 0;           // render kernel form (iscu_render_set_config)
    iscu::DevBuf dOrder;            // persistent render: frame order + work counter
    iscu::ContribScratch contrib;   // two-pass render scratch

@@ -10,16 +10,18 @@
 //
 // Kernels:
 //  PupilTablesKernel  z-independent pupil tables per request set (aperture, opd1, the opd3 obliquity factor,
-//                     Zernike + mask phase), float64 (ZernikePsf.cpp:188-231)
+//                     Zernike + mask phase), float64 (ZernikePsf.cpp:188-231); the folded transform's cosines and sines
 //  DftMatrixKernel    A (P x M) and A^T (M x P) per set, float32 phasors of float64 phases
-//  CztFp32Kernel      the plain FP32 form: one CTA per PSF, pupil phasors into shared memory, T = A U and
-//                     E = T A^T as register-tiled SIMT complex products, |E|^2, optional sum-1 normalization
+//  CztFoldKernel      the plain FP32 form: a cluster of CTAs per PSF, both products folded about the plane's centre,
+//                     |E|^2, optional sum-1 normalization
+//  PupilKernel, CGemmTiledKernel  pupils beyond shared memory: the products through global memory
 // The tensor-core form (TF32 split products on tcgen05) is in psf_tc.cu.
 
 #include "iscu_internal.h"
 #include "psf_common.cuh"
 
 #include <algorithm>
+#include <cooperative_groups.h>
 #include <cmath>
 #include <cstring>
 #include <vector>
@@ -31,35 +33,6 @@ namespace {
 constexpr double kPi = 3.14159265358979323846;
 
 // ------------------------------------------------------------------------------------------ Zernike (device, FP64)
-__device__ double Binomial(int a, int b)
-{
-   if (b < 0 || b > a)
-      return 0.0;
-   double r = 1.0;
-   for (int i = 0; i < b; ++i)
-      r = r * (a - i) / (i + 1);
-   return r;
-}
-
-// Unnormalized radial polynomial R_n^m, m >= 0 (ZernikePsf.cpp:58-67).
-__device__ double ZernikeRadial(int n, int m, double rho)
-{
-   double r = 0.0;
-   for (int k = 0; k <= (n - m) / 2; ++k)
-   {
-      const double coeff = (k % 2 == 0 ? 1.0 : -1.0) * Binomial(n - k, k) * Binomial(n - 2 * k, (n - m) / 2 - k);
-      r += coeff * pow(rho, static_cast<double>(n - 2 * k));
-   }
-   return r;
-}
-
-// ZernikeValue (ZernikePsf.cpp:74-78).
-__device__ double ZernikeValue(int n, int l, int m, double rho, double phi)
-{
-   const double radial = rho <= 1.0 ? ZernikeRadial(n, m, rho) : 0.0;
-   return radial * (l >= 0 ? cos(m * phi) : sin(m * phi));
-}
-
 __device__ double LaguerreL(int p, int a, double x)
 {
    double lm1 = 0.0, l = 1.0;
@@ -90,15 +63,67 @@ __device__ double MaskPhase(int maskModes, double maskWaist, double rhoNorm, dou
    return (re == 0.0 && im == 0.0) ? 0.0 : atan2(im, re);
 }
 
+// The folded transform. The pupil's samples k_q = q dk (q = m - M / 2) and the plane's tau dx lie symmetrically about
+// 0, so exp(i k_q x_tau) for +-q and +-tau is one cosine and one sine: with P = U[q] + U[-q], N = U[q] - U[-q],
+//   C = U[0] + sum cos(q tau) P,  S = sum sin(q tau) N,  the samples at +-tau are C +- i S,
+// on each axis: real by complex products of a quarter of the size. The aperture's radius is (M - 4) / 2 samples (dk =
+// 2 kMax / (M - 4)), so q <= Q = (M - 4) / 2. tau = t for an odd plane size (t = 0 is one sample, not two), t + 1/2 for
+// an even one.
+struct Fold
+{
+   int Q, R, nT;   // the largest q; folded rows (P of q = 0..Q, then N of q = 1..Q); sample pairs
+   __host__ __device__ Fold(int M, int P) : Q((M - 4) / 2), R(2 * Q + 1), nT((P + 1) / 2) {}
+   __host__ __device__ int Pitch() const { return (nT + 3) / 4 * 4; }        // of the table's rows
+   __host__ __device__ int Share(int c) const { return (nT + c - 1) / c; }   // pairs of a CTA of a cluster of c
+   size_t Bytes(int c) const
+   {
+      return sizeof(float4) * (static_cast<size_t>(Q + 1) * R + static_cast<size_t>(R) * (Share(c) | 1));
+   }
+};
+
+// Entry idx of set s of the folded transform's table: cs[s][q - 1][t] = cos, sin of q dk tau dx, the float64 phase
+// reduced mod 2 pi first; zeros beyond the pairs.
+__device__ void FoldTable(const SetParams& sp, int M, int P, int idx, int s, float2* __restrict__ cs)
+{
+   const Fold F(M, P);
+   const int pitch = F.Pitch();
+   if (idx >= F.Q * pitch)
+      return;
+   const int q = idx / pitch + 1, t = idx % pitch;
+   float2 v = make_float2(0.f, 0.f);
+   if (t < F.nT)
+   {
+      double sn, c;
+      sincos(ReduceTwoPi((q * sp.dk) * ((P & 1 ? t : t + 0.5) * sp.dx)), &sn, &c);
+      v = make_float2(static_cast<float>(c), static_cast<float>(sn));
+   }
+   cs[static_cast<size_t>(s) * F.Q * pitch + idx] = v;
+}
+
 // ------------------------------------------------------------------------------------------ tables
 // tables[s][idx] = (opd1, opd3Factor, zernike + mask phase); opd3Factor < 0 marks a sample outside the aperture.
-__global__ void PupilTablesKernel(const SetParams* __restrict__ sets, int M, double3* __restrict__ tables)
+// cs (nullable): the folded transform's table too, by the blocks beyond the pupil's.
+constexpr int kTableThreads = 128;
+__global__ void __launch_bounds__(kTableThreads) PupilTablesKernel(const SetParams* __restrict__ sets, int M, int P,
+                                                                   double3* __restrict__ tables,
+                                                                   float2* __restrict__ cs)
 {
    const int s = blockIdx.y;
-   const int idx = blockIdx.x * blockDim.x + threadIdx.x;
+   // the set's scalars in shared memory: the modes' loop reads them one after the other
+   __shared__ SetParams sp;
+   static_assert(sizeof(SetParams) % 8 == 0, "copied by 8 bytes");
+   for (int i = threadIdx.x; i < static_cast<int>(sizeof(SetParams) / 8); i += kTableThreads)
+      reinterpret_cast<uint64_t*>(&sp)[i] = reinterpret_cast<const uint64_t*>(sets + s)[i];
+   __syncthreads();
+   const int pupilBlocks = (M * M + kTableThreads - 1) / kTableThreads;
+   if (static_cast<int>(blockIdx.x) >= pupilBlocks)
+   {
+      FoldTable(sp, M, P, (blockIdx.x - pupilBlocks) * kTableThreads + threadIdx.x, s, cs);
+      return;
+   }
+   const int idx = blockIdx.x * kTableThreads + threadIdx.x;
    if (idx >= M * M)
       return;
-   const SetParams& sp = sets[s];
    const int iy = idx / M, ix = idx % M, c0 = M / 2;
    const double ky = (iy - c0) * sp.dk, kx = (ix - c0) * sp.dk;
    // The aperture test decides samples that sit exactly on the circle (M = 64: (30, 0), (18, 24), ...): rounded
@@ -109,16 +134,35 @@ __global__ void PupilTablesKernel(const SetParams* __restrict__ sets, int M, dou
    {
       const double kr = sqrt(kr2);
       const double rho = kr / (sp.k0 * sp.na);
-      const double phi = atan2(ky, kx);
       const double s1 = sp.na * rho / sp.ns;
       const double s3 = sp.na * rho / sp.ni;
       out.x = sp.ns * sp.depthM * sqrt(fmax(0.0, 1.0 - s1 * s1));
       out.y = sqrt(fmax(0.0, 1.0 - s3 * s3));
+      // ZernikeValue (ZernikePsf.cpp:74-78): R_n^m(rho) cos m phi (l >= 0) or sin m phi, the radial part by Horner in
+      // rho^2, the angular one from the powers of (kx + i ky) / kr (phi = 0 at the centre); no pow, atan2 or cos, whose
+      // chains made this kernel 20 us at 64 x 64 samples and 12 modes
       double zern = 0.0;
+      const double rn = rho / sp.bMax, rn2 = rn * rn;
+      const double cphi = kr > 0.0 ? kx / kr : 1.0, sphi = kr > 0.0 ? ky / kr : 0.0;
       for (int t = 0; t < sp.nModes; ++t)
-         zern += sp.coeff[t] * ZernikeValue(sp.modeN[t], sp.modeL[t], sp.modeM[t], rho / sp.bMax, phi);
+      {
+         const int n = sp.modeN[t], m = sp.modeM[t];
+         double rad = sp.radial[t][0];
+         for (int k = 1; k <= (n - m) / 2; ++k)
+            rad = rad * rn2 + sp.radial[t][k];
+         double re = 1.0, im = 0.0;
+         for (int k = 0; k < m; ++k)
+         {
+            const double r = re * cphi - im * sphi;
+            im = re * sphi + im * cphi;
+            re = r;
+            rad *= rn;
+         }
+         zern += rn <= 1.0 ? sp.coeff[t] * rad * (sp.modeL[t] >= 0 ? re : im) : 0.0;
+      }
       zern *= 2.0 * kPi;
-      const double mask = sp.doubleHelix ? MaskPhase(sp.maskModes, sp.maskWaist, rho / sp.bMax, phi) : 0.0;
+      const double mask =
+         sp.doubleHelix ? MaskPhase(sp.maskModes, sp.maskWaist, rho / sp.bMax, atan2(ky, kx)) : 0.0;
       out.z = zern + mask;
    }
    tables[static_cast<size_t>(s) * M * M + idx] = out;
@@ -144,8 +188,6 @@ __global__ void DftMatrixKernel(const SetParams* __restrict__ sets, int M, int P
 }
 
 // ------------------------------------------------------------------------------------------ plain FP32 chirp-Z
-constexpr int kCztThreads = 256;
-
 __device__ __forceinline__ void Cmac(float2& acc, float2 a, float2 b)
 {
    acc.x = fmaf(a.x, b.x, acc.x);
@@ -154,96 +196,221 @@ __device__ __forceinline__ void Cmac(float2& acc, float2 a, float2 b)
    acc.y = fmaf(a.y, b.x, acc.y);
 }
 
-// C[r][c] = sum_k L[r][k] R[k][c], rows x cols, 64 x 64 output blocks, a 4 x 4 complex tile per thread (rows
-// ty + 16 i, columns tx + 16 j: a warp reads R contiguously and L by broadcast). epi(r, c, value) stores.
-template <class Epi>
-__device__ __forceinline__ void CGemm(const float2* __restrict__ L, int ldl, const float2* __restrict__ R, int ldr,
-                                      int rows, int cols, int K, Epi epi)
-{
-   const int tx = threadIdx.x & 15, ty = threadIdx.x >> 4;
-   for (int rb = 0; rb < rows; rb += 64)
-      for (int cb = 0; cb < cols; cb += 64)
-      {
-         float2 acc[4][4];
-#pragma unroll
-         for (int i = 0; i < 4; ++i)
-#pragma unroll
-            for (int j = 0; j < 4; ++j)
-               acc[i][j] = make_float2(0.f, 0.f);
-         int ri[4], cj[4];
-#pragma unroll
-         for (int i = 0; i < 4; ++i)
-         {
-            ri[i] = min(rb + ty + 16 * i, rows - 1);
-            cj[i] = min(cb + tx + 16 * i, cols - 1);
-         }
-#pragma unroll 4
-         for (int k = 0; k < K; ++k)
-         {
-            float2 l[4], r[4];
-#pragma unroll
-            for (int i = 0; i < 4; ++i)
-            {
-               l[i] = L[static_cast<size_t>(ri[i]) * ldl + k];
-               r[i] = R[static_cast<size_t>(k) * ldr + cj[i]];
-            }
-#pragma unroll
-            for (int i = 0; i < 4; ++i)
-#pragma unroll
-               for (int j = 0; j < 4; ++j)
-                  Cmac(acc[i][j], l[i], r[j]);
-         }
-#pragma unroll
-         for (int i = 0; i < 4; ++i)
-#pragma unroll
-            for (int j = 0; j < 4; ++j)
-            {
-               const int r = rb + ty + 16 * i, c = cb + tx + 16 * j;
-               if (r < rows && c < cols)
-                  epi(r, c, acc[i][j]);
-            }
-      }
-}
+constexpr size_t kPsfScratchKept = 64u << 20;
+constexpr int kFoldThreads = 320, kFoldMaxCluster = 8;
+constexpr size_t kFoldMaxBytes = 224 * 1024;
 
-__global__ void __launch_bounds__(kCztThreads) CztFp32Kernel(const SetParams* __restrict__ sets,
-                                                               const double3* __restrict__ tables,
-                                                               const float2* __restrict__ A,
-                                                               const float2* __restrict__ At,
-                                                               const PsfItem* __restrict__ items, int M, int P,
-                                                               int normalize, float* __restrict__ out)
+// A cluster of C CTAs per PSF (grid: nPsf x C): each takes nT / C of the plane's column pairs through both products,
+// which need nothing of the others' columns, and 1/C of the pupil's phasors, written to every CTA of the cluster; the
+// plane's sum is exchanged at the end.
+//
+// What bounds it: at a stack's 49 planes, latency -- a CTA per plane left two thirds of the SMs idle through 36 x the
+// arithmetic a plane needs (64-wide blocks over 129 columns; 4.3 x more multiply-adds than the folded products). 49
+// planes of 129 x 129 from 64 pupil samples: 26 us (four CTAs a plane) against 218 us the unfolded CTA per plane; the
+// call with its tables 51 us against 262, or 950 where cudaMalloc and cudaFree are slow.
+__global__ void __launch_bounds__(kFoldThreads, 2) CztFoldKernel(const SetParams* __restrict__ sets,
+                                                                 const double3* __restrict__ tables,
+                                                                 const float2* __restrict__ cs,
+                                                                 const PsfItem* __restrict__ items, int M, int P,
+                                                                 int normalize, float* __restrict__ out)
 {
+   namespace cg = cooperative_groups;
+   cg::cluster_group cluster = cg::this_cluster();
+   const int C = static_cast<int>(cluster.num_blocks()), rank = static_cast<int>(cluster.block_rank());
+   const int psf = blockIdx.x / C, tid = threadIdx.x;
+   const Fold F(M, P);
+   const int Q = F.Q, R = F.R, nT = F.nT, pitch = F.Pitch(), share = F.Share(C), tp = share | 1;
    extern __shared__ __align__(16) unsigned char smem[];
-   float2* U = reinterpret_cast<float2*>(smem);                                  // M x M pupil phasors
-   float2* T = U + static_cast<size_t>(M) * M;                                   // P x M
-   __shared__ double sRed[kCztThreads / 32];
-   const PsfItem it = items[blockIdx.x];
+   float4* U = reinterpret_cast<float4*>(smem);         // [q][row]: (P.re, P.im, N.re, N.im) of the column pair q
+   float4* T = U + static_cast<size_t>(Q + 1) * R;      // [row][own pair]: the samples at +t and -t
+   __shared__ double sRed[kFoldThreads / 32], sPart[kFoldMaxCluster];
+   const PsfItem it = items[psf];
    const SetParams& sp = sets[it.set];
    const double3* tab = tables + static_cast<size_t>(it.set) * M * M;
-   const float2* As = A + static_cast<size_t>(it.set) * P * M;
-   const float2* Ats = At + static_cast<size_t>(it.set) * P * M;
-
-   // Pupil: phase = k0 (opd1 + ni (ti - ti0) opd3F) + zernike + mask (ZernikePsf.cpp:240-248), float64 then reduced.
-   for (int idx = threadIdx.x; idx < M * M; idx += blockDim.x)
-      U[idx] = PupilPhasor(tab[idx], sp, it.dtiM);
+   const float2* ct = cs + static_cast<size_t>(it.set) * Q * pitch;
+   const int t0 = rank * share, own = max(0, min(share, nT - t0));
+   cluster.sync();   // every CTA's shared memory is there to be written
+   // the pupil (phase = k0 (opd1 + ni (ti - ti0) opd3F) + zernike + mask, ZernikePsf.cpp:240-248, float64 then reduced),
+   // folded on both axes
+   for (int i = rank * kFoldThreads + tid; i < (Q + 1) * (Q + 1); i += C * kFoldThreads)
+   {
+      const int qy = i / (Q + 1), qx = i % (Q + 1), m0 = M / 2 * M + M / 2;
+      float2 u[2][2];
+#pragma unroll
+      for (int y = 0; y < 2; ++y)
+#pragma unroll
+         for (int x = 0; x < 2; ++x)
+         {
+            u[y][x] = PupilPhasor(tab[m0 + (y ? -qy : qy) * M + (x ? -qx : qx)], sp, it.dtiM);
+            if ((y && qy == 0) || (x && qx == 0))   // one sample on an axis, not two
+               u[y][x] = make_float2(0.f, 0.f);
+         }
+      const float2 p0 = make_float2(u[0][0].x + u[0][1].x, u[0][0].y + u[0][1].y);
+      const float2 n0 = make_float2(u[0][0].x - u[0][1].x, u[0][0].y - u[0][1].y);
+      const float2 p1 = make_float2(u[1][0].x + u[1][1].x, u[1][0].y + u[1][1].y);
+      const float2 n1 = make_float2(u[1][0].x - u[1][1].x, u[1][0].y - u[1][1].y);
+      const float4 even = make_float4(p0.x + p1.x, p0.y + p1.y, n0.x + n1.x, n0.y + n1.y);
+      const float4 odd = make_float4(p0.x - p1.x, p0.y - p1.y, n0.x - n1.x, n0.y - n1.y);
+      for (int c = 0; c < C; ++c)
+      {
+         float4* to = cluster.map_shared_rank(U, c) + static_cast<size_t>(qx) * R;
+         to[qy] = even;
+         if (qy)
+            to[Q + qy] = odd;
+      }
+   }
+   cluster.sync();
+   // T = U A^T over the folded rows: a row and four of the CTA's pairs per thread
+   for (int i = tid; i < R * ((own + 3) / 4); i += kFoldThreads)
+   {
+      const int r = i % R, g = i / R * 4;
+      float cr[4], ci[4], sr[4], si[4];
+      const float4 u0 = U[r];
+#pragma unroll
+      for (int k = 0; k < 4; ++k)
+      {
+         cr[k] = u0.x;
+         ci[k] = u0.y;
+         sr[k] = si[k] = 0.f;
+      }
+      const float2* c0 = ct + t0 + g;
+      int at[4];
+#pragma unroll
+      for (int k = 0; k < 4; ++k)
+         at[k] = min(k, own - 1 - g);
+#pragma unroll 4
+      for (int q = 1; q <= Q; ++q, c0 += pitch)
+      {
+         const float4 u = U[q * R + r];
+#pragma unroll
+         for (int k = 0; k < 4; ++k)
+         {
+            const float2 c = __ldg(c0 + at[k]);
+            cr[k] = fmaf(c.x, u.x, cr[k]);
+            ci[k] = fmaf(c.x, u.y, ci[k]);
+            sr[k] = fmaf(c.y, u.z, sr[k]);
+            si[k] = fmaf(c.y, u.w, si[k]);
+         }
+      }
+#pragma unroll
+      for (int k = 0; k < 4; ++k)
+         if (g + k < own)
+            T[r * tp + g + k] = make_float4(cr[k] - si[k], ci[k] + sr[k], cr[k] + si[k], ci[k] - sr[k]);
+   }
    __syncthreads();
-   // Row pass: T[y][m] = sum_n A[y][n] U[n][m].
-   CGemm(As, M, U, M, P, M, M, [&](int r, int c, float2 v) { T[static_cast<size_t>(r) * M + c] = v; });
-   __syncthreads();
-   // Column pass: E[y][x] = sum_m T[y][m] A[x][m]; I = |E|^2.
-   float* plane = out + static_cast<size_t>(blockIdx.x) * P * P;
+   // E = A T, I = |E|^2: a column pair and four row pairs per thread
+   float* plane = out + static_cast<size_t>(psf) * P * P;
+   const int groups = (nT + 3) / 4, half = P / 2, odd = P & 1;
    double local = 0.0;
-   CGemm(T, M, Ats, P, P, P, M, [&](int r, int c, float2 v) {
-      const float I = v.x * v.x + v.y * v.y;
-      plane[static_cast<size_t>(r) * P + c] = I;
-      local += static_cast<double>(I);
-   });
+   float I[4][4];   // [row pair][+y +x, +y -x, -y +x, -y -x] of the thread's last item
+   const int nItems = own * groups;
+   // row y = half + t (+), half - t - 1 + odd (-); columns likewise
+   auto store = [&](int i) {
+      const int c = t0 + i % own, g = i / own * 4;
+      const int xp = half + c, xm = half - c - 1 + odd;
+#pragma unroll
+      for (int k = 0; k < 4; ++k)
+         if (g + k < nT)
+         {
+            float* yp = plane + static_cast<size_t>(half + g + k) * P;
+            float* ym = plane + static_cast<size_t>(half - g - k - 1 + odd) * P;
+            yp[xp] = I[k][0];
+            yp[xm] = I[k][1];
+            ym[xp] = I[k][2];
+            ym[xm] = I[k][3];
+         }
+   };
+   for (int i = tid; i < nItems; i += kFoldThreads)
+   {
+      const int c = i % own, g = i / own * 4;
+      float cr[2][4], ci[2][4], sr[2][4], si[2][4];
+      const float4 e0 = T[c];
+#pragma unroll
+      for (int k = 0; k < 4; ++k)
+      {
+         cr[0][k] = e0.x;
+         ci[0][k] = e0.y;
+         cr[1][k] = e0.z;
+         ci[1][k] = e0.w;
+         sr[0][k] = si[0][k] = sr[1][k] = si[1][k] = 0.f;
+      }
+      const float4* c4 = reinterpret_cast<const float4*>(ct + g);
+#pragma unroll 3
+      for (int q = 1; q <= Q; ++q, c4 += pitch / 2)
+      {
+         const float4 p = T[q * tp + c], n = T[(Q + q) * tp + c];
+         const float4 a = __ldg(c4), b = __ldg(c4 + 1);
+         const float co[4] = {a.x, a.z, b.x, b.z}, sn[4] = {a.y, a.w, b.y, b.w};
+#pragma unroll
+         for (int k = 0; k < 4; ++k)
+         {
+            cr[0][k] = fmaf(co[k], p.x, cr[0][k]);
+            ci[0][k] = fmaf(co[k], p.y, ci[0][k]);
+            cr[1][k] = fmaf(co[k], p.z, cr[1][k]);
+            ci[1][k] = fmaf(co[k], p.w, ci[1][k]);
+            sr[0][k] = fmaf(sn[k], n.x, sr[0][k]);
+            si[0][k] = fmaf(sn[k], n.y, si[0][k]);
+            sr[1][k] = fmaf(sn[k], n.z, sr[1][k]);
+            si[1][k] = fmaf(sn[k], n.w, si[1][k]);
+         }
+      }
+      const bool centreX = odd && t0 + c == 0;
+#pragma unroll
+      for (int k = 0; k < 4; ++k)
+      {
+         const bool centreY = odd && g + k == 0;
+#pragma unroll
+         for (int x = 0; x < 2; ++x)
+         {
+            const float pr = cr[x][k] - si[x][k], pi = ci[x][k] + sr[x][k];
+            const float mr = cr[x][k] + si[x][k], mi = ci[x][k] - sr[x][k];
+            I[k][x] = pr * pr + pi * pi;
+            I[k][2 + x] = mr * mr + mi * mi;
+            if (g + k < nT && !(x && centreX))
+               local += static_cast<double>(I[k][x]) + (centreY ? 0.0 : static_cast<double>(I[k][2 + x]));
+         }
+      }
+      if (!normalize || i + kFoldThreads < nItems)
+         store(i);   // the last item stays in registers for its normalization
+   }
    if (!normalize)
       return;
-   const double sum = BlockSumDouble(local, sRed);
-   __syncthreads();
-   if (sum > 0.0)
-      for (int idx = threadIdx.x; idx < P * P; idx += blockDim.x)
-         plane[idx] = static_cast<float>(static_cast<double>(plane[idx]) / sum);
+   const double part = BlockSumDouble(local, sRed);
+   if (tid < C)
+      cluster.map_shared_rank(sPart, tid)[rank] = part;
+   cluster.sync();
+   double sum = 0.0;
+   for (int c = 0; c < C; ++c)
+      sum += sPart[c];
+   const double inv = sum > 0.0 ? 1.0 / sum : 1.0;
+   for (int i = tid; i < nItems; i += kFoldThreads)
+   {
+      if (i + kFoldThreads < nItems)
+      {
+         // an earlier item, back from memory (its own thread's writes)
+         const int c = t0 + i % own, g = i / own * 4;
+         const int xp = half + c, xm = half - c - 1 + odd;
+#pragma unroll
+         for (int k = 0; k < 4; ++k)
+            if (g + k < nT)
+            {
+               float* yp = plane + static_cast<size_t>(half + g + k) * P;
+               float* ym = plane + static_cast<size_t>(half - g - k - 1 + odd) * P;
+               const float v[4] = {yp[xp], yp[xm], ym[xp], ym[xm]};
+               yp[xp] = static_cast<float>(v[0] * inv);
+               yp[xm] = static_cast<float>(v[1] * inv);
+               ym[xp] = static_cast<float>(v[2] * inv);
+               ym[xm] = static_cast<float>(v[3] * inv);
+            }
+         continue;
+      }
+#pragma unroll
+      for (int k = 0; k < 4; ++k)
+#pragma unroll
+         for (int j = 0; j < 4; ++j)
+            I[k][j] = static_cast<float>(I[k][j] * inv);
+      store(i);
+   }
 }
 
 // ------------------------------------------------------------------------------------------ large pupils
@@ -360,6 +527,43 @@ __global__ void NormalizeKernel(float* __restrict__ planes, const double* __rest
 
 } // namespace
 
+// The cluster of the folded kernel: a CTA for every SM where the PSFs are few (a stack), eight column pairs a CTA at
+// least, and as many as its shared memory needs.
+static int FoldCluster(const Fold& F, uint32_t nPsf, int smCount)
+{
+   int c = 1;
+   while (c < kFoldMaxCluster && (F.Bytes(c) > kFoldMaxBytes ||
+                                  (static_cast<uint64_t>(nPsf) * c < static_cast<uint64_t>(smCount) && F.nT >= 8 * c)))
+      c *= 2;
+   return c;
+}
+
+bool FoldFits(int M, int P) { return Fold(M, P).Bytes(kFoldMaxCluster) <= kFoldMaxBytes; }
+
+// The folded FP32 chirp-Z over its tables (cs).
+static int LaunchCztFold(iscu_ctx* ctx, const SetParams* dSets, const double3* dTab, const float2* cs,
+                         const PsfItem* dItems, uint32_t nPsf, int M, int P, int normalize, float* out)
+{
+   const Fold F(M, P);
+   const int c = FoldCluster(F, nPsf, ctx->smCount);
+   ISCU_CK(cudaFuncSetAttribute(CztFoldKernel, cudaFuncAttributeMaxDynamicSharedMemorySize,
+                                static_cast<int>(kFoldMaxBytes)));
+   cudaLaunchConfig_t cfg = {};
+   cfg.gridDim = dim3(nPsf * static_cast<uint32_t>(c));
+   cfg.blockDim = dim3(kFoldThreads);
+   cfg.dynamicSmemBytes = F.Bytes(c);
+   cfg.stream = ctx->stream;
+   cudaLaunchAttribute attr = {};
+   attr.id = cudaLaunchAttributeClusterDimension;
+   attr.val.clusterDim.x = static_cast<unsigned>(c);
+   attr.val.clusterDim.y = attr.val.clusterDim.z = 1;
+   cfg.attrs = &attr;
+   cfg.numAttrs = 1;
+   ISCU_CK(cudaLaunchKernelEx(&cfg, CztFoldKernel, dSets, dTab, cs, dItems, M, P, normalize, out));
+   ISCU_CK_LAUNCH(ctx, "CztFoldKernel");
+   return ISCU_OK;
+}
+
 // The large-pupil FP32 path (global-memory products); temporaries allocated here.
 static int LaunchCztGlobalFp32(iscu_ctx* ctx, const SetParams* dSets, const double3* dTab, const float2* dA,
                                const float2* dAt, const PsfItem* dItems, uint32_t nPsf, int M, int P, int normalize,
@@ -430,6 +634,16 @@ bool GeometryFor(const iscu_psf_request& r, PsfGeometry& g, std::string& err)
    return true;
 }
 
+static double Binomial(int a, int b)
+{
+   if (b < 0 || b > a)
+      return 0.0;
+   double r = 1.0;
+   for (int i = 0; i < b; ++i)
+      r = r * (a - i) / (i + 1);
+   return r;
+}
+
 // The set parameters of a request for planes of `size` samples (ZernikePsf.cpp:166-223's scalars).
 static void MakeSetParams(const iscu_psf_request& r, int M, int size, double resLateralNm, SetParams& sp)
 {
@@ -465,6 +679,10 @@ static void MakeSetParams(const iscu_psf_request& r, int M, int size, double res
       sp.modeN[n] = nn;
       sp.modeL[n] = l;
       sp.modeM[n] = std::abs(l);
+      // R_n^m = sum_k (-1)^k C(n - k, k) C(n - 2k, (n - m) / 2 - k) rho^(n - 2k) (ZernikePsf.cpp:58-67)
+      const int half = (nn - std::abs(l)) / 2;
+      for (int q = 0; q <= half; ++q)
+         sp.radial[n][q] = (q % 2 ? -1.0 : 1.0) * Binomial(nn - q, q) * Binomial(nn - 2 * q, half - q);
       ++n;
    }
    sp.nModes = n;
@@ -506,43 +724,33 @@ int BuildPsfLibrary(iscu_ctx* ctx, const iscu_psf_request* sets, uint32_t nSets,
       items[i].dtiM = ti - sp.ti0;
    }
    const size_t tabBytes = static_cast<size_t>(nSets) * M * M * sizeof(double3);
-   const size_t matBytes = static_cast<size_t>(nSets) * P * M * sizeof(float2);
-   const size_t setBytes = nSets * sizeof(SetParams), itemBytes = nPsf * sizeof(PsfItem);
-   DevBuf dSets, dItems, dTab, dA, dAt;
-   ISCU_CK(dSets.Reserve(setBytes));
-   ISCU_CK(dItems.Reserve(itemBytes));
-   ISCU_CK(dTab.Reserve(tabBytes));
-   ISCU_CK(dA.Reserve(matBytes));
-   ISCU_CK(dAt.Reserve(matBytes));
-   ISCU_CK(cudaMemcpyAsync(dSets.p, hs.data(), setBytes, cudaMemcpyHostToDevice, ctx->stream));
-   ISCU_CK(cudaMemcpyAsync(dItems.p, items.data(), itemBytes, cudaMemcpyHostToDevice, ctx->stream));
-   PupilTablesKernel<<<dim3((M * M + 127) / 128, nSets), 128, 0, ctx->stream>>>(dSets.as<SetParams>(), M,
-                                                                                 dTab.as<double3>());
-   ISCU_CK_LAUNCH(ctx, "PupilTablesKernel");
-   DftMatrixKernel<<<dim3((P * M + 255) / 256, nSets), 256, 0, ctx->stream>>>(dSets.as<SetParams>(), M, P,
-                                                                              dA.as<float2>(), dAt.as<float2>());
-   ISCU_CK_LAUNCH(ctx, "DftMatrixKernel");
-   if (method == ISCU_CZT_TF32X3 || method == ISCU_CZT_F16X3)
-   {
-      const int rc = LaunchCztSplit(ctx, method, dSets.as<SetParams>(), dTab.as<double3>(), dA.as<float2>(), nSets,
-                                    dItems.as<PsfItem>(), nPsf, M, P, normalize, out);
-      if (rc != ISCU_OK)
-         return rc;
-   }
-   else
-   {
-      const size_t smem = (static_cast<size_t>(M) * M + static_cast<size_t>(P) * M) * sizeof(float2);
-      if (smem > 227 * 1024)
-         return LaunchCztGlobalFp32(ctx, dSets.as<SetParams>(), dTab.as<double3>(), dA.as<float2>(),
-                                    dAt.as<float2>(), dItems.as<PsfItem>(), nPsf, M, P, normalize, out);
-      ISCU_CK(cudaFuncSetAttribute(CztFp32Kernel, cudaFuncAttributeMaxDynamicSharedMemorySize,
-                                   static_cast<int>(smem)));
-      CztFp32Kernel<<<nPsf, kCztThreads, smem, ctx->stream>>>(dSets.as<SetParams>(), dTab.as<double3>(),
-                                                               dA.as<float2>(), dAt.as<float2>(),
-                                                               dItems.as<PsfItem>(), M, P, normalize, out);
-      ISCU_CK_LAUNCH(ctx, "CztFp32Kernel");
-   }
-   // The temporaries are freed when this returns; the stream must finish with them first.
+   const size_t matBytes = static_cast<size_t>(nSets) * std::max(P, 2) * M * sizeof(float2);
+   const size_t setBytes = (nSets * sizeof(SetParams) + 15) / 16 * 16, itemBytes = nPsf * sizeof(PsfItem);
+   const bool split = method == ISCU_CZT_TF32X3 || method == ISCU_CZT_F16X3, folded = !split && FoldFits(M, P);
+   // One buffer: the sets and the items (one copy), the tables, the matrices. The context keeps it up to kPsfScratchKept
+   // bytes (calls hold the context's lock and end synchronized): five allocations and frees a call took 20 to 500 us.
+   const size_t inBytes = (setBytes + itemBytes + 255) / 256 * 256, tabEnd = inBytes + (tabBytes + 255) / 256 * 256;
+   const size_t aEnd = tabEnd + (matBytes + 255) / 256 * 256, allBytes = folded ? aEnd : aEnd + matBytes;
+   DevBuf own;
+   DevBuf& buf = allBytes <= kPsfScratchKept ? ctx->psfScratch : own;
+   ISCU_CK(buf.Reserve(allBytes));
+   unsigned char* base = buf.as<unsigned char>();
+   double3* dTab = reinterpret_cast<double3*>(base + inBytes);
+   float2* dA = reinterpret_cast<float2*>(base + tabEnd);
+   float2* dAt = folded ? nullptr : reinterpret_cast<float2*>(base + aEnd);
+   std::vector<unsigned char> in(setBytes + itemBytes);
+   std::memcpy(in.data(), hs.data(), nSets * sizeof(SetParams));
+   std::memcpy(in.data() + setBytes, items.data(), itemBytes);
+   ISCU_CK(cudaMemcpyAsync(base, in.data(), in.size(), cudaMemcpyHostToDevice, ctx->stream));
+   const SetParams* dSets = reinterpret_cast<const SetParams*>(base);
+   const PsfItem* dItems = reinterpret_cast<const PsfItem*>(base + setBytes);
+   int rc = LaunchPsfTables(ctx, dSets, nSets, M, P, dTab, dA, dAt, folded);
+   if (rc == ISCU_OK)
+      rc = split ? LaunchCztSplit(ctx, method, dSets, dTab, dA, nSets, dItems, nPsf, M, P, normalize, out)
+                 : LaunchCztFp32(ctx, dSets, dTab, dA, dAt, dItems, nPsf, M, P, normalize, out);
+   if (rc != ISCU_OK)
+      return rc;
+   // The temporaries are another call's, or freed, when this returns; the stream must finish with them first.
    ISCU_CK(cudaStreamSynchronize(ctx->stream));
    return ISCU_OK;
 }
@@ -572,63 +780,57 @@ int PrepareSetParams(const iscu_psf_request* sets, uint32_t nSets, int32_t size,
    return ISCU_OK;
 }
 
-// The per-set tables and DFT matrices (once per set; a PSF plan keeps them).
 int LaunchPsfTables(iscu_ctx* ctx, const SetParams* dSets, uint32_t nSets, int M, int P, double3* dTab, float2* dA,
-                    float2* dAt)
+                    float2* dAt, bool folded)
 {
-   PupilTablesKernel<<<dim3((M * M + 127) / 128, nSets), 128, 0, ctx->stream>>>(dSets, M, dTab);
+   const Fold F(M, P);   // (Q x pitch float2 of cs fit max(P, 2) x M)
+   const int blocks = (M * M + kTableThreads - 1) / kTableThreads +
+                      (folded ? (F.Q * F.Pitch() + kTableThreads - 1) / kTableThreads : 0);
+   PupilTablesKernel<<<dim3(blocks, nSets), kTableThreads, 0, ctx->stream>>>(dSets, M, P, dTab, folded ? dA : nullptr);
    ISCU_CK_LAUNCH(ctx, "PupilTablesKernel");
+   if (folded)
+      return ISCU_OK;
    DftMatrixKernel<<<dim3((P * M + 255) / 256, nSets), 256, 0, ctx->stream>>>(dSets, M, P, dA, dAt);
    ISCU_CK_LAUNCH(ctx, "DftMatrixKernel");
    return ISCU_OK;
 }
 
-// The plain FP32 chirp-Z of nPsf items over prepared tables (shared-memory form, or the global-memory form for
-// pupils beyond shared memory).
+// The plain FP32 chirp-Z of nPsf items over prepared tables (the folded form where FoldFits, else the global-memory
+// form for pupils beyond shared memory).
 int LaunchCztFp32(iscu_ctx* ctx, const SetParams* dSets, const double3* dTab, const float2* dA, const float2* dAt,
                   const PsfItem* dItems, uint32_t nPsf, int M, int P, int normalize, float* out)
 {
-   const size_t smem = (static_cast<size_t>(M) * M + static_cast<size_t>(P) * M) * sizeof(float2);
-   if (smem > 227 * 1024)
-      return LaunchCztGlobalFp32(ctx, dSets, dTab, dA, dAt, dItems, nPsf, M, P, normalize, out);
-   ISCU_CK(cudaFuncSetAttribute(CztFp32Kernel, cudaFuncAttributeMaxDynamicSharedMemorySize, static_cast<int>(smem)));
-   CztFp32Kernel<<<nPsf, kCztThreads, smem, ctx->stream>>>(dSets, dTab, dA, dAt, dItems, M, P, normalize, out);
-   ISCU_CK_LAUNCH(ctx, "CztFp32Kernel");
-   return ISCU_OK;
+   if (FoldFits(M, P))
+      return LaunchCztFold(ctx, dSets, dTab, dA, dItems, nPsf, M, P, normalize, out);
+   return LaunchCztGlobalFp32(ctx, dSets, dTab, dA, dAt, dItems, nPsf, M, P, normalize, out);
 }
 
 int CheckFp32CztSmem(iscu_ctx* ctx, int M, int P, size_t* smem)
 {
    *smem = (static_cast<size_t>(M) * M + static_cast<size_t>(P) * M) * sizeof(float2);
-   cudaFuncAttributes fa;
-   ISCU_CK(cudaFuncGetAttributes(&fa, CztFp32Kernel));
+   constexpr size_t kBeside = 64;   // static shared memory that the limit leaves room for
    int optin = 0;
    ISCU_CK(cudaDeviceGetAttribute(&optin, cudaDevAttrMaxSharedMemoryPerBlockOptin, ctx->device));
-   if (*smem + fa.sharedSizeBytes > static_cast<size_t>(optin))
+   if (*smem + kBeside > static_cast<size_t>(optin))
       return Fail(ISCU_ERR_LIMIT, "psf library (fp32): the pupil and row pass need (M*M + P*M)*8 = " +
                                      std::to_string(*smem) + " bytes of shared memory beside the kernel's " +
-                                     std::to_string(fa.sharedSizeBytes) + ", over the device's " +
+                                     std::to_string(kBeside) + ", over the device's " +
                                      std::to_string(optin) + " per block (M = " + std::to_string(M) + ", P = " +
                                      std::to_string(P) + ")");
    return ISCU_OK;
 }
 
-// The plain FP32 pipeline (tables, DFT matrices, chirp-Z) on buffers the caller provides.
+// The plain FP32 pipeline (tables, chirp-Z) on buffers the caller provides.
 int LaunchPsfPipelineFp32(iscu_ctx* ctx, const SetParams* dSets, const PsfItem* dItems, double3* dTab, float2* dA,
                           float2* dAt, uint32_t nSets, uint32_t nPsf, int M, int P, int normalize, float* out)
 {
-   PupilTablesKernel<<<dim3((M * M + 127) / 128, nSets), 128, 0, ctx->stream>>>(dSets, M, dTab);
-   ISCU_CK_LAUNCH(ctx, "PupilTablesKernel");
-   DftMatrixKernel<<<dim3((P * M + 255) / 256, nSets), 256, 0, ctx->stream>>>(dSets, M, P, dA, dAt);
-   ISCU_CK_LAUNCH(ctx, "DftMatrixKernel");
    size_t smem = 0;
-   const int rc = CheckFp32CztSmem(ctx, M, P, &smem);
-   if (rc != ISCU_OK)
-      return rc;
-   ISCU_CK(cudaFuncSetAttribute(CztFp32Kernel, cudaFuncAttributeMaxDynamicSharedMemorySize, static_cast<int>(smem)));
-   CztFp32Kernel<<<nPsf, kCztThreads, smem, ctx->stream>>>(dSets, dTab, dA, dAt, dItems, M, P, normalize, out);
-   ISCU_CK_LAUNCH(ctx, "CztFp32Kernel");
-   return ISCU_OK;
+   int rc = CheckFp32CztSmem(ctx, M, P, &smem);   // (every shape within it folds)
+   if (rc == ISCU_OK)
+      rc = LaunchPsfTables(ctx, dSets, nSets, M, P, dTab, dA, dAt, true);
+   if (rc == ISCU_OK)
+      rc = LaunchCztFold(ctx, dSets, dTab, dA, dItems, nPsf, M, P, normalize, out);
+   return rc;
 }
 
 } // namespace iscu

@@ -15,6 +15,7 @@ struct SetParams
    double maskWaist;
    int doubleHelix, maskModes, nModes, pad;
    double coeff[28];
+   double radial[28][4];   // R_n^m's coefficients, of rho^n downwards in steps of rho^2 (n <= 6)
    int modeN[28], modeL[28], modeM[28];
 };
 
@@ -84,16 +85,20 @@ int LaunchCztTf32x3Core(iscu_ctx* ctx, const SetParams* sets, const float* ahat,
 int LaunchCztF16x3Core(iscu_ctx* ctx, const SetParams* sets, const unsigned char* ahat, int nSets,
                        const PsfItem* items, uint32_t nPsf, int M, int P, int normalize, float* out, int* dErr);
 
+// The per-set tables: the pupil's, and either the DFT matrices A (P x M) and A^T (M x P) or, where FoldFits, the folded
+// transform's cosines and sines in dA (dAt untouched).
 int LaunchPsfTables(iscu_ctx* ctx, const SetParams* dSets, uint32_t nSets, int M, int P, double3* dTab, float2* dA,
-                    float2* dAt);
+                    float2* dAt, bool folded);
+// Whether planes of P samples from M pupil samples run as the folded shared-memory kernel.
+bool FoldFits(int M, int P);
 int LaunchCztFp32(iscu_ctx* ctx, const SetParams* dSets, const double3* dTab, const float2* dA, const float2* dAt,
                   const PsfItem* dItems, uint32_t nPsf, int M, int P, int normalize, float* out);
 
 int PrepareSetParams(const iscu_psf_request* sets, uint32_t nSets, int32_t size, uint32_t maxSets, SetParams* out,
                      int* M, int* P);
-// ISCU_OK when the FP32 chirp-Z kernel's dynamic shared memory -- the pupil (M x M) and the row pass (P x M), complex
-// float -- fits beside its static shared memory in one CTA of the context's device (the per-block opt-in limit);
-// ISCU_ERR_LIMIT (naming the bytes) otherwise. *smem: the dynamic bytes.
+// ISCU_OK when the pupil (M x M) and the row pass (P x M), complex float, fit a CTA's shared memory on the context's
+// device (the per-block opt-in limit less 64 bytes); ISCU_ERR_LIMIT (naming the bytes) otherwise: the allocation-free
+// entry's limit. *smem: the bytes.
 int CheckFp32CztSmem(iscu_ctx* ctx, int M, int P, size_t* smem);
 int LaunchPsfPipelineFp32(iscu_ctx* ctx, const SetParams* dSets, const PsfItem* dItems, double3* dTab, float2* dA,
                           float2* dAt, uint32_t nSets, uint32_t nPsf, int M, int P, int normalize, float* out);

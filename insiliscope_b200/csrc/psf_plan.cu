@@ -112,12 +112,12 @@ int iscu_psf_plan_create(iscu_ctx* ctx, const iscu_psf_request* sets, uint32_t n
    const size_t M = p->M, P = p->P;
    ISCU_CK(p->sets.Reserve(n_sets * sizeof(SetParams)));
    ISCU_CK(p->tab.Reserve(n_sets * M * M * sizeof(double3)));
-   ISCU_CK(p->A.Reserve(n_sets * P * M * sizeof(float2)));
+   ISCU_CK(p->A.Reserve(n_sets * std::max<size_t>(P, 2) * M * sizeof(float2)));
    ISCU_CK(p->At.Reserve(n_sets * P * M * sizeof(float2)));
    ISCU_CK(p->err.Reserve(sizeof(int)));
    ISCU_CK(cudaMemcpyAsync(p->sets.p, hs.data(), n_sets * sizeof(SetParams), cudaMemcpyHostToDevice, ctx->stream));
    rc = LaunchPsfTables(ctx, p->sets.as<SetParams>(), n_sets, p->M, p->P, p->tab.as<double3>(), p->A.as<float2>(),
-                        p->At.as<float2>());
+                        p->At.as<float2>(), method == ISCU_CZT_FP32 && FoldFits(p->M, p->P));
    if (rc != ISCU_OK)
       return rc;
    if (method != ISCU_CZT_FP32 &&

@@ -182,3 +182,28 @@ def test_plan_run_in_chunks_matches_device_run(engine, method):
     with pytest.raises(IscuError):
         plan.run(bad, L.defocus_nm)
     plan.close()
+
+
+@pytest.mark.parametrize("M,size,n", [(8, 1, 2), (9, 2, 3), (33, 7, 1), (64, 129, 3), (64, 130, 200), (100, 65, 20),
+                                      (128, 129, 2), (127, 64, 40), (16, 300, 1)])
+def test_folded_planes_vs_oracle(engine, oracle, M, size, n):
+    """The folded FP32 form over odd and even pupils and planes, one plane to more than the SMs (clusters of 8 to 1),
+    sizes with a remainder in every split, normalized and not, two sets with aberrations that are neither even nor odd,
+    from the library and from a plan; a double-helix mask in the second set."""
+    from insiliscope_b200.engine import PsfPlan
+    rng = np.random.default_rng(M + size)
+    zern = [0.0, 0.0, 0.0] + list(rng.normal(0.0, 0.08, 25))
+    sets = [PsfParams(wavelength_nm=670.0, na=1.4, sample_index=1.33, sample_depth_nm=300.0, pixel_size_nm=100.0,
+                      zernike=zern, oversampling=3, kernel_half_width_px=8, nz=3, pupil_samples=M),
+            PsfParams(wavelength_nm=580.0, na=1.3, pixel_size_nm=110.0, oversampling=4, kernel_half_width_px=8, nz=3,
+                      double_helix=True, pupil_samples=M)]
+    set_of = np.arange(n, dtype=np.uint32) % 2
+    dz = rng.uniform(-500.0, 500.0, n)
+    plan = PsfPlan(engine, sets, size=size)
+    for normalize in (True, False):
+        got = engine.psf_library_dev(sets, set_of, dz, size=size, normalize=normalize).cpu().numpy()
+        assert np.array_equal(plan.run(set_of, dz, normalize=normalize), got)
+        for i in range(0, n, max(1, n // 4)):
+            want = oracle.psf_planes(sets[set_of[i]], dz[i:i + 1] * 1e-9, size=size, normalize=normalize)
+            assert _max_rel(got[i:i + 1], want) <= TOL, (i, normalize)
+    plan.close()
