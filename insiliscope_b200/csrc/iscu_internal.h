@@ -181,7 +181,7 @@ struct StaticView
 // origin) groups, and every emitter's float contribution to each pixel of its square.
 struct ContribScratch
 {
-   DevBuf rec, grec, keys, list, contrib, ctr;
+   DevBuf rec, grec, keys, list, chunks, contrib, ctr;
 };
 
 // One I/O slot of the event render (iscu_render_events[_async]): the batch's device staging (events, bucket and

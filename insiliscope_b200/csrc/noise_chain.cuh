@@ -80,11 +80,11 @@ static __device__ __noinline__ uint32_t NoisePixelExact(float photonValue, uint3
 // ------------------------------------------------------------------------------------------------ the fast chain
 // NoisePixel is the same chain with every decision taken in float32 where it is sure, so the ADU are the float64
 // chain's bits. What bounds the chain is the issue and integer rate of the Knuth loop's hashes (its trip count is the
-// reference's by definition), so the loop carries nothing in float64: 29 instructions a hash against 44, one word of
+// reference's by definition), so the loop carries nothing in float64: 28 instructions a hash against 44, one word of
 // the stream selected instead of queued, no float64 exponential, logarithm, quotient or conversion (a conversion
 // issues at a quarter of the float64 rate). Error bounds, each stated where it is used, are at least 1.4 times what the
 // operations' documented bounds add up to; in doubt (about one pixel in 10^4) the float64 chain decides. Measured: the
-// sCMOS noise of 16 frames of 512 x 512 px 159 -> 97 us a call, the EMCCD noise of 64 such frames 0.66 -> 0.36 ms.
+// sCMOS noise of 16 frames of 512 x 512 px 159 -> 94 us a call, the EMCCD noise of 64 such frames 0.66 -> 0.35 ms.
 
 __device__ __forceinline__ float Ex2Approx(float x)
 {
@@ -115,6 +115,22 @@ __device__ __forceinline__ float RcpApprox(float x)
 __device__ __forceinline__ float UniformF(uint32_t x)
 {
    return __uint_as_float(__funnelshift_r(x, 0x7fu, 9)) - 0.999999940395355224609375f;
+}
+
+// The product of the four words' uniforms, two lanes at a time (each rounds as the one-lane instruction).
+__device__ __forceinline__ float UniformProduct(const uint32_t (&w)[4])
+{
+   const uint64_t c = 0xBF7FFFFFBF7FFFFFull;   // -(1 - 2^-24), twice
+   uint64_t x, y;
+   asm("{.reg .b64 t; mov.b64 t, {%1, %2}; add.rn.f32x2 %0, t, %3;}"
+       : "=l"(x)
+       : "r"(__funnelshift_r(w[0], 0x7fu, 9)), "r"(__funnelshift_r(w[1], 0x7fu, 9)), "l"(c));
+   asm("{.reg .b64 t; mov.b64 t, {%1, %2}; add.rn.f32x2 %0, t, %3;}"
+       : "=l"(y)
+       : "r"(__funnelshift_r(w[2], 0x7fu, 9)), "r"(__funnelshift_r(w[3], 0x7fu, 9)), "l"(c));
+   uint64_t z;
+   asm("mul.rn.f32x2 %0, %1, %2;" : "=l"(z) : "l"(x), "l"(y));
+   return __uint_as_float(static_cast<uint32_t>(z)) * __uint_as_float(static_cast<uint32_t>(z >> 32));
 }
 
 // A pixel's hashes by counter. Before its first exclusive-or the permutation's words d, a and b are linear in the
@@ -213,33 +229,31 @@ __device__ __forceinline__ uint16_t NoisePixel(float photonValue, uint32_t i, co
    if (lf <= 59.9999f && lf >= 1e-6f)
    {
       // Knuth. L within 1.2e-5 + 4e-6 (lambda's error, the argument's rounding, ex2.approx) of exp(-mean); the
-      // product within 2^-24 per factor of the float64 one, 256 factors at most here (1.6e-5): the margin is 6e-5.
+      // product within 2^-24 per factor of the float64 one, 256 factors at most here (1.6e-5), and two more for the
+      // block's start below: the margin is 6e-5.
       const float L = Ex2Approx(lf * -1.44269504f), hi = L * 1.00006f, lo = L * 0.99994f;
       const uint32_t mul = 1664525u, inc = 1013904223u, sa = (frame * mul + inc) * mul;
       uint32_t d = inc, a = H.a0, b = H.b0, w[4];
-      float p = 1.f, u0, u2, p2, p4;
-      int blk = 0;
-      for (;; ++blk)
+      float p4 = 1.f, prod;
+      do
       {
          H.Finish(d, a, b, w);
-         u0 = UniformF(w[0]);
-         u2 = UniformF(w[2]);
-         p2 = u0 * UniformF(w[1]);
-         p4 = p * (p2 * (u2 * UniformF(w[3])));
+         prod = UniformProduct(w);
+         p4 *= prod;
          d += mul;
          a += sa;
          b += H.sb;
-         if (!(p4 > hi) || blk == 63)
-            break;
-         p = p4;
-      }
+      } while (p4 > hi);   // (each factor is below 1)
+      // d is linear in the counter: the blocks drawn, from mul's inverse mod 2^32; the product before the last block
+      const uint32_t drawn = (d - inc) * 0xFEE058C5u;
+      const float p = p4 * RcpApprox(prod), u0 = UniformF(w[0]), u2 = UniformF(w[2]), p2 = u0 * UniformF(w[1]);
       // the block's first product at or below L: its factor ends the draw
       const float q1 = p * u0, q2 = p * p2, q3 = q2 * u2;
       const bool o1 = q1 > hi, o2 = o1 && q2 > hi, o3 = o2 && q3 > hi;
       const float last = o3 ? p4 : (o2 ? q3 : (o1 ? q2 : q1));
-      ok = ok && last < lo;
+      ok = ok && last < lo && drawn <= 64u && p4 > 1e-36f;   // (a subnormal product has lost its places)
       const int n = o3 ? 3 : (o2 ? 2 : (o1 ? 1 : 0));
-      pos = 4 * blk + n;
+      pos = 4 * (drawn - 1) + n;
       ne = static_cast<float>(pos);
       ++pos;
       if (!cam.emccd)

@@ -9,8 +9,8 @@
 //     (slot, plane, bx, by) counted;
 //  2. the groups' offsets (one CTA scan) and 3. each emitter listed under its group;
 //  4. contributions: a CTA takes a group's block of square pixels and up to 64 of its emitters; each thread loads its
-//     pixel's taps into registers once and computes every emitter's float contribution, in the reference's operation
-//     order, into HBM (emitter-major, one float per pixel of the square);
+//     pixel's taps into registers once and computes every emitter's float contribution -- the reference's value, from
+//     a fused sum where that rounds alike -- into HBM (emitter-major, one float per pixel of the square);
 //  5. gather (one CTA per frame tile, or a persistent grid heaviest frame first): every pixel adds, in the frame's
 //     emitter order, the contributions of the emitters whose square (and halo cut) covers it -- the same float
 //     additions in the same order as RenderPhotonImage (SMLMSimulation.cpp:103-160) -- then the noise chain
@@ -31,24 +31,13 @@ namespace iscu {
 
 namespace {
 
-constexpr int kE = 64;          // emitters per contribution work item
-// Contribution CTAs: at most 384 computing threads and a staging warp, two per SM (72 registers: the 16 float64 taps
-// in registers without spills). A 33 x 33 square is three pixel blocks, so a group's per-item work (its taps from L2,
-// its geometry, the barrier) is paid three times rather than five as with 224-thread CTAs four to an SM, while the
-// other CTA keeps the FP64 pipe busy through one CTA's barrier.
-constexpr int kMaxCT = 384;
-constexpr int kContribPerSm = 2;
+constexpr int kE = 64;          // emitters per contribution chunk
+// Contribution CTAs: at most kMaxCT computing threads and a staging warp.
+constexpr int kMaxCT = 192;
+constexpr int kContribPerSm = 4;
 constexpr int kGT = 256;        // gather CTA size (one thread per pixel of the tile)
+constexpr int kGList = 64;       // a warp's list: worked off when the next 32 emitters may not fit
 constexpr int kGChunk = 256;    // gather staging chunk
-
-// One emitter's setup, as the contribution pass reads it.
-struct SplatRec
-{
-   double photons;
-   double wx[4], wy[4];
-   int bx, by;
-   int key, plane;
-};
 
 // The group keys: slot s owns keys [base[s], base[s + 1]); key base[s] + (plane n1 + (by - lo)) n1 + (bx - lo) is the
 // group (s, plane, bx, by); the slot's last key collects tap origins outside [lo, lo + n1) (none arise from finite
@@ -58,7 +47,6 @@ struct KeyMap
    int base[ISCU_MAX_KERNELS + 1];
    int lo[ISCU_MAX_KERNELS];
    int n1[ISCU_MAX_KERNELS];
-   int pbs[ISCU_MAX_KERNELS];    // pixel blocks of a group's square (ceil(side^2 / contribution CTA size))
    int side[ISCU_MAX_KERNELS];   // splat square side, 2 camRad + 1
 };
 
@@ -84,49 +72,44 @@ struct SetupArgs
    uint32_t n;
    Kernels K;
    KeyMap km;
-   SplatRec* rec;
+   int* key;          // per emitter; -1: not splatted
    int4* grec;        // per emitter (x0, y0, slot, plane); slot -1: not splatted
    uint32_t* count;   // per key
 };
+
+// An emitter's slot, SplatSetup and key (false: not splatted).
+__device__ __forceinline__ bool SetupEmitter(const Kernels& K, const KeyMap& km, const iscu_emitter& em, int& slot,
+                                             int& plane, int& key, StagedEmitter& s)
+{
+   slot = static_cast<int>(static_cast<uint32_t>(em.plane) >> 16);
+   plane = em.plane & 0xffff;
+   if (!(slot < ISCU_MAX_KERNELS && em.photons > 0.0 && K.k[slot].sums64 && plane < K.k[slot].nz &&
+         PositionOk(em.x_px, em.y_px)))
+      return false;
+   s.x0 = static_cast<int>(RoundHalfUp(em.x_px));
+   s.y0 = static_cast<int>(RoundHalfUp(em.y_px));
+   SetupWeights(K.k[slot], em.x_px, em.y_px, s);
+   const int n1 = km.n1[slot], cy = s.by - km.lo[slot], cx = s.bx - km.lo[slot];
+   key = (cy >= 0 && cy < n1 && cx >= 0 && cx < n1) ? km.base[slot] + (plane * n1 + cy) * n1 + cx
+                                                    : km.base[slot + 1] - 1;
+   return true;
+}
 
 __global__ void ContribSetupKernel(SetupArgs a)
 {
    const uint32_t g = blockIdx.x * blockDim.x + threadIdx.x;
    bool valid = false;
-   int key = 0;
+   int key = -1;
    if (g < a.n)
    {
-      const iscu_emitter em = a.ems[g];
-      const int slot = static_cast<int>(static_cast<uint32_t>(em.plane) >> 16), plane = em.plane & 0xffff;
+      int slot = 0, plane = 0;
+      StagedEmitter s;
       int4 gr = make_int4(0, 0, -1, 0);
-      if (slot < ISCU_MAX_KERNELS && em.photons > 0.0 && a.K.k[slot].sums64 && plane < a.K.k[slot].nz &&
-          PositionOk(em.x_px, em.y_px))
-      {
-         const KernelView& kv = a.K.k[slot];
-         StagedEmitter s;
-         s.x0 = static_cast<int>(RoundHalfUp(em.x_px));
-         s.y0 = static_cast<int>(RoundHalfUp(em.y_px));
-         SetupWeights(kv, em.x_px, em.y_px, s);
-         SplatRec r;
-         r.photons = em.photons;
-#pragma unroll
-         for (int k = 0; k < 4; ++k)
-         {
-            r.wx[k] = s.wx[k];
-            r.wy[k] = s.wy[k];
-         }
-         r.bx = s.bx;
-         r.by = s.by;
-         r.plane = plane;
-         const int n1 = a.km.n1[slot], cy = s.by - a.km.lo[slot], cx = s.bx - a.km.lo[slot];
-         key = (cy >= 0 && cy < n1 && cx >= 0 && cx < n1) ? a.km.base[slot] + (plane * n1 + cy) * n1 + cx
-                                                          : a.km.base[slot + 1] - 1;
-         r.key = key;
-         a.rec[g] = r;
+      valid = SetupEmitter(a.K, a.km, a.ems[g], slot, plane, key, s);
+      if (valid)
          gr = make_int4(s.x0, s.y0, slot, plane);
-         valid = true;
-      }
       a.grec[g] = gr;
+      a.key[g] = valid ? key : -1;
    }
    const unsigned vm = __ballot_sync(0xffffffffu, valid);
    if (valid)
@@ -139,14 +122,14 @@ __global__ void ContribSetupKernel(SetupArgs a)
 
 // ------------------------------------------------------------------------------------------------ 2. offsets
 // One CTA of 1024 threads, kScanPer consecutive keys a thread per pass of 4,096 keys (one round trip for the counts):
-// start[k] = exclusive sum of count, itemStart[k] = exclusive sum of the keys' work items (ceil(count / kE) emitter
-// chunks x the slot's pixel blocks), itemKey[i] = k for each of key k's items; itemStart[nKeys] and ctr[0] = the
-// total; ctr[1] = 0.
+// start[k] = exclusive sum of count, chunkStart[k] = exclusive sum of the keys' chunks (ceil(count / kE)); ctr[0] = the
+// chunks' total; ctr[1] = 0. (The chunks' records are written by the scatter: one thread listing all of a key's work in
+// turn took 14 of this kernel's 26 us on the two-colour movie.)
 constexpr int kScanPer = 4;
 __global__ void __launch_bounds__(1024) ContribScanKernel(KeyMap km, const uint32_t* __restrict__ count,
                                                           uint32_t* __restrict__ start, uint32_t* __restrict__ cursor,
-                                                          uint32_t* __restrict__ itemStart,
-                                                          uint32_t* __restrict__ itemKey, uint32_t* __restrict__ ctr)
+                                                          uint32_t* __restrict__ chunkStart,
+                                                          uint32_t* __restrict__ ctr)
 {
    const int nKeys = km.base[ISCU_MAX_KERNELS];
    const int lane = threadIdx.x & 31, warp = threadIdx.x >> 5;
@@ -165,7 +148,7 @@ __global__ void __launch_bounds__(1024) ContribScanKernel(KeyMap km, const uint3
 #pragma unroll
       for (int j = 0; j < kScanPer; ++j)
       {
-         it[j] = c[j] ? ((c[j] + kE - 1) / kE) * static_cast<uint32_t>(km.pbs[SlotOfKey(km, kb + j)]) : 0u;
+         it[j] = (c[j] + kE - 1) / kE;
          tc += c[j];
          ti += it[j];
       }
@@ -213,9 +196,7 @@ __global__ void __launch_bounds__(1024) ContribScanKernel(KeyMap km, const uint3
          {
             start[k] = ec;
             cursor[k] = ec;
-            itemStart[k] = ei;
-            for (uint32_t q = 0; q < it[j]; ++q)
-               itemKey[ei + q] = static_cast<uint32_t>(k);
+            chunkStart[k] = ei;
          }
          ec += c[j];
          ei += it[j];
@@ -230,7 +211,6 @@ __global__ void __launch_bounds__(1024) ContribScanKernel(KeyMap km, const uint3
    }
    if (threadIdx.x == 0)
    {
-      itemStart[nKeys] = carry[1];
       ctr[0] = carry[1];
       ctr[1] = 0;
    }
@@ -238,20 +218,53 @@ __global__ void __launch_bounds__(1024) ContribScanKernel(KeyMap km, const uint3
 
 // ------------------------------------------------------------------------------------------------ 3. lists
 // An emitter as the contribution pass stages it; the lists hold these records in group order.
-struct CStage
+struct __align__(16) CStage
 {
-   double photons;
-   double wx[4], wy[4];
+   double wx[4], wp[4];   // the column weights; the row weights times the photons
    uint32_t g;
-   int bx, by, plane;
+   float thr;             // 2^-10 x 1.6 photons: below thr x the taps' largest magnitude a sum cancels too much
+   int bx, by;
+   double photons;
+   double wy[4];
+   int plane, pad;
+};
+static_assert(sizeof(CStage) == 128, "8 x 16 bytes");
+
+// Up to kE emitters of one group, with what is the same for the group's pixels: worked out once a chunk (the tap
+// offsets' divisions alone were 400 instructions a thread and work item, a third of the contribution pass).
+struct __align__(16) CChunk
+{
+   int off[16];          // tap (j, i)'s offset in the phase layout from a pixel's own word
+   const double* base;   // the plane's words of the phase layout
+   int first, cnt;       // stage records
+   int slot, plane;
+   int kind;             // 0 the misc group; 1 tap origins beyond the phase layout; 2 within it
+   float invSide;
+   int pad[8];
+};
+static_assert(sizeof(CChunk) == 128, "8 x 16 bytes");
+
+struct ScatterArgs
+{
+   const iscu_emitter* ems;
+   uint32_t n;
+   Kernels K;
+   KeyMap km;
+   const int* key;
+   const uint32_t* count;
+   const uint32_t* start;
+   uint32_t* cursor;
+   const uint32_t* chunkStart;
+   CStage* stage;
+   CChunk* chunk;
 };
 
-__global__ void ContribScatterKernel(uint32_t n, const SplatRec* __restrict__ rec, const int4* __restrict__ grec,
-                                     uint32_t* __restrict__ cursor, CStage* __restrict__ stage)
+// Each emitter's record in its group's list; the first emitter of a chunk writes the chunk's.
+__global__ void ContribScatterKernel(ScatterArgs a)
 {
    const uint32_t g = blockIdx.x * blockDim.x + threadIdx.x;
-   const bool valid = g < n && grec[g].z >= 0;
-   const int key = valid ? rec[g].key : 0;
+   const int key = g < a.n ? a.key[g] : -1;
+   const bool valid = key >= 0;
    const unsigned vm = __ballot_sync(0xffffffffu, valid);
    if (!valid)
       return;
@@ -260,22 +273,52 @@ __global__ void ContribScatterKernel(uint32_t n, const SplatRec* __restrict__ re
    const int leader = __ffs(peers) - 1;
    uint32_t base = 0;
    if (lane == leader)
-      base = atomicAdd(&cursor[key], static_cast<uint32_t>(__popc(peers)));
+      base = atomicAdd(&a.cursor[key], static_cast<uint32_t>(__popc(peers)));
    base = __shfl_sync(peers, base, leader);
-   const SplatRec& r = rec[g];
-   CStage s;
-   s.photons = r.photons;
+   const uint32_t at = base + __popc(peers & ((1u << lane) - 1u));
+   const iscu_emitter em = a.ems[g];
+   int slot = 0, plane = 0, k2 = 0;
+   StagedEmitter s;
+   SetupEmitter(a.K, a.km, em, slot, plane, k2, s);
+   CStage c;
 #pragma unroll
    for (int k = 0; k < 4; ++k)
    {
-      s.wx[k] = r.wx[k];
-      s.wy[k] = r.wy[k];
+      c.wx[k] = s.wx[k];
+      c.wy[k] = s.wy[k];
+      c.wp[k] = em.photons * s.wy[k];
    }
-   s.g = g;
-   s.bx = r.bx;
-   s.by = r.by;
-   s.plane = r.plane;
-   stage[base + __popc(peers & ((1u << lane) - 1u))] = s;
+   c.photons = em.photons;
+   c.thr = static_cast<float>(em.photons * (1.6 / 1024.0));
+   c.g = g;
+   c.bx = s.bx;
+   c.by = s.by;
+   c.plane = plane;
+   c.pad = 0;
+   a.stage[at] = c;
+   const uint32_t pos = at - a.start[key];
+   if (pos % kE != 0)
+      return;
+   const KernelView& kv = a.K.k[slot];
+   const int os = kv.os, nt = TapsOf(kv), ext = kv.nb * os, span = kv.camRad * os, nb2 = kv.nb * kv.nb;
+   const int R = s.by + os - 1 + kv.padLo, C = s.bx + os - 1 + kv.padLo;
+   const bool misc = key == a.km.base[slot + 1] - 1;
+   const bool fits = !misc && kv.phase && R - span >= 0 && R + span + nt - 1 < ext && C - span >= 0 &&
+                     C + span + nt - 1 < ext;
+   CChunk h;
+#pragma unroll
+   for (int j = 0; j < 4; ++j)
+#pragma unroll
+      for (int i = 0; i < 4; ++i)
+         h.off[4 * j + i] = fits ? ((R + j) % os * os + (C + i) % os) * nb2 + (R + j) / os * kv.nb + (C + i) / os : 0;
+   h.base = kv.phase + static_cast<size_t>(misc ? 0 : plane) * os * os * nb2;
+   h.first = static_cast<int>(at);
+   h.cnt = static_cast<int>(min(static_cast<uint32_t>(kE), a.count[key] - pos));
+   h.slot = slot;
+   h.plane = plane;
+   h.kind = misc ? 0 : (fits ? 2 : 1);
+   h.invSide = 1.f / static_cast<float>(a.km.side[slot]);
+   a.chunk[a.chunkStart[key] + pos / kE] = h;
 }
 
 // ------------------------------------------------------------------------------------------------ 4. contributions
@@ -283,12 +326,10 @@ struct ContribArgs
 {
    KeyMap km;
    Kernels K;
-   const uint32_t* count;
-   const uint32_t* start;
-   const uint32_t* itemStart;
-   const uint32_t* itemKey;
+   const CChunk* chunk;
    const CStage* stage;  // the emitters in group order
-   uint32_t* ctr;        // [0] work items, [1] the next item
+   uint32_t* ctr;        // [0] chunks, [1] the next work item
+   uint32_t blocks;      // pixel blocks of the largest square: work items per chunk
    float* contrib;       // emitter g's square at contrib[g S ..]
    uint32_t S;
 };
@@ -314,6 +355,41 @@ __device__ __forceinline__ double RegisterTaps(const double (&t)[4][4], const CS
    for (int j = 1; j < NT; ++j)
       sum += e.wy[j] * row[j];
    return sum;
+}
+
+// The same sum with the photons in the row weights and fused multiply-adds: 20 float64 instructions against 36. It and
+// photons x RegisterTaps differ by at most 21 roundings of A = sum |wp wx B|, below 2^-48 A.
+template <int NT>
+__device__ __forceinline__ double FusedTaps(const double (&t)[4][4], const CStage& e)
+{
+   double sum = 0.0;
+#pragma unroll
+   for (int j = 0; j < NT; ++j)
+   {
+      double r = e.wx[0] * t[j][0];
+#pragma unroll
+      for (int i = 1; i < NT; ++i)
+         r = fma(e.wx[i], t[j][i], r);
+      sum = j == 0 ? e.wp[0] * r : fma(e.wp[j], r, sum);
+   }
+   return sum;
+}
+
+// The contribution float(photons x sum) of the reference's operation order, from the fused sum c where c rounds to
+// the same float surely: A <= 1.5625 photons x the taps' largest magnitude (the weights' magnitudes sum to at most
+// 1.25 per axis), so with |c| at least 2^-10 x 1.6 photons x that magnitude the two sums lie within 2^-38 |c| of each
+// other, 2^15 of c's last places, and round alike unless a float's midpoint (bit 28 alone of the 29 dropped) is that
+// near. In doubt (one in 8,000, and where the taps cancel or the photons are extreme) in the reference's order. `big`:
+// the magnitude, at least; `small`: the least |c| taken (-1 where every tap is 0).
+template <int NT>
+__device__ __forceinline__ float Contribution(const double (&t)[4][4], const CStage& e, float big, float small)
+{
+   const double c = FusedTaps<NT>(t, e);
+   const float f = static_cast<float>(c), least = fmaf(e.thr, big, small);
+   const unsigned near = static_cast<unsigned>(__double2loint(c)) * 8u + (0x80000000u + (1u << 18));
+   if (near > (1u << 19) && fabsf(f) >= least && least < 1e30f)
+      return f;
+   return static_cast<float>(e.photons * RegisterTaps<NT>(t, e));
 }
 
 // Any tap origin, from the row-major float64 sums with the reference's bounds (the misc group).
@@ -350,131 +426,151 @@ __device__ __forceinline__ bool HaloKeeps(const KernelView& kv, int plane, int d
 }
 
 template <int NT>
-__device__ __forceinline__ void GroupContrib(const ContribArgs& a, const KernelView& kv, const CStage* sE, int cnt,
-                                             int plane, int bx, int by, int p, int dx, int dy, bool active)
+__device__ __forceinline__ void GroupContrib(const ContribArgs& a, const KernelView& kv, const CChunk& it,
+                                             const CStage* E, int p, int dx, int dy, bool active)
 {
-   const int os = kv.os, ext = kv.nb * os, span = kv.camRad * os;
-   const int R = by + os - 1 + kv.padLo, C = bx + os - 1 + kv.padLo;
-   const bool fits = kv.phase && R - span >= 0 && R + span + NT - 1 < ext && C - span >= 0 &&
-                     C + span + NT - 1 < ext;
-   if (!fits)
+   const int cnt = it.cnt;
+   if (it.kind == 1)
    {
       for (int k = 0; k < cnt; ++k)
          if (active)
-            a.contrib[static_cast<size_t>(sE[k].g) * a.S + p] =
-               static_cast<float>(sE[k].photons * BoundedTaps(kv, sE[k], NT, dx, dy));
+            a.contrib[static_cast<size_t>(E[k].g) * a.S + p] =
+               static_cast<float>(E[k].photons * BoundedTaps(kv, E[k], NT, dx, dy));
       return;
    }
    double t[4][4];
-   const int nb = kv.nb, nb2 = nb * nb;
-   const double* base = kv.phase + static_cast<size_t>(plane) * os * os * nb2 + (active ? dy * nb + dx : 0);
+   const double* base = it.base + (active ? dy * kv.nb + dx : 0);
 #pragma unroll
    for (int j = 0; j < NT; ++j)
 #pragma unroll
       for (int i = 0; i < NT; ++i)
-         t[j][i] = __ldg(base + ((R + j) % os * os + (C + i) % os) * nb2 + ((R + j) / os) * nb + (C + i) / os);
+         t[j][i] = __ldg(base + it.off[4 * j + i]);
+   // an upper bound of the taps' magnitudes from their high words
+   int hi = 0;
+#pragma unroll
+   for (int j = 0; j < NT; ++j)
+#pragma unroll
+      for (int i = 0; i < NT; ++i)
+         hi = max(hi, __double2hiint(t[j][i]) & 0x7fffffff);
+   const float big = hi ? static_cast<float>(__hiloint2double(hi + 1, 0)) : 0.f, small = hi ? 1e-30f : -1.f;
    float* out = a.contrib + p;
-   // two emitters per step: independent FP64 chains in flight
    int k = 0;
    for (; k + 1 < cnt; k += 2)
    {
-      const CStage& e0 = sE[k];
-      const CStage& e1 = sE[k + 1];
-      const double s0 = RegisterTaps<NT>(t, e0);
-      const double s1 = RegisterTaps<NT>(t, e1);
+      const CStage& e0 = E[k];
+      const CStage& e1 = E[k + 1];
+      const float v0 = Contribution<NT>(t, e0, big, small);
+      const float v1 = Contribution<NT>(t, e1, big, small);
       if (active)
       {
-         out[static_cast<size_t>(e0.g) * a.S] = static_cast<float>(e0.photons * s0);
-         out[static_cast<size_t>(e1.g) * a.S] = static_cast<float>(e1.photons * s1);
+         out[static_cast<size_t>(e0.g) * a.S] = v0;
+         out[static_cast<size_t>(e1.g) * a.S] = v1;
       }
    }
    if (k < cnt && active)
-      out[static_cast<size_t>(sE[k].g) * a.S] = static_cast<float>(sE[k].photons * RegisterTaps<NT>(t, sE[k]));
+      out[static_cast<size_t>(E[k].g) * a.S] = Contribution<NT>(t, E[k], big, small);
 }
 
-// The work item's key, first stage record, record count and pixel block (key -1: no items left).
-__device__ __forceinline__ void FetchItem(const ContribArgs& a, int* info)
-{
-   const uint32_t item = atomicAdd(&a.ctr[1], 1u);
-   int key = -1, first = 0, cnt = 0, pbi = 0;
-   if (item < a.ctr[0])
-   {
-      key = static_cast<int>(a.itemKey[item]);
-      const int pbs = a.km.pbs[SlotOfKey(a.km, key)];
-      const uint32_t local = item - a.itemStart[key];
-      pbi = static_cast<int>(local % pbs);
-      const uint32_t chunk = local / pbs;
-      first = static_cast<int>(a.start[key] + chunk * kE);
-      cnt = static_cast<int>(min(static_cast<uint32_t>(kE), a.count[key] - chunk * kE));
-   }
-   info[0] = key;
-   info[1] = first;
-   info[2] = cnt;
-   info[3] = pbi;
-}
-
-// blockDim.x = computing threads + one staging warp: while the others compute item i, the last warp fetches item
-// i + 1 and stages its emitters into the other buffer.
+// blockDim.x = computing threads + one staging warp, three buffers: while the others compute item i, the staging warp
+// has item i + 1's emitters arriving, issues item i + 2's copy, whose chunk it asked for an item ago, and asks for item
+// i + 3's chunk and number i + 4, so that each of these round trips has an item's time. (Fetched one after the other
+// within an item they took longer than the item's work.) An item is one block of computing threads' pixels of a chunk.
 __global__ void __launch_bounds__(kMaxCT + 32, kContribPerSm) ContribKernel(ContribArgs a)
 {
-   __shared__ CStage sE[2][kE];
-   __shared__ int sInfo[2][4];
+   __shared__ CStage sE[3][kE];
+   __shared__ CChunk sChunk[3];
+   __shared__ uint32_t sItem[3];
    const int nc = static_cast<int>(blockDim.x) - 32;   // computing threads
    const bool stager = static_cast<int>(threadIdx.x) >= nc;
    const int sl = static_cast<int>(threadIdx.x) - nc;  // lane of the staging warp
+   const uint32_t items = a.ctr[0] * a.blocks;
+   constexpr int kHead = static_cast<int>(sizeof(CChunk) / 16), kRec = static_cast<int>(sizeof(CStage) / 16);
+   uint32_t ahead = 0, asked = 0;      // lane 0: the number asked for; the item whose chunk is on its way
+   int4 head = make_int4(0, 0, 0, 0);  // that chunk's 16 bytes of this lane
+   auto number = [&] {
+      if (sl == 0)
+         ahead = atomicAdd(&a.ctr[1], 1u);
+   };
+   auto askChunk = [&] {
+      asked = __shfl_sync(0xffffffffu, ahead, 0);
+      if (asked < items && sl < kHead)
+         head = __ldg(reinterpret_cast<const int4*>(a.chunk + asked / a.blocks) + sl);
+   };
+   auto copy = [&](int buf) {
+      if (sl == 0)
+         sItem[buf] = asked;
+      if (asked < items)
+      {
+         if (sl < kHead)
+            reinterpret_cast<int4*>(&sChunk[buf])[sl] = head;
+         __syncwarp();
+         const int n = sChunk[buf].cnt * kRec;
+         const int4* from = reinterpret_cast<const int4*>(a.stage + sChunk[buf].first);
+         const uint32_t to = static_cast<uint32_t>(__cvta_generic_to_shared(sE[buf]));
+         for (int t = sl; t < n; t += 32)
+            asm volatile("cp.async.cg.shared.global [%0], [%1], 16;" ::"r"(to + 16u * t), "l"(from + t) : "memory");
+      }
+      asm volatile("cp.async.commit_group;" ::: "memory");
+   };
    if (stager)
    {
-      if (sl == 0)
-         FetchItem(a, sInfo[0]);
-      __syncwarp();
-      for (int t = sl; t < sInfo[0][2]; t += 32)
-         sE[0][t] = a.stage[sInfo[0][1] + t];
+      number();
+      askChunk();
+      number();
+      copy(0);
+      askChunk();
+      number();
+      copy(1);
+      askChunk();
+      number();
+      asm volatile("cp.async.wait_group 1;" ::: "memory");
    }
    __syncthreads();
-   for (int cur = 0;; cur ^= 1)
+   for (int cur = 0;; cur = cur == 2 ? 0 : cur + 1)
    {
-      const int key = sInfo[cur][0], cnt = sInfo[cur][2], pbi = sInfo[cur][3];
-      if (key < 0)
+      const uint32_t item = sItem[cur];
+      if (item >= items)
          return;
       if (stager)
       {
-         if (sl == 0)
-            FetchItem(a, sInfo[cur ^ 1]);
-         __syncwarp();
-         if (sInfo[cur ^ 1][0] >= 0)
-            for (int t = sl; t < sInfo[cur ^ 1][2]; t += 32)
-               sE[cur ^ 1][t] = a.stage[sInfo[cur ^ 1][1] + t];
+         copy(cur == 0 ? 2 : cur - 1);   // item i + 2 (the buffer of item i - 1, done)
+         askChunk();
+         number();
+         asm volatile("cp.async.wait_group 1;" ::: "memory");   // item i + 1 is there
       }
       else
       {
-         const int slot = SlotOfKey(a.km, key);
+         const CChunk& it = sChunk[cur];
+         const int slot = it.slot;
          const KernelView& kv = a.K.k[slot];
          const int side = a.km.side[slot], cr = kv.camRad;
-         const int p = pbi * nc + static_cast<int>(threadIdx.x);
+         const int p = static_cast<int>(item % a.blocks) * nc + static_cast<int>(threadIdx.x);
          const bool inSquare = p < side * side;
-         const int dx = inSquare ? p % side - cr : 0, dy = inSquare ? p / side - cr : 0;
+         // p / side: the quotient's fraction is at least half a 1 / side from a whole number, the float product's error
+         // below that for squares of up to 4 M pixels; larger ones divide
+         int row = static_cast<int>((static_cast<float>(p) + 0.5f) * it.invSide);
+         if (side > 2000)
+            row = p / side;
+         const int dx = inSquare ? p - row * side - cr : 0, dy = inSquare ? row - cr : 0;
          const int nt = TapsOf(kv);
-         const int local = key - a.km.base[slot];
          const CStage* E = sE[cur];
-         if (key == a.km.base[slot + 1] - 1)
+         if (__any_sync(0xffffffffu, inSquare))
          {
-            // the misc group: every emitter with its own plane and tap origin
-            for (int k = 0; k < cnt; ++k)
-               if (inSquare && HaloKeeps(kv, E[k].plane, dx, dy))
-                  a.contrib[static_cast<size_t>(E[k].g) * a.S + p] =
-                     static_cast<float>(E[k].photons * BoundedTaps(kv, E[k], nt, dx, dy));
-         }
-         else
-         {
-            const int n1 = a.km.n1[slot], plane = local / (n1 * n1), cls = local % (n1 * n1);
-            const int by = a.km.lo[slot] + cls / n1, bx = a.km.lo[slot] + cls % n1;
-            const bool active = inSquare && HaloKeeps(kv, plane, dx, dy);
-            if (nt == 4)
-               GroupContrib<4>(a, kv, E, cnt, plane, bx, by, p, dx, dy, active);
+            const bool active = inSquare && (it.kind == 0 || HaloKeeps(kv, it.plane, dx, dy));
+            if (it.kind == 0)
+            {
+               // the misc group: every emitter with its own plane and tap origin
+               for (int k = 0; k < it.cnt; ++k)
+                  if (inSquare && HaloKeeps(kv, E[k].plane, dx, dy))
+                     a.contrib[static_cast<size_t>(E[k].g) * a.S + p] =
+                        static_cast<float>(E[k].photons * BoundedTaps(kv, E[k], nt, dx, dy));
+            }
+            else if (nt == 4)
+               GroupContrib<4>(a, kv, it, E, p, dx, dy, active);
             else if (nt == 2)
-               GroupContrib<2>(a, kv, E, cnt, plane, bx, by, p, dx, dy, active);
+               GroupContrib<2>(a, kv, it, E, p, dx, dy, active);
             else
-               GroupContrib<1>(a, kv, E, cnt, plane, bx, by, p, dx, dy, active);
+               GroupContrib<1>(a, kv, it, E, p, dx, dy, active);
          }
       }
       __syncthreads();
@@ -482,13 +578,13 @@ __global__ void __launch_bounds__(kMaxCT + 32, kContribPerSm) ContribKernel(Cont
 }
 
 // ------------------------------------------------------------------------------------------------ 5. gather
-struct GStage
+// A staged emitter as one warp adds it: its contribution to the warp's first pixel (counted from the square's pitch, so
+// perhaps outside the square), the pitch, and the warp's pixels that its square and halo cut cover.
+struct __align__(16) GEntry
 {
-   const float* centre;   // the emitter's contributions at its square's centre pixel: contrib + g S + cr side + cr
-   int x0, y0;            // (the first 16 bytes: what every pixel's test and address read)
-   int cr, side;
-   const int16_t* lo;     // halo cut of the emitter's plane, by dy + cr; null: the whole square
-   const int16_t* hi;
+   const float* first;
+   int side;
+   unsigned covers;
 };
 
 struct GatherArgs
@@ -511,33 +607,24 @@ struct GatherArgs
 
 // Stages one chunk of a frame's emitters whose square reaches the tile, in list order. Every thread calls it.
 __device__ __forceinline__ int GatherStage(const GatherArgs& a, uint32_t start, uint32_t count, int tx0, int ty0,
-                                           int tx1, int ty1, GStage* sG, int* sWarp, bool& anyHalo)
+                                           int tx1, int ty1, int4* sG, uint32_t* sId, int* sWarp)
 {
    const int t = threadIdx.x, lane = t & 31, warp = t >> 5;
    bool keep = false;
-   GStage s;
+   int4 gr = make_int4(0, 0, -1, 0);
    if (static_cast<uint32_t>(t) < count)
    {
-      const uint32_t g = start + t;
-      const int4 gr = a.grec[g];
+      gr = a.grec[start + t];
       if (gr.z >= 0)
       {
-         const KernelView& kv = a.K.k[gr.z];
-         const int cr = kv.camRad;
+         const int cr = a.K.k[gr.z].camRad;
          keep = gr.x + cr >= tx0 && gr.x - cr <= tx1 && gr.y + cr >= ty0 && gr.y - cr <= ty1;
-         s.x0 = gr.x;
-         s.y0 = gr.y;
-         s.cr = cr;
-         s.side = 2 * cr + 1;
-         s.centre = a.contrib + static_cast<size_t>(g) * a.S + static_cast<size_t>(cr) * s.side + cr;
-         s.lo = kv.spanLo ? kv.spanLo + gr.w * s.side : nullptr;
-         s.hi = kv.spanHi ? kv.spanHi + gr.w * s.side : nullptr;
       }
    }
    const unsigned ballot = __ballot_sync(0xffffffffu, keep);
    if (lane == 0)
       sWarp[warp] = __popc(ballot);
-   anyHalo = __syncthreads_or(keep && s.lo != nullptr) != 0;
+   __syncthreads();
    int base = 0, total = 0;
 #pragma unroll
    for (int w = 0; w < kGT / 32; ++w)
@@ -547,75 +634,72 @@ __device__ __forceinline__ int GatherStage(const GatherArgs& a, uint32_t start, 
       total += c;
    }
    if (keep)
-      sG[base + __popc(ballot & ((1u << lane) - 1u))] = s;
+   {
+      base += __popc(ballot & ((1u << lane) - 1u));
+      sG[base] = gr;
+      sId[base] = start + t;
+   }
    __syncthreads();
    return total;
 }
 
-__device__ __forceinline__ int GatherWarpList(const GStage* sG, int kept, int wx0, int wx1, int wy0, int wy1,
-                                              uint16_t* list)
+// The pixels of the warp's CW x 32 / CW rectangle at (wx0, wy0) that emitter gr's square and halo cut cover, a bit per
+// lane.
+template <int CW>
+__device__ __forceinline__ unsigned Covers(const KernelView& kv, const int4& gr, int wx0, int wy0)
 {
-   const int lane = threadIdx.x & 31;
-   int n = 0;
-   for (int b = 0; b < kept; b += 32)
+   const int cr = kv.camRad, x0 = gr.x - wx0;
+   const int lo = max(0, x0 - cr), hi = min(CW - 1, x0 + cr);
+   unsigned m = 0;
+#pragma unroll
+   for (int r = 0; r < 32 / CW; ++r)
    {
-      const int k = b + lane;
-      bool hit = false;
-      if (k < kept)
+      const int dy = wy0 + r - gr.y;
+      if (dy < -cr || dy > cr)
+         continue;
+      int l = lo, h = hi;
+      if (kv.spanLo)
       {
-         const GStage& e = sG[k];
-         hit = e.x0 + e.cr >= wx0 && e.x0 - e.cr <= wx1 && e.y0 + e.cr >= wy0 && e.y0 - e.cr <= wy1;
+         const int at = gr.w * (2 * cr + 1) + dy + cr;
+         l = max(l, x0 + kv.spanLo[at]);
+         h = min(h, x0 + kv.spanHi[at]);
       }
-      const unsigned bal = __ballot_sync(0xffffffffu, hit);
-      if (hit)
-         list[n + __popc(bal & ((1u << lane) - 1u))] = static_cast<uint16_t>(k);
-      n += __popc(bal);
+      if (l <= h)
+         m |= ((2u << h) - (1u << l)) << (r * CW & 31);
    }
-   __syncwarp();
-   return n;
+   return m;
 }
 
-// Whether the emitter's square and halo cut cover pixel (X, Y); the contribution's address if so.
-template <bool kHalo>
-__device__ __forceinline__ bool GatherCovers(const GStage& e, int X, int Y, const float*& src)
+// A pixel's adds of the warp's entries, in list order, four loads in flight. The lanes' tests are worked out once an
+// entry, a lane per emitter, when the list is made; an add is a shared load, a bit test, the address and the load (a
+// test of the pixel against the square and the cut for each emitter took twice the instructions: the gather's part of
+// the two-colour movie 1.5 -> WHAT ms).
+__device__ __forceinline__ float GatherAdds(const GEntry* list, int n, unsigned bit, int lx, int ly, float acc)
 {
-   const int dx = X - e.x0, dy = Y - e.y0, cr = e.cr;
-   const unsigned w = static_cast<unsigned>(2 * cr);   // |dx|, |dy| <= cr as one unsigned compare each
-   if (static_cast<unsigned>(dx + cr) > w || static_cast<unsigned>(dy + cr) > w)
-      return false;
-   if (kHalo && e.lo && (dx < e.lo[dy + cr] || dx > e.hi[dy + cr]))
-      return false;
-   src = e.centre + dy * e.side + dx;
-   return true;
-}
-
-// A pixel's adds of the warp list's contributions, in list order, four loads in flight.
-template <bool kHalo>
-__device__ __forceinline__ float GatherAdds(const GStage* sG, const uint16_t* list, int n, int X, int Y, float acc)
-{
-   int m = 0;
-   for (; m + 4 <= n; m += 4)
+   for (int m = 0; m < n; m += 4)
    {
       float v[4];
-      bool in[4];
 #pragma unroll
       for (int u = 0; u < 4; ++u)
       {
-         const float* src = nullptr;
-         in[u] = GatherCovers<kHalo>(sG[list[m + u]], X, Y, src);
-         v[u] = in[u] ? __ldg(src) : 0.0f;
+         const GEntry e = list[m + u];   // (the list ends in entries that cover nothing)
+         v[u] = e.covers & bit ? __ldg(e.first + (ly * e.side + lx)) : 0.0f;   // (acc is never -0: adding 0 keeps it)
       }
 #pragma unroll
       for (int u = 0; u < 4; ++u)
-         if (in[u])
-            acc += v[u];
+         acc += v[u];
    }
-   for (; m < n; ++m)
-   {
-      const float* src = nullptr;
-      if (GatherCovers<kHalo>(sG[list[m]], X, Y, src))
-         acc += __ldg(src);
-   }
+   return acc;
+}
+
+// Every lane of the warp calls it.
+__device__ __forceinline__ float GatherFlush(GEntry* list, int n, int lane, unsigned bit, int lx, int ly, float acc)
+{
+   if (lane < 4 && (n & 3))
+      list[n + lane] = GEntry{nullptr, 0, 0u};
+   __syncwarp();
+   acc = GatherAdds(list, n, bit, lx, ly, acc);
+   __syncwarp();
    return acc;
 }
 
@@ -626,17 +710,19 @@ __global__ void __launch_bounds__(kGT, 6) GatherTilesKernel(GatherArgs a)
 {
    static_assert(TX * TY == kGT, "one thread per pixel of the tile");
    static_assert(TX % 32 == 0 || 32 % TX == 0, "a warp covers a rectangle of the tile");
-   __shared__ GStage sG[kGChunk];
-   __shared__ uint16_t sList[kGT / 32][kGChunk];
+   __shared__ int4 sG[kGChunk];
+   __shared__ uint32_t sId[kGChunk];
+   __shared__ GEntry sList[kGT / 32][kGList];
    __shared__ int sWarp[kGT / 32];
    __shared__ uint32_t sItem;
    const int W = static_cast<int>(a.st.width), H = static_cast<int>(a.st.height);
    const uint32_t tilesX = (W + TX - 1) / TX, tilesY = (H + TY - 1) / TY, tilesPerFrame = tilesX * tilesY;
    const uint32_t total = a.nFrames * tilesPerFrame;
    const int warp = threadIdx.x >> 5;
-   uint16_t* list = sList[warp];
-   const int wcx = TX >= 32 ? (32 * warp) % TX : 0, wcw = TX >= 32 ? 32 : TX;
-   const int wry = (32 * warp) / TX, wrh = TX >= 32 ? 1 : 32 / TX;
+   GEntry* list = sList[warp];
+   constexpr int CW = TX >= 32 ? 32 : TX;   // a warp's pixels: CW x 32 / CW
+   const int lane = threadIdx.x & 31, lx = lane % CW, ly = lane / CW;
+   const int wcx = TX >= 32 ? (32 * warp) % TX : 0, wry = (32 * warp) / TX;
    for (;;)
    {
       uint32_t f, tile;
@@ -666,17 +752,38 @@ __global__ void __launch_bounds__(kGT, 6) GatherTilesKernel(GatherArgs a)
       const uint32_t i = static_cast<uint32_t>(Y) * a.st.width + static_cast<uint32_t>(X);
       const int wx0 = tx0 + wcx, wy0 = ty0 + wry;
       float acc = inside ? Background(a.st, i, fr.bg_scale) : 0.0f;
+      int listed = 0;
       for (uint32_t e0 = 0; e0 < emCount; e0 += kGChunk)
       {
          const uint32_t cnt = min(static_cast<uint32_t>(kGChunk), emCount - e0);
-         bool anyHalo = false;
-         const int kept = GatherStage(a, fr.em_start + e0, cnt, tx0, ty0, tx1, ty1, sG, sWarp, anyHalo);
-         const int n = GatherWarpList(sG, kept, wx0, wx0 + wcw - 1, wy0, wy0 + wrh - 1, list);
-         // the chunk's adds in list order; the halo test only where a staged emitter has a cut (the same for the CTA)
-         if (inside)
-            acc = anyHalo ? GatherAdds<true>(sG, list, n, X, Y, acc) : GatherAdds<false>(sG, list, n, X, Y, acc);
+         const int kept = GatherStage(a, fr.em_start + e0, cnt, tx0, ty0, tx1, ty1, sG, sId, sWarp);
+         for (int k0 = 0; k0 < kept; k0 += 32)
+         {
+            // the staged emitters that cover a pixel of the warp, a lane per emitter
+            GEntry e{nullptr, 0, 0u};
+            if (k0 + lane < kept)
+            {
+               const int4 gr = sG[k0 + lane];
+               const KernelView& kv = a.K.k[gr.z];
+               e.covers = Covers<CW>(kv, gr, wx0, wy0);
+               e.side = 2 * kv.camRad + 1;
+               e.first = a.contrib + static_cast<size_t>(sId[k0 + lane]) * a.S +
+                         ((wy0 - gr.y + kv.camRad) * e.side + wx0 - gr.x + kv.camRad);
+            }
+            const unsigned hit = __ballot_sync(0xffffffffu, e.covers != 0u);
+            if (e.covers)
+               list[listed + __popc(hit & ((1u << lane) - 1u))] = e;
+            listed += __popc(hit);
+            __syncwarp();
+            if (listed > kGList - 36)   // (32 more, and the entries that end a list)
+            {
+               acc = GatherFlush(list, listed, lane, inside ? 1u << lane : 0u, lx, ly, acc);
+               listed = 0;
+            }
+         }
          __syncthreads();
       }
+      acc = GatherFlush(list, listed, lane, inside ? 1u << lane : 0u, lx, ly, acc);
       if (inside)
       {
          const size_t o = static_cast<size_t>(f) * a.st.width * a.st.height + i;
@@ -713,7 +820,7 @@ namespace {
 struct ContribGeometry
 {
    KeyMap km = {};
-   int nKeys = 0, ct = 32;
+   int nKeys = 0, ct = 32, blocks = 1;   // computing threads of a contribution CTA; its blocks of the largest square
    size_t S = 1;
 };
 
@@ -735,22 +842,16 @@ ContribGeometry GeometryOf(const iscu_ctx* ctx)
       maxS2 = std::max(maxS2, side * side);
    }
    G.km.base[ISCU_MAX_KERNELS] = G.nKeys;
-   const int blocks = (maxS2 + kMaxCT - 1) / kMaxCT;
-   G.ct = std::min(kMaxCT, ((maxS2 + blocks - 1) / blocks + 31) / 32 * 32);
-   for (int s = 0; s < ISCU_MAX_KERNELS; ++s)
-      G.km.pbs[s] = std::max(1, (G.km.side[s] * G.km.side[s] + G.ct - 1) / G.ct);
+   G.blocks = (maxS2 + kMaxCT - 1) / kMaxCT;
+   G.ct = std::min(kMaxCT, ((maxS2 + G.blocks - 1) / G.blocks + 31) / 32 * 32);
    G.S = static_cast<size_t>(maxS2);
    return G;
 }
 
-// An upper bound of the work items: every key's emitter chunks (one partial chunk per key at most) times the largest
-// number of pixel blocks.
-size_t MaxItems(const ContribGeometry& G, uint32_t nEm)
+// An upper bound of the chunks: the full ones and one partial chunk per key, no more than emitters.
+size_t MaxChunks(const ContribGeometry& G, uint32_t nEm)
 {
-   int maxPbs = 1;
-   for (int s = 0; s < ISCU_MAX_KERNELS; ++s)
-      maxPbs = std::max(maxPbs, G.km.pbs[s]);
-   return (static_cast<size_t>(nEm) / kE + static_cast<size_t>(G.nKeys) + 1) * static_cast<size_t>(maxPbs);
+   return std::min<size_t>(nEm, static_cast<size_t>(nEm) / kE + static_cast<size_t>(G.nKeys)) + 1;
 }
 
 } // namespace
@@ -769,11 +870,12 @@ int ReserveContrib(iscu_ctx* ctx, uint32_t nEm, ContribScratch& sc)
       return Fail(ISCU_ERR_LIMIT, "two-pass render: contributions of " + std::to_string(nEm) + " emitters need " +
                                      std::to_string(contribBytes >> 20) + " MiB, over the limit");
    const size_t n = std::max<uint32_t>(nEm, 1u);
-   ISCU_CK(sc.rec.Reserve(n * sizeof(SplatRec)));
+   ISCU_CK(sc.rec.Reserve(n * sizeof(int)));
    ISCU_CK(sc.grec.Reserve(n * sizeof(int4)));
    ISCU_CK(sc.list.Reserve(n * sizeof(CStage)));
    ISCU_CK(sc.contrib.Reserve(std::max<size_t>(contribBytes, 16)));
-   ISCU_CK(sc.keys.Reserve((4 * static_cast<size_t>(G.nKeys) + 1 + MaxItems(G, nEm)) * sizeof(uint32_t)));
+   ISCU_CK(sc.keys.Reserve(std::max<size_t>(4 * static_cast<size_t>(G.nKeys), 4) * sizeof(uint32_t)));
+   ISCU_CK(sc.chunks.Reserve(MaxChunks(G, nEm) * sizeof(CChunk)));
    ISCU_CK(sc.ctr.Reserve(4 * sizeof(uint32_t)));
    return ISCU_OK;
 }
@@ -789,7 +891,7 @@ int LaunchContribRender(iscu_ctx* ctx, int tileConfig, const iscu_emitter* ems, 
       return rcReserve;
    const ContribGeometry G = GeometryOf(ctx);
    const KeyMap& km = G.km;
-   const int nKeys = G.nKeys, ct = G.ct;
+   const int nKeys = G.nKeys;
    const size_t S = G.S;
    cudaEvent_t* marks = RenderMarks(ctx);
    if (marks)
@@ -797,32 +899,28 @@ int LaunchContribRender(iscu_ctx* ctx, int tileConfig, const iscu_emitter* ems, 
    uint32_t* count = sc.keys.as<uint32_t>();
    uint32_t* start = count + nKeys;
    uint32_t* cursor = start + nKeys;
-   uint32_t* itemStart = cursor + nKeys;
-   uint32_t* itemKey = itemStart + nKeys + 1;
+   uint32_t* chunkStart = cursor + nKeys;
    const Kernels K = KernelsOfCtx(ctx);
    if (nEm > 0)
    {
       if (nKeys > 0)
          ISCU_CK(cudaMemsetAsync(count, 0, static_cast<size_t>(nKeys) * sizeof(uint32_t), ctx->stream));
-      SetupArgs sa{ems, nEm, K, km, sc.rec.as<SplatRec>(), sc.grec.as<int4>(), count};
+      SetupArgs sa{ems, nEm, K, km, sc.rec.as<int>(), sc.grec.as<int4>(), count};
       ContribSetupKernel<<<(nEm + 255) / 256, 256, 0, ctx->stream>>>(sa);
       ISCU_CK_LAUNCH(ctx, "ContribSetupKernel");
       if (nKeys > 0)
       {
-         ContribScanKernel<<<1, 1024, 0, ctx->stream>>>(km, count, start, cursor, itemStart, itemKey,
-                                                        sc.ctr.as<uint32_t>());
+         ContribScanKernel<<<1, 1024, 0, ctx->stream>>>(km, count, start, cursor, chunkStart, sc.ctr.as<uint32_t>());
          ISCU_CK_LAUNCH(ctx, "ContribScanKernel");
-         ContribScatterKernel<<<(nEm + 255) / 256, 256, 0, ctx->stream>>>(nEm, sc.rec.as<SplatRec>(),
-                                                                           sc.grec.as<int4>(), cursor,
-                                                                           sc.list.as<CStage>());
+         ScatterArgs xa{ems,    nEm,        K, km, sc.rec.as<int>(), count, start, cursor, chunkStart,
+                        sc.list.as<CStage>(), sc.chunks.as<CChunk>()};
+         ContribScatterKernel<<<(nEm + 255) / 256, 256, 0, ctx->stream>>>(xa);
          ISCU_CK_LAUNCH(ctx, "ContribScatterKernel");
          if (marks)
             ISCU_CK(cudaEventRecord(marks[1], ctx->stream));
-         ContribArgs ca{km, K, count, start, itemStart, itemKey, sc.list.as<CStage>(), sc.ctr.as<uint32_t>(),
-                        sc.contrib.as<float>(), static_cast<uint32_t>(S)};
-         int perSm = 0;
-         ISCU_CK(cudaOccupancyMaxActiveBlocksPerMultiprocessor(&perSm, ContribKernel, ct + 32, 0));
-         ContribKernel<<<std::max(1, perSm) * ctx->smCount, ct + 32, 0, ctx->stream>>>(ca);
+         ContribArgs ca{km, K, sc.chunks.as<CChunk>(), sc.list.as<CStage>(), sc.ctr.as<uint32_t>(),
+                        static_cast<uint32_t>(G.blocks), sc.contrib.as<float>(), static_cast<uint32_t>(S)};
+         ContribKernel<<<kContribPerSm * ctx->smCount, G.ct + 32, 0, ctx->stream>>>(ca);
          ISCU_CK_LAUNCH(ctx, "ContribKernel");
       }
    }
