@@ -32,7 +32,8 @@ namespace iscu {
 namespace {
 
 constexpr int kE = 64;          // emitters per contribution chunk
-// Contribution CTAs: at most kMaxCT computing threads and a staging warp.
+// Contribution CTAs: at most kMaxCT computing threads and a staging warp, four per SM (72 registers: the 16 float64 taps
+// in registers). A 33 x 33 square is six pixel blocks; 224 x 3, 256 x 3 and 352 x 2 threads measured 1.5 to 6 % more.
 constexpr int kMaxCT = 192;
 constexpr int kContribPerSm = 4;
 constexpr int kGT = 256;        // gather CTA size (one thread per pixel of the tile)
@@ -49,16 +50,6 @@ struct KeyMap
    int n1[ISCU_MAX_KERNELS];
    int side[ISCU_MAX_KERNELS];   // splat square side, 2 camRad + 1
 };
-
-__device__ __forceinline__ int SlotOfKey(const KeyMap& km, int key)
-{
-   int s = 0;
-#pragma unroll
-   for (int t = 1; t < ISCU_MAX_KERNELS; ++t)
-      if (key >= km.base[t])
-         s = t;
-   return s;
-}
 
 __device__ __forceinline__ int TapsOf(const KernelView& kv)
 {
@@ -474,7 +465,15 @@ __device__ __forceinline__ void GroupContrib(const ContribArgs& a, const KernelV
 // blockDim.x = computing threads + one staging warp, three buffers: while the others compute item i, the staging warp
 // has item i + 1's emitters arriving, issues item i + 2's copy, whose chunk it asked for an item ago, and asks for item
 // i + 3's chunk and number i + 4, so that each of these round trips has an item's time. (Fetched one after the other
-// within an item they took longer than the item's work.) An item is one block of computing threads' pixels of a chunk.
+// within an item they took longer than a short item's work.) An item is one block of computing threads' pixels of a
+// chunk.
+//
+// What bounds it: the emitter loop, 86 cycles a warp's contribution and scheduler where its 20 float64 operations and
+// the conversion need 56 (a float64 operation issues every 2.35 cycles, a conversion takes 8.5); 54 instructions in all,
+// the FP64 pipe at 39 %. Taps, chunk and barriers are 20 % on the dSTORM movie, 9 % on the two-colour one. 35 M
+// contributions of the dSTORM movie 136 -> 122 us, 484 M of the two-colour movie 1.55 -> 1.27 ms against unfused sums
+// with each thread's own tap offsets. Building the float from the double's bits instead of converting, and two or four
+// emitters without a branch between them, measured 5 to 40 % slower (more integer instructions; spilled taps).
 __global__ void __launch_bounds__(kMaxCT + 32, kContribPerSm) ContribKernel(ContribArgs a)
 {
    __shared__ CStage sE[3][kE];
@@ -579,12 +578,14 @@ __global__ void __launch_bounds__(kMaxCT + 32, kContribPerSm) ContribKernel(Cont
 
 // ------------------------------------------------------------------------------------------------ 5. gather
 // A staged emitter as one warp adds it: its contribution to the warp's first pixel (counted from the square's pitch, so
-// perhaps outside the square), the pitch, and the warp's pixels that its square and halo cut cover.
+// perhaps outside the square), the pitch, and the pixels of the warp's kSub rectangles that its square and halo cut
+// cover.
+template <int kSub>
 struct __align__(16) GEntry
 {
    const float* first;
    int side;
-   unsigned covers;
+   unsigned covers[kSub];
 };
 
 struct GatherArgs
@@ -670,57 +671,68 @@ __device__ __forceinline__ unsigned Covers(const KernelView& kv, const int4& gr,
    return m;
 }
 
-// A pixel's adds of the warp's entries, in list order, four loads in flight. The lanes' tests are worked out once an
-// entry, a lane per emitter, when the list is made; an add is a shared load, a bit test, the address and the load (a
-// test of the pixel against the square and the cut for each emitter took twice the instructions: the gather's part of
-// the two-colour movie 1.5 -> WHAT ms).
-__device__ __forceinline__ float GatherAdds(const GEntry* list, int n, unsigned bit, int lx, int ly, float acc)
+// A thread's pixels' adds of the warp's entries, in list order, four entries' loads in flight. The lanes' tests are
+// worked out once an entry, a lane per emitter, when the list is made, so that an add is a shared load, a bit test, the
+// address and the load, the first and the last two shared by the kSub pixels (TX apart).
+template <int TX, int kSub>
+__device__ __forceinline__ void GatherAdds(const GEntry<kSub>* list, int n, const unsigned (&bit)[kSub], int lx, int ly,
+                                           float (&acc)[kSub])
 {
    for (int m = 0; m < n; m += 4)
    {
-      float v[4];
+      float v[4][kSub];
 #pragma unroll
       for (int u = 0; u < 4; ++u)
       {
-         const GEntry e = list[m + u];   // (the list ends in entries that cover nothing)
-         v[u] = e.covers & bit ? __ldg(e.first + (ly * e.side + lx)) : 0.0f;   // (acc is never -0: adding 0 keeps it)
+         const GEntry<kSub>& e = list[m + u];   // (the list ends in entries that cover nothing)
+         const float* p = e.first + (ly * e.side + lx);
+#pragma unroll
+         for (int q = 0; q < kSub; ++q)
+            v[u][q] = e.covers[q] & bit[q] ? __ldg(p + q * TX) : 0.0f;   // (acc is never -0: adding 0 keeps it)
       }
 #pragma unroll
       for (int u = 0; u < 4; ++u)
-         acc += v[u];
+#pragma unroll
+         for (int q = 0; q < kSub; ++q)
+            acc[q] += v[u][q];
    }
-   return acc;
 }
 
 // Every lane of the warp calls it.
-__device__ __forceinline__ float GatherFlush(GEntry* list, int n, int lane, unsigned bit, int lx, int ly, float acc)
+template <int TX, int kSub>
+__device__ __forceinline__ void GatherFlush(GEntry<kSub>* list, int n, int lane, const unsigned (&bit)[kSub], int lx,
+                                            int ly, float (&acc)[kSub])
 {
    if (lane < 4 && (n & 3))
-      list[n + lane] = GEntry{nullptr, 0, 0u};
+      list[n + lane] = GEntry<kSub>{};
    __syncwarp();
-   acc = GatherAdds(list, n, bit, lx, ly, acc);
+   GatherAdds<TX, kSub>(list, n, bit, lx, ly, acc);
    __syncwarp();
-   return acc;
 }
 
-// Six CTAs per SM (40 registers; the noise chain spills a little): the gather's loads and the Knuth loops are latency-
-// bound, and the extra warps hide more than the spills cost (C0 tiles 0.228 -> 0.211 ms, C3 4.60 -> 4.12 ms).
-template <int TX, int TY, bool kNoise, bool kPersistent>
+// kSub: a CTA's tile is kSub tiles of TX x TY side by side, a thread's pixels TX apart: what a CTA does for a chunk of
+// emitters (staging, the warps' lists) is half the gather's instructions at 256 x 256 px and 430 emitters a frame, and
+// two pixels share it. Six CTAs per SM (40 registers; the noise chain spills a little): the gather's loads and the Knuth
+// loops are latency-bound, and the extra warps hide more than the spills cost. Issue-bound (83 %; half of it the noise
+// chain): dSTORM movie 139 -> 118 us, two-colour movie 2.85 -> 2.19 ms, against a test of the pixel's distances for each
+// emitter and one tile a CTA.
+template <int TX, int TY, bool kNoise, bool kPersistent, int kSub>
 __global__ void __launch_bounds__(kGT, 6) GatherTilesKernel(GatherArgs a)
 {
    static_assert(TX * TY == kGT, "one thread per pixel of the tile");
    static_assert(TX % 32 == 0 || 32 % TX == 0, "a warp covers a rectangle of the tile");
    __shared__ int4 sG[kGChunk];
    __shared__ uint32_t sId[kGChunk];
-   __shared__ GEntry sList[kGT / 32][kGList];
+   __shared__ GEntry<kSub> sList[kGT / 32][kGList];
    __shared__ int sWarp[kGT / 32];
    __shared__ uint32_t sItem;
    const int W = static_cast<int>(a.st.width), H = static_cast<int>(a.st.height);
-   const uint32_t tilesX = (W + TX - 1) / TX, tilesY = (H + TY - 1) / TY, tilesPerFrame = tilesX * tilesY;
+   constexpr int kTX = kSub * TX;
+   const uint32_t tilesX = (W + kTX - 1) / kTX, tilesY = (H + TY - 1) / TY, tilesPerFrame = tilesX * tilesY;
    const uint32_t total = a.nFrames * tilesPerFrame;
    const int warp = threadIdx.x >> 5;
-   GEntry* list = sList[warp];
-   constexpr int CW = TX >= 32 ? 32 : TX;   // a warp's pixels: CW x 32 / CW
+   GEntry<kSub>* list = sList[warp];
+   constexpr int CW = TX >= 32 ? 32 : TX;   // a warp's pixels: CW x 32 / CW, kSub times
    const int lane = threadIdx.x & 31, lx = lane % CW, ly = lane / CW;
    const int wcx = TX >= 32 ? (32 * warp) % TX : 0, wry = (32 * warp) / TX;
    for (;;)
@@ -745,13 +757,20 @@ __global__ void __launch_bounds__(kGT, 6) GatherTilesKernel(GatherArgs a)
       }
       const iscu_frame fr = a.frames[f];
       const uint32_t emCount = fr.em_start < a.nEm ? min(fr.em_count, a.nEm - fr.em_start) : 0u;
-      const int tx0 = static_cast<int>(tile % tilesX) * TX, ty0 = static_cast<int>(tile / tilesX) * TY;
+      const int tx0 = static_cast<int>(tile % tilesX) * kTX, ty0 = static_cast<int>(tile / tilesX) * TY;
       const int X = tx0 + static_cast<int>(threadIdx.x % TX), Y = ty0 + static_cast<int>(threadIdx.x / TX);
-      const int tx1 = min(tx0 + TX, W) - 1, ty1 = min(ty0 + TY, H) - 1;
-      const bool inside = X < W && Y < H;
+      const int tx1 = min(tx0 + kTX, W) - 1, ty1 = min(ty0 + TY, H) - 1;
       const uint32_t i = static_cast<uint32_t>(Y) * a.st.width + static_cast<uint32_t>(X);
       const int wx0 = tx0 + wcx, wy0 = ty0 + wry;
-      float acc = inside ? Background(a.st, i, fr.bg_scale) : 0.0f;
+      float acc[kSub];
+      unsigned bit[kSub];
+#pragma unroll
+      for (int q = 0; q < kSub; ++q)
+      {
+         const bool inside = X + q * TX < W && Y < H;
+         bit[q] = inside ? 1u << lane : 0u;
+         acc[q] = inside ? Background(a.st, i + q * TX, fr.bg_scale) : 0.0f;
+      }
       int listed = 0;
       for (uint32_t e0 = 0; e0 < emCount; e0 += kGChunk)
       {
@@ -760,39 +779,54 @@ __global__ void __launch_bounds__(kGT, 6) GatherTilesKernel(GatherArgs a)
          for (int k0 = 0; k0 < kept; k0 += 32)
          {
             // the staged emitters that cover a pixel of the warp, a lane per emitter
-            GEntry e{nullptr, 0, 0u};
+            GEntry<kSub> e{};
+            unsigned any = 0;
             if (k0 + lane < kept)
             {
                const int4 gr = sG[k0 + lane];
                const KernelView& kv = a.K.k[gr.z];
-               e.covers = Covers<CW>(kv, gr, wx0, wy0);
+#pragma unroll
+               for (int q = 0; q < kSub; ++q)
+                  any |= e.covers[q] = Covers<CW>(kv, gr, wx0 + q * TX, wy0);
                e.side = 2 * kv.camRad + 1;
                e.first = a.contrib + static_cast<size_t>(sId[k0 + lane]) * a.S +
                          ((wy0 - gr.y + kv.camRad) * e.side + wx0 - gr.x + kv.camRad);
             }
-            const unsigned hit = __ballot_sync(0xffffffffu, e.covers != 0u);
-            if (e.covers)
+            const unsigned hit = __ballot_sync(0xffffffffu, any != 0u);
+            if (any)
                list[listed + __popc(hit & ((1u << lane) - 1u))] = e;
             listed += __popc(hit);
             __syncwarp();
             if (listed > kGList - 36)   // (32 more, and the entries that end a list)
             {
-               acc = GatherFlush(list, listed, lane, inside ? 1u << lane : 0u, lx, ly, acc);
+               GatherFlush<TX, kSub>(list, listed, lane, bit, lx, ly, acc);
                listed = 0;
             }
          }
          __syncthreads();
       }
-      acc = GatherFlush(list, listed, lane, inside ? 1u << lane : 0u, lx, ly, acc);
-      if (inside)
+      GatherFlush<TX, kSub>(list, listed, lane, bit, lx, ly, acc);
+      // (one copy of the noise chain, gone through kSub times)
+#pragma unroll 1
+      for (int q = 0; q < kSub; ++q)
       {
-         const size_t o = static_cast<size_t>(f) * a.st.width * a.st.height + i;
+         float v = acc[0];
+         unsigned in = bit[0];
+#pragma unroll
+         for (int r = 1; r < kSub; ++r)
+         {
+            v = q == r ? acc[r] : v;
+            in = q == r ? bit[r] : in;
+         }
+         if (!in)
+            continue;
+         const size_t o = static_cast<size_t>(f) * a.st.width * a.st.height + i + q * TX;
          if (a.photonsOut)
-            a.photonsOut[o] = acc;
+            a.photonsOut[o] = v;
          if (kNoise)
          {
             CounterRng u(a.seed, fr.frame);
-            a.aduOut[o] = NoisePixel(acc, i, a.cam, a.st, u);
+            a.aduOut[o] = NoisePixel(v, i + q * TX, a.cam, a.st, u);
          }
       }
       if (!kPersistent)
@@ -801,14 +835,14 @@ __global__ void __launch_bounds__(kGT, 6) GatherTilesKernel(GatherArgs a)
 }
 
 using GatherFn = void (*)(GatherArgs);
-template <bool kNoise, bool kPersistent>
+template <bool kNoise, bool kPersistent, int kSub>
 GatherFn GatherTile(int tile)
 {
    switch (tile)
    {
-   case 0: return GatherTilesKernel<16, 16, kNoise, kPersistent>;
-   case 1: return GatherTilesKernel<32, 8, kNoise, kPersistent>;
-   default: return GatherTilesKernel<8, 32, kNoise, kPersistent>;
+   case 0: return GatherTilesKernel<16, 16, kNoise, kPersistent, kSub>;
+   case 1: return GatherTilesKernel<32, 8, kNoise, kPersistent, kSub>;
+   default: return GatherTilesKernel<8, 32, kNoise, kPersistent, kSub>;
    }
 }
 constexpr int kTileW[3] = {16, 32, 8}, kTileH[3] = {16, 8, 32};
@@ -945,9 +979,26 @@ int LaunchContribRender(iscu_ctx* ctx, int tileConfig, const iscu_emitter* ems, 
    ga.aduOut = cam ? adu : nullptr;
    const int tile = tileConfig % 3;
    const bool persistent = tileConfig / 3 == 1;
-   const int tw = kTileW[tile], th = kTileH[tile];
-   GatherFn fn = cam ? (persistent ? GatherTile<true, true>(tile) : GatherTile<true, false>(tile))
-                     : (persistent ? GatherTile<false, true>(tile) : GatherTile<false, false>(tile));
+   // four or two tiles a CTA where that leaves CTAs enough to even out the last round (six run on an SM): four from 48
+   // an SM (two-colour movie, 442: tiles pass 2.19 ms against 2.39 with two and 2.85 with one; dSTORM movie, 22: 122
+   // against 118.5 and 128 us), two from 12
+   const int th = kTileH[tile];
+   const auto tilesOf = [&](int tw) { return (ga.st.width + tw - 1) / tw * ((ga.st.height + th - 1) / th); };
+   int sub = 1;
+   for (int q = persistent ? 1 : 4; q > 1 && sub == 1; q /= 2)
+      if (static_cast<uint64_t>(tilesOf(q * kTileW[tile])) * nFrames >=
+          static_cast<uint64_t>(q == 4 ? 48 : 12) * ctx->smCount)
+         sub = q;
+   const int tw = kTileW[tile] * sub;
+   GatherFn fn = nullptr;
+   if (persistent)
+      fn = cam ? GatherTile<true, true, 1>(tile) : GatherTile<false, true, 1>(tile);
+   else if (sub == 4)
+      fn = cam ? GatherTile<true, false, 4>(tile) : GatherTile<false, false, 4>(tile);
+   else if (sub == 2)
+      fn = cam ? GatherTile<true, false, 2>(tile) : GatherTile<false, false, 2>(tile);
+   else
+      fn = cam ? GatherTile<true, false, 1>(tile) : GatherTile<false, false, 1>(tile);
    if (persistent)
    {
       int rc = LaunchFrameOrder(ctx, frames, nFrames, orderBuf);
@@ -957,9 +1008,8 @@ int LaunchContribRender(iscu_ctx* ctx, int tileConfig, const iscu_emitter* ems, 
       ga.counter = orderBuf + ((nFrames + 3) & ~3u);
       int perSm = 0;
       ISCU_CK(cudaOccupancyMaxActiveBlocksPerMultiprocessor(&perSm, fn, kGT, 0));
-      const uint32_t tiles = ((ga.st.width + tw - 1) / tw) * ((ga.st.height + th - 1) / th);
       const uint32_t grid = std::min<uint32_t>(static_cast<uint32_t>(std::max(1, perSm) * ctx->smCount),
-                                               tiles * nFrames);
+                                               tilesOf(tw) * nFrames);
       fn<<<grid, kGT, 0, ctx->stream>>>(ga);
    }
    else
