@@ -7,7 +7,7 @@
 //
 //  1. setup (one thread per emitter): SplatSetup (PsfGeneratorBridge.cpp:1382-1422), and the emitter's group
 //     (slot, plane, bx, by) counted;
-//  2. the groups' offsets (one CTA scan) and 3. each emitter listed under its group;
+//  2. the groups' offsets (a scan by the last CTA of the setup) and 3. each emitter listed under its group;
 //  4. contributions: a CTA takes a group's block of square pixels and up to 64 of its emitters; each thread loads its
 //     pixel's taps into registers once and computes every emitter's float contribution -- the reference's value, from
 //     a fused sum where that rounds alike -- into HBM (emitter-major, one float per pixel of the square);
@@ -65,7 +65,11 @@ struct SetupArgs
    KeyMap km;
    int* key;          // per emitter; -1: not splatted
    int4* grec;        // per emitter (x0, y0, slot, plane); slot -1: not splatted
-   uint32_t* count;   // per key
+   uint32_t* count;   // per key, zero beforehand; then the CTAs done, zero beforehand
+   uint32_t* start;   // the offsets (ScanKeys)
+   uint32_t* cursor;
+   uint32_t* chunkStart;
+   uint32_t* ctr;
 };
 
 // An emitter's slot, SplatSetup and key (false: not splatted).
@@ -86,7 +90,83 @@ __device__ __forceinline__ bool SetupEmitter(const Kernels& K, const KeyMap& km,
    return true;
 }
 
-__global__ void ContribSetupKernel(SetupArgs a)
+// 2. The offsets, by one CTA of kSetupThreads threads, kScanPer consecutive keys a thread and pass: start[k] = cursor[k] =
+// exclusive sum of count, chunkStart[k] = exclusive sum of the keys' chunks (ceil(count / kE)); ctr[0] = the chunks'
+// total; ctr[1] = 0. (The chunks' records are written by the scatter: one thread listing all of a key's work in turn
+// took 14 of 26 us on the two-colour movie.)
+constexpr int kSetupThreads = 512, kScanPer = 8;
+__device__ __forceinline__ void ScanKeys(const SetupArgs& a)
+{
+   constexpr int kWarps = kSetupThreads / 32;
+   const int nKeys = a.km.base[ISCU_MAX_KERNELS];
+   const int lane = threadIdx.x & 31, warp = threadIdx.x >> 5;
+   __shared__ uint32_t sw[2][kWarps];
+   uint32_t carryC = 0, carryI = 0;
+   for (int k0 = 0; k0 < nKeys; k0 += kSetupThreads * kScanPer)
+   {
+      const int kb = k0 + static_cast<int>(threadIdx.x) * kScanPer;
+      uint32_t c[kScanPer], it[kScanPer], tc = 0, ti = 0;
+#pragma unroll
+      for (int j = 0; j < kScanPer; ++j)
+         c[j] = kb + j < nKeys ? __ldcg(a.count + kb + j) : 0u;
+#pragma unroll
+      for (int j = 0; j < kScanPer; ++j)
+      {
+         it[j] = (c[j] + kE - 1) / kE;
+         tc += c[j];
+         ti += it[j];
+      }
+      uint32_t xc = tc, xi = ti;   // inclusive warp scans of the threads' totals
+#pragma unroll
+      for (int d = 1; d < 32; d <<= 1)
+      {
+         const uint32_t u = __shfl_up_sync(0xffffffffu, xc, d), v = __shfl_up_sync(0xffffffffu, xi, d);
+         if (lane >= d)
+         {
+            xc += u;
+            xi += v;
+         }
+      }
+      __syncthreads();   // the pass before has read sw
+      if (lane == 31)
+      {
+         sw[0][warp] = xc;
+         sw[1][warp] = xi;
+      }
+      __syncthreads();
+      uint32_t ec = carryC + xc - tc, ei = carryI + xi - ti;
+#pragma unroll
+      for (int w = 0; w < kWarps; ++w)
+      {
+         ec += w < warp ? sw[0][w] : 0u;
+         ei += w < warp ? sw[1][w] : 0u;
+         carryC += sw[0][w];
+         carryI += sw[1][w];
+      }
+#pragma unroll
+      for (int j = 0; j < kScanPer; ++j)
+      {
+         const int k = kb + j;
+         if (k < nKeys)
+         {
+            a.start[k] = ec;
+            a.cursor[k] = ec;
+            a.chunkStart[k] = ei;
+         }
+         ec += c[j];
+         ei += it[j];
+      }
+   }
+   if (threadIdx.x == 0)
+   {
+      a.ctr[0] = carryI;
+      a.ctr[1] = 0;
+   }
+}
+
+// The emitters' keys, counted; the last CTA to finish works out the keys' offsets (a launch of one CTA for them was 7 us
+// on its own).
+__global__ void __launch_bounds__(kSetupThreads) ContribSetupKernel(SetupArgs a)
 {
    const uint32_t g = blockIdx.x * blockDim.x + threadIdx.x;
    bool valid = false;
@@ -109,102 +189,16 @@ __global__ void ContribSetupKernel(SetupArgs a)
       if ((threadIdx.x & 31) == __ffs(peers) - 1)
          atomicAdd(&a.count[key], static_cast<uint32_t>(__popc(peers)));
    }
-}
-
-// ------------------------------------------------------------------------------------------------ 2. offsets
-// One CTA of 1024 threads, kScanPer consecutive keys a thread per pass of 4,096 keys (one round trip for the counts):
-// start[k] = exclusive sum of count, chunkStart[k] = exclusive sum of the keys' chunks (ceil(count / kE)); ctr[0] = the
-// chunks' total; ctr[1] = 0. (The chunks' records are written by the scatter: one thread listing all of a key's work in
-// turn took 14 of this kernel's 26 us on the two-colour movie.)
-constexpr int kScanPer = 4;
-__global__ void __launch_bounds__(1024) ContribScanKernel(KeyMap km, const uint32_t* __restrict__ count,
-                                                          uint32_t* __restrict__ start, uint32_t* __restrict__ cursor,
-                                                          uint32_t* __restrict__ chunkStart,
-                                                          uint32_t* __restrict__ ctr)
-{
-   const int nKeys = km.base[ISCU_MAX_KERNELS];
-   const int lane = threadIdx.x & 31, warp = threadIdx.x >> 5;
-   __shared__ uint32_t sw[2][32];
-   __shared__ uint32_t carry[2];
-   if (threadIdx.x == 0)
-      carry[0] = carry[1] = 0;
+   __shared__ bool last;
+   __threadfence();   // the counts before the CTA's arrival
    __syncthreads();
-   for (int k0 = 0; k0 < nKeys; k0 += 1024 * kScanPer)
-   {
-      const int kb = k0 + static_cast<int>(threadIdx.x) * kScanPer;
-      uint32_t c[kScanPer], it[kScanPer], tc = 0, ti = 0;
-#pragma unroll
-      for (int j = 0; j < kScanPer; ++j)
-         c[j] = kb + j < nKeys ? count[kb + j] : 0u;
-#pragma unroll
-      for (int j = 0; j < kScanPer; ++j)
-      {
-         it[j] = (c[j] + kE - 1) / kE;
-         tc += c[j];
-         ti += it[j];
-      }
-      uint32_t xc = tc, xi = ti;   // inclusive warp scans of the threads' totals
-#pragma unroll
-      for (int d = 1; d < 32; d <<= 1)
-      {
-         const uint32_t u = __shfl_up_sync(0xffffffffu, xc, d), v = __shfl_up_sync(0xffffffffu, xi, d);
-         if (lane >= d)
-         {
-            xc += u;
-            xi += v;
-         }
-      }
-      if (lane == 31)
-      {
-         sw[0][warp] = xc;
-         sw[1][warp] = xi;
-      }
-      __syncthreads();
-      if (warp == 0)
-      {
-         uint32_t u = sw[0][lane], v = sw[1][lane];
-#pragma unroll
-         for (int d = 1; d < 32; d <<= 1)
-         {
-            const uint32_t pu = __shfl_up_sync(0xffffffffu, u, d), pv = __shfl_up_sync(0xffffffffu, v, d);
-            if (lane >= d)
-            {
-               u += pu;
-               v += pv;
-            }
-         }
-         sw[0][lane] = u;
-         sw[1][lane] = v;
-      }
-      __syncthreads();
-      uint32_t ec = carry[0] + (warp ? sw[0][warp - 1] : 0u) + xc - tc;
-      uint32_t ei = carry[1] + (warp ? sw[1][warp - 1] : 0u) + xi - ti;
-#pragma unroll
-      for (int j = 0; j < kScanPer; ++j)
-      {
-         const int k = kb + j;
-         if (k < nKeys)
-         {
-            start[k] = ec;
-            cursor[k] = ec;
-            chunkStart[k] = ei;
-         }
-         ec += c[j];
-         ei += it[j];
-      }
-      __syncthreads();
-      if (threadIdx.x == 1023)
-      {
-         carry[0] = ec;
-         carry[1] = ei;
-      }
-      __syncthreads();
-   }
    if (threadIdx.x == 0)
-   {
-      ctr[0] = carry[1];
-      ctr[1] = 0;
-   }
+      last = atomicAdd(a.count + a.km.base[ISCU_MAX_KERNELS], 1u) == gridDim.x - 1;
+   __syncthreads();
+   if (!last)
+      return;
+   __threadfence();
+   ScanKeys(a);
 }
 
 // ------------------------------------------------------------------------------------------------ 3. lists
@@ -297,11 +291,21 @@ __global__ void ContribScatterKernel(ScatterArgs a)
    const bool fits = !misc && kv.phase && R - span >= 0 && R + span + nt - 1 < ext && C - span >= 0 &&
                      C + span + nt - 1 < ext;
    CChunk h;
+   int off[2][4];   // each axis' taps: the phase's plane and word
+   int row = R / os, ph = R - row * os, col = C / os, cph = C - col * os;
+#pragma unroll
+   for (int j = 0; j < 4; ++j)
+   {
+      off[0][j] = ph * os * nb2 + row * kv.nb;
+      off[1][j] = cph * nb2 + col;
+      ph = ph + 1 == os ? (++row, 0) : ph + 1;
+      cph = cph + 1 == os ? (++col, 0) : cph + 1;
+   }
 #pragma unroll
    for (int j = 0; j < 4; ++j)
 #pragma unroll
       for (int i = 0; i < 4; ++i)
-         h.off[4 * j + i] = fits ? ((R + j) % os * os + (C + i) % os) * nb2 + (R + j) / os * kv.nb + (C + i) / os : 0;
+         h.off[4 * j + i] = fits ? off[0][j] + off[1][i] : 0;
    h.base = kv.phase + static_cast<size_t>(misc ? 0 : plane) * os * os * nb2;
    h.first = static_cast<int>(at);
    h.cnt = static_cast<int>(min(static_cast<uint32_t>(kE), a.count[key] - pos));
@@ -486,22 +490,24 @@ __global__ void __launch_bounds__(kMaxCT + 32, kContribPerSm) ContribKernel(Cont
    constexpr int kHead = static_cast<int>(sizeof(CChunk) / 16), kRec = static_cast<int>(sizeof(CStage) / 16);
    uint32_t ahead = 0, asked = 0;      // lane 0: the number asked for; the item whose chunk is on its way
    int4 head = make_int4(0, 0, 0, 0);  // that chunk's 16 bytes of this lane
+   // (a CTA's first three items are its own; the counter hands out the rest)
    auto number = [&] {
       if (sl == 0)
-         ahead = atomicAdd(&a.ctr[1], 1u);
+         ahead = 3 * gridDim.x + atomicAdd(&a.ctr[1], 1u);
    };
-   auto askChunk = [&] {
-      asked = __shfl_sync(0xffffffffu, ahead, 0);
-      if (asked < items && sl < kHead)
-         head = __ldg(reinterpret_cast<const int4*>(a.chunk + asked / a.blocks) + sl);
+   auto chunk = [&](uint32_t i) {
+      int4 h = make_int4(0, 0, 0, 0);
+      if (i < items && sl < kHead)
+         h = __ldg(reinterpret_cast<const int4*>(a.chunk + i / a.blocks) + sl);
+      return h;
    };
-   auto copy = [&](int buf) {
+   auto copy = [&](int buf, uint32_t i, const int4& h) {
       if (sl == 0)
-         sItem[buf] = asked;
-      if (asked < items)
+         sItem[buf] = i;
+      if (i < items)
       {
          if (sl < kHead)
-            reinterpret_cast<int4*>(&sChunk[buf])[sl] = head;
+            reinterpret_cast<int4*>(&sChunk[buf])[sl] = h;
          __syncwarp();
          const int n = sChunk[buf].cnt * kRec;
          const int4* from = reinterpret_cast<const int4*>(a.stage + sChunk[buf].first);
@@ -514,14 +520,12 @@ __global__ void __launch_bounds__(kMaxCT + 32, kContribPerSm) ContribKernel(Cont
    if (stager)
    {
       number();
-      askChunk();
-      number();
-      copy(0);
-      askChunk();
-      number();
-      copy(1);
-      askChunk();
-      number();
+      const uint32_t i0 = blockIdx.x, i1 = i0 + gridDim.x;
+      asked = i1 + gridDim.x;
+      const int4 h0 = chunk(i0), h1 = chunk(i1);
+      head = chunk(asked);
+      copy(0, i0, h0);
+      copy(1, i1, h1);
       asm volatile("cp.async.wait_group 1;" ::: "memory");
    }
    __syncthreads();
@@ -532,8 +536,9 @@ __global__ void __launch_bounds__(kMaxCT + 32, kContribPerSm) ContribKernel(Cont
          return;
       if (stager)
       {
-         copy(cur == 0 ? 2 : cur - 1);   // item i + 2 (the buffer of item i - 1, done)
-         askChunk();
+         copy(cur == 0 ? 2 : cur - 1, asked, head);   // item i + 2 (the buffer of item i - 1, done)
+         asked = __shfl_sync(0xffffffffu, ahead, 0);
+         head = chunk(asked);
          number();
          asm volatile("cp.async.wait_group 1;" ::: "memory");   // item i + 1 is there
       }
@@ -908,7 +913,7 @@ int ReserveContrib(iscu_ctx* ctx, uint32_t nEm, ContribScratch& sc)
    ISCU_CK(sc.grec.Reserve(n * sizeof(int4)));
    ISCU_CK(sc.list.Reserve(n * sizeof(CStage)));
    ISCU_CK(sc.contrib.Reserve(std::max<size_t>(contribBytes, 16)));
-   ISCU_CK(sc.keys.Reserve(std::max<size_t>(4 * static_cast<size_t>(G.nKeys), 4) * sizeof(uint32_t)));
+   ISCU_CK(sc.keys.Reserve((4 * static_cast<size_t>(G.nKeys) + 1) * sizeof(uint32_t)));
    ISCU_CK(sc.chunks.Reserve(MaxChunks(G, nEm) * sizeof(CChunk)));
    ISCU_CK(sc.ctr.Reserve(4 * sizeof(uint32_t)));
    return ISCU_OK;
@@ -930,22 +935,20 @@ int LaunchContribRender(iscu_ctx* ctx, int tileConfig, const iscu_emitter* ems, 
    cudaEvent_t* marks = RenderMarks(ctx);
    if (marks)
       ISCU_CK(cudaEventRecord(marks[0], ctx->stream));
-   uint32_t* count = sc.keys.as<uint32_t>();
-   uint32_t* start = count + nKeys;
+   uint32_t* count = sc.keys.as<uint32_t>();   // and the CTAs done
+   uint32_t* start = count + nKeys + 1;
    uint32_t* cursor = start + nKeys;
    uint32_t* chunkStart = cursor + nKeys;
    const Kernels K = KernelsOfCtx(ctx);
    if (nEm > 0)
    {
-      if (nKeys > 0)
-         ISCU_CK(cudaMemsetAsync(count, 0, static_cast<size_t>(nKeys) * sizeof(uint32_t), ctx->stream));
-      SetupArgs sa{ems, nEm, K, km, sc.rec.as<int>(), sc.grec.as<int4>(), count};
-      ContribSetupKernel<<<(nEm + 255) / 256, 256, 0, ctx->stream>>>(sa);
+      ISCU_CK(cudaMemsetAsync(count, 0, (static_cast<size_t>(nKeys) + 1) * sizeof(uint32_t), ctx->stream));
+      SetupArgs sa{ems,   nEm,   K,      km,         sc.rec.as<int>(), sc.grec.as<int4>(),
+                   count, start, cursor, chunkStart, sc.ctr.as<uint32_t>()};
+      ContribSetupKernel<<<(nEm + kSetupThreads - 1) / kSetupThreads, kSetupThreads, 0, ctx->stream>>>(sa);
       ISCU_CK_LAUNCH(ctx, "ContribSetupKernel");
       if (nKeys > 0)
       {
-         ContribScanKernel<<<1, 1024, 0, ctx->stream>>>(km, count, start, cursor, chunkStart, sc.ctr.as<uint32_t>());
-         ISCU_CK_LAUNCH(ctx, "ContribScanKernel");
          ScatterArgs xa{ems,    nEm,        K, km, sc.rec.as<int>(), count, start, cursor, chunkStart,
                         sc.list.as<CStage>(), sc.chunks.as<CChunk>()};
          ContribScatterKernel<<<(nEm + 255) / 256, 256, 0, ctx->stream>>>(xa);
