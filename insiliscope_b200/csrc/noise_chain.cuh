@@ -16,10 +16,13 @@ struct PixelCamera
    int emccd;
 };
 
-// The float64 chain of sensor pixel `pix` of the frame that `u` is keyed to, its roundings and decisions taken from
-// the float32 normal where that is sure. Out of line: NoisePixel comes here where its float32 decisions are in doubt.
+// The float64 chain of sensor pixel `pix` of frame `frame`, its roundings and decisions taken from the float32 normal
+// where that is sure. Out of line: NoisePixel comes here where its float32 decisions are in doubt. pos: the words of the
+// stream that the Poisson draw of `electrons` took, where that draw is sure (kNoDraw: it is not); the chain goes on from
+// there, since in a small image the few pixels that come here are the last to end.
+constexpr uint32_t kNoDraw = 0xFFFFFFFFu;
 static __device__ __noinline__ uint32_t NoisePixelExact(float photonValue, uint32_t pix, uint32_t seed, uint32_t frame,
-                                                 PixelCamera cam)
+                                                        PixelCamera cam, float electrons, uint32_t pos)
 {
    CounterRng u(seed, frame);
    u.Pixel(pix);
@@ -27,7 +30,15 @@ static __device__ __noinline__ uint32_t NoisePixelExact(float photonValue, uint3
    const double photons = pv > 0.0 ? pv : 0.0;   // std::max(0.0, v)
    if (cam.emccd)
    {
-      const double ne = CounterPoisson(photons * cam.qe + cam.dark + cam.cic, u);
+      double ne = electrons;
+      if (pos == kNoDraw)
+         ne = CounterPoisson(photons * cam.qe + cam.dark + cam.cic, u);
+      else
+      {
+         u.ctr = pos >> 2;
+         for (uint32_t i = 0; i < (pos & 3u); ++i)
+            u.Uniform();
+      }
       const double readE = cam.readNoise / cam.emGain, gain = cam.gain, offset = cam.offset;
       // The register's Gamma with float32 decisions (GammaSure), else CounterGamma from the saved stream; then the
       // rounding (before the clamp) from the float32 read-noise normal when no boundary is within the bound of both
@@ -171,18 +182,18 @@ struct PixelHashes
       const uint32_t mul = 1664525u, inc = 1013904223u;
       Finish(inc + ctr * mul, a0 + ctr * ((frame * mul + inc) * mul), b0 + ctr * sb, w);
    }
-   // Words pos .. pos + 2 of the stream.
-   __device__ __forceinline__ void Words3(uint32_t frame, uint32_t pos, uint32_t& w0, uint32_t& w1, uint32_t& w2) const
+   // Words pos .. pos + 4 of the stream: always within two hashes.
+   __device__ __forceinline__ void Words(uint32_t frame, uint32_t pos, uint32_t (&w)[5]) const
    {
       uint32_t lo[4], hi[4];
       At(frame, pos >> 2, lo);
       At(frame, (pos >> 2) + 1, hi);
       const bool odd = pos & 1, two = pos & 2;
-      const uint32_t x0 = odd ? lo[1] : lo[0], x1 = odd ? lo[2] : lo[1], x2 = odd ? lo[3] : lo[2],
-                     x3 = odd ? hi[0] : lo[3], x4 = odd ? hi[1] : hi[0];
-      w0 = two ? x2 : x0;
-      w1 = two ? x3 : x1;
-      w2 = two ? x4 : x2;
+      const uint32_t x[7] = {odd ? lo[1] : lo[0], odd ? lo[2] : lo[1], odd ? lo[3] : lo[2], odd ? hi[0] : lo[3],
+                             odd ? hi[1] : hi[0], odd ? hi[2] : hi[1], odd ? hi[3] : hi[2]};
+#pragma unroll
+      for (int i = 0; i < 5; ++i)
+         w[i] = two ? x[i + 2] : x[i];
    }
 };
 
@@ -224,7 +235,7 @@ __device__ __forceinline__ uint16_t NoisePixel(float photonValue, uint32_t i, co
    bool ok = cam.fast != 0;
    float ne = 0.f;
    uint32_t pos = 0;          // words of the stream consumed
-   uint32_t g1 = 0, g2 = 0;   // sCMOS: the read noise's words
+   uint32_t g1 = 0, g2 = 0;   // the read noise's words
    const PixelHashes H(seed, frame, pix);
    if (lf <= 59.9999f && lf >= 1e-6f)
    {
@@ -245,15 +256,15 @@ __device__ __forceinline__ uint16_t NoisePixel(float photonValue, uint32_t i, co
          b += H.sb;
       } while (p4 > hi);   // (each factor is below 1)
       // d is linear in the counter: the blocks drawn, from mul's inverse mod 2^32; the product before the last block
-      const uint32_t drawn = (d - inc) * 0xFEE058C5u;
+      const uint32_t blocks = (d - inc) * 0xFEE058C5u;
       const float p = p4 * RcpApprox(prod), u0 = UniformF(w[0]), u2 = UniformF(w[2]), p2 = u0 * UniformF(w[1]);
       // the block's first product at or below L: its factor ends the draw
       const float q1 = p * u0, q2 = p * p2, q3 = q2 * u2;
       const bool o1 = q1 > hi, o2 = o1 && q2 > hi, o3 = o2 && q3 > hi;
       const float last = o3 ? p4 : (o2 ? q3 : (o1 ? q2 : q1));
-      ok = ok && last < lo && drawn <= 64u && p4 > 1e-36f;   // (a subnormal product has lost its places)
+      ok = ok && last < lo && blocks <= 64u && p4 > 1e-36f;   // (a subnormal product has lost its places)
       const int n = o3 ? 3 : (o2 ? 2 : (o1 ? 1 : 0));
-      pos = 4 * (drawn - 1) + n;
+      pos = 4 * (blocks - 1) + n;
       ne = static_cast<float>(pos);
       ++pos;
       if (!cam.emccd)
@@ -297,36 +308,45 @@ __device__ __forceinline__ uint16_t NoisePixel(float photonValue, uint32_t i, co
          g2 = w[1];
       }
    }
+   const uint32_t drawn = ok ? pos : kNoDraw;
    const float ig = RcpApprox(gainF), aig = fabsf(ig);
    if (cam.emccd)
    {
       // The register's Gamma (CounterGamma's steps and draws): x within e; t = 1 + c x within dt; v = t^3 within dv;
       // the squeeze and the logarithmic test each within a bound of their terms' errors.
       float out = 0.f, outErr = 0.f;
-      if (ne > 0.f && ok)
+      uint32_t w[5];
+      if (!(ne > 0.f))
+      {
+         H.Words(frame, pos, w);
+         g1 = w[0];
+         g2 = w[1];
+      }
+      else if (ok)
       {
          const float d = ne - 0.333333333f, c = RsqrtApprox(9.f * d);
          ok = false;
          for (int it = 0; it < 16; ++it)
          {
-            uint32_t w1, w2, w3;
-            H.Words3(frame, pos, w1, w2, w3);
-            const NormalF z = DrawNormalF(w1, w2);
+            H.Words(frame, pos, w);
+            g1 = w[3];   // the read noise's words, if this draw is taken
+            g2 = w[4];
+            const NormalF z = DrawNormalF(w[0], w[1]);
             const float x = z.g, cx = c * x, t = 1.f + cx, dt = fmaf(c, z.e, fmaf(5e-7f, fabsf(cx), 1.3e-7f));
             const bool negative = t + dt <= 0.f;   // drawn again before its third uniform
             pos += negative ? 2 : 3;
             if (negative)
                continue;
             const float tt = t + dt, v = t * t * t, dv = fmaf(3.f * tt * tt, dt, 2.5e-7f * v);
-            const float w = UniformF(w3), x2 = x * x, ax = fabsf(x) + z.e;
+            const float uw = UniformF(w[2]), x2 = x * x, ax = fabsf(x) + z.e;
             const float s = fmaf(-0.0331f * x2, x2, 1.f);
             const float ds = fmaf(0.14f * ax * ax * ax, z.e, fmaf(4e-8f * x2, x2, 4e-7f));
             out = d * v;
             outErr = fmaf(d, dv, 3.6e-7f * out);
-            ok = t > dt && w < s - ds;
-            if (ok || !(t > dt) || !(w >= s + ds))
+            ok = t > dt && uw < s - ds;
+            if (ok || !(t > dt) || !(uw >= s + ds))
                break;
-            const float lw = 0.693147181f * Lg2Approx(w), lv = 0.693147181f * Lg2Approx(v);
+            const float lw = 0.693147181f * Lg2Approx(uw), lv = 0.693147181f * Lg2Approx(v);
             const float rhs = fmaf(0.5f, x2, d * (1.f - v + lv));
             const float iv = RcpApprox(v);
             const float alw = fabsf(lw), alv = fabsf(lv);
@@ -339,9 +359,7 @@ __device__ __forceinline__ uint16_t NoisePixel(float photonValue, uint32_t i, co
       }
       if (ok)
       {
-         uint32_t w1, w2, w3;
-         H.Words3(frame, pos, w1, w2, w3);
-         const NormalF z = DrawNormalF(w1, w2);
+         const NormalF z = DrawNormalF(g1, g2);
          const float rn = readF * cam.invEmF, rz = rn * z.g;
          const float af = fmaf(out + rz, ig, offF);
          const float m = aig * (outErr + fabsf(rn) * z.e) + 1.2e-6f * fmaf(out + fabsf(rz), aig, fabsf(offF));
@@ -376,7 +394,8 @@ __device__ __forceinline__ uint16_t NoisePixel(float photonValue, uint32_t i, co
    return static_cast<uint16_t>(NoisePixelExact(
       photonValue, pix, seed, frame,
       {cam.qe, cam.dark, cam.cic, cam.emGain, cam.maxAdu, st.readNoise ? static_cast<double>(readF) : cam.readNoise,
-       st.gain ? static_cast<double>(gainF) : cam.gain, static_cast<double>(offF), cam.emccd}));
+       st.gain ? static_cast<double>(gainF) : cam.gain, static_cast<double>(offF), cam.emccd},
+      ne, drawn));
 }
 
 } // namespace iscu
