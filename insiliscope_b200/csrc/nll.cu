@@ -19,6 +19,7 @@
 #include "iscu_internal.h"
 #include "psf_common.cuh"
 
+#include <algorithm>
 #include <cmath>
 #include <memory>
 #include <vector>
@@ -33,7 +34,6 @@ struct iscu_nll_model
    iscu::DevBuf basis;     // J x M*M float64: 2 pi Z_j
    iscu::DevBuf cs;        // the folded transform's cosines and sines (NllTables)
    iscu::DevBuf zphase;    // M*M float64: 2 pi sum c_j Z_j of the current evaluation
-   iscu::DevBuf zern;      // J float64
 };
 
 namespace iscu {
@@ -97,16 +97,48 @@ __device__ __forceinline__ void BlockSums(double (&v)[NV], double* red)
    }
 }
 
-__global__ void ZernPhaseKernel(const double* __restrict__ basis, const double* __restrict__ zern, int J, int MM,
-                                double* __restrict__ zphase)
+// What an evaluation needs before its emitters, in one launch (a copy, four clears and a kernel of their own were half a
+// live fit's time on the device): the Zernike phase of every pupil sample, and the accumulated outputs cleared.
+struct PrepareArgs
 {
-   const int m = blockIdx.x * blockDim.x + threadIdx.x;
-   if (m >= MM)
-      return;
-   double s = 0.0;
-   for (int j = 0; j < J; ++j)
-      s += zern[j] * basis[static_cast<size_t>(j) * MM + m];
-   zphase[m] = s;
+   const double* basis;
+   int J, MM;
+   const double* zernDev;   // nullable: the coefficients are in `zern`
+   double zern[kMaxJ];
+   double* zphase;
+   double* nll;
+   int* err;
+   double* gBg;             // nullable
+   uint32_t nFrames;
+   double* gZern;           // nullable
+};
+
+__global__ void __launch_bounds__(256) NllPrepareKernel(PrepareArgs a)
+{
+   __shared__ double z[kMaxJ];
+   if (threadIdx.x < kMaxJ)
+      z[threadIdx.x] = static_cast<int>(threadIdx.x) >= a.J ? 0.0
+                       : a.zernDev                         ? a.zernDev[threadIdx.x]
+                                                           : a.zern[threadIdx.x];
+   __syncthreads();
+   const uint32_t i = blockIdx.x * blockDim.x + threadIdx.x;
+   if (static_cast<int>(i) < a.MM)
+   {
+      double s = 0.0;
+#pragma unroll 8
+      for (int j = 0; j < a.J; ++j)
+         s += z[j] * a.basis[static_cast<size_t>(j) * a.MM + i];
+      a.zphase[i] = s;
+   }
+   if (i == 0)
+   {
+      *a.nll = 0.0;
+      *a.err = 0;
+   }
+   if (a.gZern && static_cast<int>(i) < a.J)
+      a.gZern[i] = 0.0;
+   if (a.gBg && i < a.nFrames)
+      a.gBg[i] = 0.0;
 }
 
 struct NllArgs
@@ -760,7 +792,6 @@ int iscu_nll_model_create(iscu_ctx* ctx, const iscu_nll_spec* spec, iscu_nll_mod
    ISCU_CK(mdl->basis.Reserve(std::max<size_t>(basis.size(), 1) * sizeof(double)));
    ISCU_CK(mdl->cs.Reserve(sizeof(NllTables)));
    ISCU_CK(mdl->zphase.Reserve(MM * sizeof(double)));
-   ISCU_CK(mdl->zern.Reserve(kMaxJ * sizeof(double)));
    ISCU_CK(cudaMemcpyAsync(mdl->samples.p, samp.data(), samp.size() * sizeof(double), cudaMemcpyHostToDevice,
                            ctx->stream));
    if (!basis.empty())
@@ -807,25 +838,29 @@ int iscu_nll_eval_dev(iscu_nll_model* model, uint32_t n_emitters, const float* p
    iscu_ctx* ctx = model->ctx;
    std::lock_guard<std::recursive_mutex> lock(ctx->mu);
    ClearError();
-   const int MM = model->M * model->M;
+   PrepareArgs pa = {};
+   pa.basis = model->basis.as<double>();
+   pa.J = model->J;
+   pa.MM = model->M * model->M;
    if (model->J)
    {
-      ISCU_CK(cudaMemcpyAsync(model->zern.p, zern, model->J * sizeof(double), cudaMemcpyHostToDevice, ctx->stream));
-      ZernPhaseKernel<<<(MM + 255) / 256, 256, 0, ctx->stream>>>(model->basis.as<double>(), model->zern.as<double>(),
-                                                                  model->J, MM, model->zphase.as<double>());
-      ISCU_CK_LAUNCH(ctx, "ZernPhaseKernel");
+      cudaPointerAttributes where = {};
+      if (cudaPointerGetAttributes(&where, zern) != cudaSuccess)
+         cudaGetLastError();   // not a pointer that CUDA knows: the host's
+      if (where.type == cudaMemoryTypeDevice)
+         pa.zernDev = zern;
+      else
+         std::copy(zern, zern + model->J, pa.zern);
    }
-   else
-      ISCU_CK(cudaMemsetAsync(model->zphase.p, 0, MM * sizeof(double), ctx->stream));
-   ISCU_CK(cudaMemsetAsync(nll_dev, 0, sizeof(double), ctx->stream));
-   ISCU_CK(cudaMemsetAsync(err_dev, 0, sizeof(int32_t), ctx->stream));
-   if (grad)
-   {
-      if (n_frames)
-         ISCU_CK(cudaMemsetAsync(grad_bg_dev, 0, n_frames * sizeof(double), ctx->stream));
-      if (model->J)
-         ISCU_CK(cudaMemsetAsync(grad_zern_dev, 0, model->J * sizeof(double), ctx->stream));
-   }
+   pa.zphase = model->zphase.as<double>();
+   pa.nll = nll_dev;
+   pa.err = err_dev;
+   pa.nFrames = n_frames;
+   pa.gBg = grad ? grad_bg_dev : nullptr;
+   pa.gZern = grad ? grad_zern_dev : nullptr;
+   const uint32_t cover = std::max(static_cast<uint32_t>(pa.MM), grad ? n_frames : 0u);
+   NllPrepareKernel<<<(cover + 255) / 256, 256, 0, ctx->stream>>>(pa);
+   ISCU_CK_LAUNCH(ctx, "NllPrepareKernel");
    if (n_emitters == 0)
       return ISCU_OK;
    NllArgs a;

@@ -136,3 +136,40 @@ def test_sample_groupings_match_oracle(engine, roi, n):
         for col in range(want.shape[1]):
             assert np.max(np.abs(have[:, col] - want[:, col])) <= 1e-4 * np.max(np.abs(want[:, col])), col
     model.close()
+
+
+def test_autograd_forms(problem):
+    """The autograd function's paths: no gradient wanted (the likelihood alone, the same value), Zernike coefficients on
+    the device and on the host in either precision, a scaled loss, a second backward, a differentiated backward, and
+    an input changed in place in between, which autograd refuses."""
+    model, prob, counts, ospec, t = problem
+    p, fr, bg, k = _dev(prob, counts)
+    want, _, (gp, gb, gz) = model.evaluate(p, fr, bg, prob.zern, k, grad=True)
+    with torch.no_grad():
+        quiet = poisson_nll(model, p.clone().requires_grad_(True), bg, torch.from_numpy(prob.zern), k, fr)
+    assert not quiet.requires_grad and abs(float(quiet) - want) <= 1e-12 * abs(want)
+    for device, dtype in (("cuda", torch.float64), ("cuda", torch.float32), ("cpu", torch.float64), ("cpu", torch.float32)):
+        z = torch.tensor(prob.zern, dtype=dtype, device=device, requires_grad=True)
+        q = p.clone().requires_grad_(True)
+        b = bg.clone().requires_grad_(True)
+        zval = z.detach().double().cpu().numpy()
+        _, _, (wp, wb, wz) = model.evaluate(p, fr, bg, zval, k, grad=True)
+        loss = poisson_nll(model, q, b, z, k, fr)
+        (0.3 * loss).backward(retain_graph=True)
+        (0.7 * loss).backward()
+        assert loss.dtype == torch.float64 and loss.dim() == 0 and loss.device == q.device
+        assert z.grad.dtype == dtype and z.grad.device.type == device
+        assert torch.allclose(q.grad, wp, rtol=1e-6, atol=0)
+        assert torch.allclose(b.grad.double(), wb, rtol=1e-6)
+        assert torch.allclose(z.grad.double().cpu(), wz.cpu(), rtol=1e-6)
+    s = torch.tensor(2.0, dtype=torch.float64, device="cuda", requires_grad=True)
+    q = p.clone().requires_grad_(True)
+    g, = torch.autograd.grad(s * poisson_nll(model, q, bg, torch.from_numpy(prob.zern), k, fr), q, create_graph=True)
+    d, = torch.autograd.grad(g.sum(), s)
+    assert torch.allclose(d, gp.double().sum(), rtol=1e-5)
+    q = p.clone().requires_grad_(True)
+    loss = poisson_nll(model, q, bg, torch.from_numpy(prob.zern), k, fr)
+    with torch.no_grad():
+        q.add_(1.0)
+    with pytest.raises(RuntimeError):
+        loss.backward()
