@@ -54,32 +54,33 @@ __device__ __forceinline__ bool Covers(const StagedEmitter& e, int X, int Y, int
    return true;
 }
 
-// The 16 taps of a fast emitter for the pixel p words from its centre pixel in the phase layout: the reference's
+// The NT x NT taps of a fast emitter for the pixel p words from its centre pixel in the phase layout: the reference's
 // row = 0; row += wx[i] B; sum += wy[j] row, unrolled. Taps outside the bw x bw array read the layout's zero margin
 // where the reference skips them, and the sums start from the first product instead of 0: both change at most the
 // sign of a zero partial sum, which the final float add cannot see (a pixel that starts at a background other than
 // -0 is never -0).
+template <int NT>
 __device__ __forceinline__ double PhaseTaps(const StagedEmitter& e, int p)
 {
-   int q[4];
+   int q[NT];
 #pragma unroll
-   for (int i = 0; i < 4; ++i)
+   for (int i = 0; i < NT; ++i)
       q[i] = p + e.xb[i];
-   double row[4];
+   double row[NT];
 #pragma unroll
-   for (int j = 0; j < 4; ++j)
+   for (int j = 0; j < NT; ++j)
    {
       const double* pr = e.row[j];
       double r = e.wx[0] * __ldg(pr + q[0]);
-      r += e.wx[1] * __ldg(pr + q[1]);
-      r += e.wx[2] * __ldg(pr + q[2]);
-      r += e.wx[3] * __ldg(pr + q[3]);
+#pragma unroll
+      for (int i = 1; i < NT; ++i)
+         r += e.wx[i] * __ldg(pr + q[i]);
       row[j] = r;
    }
    double sum = e.wy[0] * row[0];
-   sum += e.wy[1] * row[1];
-   sum += e.wy[2] * row[2];
-   sum += e.wy[3] * row[3];
+#pragma unroll
+   for (int j = 1; j < NT; ++j)
+      sum += e.wy[j] * row[j];
    return sum;
 }
 
@@ -111,7 +112,13 @@ __device__ __forceinline__ void SplatSingle(const StagedEmitter& e, const Kernel
    int dx, dy;
    if (!inside || !Covers(e, X, Y, dx, dy))
       return;
-   const double sum = e.fast ? PhaseTaps(e, dy * e.nb + dx) : GeneralTaps(e, K.k[e.slot], dx, dy);
+   // (a linear splat's 2 x 2 taps from the row-major sums, os words apart across the lanes and in loops of their own,
+   // took the events of 60 EMCCD frames of 131 x 97 px WHAT)
+   const int p = dy * e.nb + dx;
+   const double sum = !e.fast          ? GeneralTaps(e, K.k[e.slot], dx, dy)
+                      : e.nTaps == 4   ? PhaseTaps<4>(e, p)
+                      : e.nTaps == 2   ? PhaseTaps<2>(e, p)
+                                       : PhaseTaps<1>(e, p);
    acc += static_cast<float>(e.photons * sum);
 }
 
@@ -153,11 +160,11 @@ __device__ __forceinline__ int StageChunk(const iscu_emitter* __restrict__ ems, 
       s.spanLo = kv.spanLo ? kv.spanLo + s.plane * sq : nullptr;
       s.spanHi = kv.spanHi ? kv.spanHi + s.plane * sq : nullptr;
       // The phase layout serves the splat when every tap of every pixel of its square lies inside it (rows
-      // R + dy os + j, columns C + dx os + i in padded coordinates, |dx|, |dy| <= camRad, i, j < 4).
+      // R + dy os + j, columns C + dx os + i in padded coordinates, |dx|, |dy| <= camRad, i, j < nTaps).
       const int os = kv.os, ext = kv.nb * os, span = kv.camRad * os;
       const int R = s.by + os - 1 + kv.padLo, Cc = s.bx + os - 1 + kv.padLo;
-      s.fast = kv.phase && s.nTaps == 4 && R - span >= 0 && R + span + 3 < ext && Cc - span >= 0 &&
-               Cc + span + 3 < ext;
+      s.fast = kv.phase && R - span >= 0 && R + span + s.nTaps - 1 < ext && Cc - span >= 0 &&
+               Cc + span + s.nTaps - 1 < ext;
       if (s.fast)
       {
          const int nb2 = kv.nb * kv.nb;
@@ -288,14 +295,14 @@ __global__ void __launch_bounds__(kThreads, kPair ? 2 : 3) RenderTilesKernel(Ren
          {
             const StagedEmitter& ea = sEm[list[m]];
             const StagedEmitter& eb = sEm[list[m + 1]];
-            if (ea.fast && eb.fast)
+            if (ea.fast && eb.fast && ea.nTaps == 4 && eb.nTaps == 4)
             {
                int dxa, dya, dxb, dyb;
                const bool ina = inside && Covers(ea, X, Y, dxa, dya);
                const bool inb = inside && Covers(eb, X, Y, dxb, dyb);
                // a pixel outside a square reads the centre pixel's taps (in the layout) and adds nothing
-               const double sa = PhaseTaps(ea, ina ? dya * ea.nb + dxa : 0);
-               const double sb = PhaseTaps(eb, inb ? dyb * eb.nb + dxb : 0);
+               const double sa = PhaseTaps<4>(ea, ina ? dya * ea.nb + dxa : 0);
+               const double sb = PhaseTaps<4>(eb, inb ? dyb * eb.nb + dxb : 0);
                if (ina)
                   acc += static_cast<float>(ea.photons * sa);
                if (inb)

@@ -46,7 +46,7 @@ struct StagedEmitter
    const int16_t* spanLo;   // halo cut of the emitter's plane, indexed by dy + camRad; null: the whole square
    const int16_t* spanHi;
    int bx, by, plane;
-   uint8_t nTaps, slot, fast, pad;   // fast: a 4 x 4 splat whose taps all lie in the phase layout
+   uint8_t nTaps, slot, fast, pad;   // fast: a splat whose taps all lie in the phase layout
 };
 
 // Positions the splat accepts: finite and within +-1e9 pixels (beyond, the centre pixel leaves the int range).
