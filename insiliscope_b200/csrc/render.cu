@@ -113,7 +113,7 @@ __device__ __forceinline__ void SplatSingle(const StagedEmitter& e, const Kernel
    if (!inside || !Covers(e, X, Y, dx, dy))
       return;
    // (a linear splat's 2 x 2 taps from the row-major sums, os words apart across the lanes and in loops of their own,
-   // took the events of 60 EMCCD frames of 131 x 97 px WHAT)
+   // took the events of 60 EMCCD frames of 131 x 97 px from 157 to 180 us a call)
    const int p = dy * e.nb + dx;
    const double sum = !e.fast          ? GeneralTaps(e, K.k[e.slot], dx, dy)
                       : e.nTaps == 4   ? PhaseTaps<4>(e, p)
@@ -237,9 +237,11 @@ struct RenderArgs
    uint16_t* aduOut;
 };
 
-// kPair: two emitters per step (their taps in flight together; 2 CTAs per SM by registers), else one (3 CTAs).
+// kPair: two emitters per step (their taps in flight together; 2 CTAs per SM by registers), else one (4 CTAs: the noise
+// chain spills a little, but the taps' latency is what bounds the pass: 200 frames of 128 x 128 px, 160 emitters each,
+// 591 us with three, 521 with four; the events of 60 EMCCD frames of 131 x 97 px 160 and 154).
 template <int TX, int TY, bool kNoise, bool kPersistent, bool kPair>
-__global__ void __launch_bounds__(kThreads, kPair ? 2 : 3) RenderTilesKernel(RenderArgs a)
+__global__ void __launch_bounds__(kThreads, kPair ? 2 : 4) RenderTilesKernel(RenderArgs a)
 {
    static_assert(TX * TY == kThreads, "one thread per pixel of the tile");
    static_assert(TX % 32 == 0 || 32 % TX == 0, "a warp covers a rectangle of the tile");
