@@ -237,11 +237,34 @@ struct RenderArgs
    uint16_t* aduOut;
 };
 
-// kPair: two emitters per step (their taps in flight together; 2 CTAs per SM by registers), else one (4 CTAs: the noise
-// chain spills a little, but the taps' latency is what bounds the pass: 200 frames of 128 x 128 px, 160 emitters each,
-// 591 us with three, 521 with four; the events of 60 EMCCD frames of 131 x 97 px 160 and 154).
-template <int TX, int TY, bool kNoise, bool kPersistent, bool kPair>
-__global__ void __launch_bounds__(kThreads, kPair ? 2 : 4) RenderTilesKernel(RenderArgs a)
+// kStep emitters' contributions to pixel (X, Y), their taps in flight together, added in list order; entries at or
+// past n, and those that do not cover the pixel, read the centre pixel's taps (in the layout) and add nothing.
+template <int NT, int kStep>
+__device__ __forceinline__ void SplatStep(const StagedEmitter* sEm, const uint16_t* list, int m, int n, bool inside, int X,
+                                          int Y, float& acc)
+{
+   double sum[kStep];
+   bool in[kStep];
+#pragma unroll
+   for (int u = 0; u < kStep; ++u)
+   {
+      const StagedEmitter& e = sEm[list[min(m + u, n - 1)]];
+      int dx, dy;
+      in[u] = inside && m + u < n && Covers(e, X, Y, dx, dy);
+      sum[u] = PhaseTaps<NT>(e, in[u] ? dy * e.nb + dx : 0);
+   }
+#pragma unroll
+   for (int u = 0; u < kStep; ++u)
+      if (in[u])
+         acc += static_cast<float>(sEm[list[m + u]].photons * sum[u]);
+}
+
+// kStep emitters at a time: 1 at four CTAs per SM (the noise chain spills a little, but the taps' latency is what bounds
+// the pass: 200 frames of 128 x 128 px, 160 emitters each, 591 us with three, 521 with four; the events of 60 EMCCD
+// frames of 131 x 97 px 160 and 154); 2 at two per SM, for batches whose CTAs are all resident at that (LaunchConfig),
+// where a warp's own chain of taps is the time. 4 at one CTA per SM gained nothing on 2.
+template <int TX, int TY, bool kNoise, bool kPersistent, int kStep>
+__global__ void __launch_bounds__(kThreads, kStep == 1 ? 4 : 2) RenderTilesKernel(RenderArgs a)
 {
    static_assert(TX * TY == kThreads, "one thread per pixel of the tile");
    static_assert(TX % 32 == 0 || 32 % TX == 0, "a warp covers a rectangle of the tile");
@@ -291,33 +314,29 @@ __global__ void __launch_bounds__(kThreads, kPair ? 2 : 4) RenderTilesKernel(Ren
          const uint32_t cnt = min(static_cast<uint32_t>(kChunk), emCount - e0);
          const int kept = StageChunk(a.ems, fr.em_start + e0, cnt, a.K, tx0, ty0, tx1, ty1, sEm, sWarp);
          const int n = WarpList(sEm, kept, wx0, wx0 + wcw - 1, wy0, wy0 + wrh - 1, list);
-         // Two emitters per step, their taps independent (more loads in flight), their adds in list order.
-         int m = 0;
-         for (; kPair && m + 1 < n; m += 2)
-         {
-            const StagedEmitter& ea = sEm[list[m]];
-            const StagedEmitter& eb = sEm[list[m + 1]];
-            if (ea.fast && eb.fast && ea.nTaps == 4 && eb.nTaps == 4)
+         if (kStep == 1)
+            for (int m = 0; m < n; ++m)
+               SplatSingle(sEm[list[m]], a.K, inside, X, Y, acc);
+         else
+            for (int m = 0; m < n; m += kStep)
             {
-               int dxa, dya, dxb, dyb;
-               const bool ina = inside && Covers(ea, X, Y, dxa, dya);
-               const bool inb = inside && Covers(eb, X, Y, dxb, dyb);
-               // a pixel outside a square reads the centre pixel's taps (in the layout) and adds nothing
-               const double sa = PhaseTaps<4>(ea, ina ? dya * ea.nb + dxa : 0);
-               const double sb = PhaseTaps<4>(eb, inb ? dyb * eb.nb + dxb : 0);
-               if (ina)
-                  acc += static_cast<float>(ea.photons * sa);
-               if (inb)
-                  acc += static_cast<float>(eb.photons * sb);
+               // together where all are fast with the same taps (the same for the warp's lanes)
+               const int nt = sEm[list[m]].nTaps;
+               bool alike = true;
+#pragma unroll
+               for (int u = 0; u < kStep; ++u)
+               {
+                  const StagedEmitter& e = sEm[list[min(m + u, n - 1)]];
+                  alike = alike && e.fast && e.nTaps == nt;
+               }
+               if (alike && nt == 4)
+                  SplatStep<4, kStep>(sEm, list, m, n, inside, X, Y, acc);
+               else if (alike && nt == 2)
+                  SplatStep<2, kStep>(sEm, list, m, n, inside, X, Y, acc);
+               else
+                  for (int u = m; u < min(m + kStep, n); ++u)
+                     SplatSingle(sEm[list[u]], a.K, inside, X, Y, acc);
             }
-            else
-            {
-               SplatSingle(ea, a.K, inside, X, Y, acc);
-               SplatSingle(eb, a.K, inside, X, Y, acc);
-            }
-         }
-         for (; m < n; ++m)
-            SplatSingle(sEm[list[m]], a.K, inside, X, Y, acc);
          __syncthreads();
       }
       if (inside)
@@ -383,28 +402,28 @@ __global__ void SumsToDoubleKernel(const float* __restrict__ in, size_t n, doubl
 }
 
 // The forms: config % 3 the tile (16 x 16, 32 x 8, 8 x 32), (config / 3) % 2 grid or persistent, config / 6 one or
-// two emitters per step.
+// two emitters per step (few: two in every grid form; the same bits in all).
 using RenderFn = void (*)(RenderArgs);
-template <bool kNoise, bool kPersistent, bool kPair>
+template <bool kNoise, bool kPersistent, int kStep>
 RenderFn TileVariant(int tile)
 {
    switch (tile)
    {
-   case 0: return RenderTilesKernel<16, 16, kNoise, kPersistent, kPair>;
-   case 1: return RenderTilesKernel<32, 8, kNoise, kPersistent, kPair>;
-   default: return RenderTilesKernel<8, 32, kNoise, kPersistent, kPair>;
+   case 0: return RenderTilesKernel<16, 16, kNoise, kPersistent, kStep>;
+   case 1: return RenderTilesKernel<32, 8, kNoise, kPersistent, kStep>;
+   default: return RenderTilesKernel<8, 32, kNoise, kPersistent, kStep>;
    }
 }
 template <bool kNoise>
-RenderFn Variant(int config)
+RenderFn Variant(int config, bool few)
 {
    const int tile = config % 3;
    switch (config / 3)
    {
-   case 0: return TileVariant<kNoise, false, false>(tile);
-   case 1: return TileVariant<kNoise, true, false>(tile);
-   case 2: return TileVariant<kNoise, false, true>(tile);
-   default: return TileVariant<kNoise, true, true>(tile);
+   case 0: return few ? TileVariant<kNoise, false, 2>(tile) : TileVariant<kNoise, false, 1>(tile);
+   case 1: return TileVariant<kNoise, true, 1>(tile);
+   case 2: return TileVariant<kNoise, false, 2>(tile);
+   default: return TileVariant<kNoise, true, 2>(tile);
    }
 }
 constexpr int kTileW[3] = {16, 32, 8}, kTileH[3] = {16, 8, 32};
@@ -442,7 +461,12 @@ int LaunchConfig(iscu_ctx* ctx, int config, const iscu_emitter* ems, uint32_t nE
    a.aduOut = cam ? adu : nullptr;
    const bool persistent = (config / 3) % 2 == 1;
    const int tw = kTileW[config % 3], th = kTileH[config % 3];
-   RenderFn fn = cam ? Variant<true>(config) : Variant<false>(config);
+   const uint64_t ctas = static_cast<uint64_t>((a.st.width + tw - 1) / tw) * ((a.st.height + th - 1) / th) * nFrames;
+   // Two emitters a step where every CTA is resident even so: one frame of 64 x 64 px (16 CTAs) 32.8 us with one, 28.9
+   // with two, four of 128 x 128 (256) 38.3 and 33.1; past the line there is nothing to gain (six, 384 CTAs, 37.0 and
+   // 37.6; eight 38.1 and 39.9).
+   const bool few = ctas <= 2ull * ctx->smCount;
+   RenderFn fn = cam ? Variant<true>(config, few) : Variant<false>(config, few);
    if (persistent)
    {
       const int rc = LaunchFrameOrder(ctx, frames, nFrames, orderBuf);

@@ -255,3 +255,41 @@ def test_contributions_equal_the_one_pass_sums(engine, interp, halo):
     for config, (ph, adu) in out.items():
         assert np.array_equal(ph, out[0][0], equal_nan=True), config
         assert np.array_equal(adu, out[0][1]), config
+
+
+@pytest.mark.parametrize("per", [(1,), (2, 0, 3), (65, 2047, 2049, 64)])
+def test_small_batches_equal_the_one_emitter_step(engine, per):
+    """A batch whose CTAs are all resident takes two emitters a step where they have the same taps (here cubic, linear,
+    nearest and off-band emitters mixed, odd counts, both sides of a chunk); the persistent form takes one: the same
+    bits, also next to the same frames in a batch over the line."""
+    import torch
+    rng = np.random.default_rng(len(per))
+    half, os_ = 6, 4
+    n = 2 * half * os_ + 1
+    planes = rng.uniform(0.0, 1e-3, (3, n, n)).astype(np.float32)
+    for slot, interp in enumerate((INTERP_CUBIC, INTERP_LINEAR, INTERP_NEAREST)):
+        engine.kernel_set_planes(slot, planes, os_, 25.0, interp)
+    w, h, total = 49, 35, sum(per)
+    em = np.zeros(total, EMITTER_DTYPE)
+    em["x_px"] = rng.uniform(-half, w + half, total)
+    em["y_px"] = rng.uniform(-half, h + half, total)
+    em["photons"] = rng.uniform(1.0, 3000.0, total)
+    em["plane"] = rng.integers(0, 3, total) + 65536 * np.where(rng.uniform(size=total) < 0.7, 0, rng.integers(0, 3, total))
+    engine.set_static(w, h, flat_bg=10.0)
+    cam = CameraParams(gain=2.0, read_noise_e=1.5)
+    dem = torch.from_numpy(em.view(np.uint8)).cuda()
+    out = []
+    for config, empty in ((0, 0), (3, 0), (0, 60)):
+        fr = frames_table(np.concatenate([np.array(per), np.zeros(empty, int)]))
+        dfr = torch.from_numpy(fr.view(np.uint8)).cuda()
+        ph = torch.empty((len(fr), h, w), dtype=torch.float32, device="cuda")
+        adu = torch.empty((len(fr), h, w), dtype=torch.uint16, device="cuda")
+        try:
+            engine.set_render_config(config)
+            engine.render_frames_dev(dem, dfr, len(fr), cam, 5, ph, adu)
+        finally:
+            engine.set_render_config(0)
+        out.append((ph.cpu().numpy()[: len(per)], adu.cpu().numpy()[: len(per)]))
+    for got in out[1:]:
+        assert np.array_equal(got[0].view(np.uint32), out[0][0].view(np.uint32))
+        assert np.array_equal(got[1], out[0][1])
