@@ -160,12 +160,7 @@ namespace {
 #ifndef ISCU_WF_MIN_CTAS
 #define ISCU_WF_MIN_CTAS 2
 #endif
-// Stage buffers of the z pass: 2 = persistent CTAs copying the next column block in while transforming one; 1 = a
-// CTA per column block.
-#ifndef ISCU_WF_Z_STAGES
-#define ISCU_WF_Z_STAGES 1
-#endif
-// Columns per z block with one stage buffer (a power of two).
+// Columns per z block (a power of two).
 #ifndef ISCU_WF_Z_COLUMNS
 #define ISCU_WF_Z_COLUMNS 32
 #endif
@@ -173,6 +168,7 @@ constexpr int kThreads = 256;
 constexpr int kMinCtas = ISCU_WF_MIN_CTAS;
 constexpr size_t kSmemBudget = 100 * 1024;   // lines per CTA are sized to this
 constexpr size_t kSmemMax = 227 * 1024;
+constexpr size_t kSmemThird = 74 * 1024;   // dynamic shared memory of a CTA that leaves room for two more on its SM
 constexpr size_t kSmemPair = 112 * 1024;   // dynamic shared memory of a CTA that leaves room for a second on its SM
 
 __device__ __forceinline__ float2 Cadd(float2 a, float2 b) { return make_float2(a.x + b.x, a.y + b.y); }
@@ -629,52 +625,36 @@ __global__ void __launch_bounds__(kThreads, kMinCtas) YInverseKernel(const float
    ISCU_RADIX_SWITCH(P.r[0], (YLast<R>(S, rows, d.nyv, oy, nb, LogQ(P, 0), GroupTw(P, twg, 0))));
 }
 
-// The asynchronous copies of one block of columns into a stage buffer: B's nzv planes at in[n BZ + b] and, when
-// convolving, the PSF spectrum's GZ planes after them. 16-byte copies of column pairs (nb is even whenever BZ >= 2:
-// GY and BZ are powers of two, GY >= 4), else 8-byte ones.
-template <bool kConvolve>
-__device__ __forceinline__ void ZPrefetch(const float2* __restrict__ B, const float2* __restrict__ Kh, size_t plane, size_t col,
-                          int nzv, int GZ, int nb, int BZ, int logBZ, float2* in)
+// The asynchronous copies of one block of columns of `planes` planes, column b of plane n to dst[n BZ + b]: 16-byte
+// copies of column pairs (nb is even whenever BZ >= 2: GY and BZ are powers of two, GY >= 4), else 8-byte ones.
+__device__ __forceinline__ void ZPrefetch(const float2* __restrict__ src, size_t plane, int planes, int nb, int BZ,
+                                          int logBZ, float2* dst)
 {
-   float2* ks = in + (static_cast<size_t>(nzv) << logBZ);
    if ((nb & 1) == 0)
    {
       const int logPairs = logBZ - 1, pairs = BZ >> 1;
-      for (int t = threadIdx.x; t < (nzv << logPairs); t += blockDim.x)
+      for (int t = threadIdx.x; t < (planes << logPairs); t += blockDim.x)
       {
          const int n = t >> logPairs, b = (t & (pairs - 1)) << 1;
          if (b < nb)
-            CopyAsync16(in + (n << logBZ) + b, B + n * plane + col + b);
+            CopyAsync16(dst + (n << logBZ) + b, src + n * plane + b);
       }
-      if (kConvolve)
-         for (int t = threadIdx.x; t < (GZ << logPairs); t += blockDim.x)
-         {
-            const int n = t >> logPairs, b = (t & (pairs - 1)) << 1;
-            if (b < nb)
-               CopyAsync16(ks + (n << logBZ) + b, Kh + n * plane + col + b);
-         }
    }
    else
    {
-      for (int t = threadIdx.x; t < (nzv << logBZ); t += blockDim.x)
+      for (int t = threadIdx.x; t < (planes << logBZ); t += blockDim.x)
       {
          const int n = t >> logBZ, b = t & (BZ - 1);
          if (b < nb)
-            CopyAsync8(in + t, B + n * plane + col + b);
+            CopyAsync8(dst + t, src + n * plane + b);
       }
-      if (kConvolve)
-         for (int t = threadIdx.x; t < (GZ << logBZ); t += blockDim.x)
-         {
-            const int n = t >> logBZ, b = t & (BZ - 1);
-            if (b < nb)
-               CopyAsync8(ks + t, Kh + n * plane + col + b);
-         }
    }
 }
 
-// Z forward group 0: the block's columns from its stage buffer (lanes walk the columns), DIF group, twiddles.
+// Z forward group 0 in place (a task's points are its own slots; planes from nzv on are zero and not read), lanes
+// walking the columns: DIF group, twiddles.
 template <int R, bool kHalf>
-__device__ __forceinline__ void ZFirst(const ColAddr& S, const float2* in, int nzv, int nb, int BL, int logBL, int logQ,
+__device__ __forceinline__ void ZFirst(const ColAddr& S, int nzv, int nb, int BL, int logBL, int logQ,
                        const float2* __restrict__ tw)
 {
    const int q = 1 << logQ, total = BL << logQ;
@@ -688,7 +668,7 @@ __device__ __forceinline__ void ZFirst(const ColAddr& S, const float2* in, int n
       for (int m = 0; m < (kHalf ? R / 2 : R); ++m)
       {
          const int n = j + m * q;
-         v[m] = n < nzv ? in[(n << logBL) + b] : make_float2(0.f, 0.f);
+         v[m] = n < nzv ? S(b, n) : make_float2(0.f, 0.f);
       }
       DifReg<R, false, kHalf>(v);
       if (tw)
@@ -772,85 +752,57 @@ __device__ __forceinline__ void ZLast(const ColAddr& S, float2* __restrict__ B, 
 }
 
 // Columns along z of B (nzv planes) -> GZ-point forward FFT -> either the PSF spectrum Kh[pz][k][p] (all GZ planes,
-// forward only) or, times Kh, the inverse FFT cropped to planes [oz, oz + nzv) back into B. Persistent: CTA c takes
-// column blocks c, c + gridDim.x, ... (block blk: k = blk / blocksPerK, columns from p0 = (blk % blocksPerK) BZ),
-// and with stages = 2 the next block's B planes and PSF spectrum are copied into shared memory while this one is
-// transformed (stages = 1 where two stage buffers do not fit: the copies then follow the block). BZ a power of two;
-// smem (GZ + stages (nzv + GZ when convolving)) BZ float2, column layout.
+// forward only) or, times Kh, the inverse FFT cropped to planes [oz, oz + nzv) back into B. CTA blk takes columns from
+// p0 = (blk % blocksPerK) BZ of k = blk / blocksPerK, BZ a power of two; smem GZ BZ float2 (twice that when convolving:
+// the PSF spectrum's planes follow), column layout. B's planes are copied to the slots that group 0 reads, so the
+// transform is in place; the PSF spectrum arrives behind group 0. Latency bounds the pass (two CTAs an SM issue in 64 %
+// of the cycles), so the codelets are held to three: a 64-plane series of 512 x 512 px (513 x 1024 columns of 128) 252
+// us, 320 with a separate buffer for B's planes and two CTAs.
 template <bool kConvolve, int kLogN>
-__global__ void __launch_bounds__(kThreads, kMinCtas) ZKernel(float2* __restrict__ B, Dims d, int BZ, int logBZ,
-                                                              int blocksPerK, int nBlocks, int stages, int oz,
-                                                              const float2* __restrict__ twg, float2* __restrict__ Kh)
+__global__ void __launch_bounds__(kThreads, kLogN ? 3 : kMinCtas) ZKernel(float2* __restrict__ B, Dims d, int BZ, int logBZ,
+                                                                          int blocksPerK, int oz,
+                                                                          const float2* __restrict__ twg,
+                                                                          float2* __restrict__ Kh)
 {
    extern __shared__ float2 s[];
    const size_t plane = static_cast<size_t>(d.NK) * d.GY;
    const LinePlan P = Fixed<kLogN, 2>(d.pz);
    const int GZ = 1 << P.logN;
    const ColAddr S{s, BZ};
-   const size_t stageElems = static_cast<size_t>(d.nzv + (kConvolve ? GZ : 0)) << logBZ;
-   float2* stage0 = s + (static_cast<size_t>(GZ) << logBZ);
+   float2* KS = s + (static_cast<size_t>(GZ) << logBZ);
    const int logQ0 = LogQ(P, 0);
    const float2* tw0 = GroupTw(P, twg, 0);
-   const bool half = 2 * d.nzv <= (1 << P.logN), single = P.groups == 1;
-   auto colOf = [&](int blk, int& nb) {
-      const int k = blk / blocksPerK, p0 = (blk - k * blocksPerK) << logBZ;
-      nb = min(BZ, d.GY - p0);
-      return static_cast<size_t>(k) * d.GY + p0;
-   };
-   int blk = blockIdx.x;
-   if (blk < nBlocks)
-   {
-      int nb;
-      const size_t col = colOf(blk, nb);
-      ZPrefetch<kConvolve>(B, Kh, plane, col, d.nzv, GZ, nb, BZ, logBZ, stage0);
-   }
+   const bool half = 2 * d.nzv <= GZ, single = P.groups == 1;
+   const int k = blockIdx.x / blocksPerK, p0 = (blockIdx.x - k * blocksPerK) << logBZ, nb = min(BZ, d.GY - p0);
+   const size_t col = static_cast<size_t>(k) * d.GY + p0;
+   ZPrefetch(B + col, plane, d.nzv, nb, BZ, logBZ, s);
    CopyAsyncCommit();
-   for (int i = 0; blk < nBlocks; ++i, blk += gridDim.x)
+   if (kConvolve)
+      ZPrefetch(Kh + col, plane, GZ, nb, BZ, logBZ, KS);
+   CopyAsyncCommit();
+   CopyAsyncWaitPrior();   // B's planes
+   __syncthreads();
+   if (half)
+      ISCU_RADIX_SWITCH16(P.r[0], (ZFirst<R, true>(S, d.nzv, nb, BZ, logBZ, logQ0, tw0)))
+   else
+      ISCU_RADIX_SWITCH16(P.r[0], (ZFirst<R, false>(S, d.nzv, nb, BZ, logBZ, logQ0, tw0)))
+   CopyAsyncWait();   // the PSF spectrum
+   __syncthreads();
+   for (int g = 1; g < P.groups - 1; ++g)
    {
-      const int buf = stages == 2 ? (i & 1) : 0, next = blk + gridDim.x;
-      if (stages == 2 && next < nBlocks)
-      {
-         int nbn;
-         const size_t coln = colOf(next, nbn);
-         ZPrefetch<kConvolve>(B, Kh, plane, coln, d.nzv, GZ, nbn, BZ, logBZ, stage0 + (buf ^ 1) * stageElems);
-      }
-      CopyAsyncCommit();
-      CopyAsyncWaitPrior();   // this block's copies (the group before the one just committed)
+      ISCU_RADIX_SWITCH16(P.r[g],
+                        (SmemGroup<R, false, true>(S, nb, BZ, logBZ, P.logN, LogQ(P, g), GroupTw(P, twg, g))));
       __syncthreads();
-      int nb;
-      const size_t col = colOf(blk, nb);
-      const float2* in = stage0 + buf * stageElems;
-      const float2* KS = in + (static_cast<size_t>(d.nzv) << logBZ);
-      if (half)
-         ISCU_RADIX_SWITCH16(P.r[0], (ZFirst<R, true>(S, in, d.nzv, nb, BZ, logBZ, logQ0, tw0)))
-      else
-         ISCU_RADIX_SWITCH16(P.r[0], (ZFirst<R, false>(S, in, d.nzv, nb, BZ, logBZ, logQ0, tw0)))
-      __syncthreads();
-      for (int g = 1; g < P.groups - 1; ++g)
-      {
-         ISCU_RADIX_SWITCH16(P.r[g],
-                           (SmemGroup<R, false, true>(S, nb, BZ, logBZ, P.logN, LogQ(P, g), GroupTw(P, twg, g))));
-         __syncthreads();
-      }
-      ISCU_RADIX_SWITCH16(P.r[P.groups - 1],
-                        (ZTurn<R, kConvolve>(S, KS, Kh, plane, col, nb, BZ, logBZ, P.logN, !single, true)));
-      if (kConvolve)
-      {
-         __syncthreads();
-         if (!single)
-            InverseRest<true, true>(P, twg, S, nb, BZ, logBZ, P.groups - 2, 1);
-         ISCU_RADIX_SWITCH16(P.r[0], (ZLast<R>(S, B, plane, col, d.nzv, oz, nb, BZ, logBZ, logQ0, tw0, !single)));
-      }
-      __syncthreads();   // the block's shared memory (S and its stage buffer) is free again
-      if (stages == 1 && next < nBlocks)
-      {
-         int nbn;
-         const size_t coln = colOf(next, nbn);
-         ZPrefetch<kConvolve>(B, Kh, plane, coln, d.nzv, GZ, nbn, BZ, logBZ, stage0);
-         CopyAsyncCommit();
-      }
    }
-   CopyAsyncWait();
+   ISCU_RADIX_SWITCH16(P.r[P.groups - 1],
+                     (ZTurn<R, kConvolve>(S, KS, Kh, plane, col, nb, BZ, logBZ, P.logN, !single, true)));
+   if (kConvolve)
+   {
+      __syncthreads();
+      if (!single)
+         InverseRest<true, true>(P, twg, S, nb, BZ, logBZ, P.groups - 2, 1);
+      ISCU_RADIX_SWITCH16(P.r[0], (ZLast<R>(S, B, plane, col, d.nzv, oz, nb, BZ, logBZ, logQ0, tw0, !single)));
+   }
 }
 
 // X inverse, the last DIF group's inverse (span 1, no twiddles) straight from A: Z'[k] = (X[k] + conj X[H-k]) +
@@ -1269,21 +1221,17 @@ int YLines(const LinePlan& P)
    const int N = 1 << P.logN;
    return std::max<int>(1, std::min<int>(std::max(1, 8192 / N), static_cast<int>(kSmemBudget / RowBytes(P))));
 }
-// The z pass's column blocks: BZ columns per block (a power of two), `stages` stage buffers, the persistent grid.
+// The z pass's column blocks: BZ columns per block (a power of two).
 struct ZLaunch
 {
-   int BZ = 1, logBZ = 0, stages = 1, blocksPerK = 1, nBlocks = 1, grid = 1;
+   int BZ = 1, logBZ = 0, blocksPerK = 1, nBlocks = 1;
    size_t smem = 0;
 };
 
-size_t ZSmem(const Dims& d, int BZ, int stages, bool convolve)
+size_t ZSmem(const Dims& d, int BZ, bool convolve)
 {
-   return (static_cast<size_t>(d.GZ) + stages * static_cast<size_t>(d.nzv + (convolve ? d.GZ : 0))) * BZ *
-          sizeof(float2);
+   return static_cast<size_t>(convolve ? 2 : 1) * d.GZ * BZ * sizeof(float2);
 }
-
-template <bool kConvolve, int kLogN>
-int ZPlan(const iscu_ctx* ctx, const Dims& d, ZLaunch& z);
 
 // Codelets: the transform lengths each pass is compiled for (log2 of X's half length H, of GY, of GZ); any other
 // length runs the runtime-plan kernel (K = 0).
@@ -1355,25 +1303,19 @@ int SetFftSmem(int logH, int logGY, int logGZ)
    return ISCU_OK;
 }
 
-template <bool kConvolve, int kLogN>
-int ZPlan(const iscu_ctx* ctx, const Dims& d, ZLaunch& z)
+int ZPlan(const Dims& d, bool convolve, ZLaunch& z)
 {
-   // 16 columns per block (8 when the buffers would pass the budget, ...), double-buffered where that fits
-   z.BZ = ISCU_WF_Z_STAGES == 2 ? 16 : ISCU_WF_Z_COLUMNS;
-   z.stages = ISCU_WF_Z_STAGES;
-   while (z.BZ > 1 && ZSmem(d, z.BZ, z.stages, kConvolve) > kSmemBudget)
+   // as many columns as leave room for three CTAs an SM
+   z.BZ = ISCU_WF_Z_COLUMNS;
+   while (z.BZ > 1 && ZSmem(d, z.BZ, convolve) > kSmemThird)
       z.BZ >>= 1;
-   if (ZSmem(d, z.BZ, z.stages, kConvolve) > kSmemBudget)
-      z.stages = 1;
-   z.smem = ZSmem(d, z.BZ, z.stages, kConvolve);
-   if (z.smem > kSmemMax)
+   z.smem = ZSmem(d, z.BZ, convolve);
+   // the lengths taken leave room for the column's input as well
+   if (z.smem + static_cast<size_t>(d.nzv) * z.BZ * sizeof(float2) > kSmemMax)
       return Fail(ISCU_ERR_LIMIT, "widefield plan: a z column block does not fit in shared memory");
    z.logBZ = Log2(z.BZ);
    z.blocksPerK = (d.GY + z.BZ - 1) / z.BZ;
    z.nBlocks = z.blocksPerK * d.NK;
-   int perSm = 0;
-   ISCU_CK(cudaOccupancyMaxActiveBlocksPerMultiprocessor(&perSm, ZKernel<kConvolve, kLogN>, kThreads, z.smem));
-   z.grid = z.stages == 2 ? std::max(1, std::min(z.nBlocks, std::max(1, perSm) * ctx->smCount)) : z.nBlocks;
    return ISCU_OK;
 }
 
@@ -1391,10 +1333,9 @@ static int ConvolveToA(iscu_wf_plan* p, const float* density)
       return rc;
    p->Mark(2);
    int rc2 = ISCU_OK;
-   ISCU_WF_Z_CODELETS(d.logGZ, ZLaunch zl; rc2 = ZPlan<true, K>(ctx, d, zl); if (rc2 != ISCU_OK) return rc2;
-                      (ZKernel<true, K><<<zl.grid, kThreads, zl.smem, ctx->stream>>>(
-                         p->B.as<float2>(), d, zl.BZ, zl.logBZ, zl.blocksPerK, zl.nBlocks, zl.stages,
-                         static_cast<int>(p->kz / 2), twg, p->Kh.as<float2>())));
+   ISCU_WF_Z_CODELETS(d.logGZ, ZLaunch zl; rc2 = ZPlan(d, true, zl); if (rc2 != ISCU_OK) return rc2;
+                      (ZKernel<true, K><<<zl.nBlocks, kThreads, zl.smem, ctx->stream>>>(
+                         p->B.as<float2>(), d, zl.BZ, zl.logBZ, zl.blocksPerK, static_cast<int>(p->kz / 2), twg, p->Kh.as<float2>())));
    ISCU_CK_LAUNCH(ctx, "ZKernel<convolve>");
    p->Mark(3);
    const int BK = YLines(d.py);
@@ -1646,10 +1587,10 @@ int MakePlan(iscu_ctx* ctx, uint32_t nx, uint32_t ny, uint32_t nz, const float* 
    rc = ForwardXY(p.get(), psf, dk, p->A.as<float2>(), p->B.as<float2>());
    if (rc != ISCU_OK)
       return rc;
-   ISCU_WF_Z_CODELETS(dk.logGZ, ZLaunch zl; rc = ZPlan<false, K>(ctx, dk, zl); if (rc != ISCU_OK) return rc;
-                      (ZKernel<false, K><<<zl.grid, kThreads, zl.smem, ctx->stream>>>(
-                         p->B.as<float2>(), dk, zl.BZ, zl.logBZ, zl.blocksPerK, zl.nBlocks, zl.stages, 0,
-                         p->twg.as<float2>(), p->Kh.as<float2>())));
+   ISCU_WF_Z_CODELETS(dk.logGZ, ZLaunch zl; rc = ZPlan(dk, false, zl); if (rc != ISCU_OK) return rc;
+                      (ZKernel<false, K><<<zl.nBlocks, kThreads, zl.smem, ctx->stream>>>(
+                         p->B.as<float2>(), dk, zl.BZ, zl.logBZ, zl.blocksPerK, 0, p->twg.as<float2>(),
+                         p->Kh.as<float2>())));
    ISCU_CK_LAUNCH(ctx, "ZKernel<spectrum>");
    ISCU_CK(cudaStreamSynchronize(ctx->stream));
    out = std::move(p);
