@@ -504,19 +504,23 @@ __global__ void __launch_bounds__(kThreads, kMinCtas) XForwardKernel(const float
       ISCU_RADIX_SWITCH(P.r[0], (XFirst<R, false>(S, src, d.nxv, nb, logQ0, tw0, pairs)))
    __syncthreads();
    ForwardRest<true>(P, twg, S, nb, BY, logBY);
-   // X[k] = ((Z[k] + conj Z[H-k]) - i W_GX^k (Z[k] - conj Z[H-k])) / 2, Z in bit-reversed order
-   for (int t = threadIdx.x; t < (H + 1) * BY; t += blockDim.x)
+   // X[k] = ((Z[k] + conj Z[H-k]) - i W_GX^k (Z[k] - conj Z[H-k])) / 2, Z in bit-reversed order, and X[H-k] from the
+   // same two values: (e, o, W) there are (conj e, -conj o, -conj W). 64 planes of 512 x 512 px: 73 us, 91 with each
+   // bin by itself (the pass is bound by instructions and latency: 31 us of bytes).
+   float2* out = A + static_cast<size_t>(z) * d.NK * d.nyv + y0;
+   for (int t = threadIdx.x; t < (H / 2 + 1) << logBY; t += blockDim.x)
    {
       const int k = t >> logBY, b = t & (BY - 1);
       if (b >= nb)
          continue;
-      const float2 zk = S(b, Rev(k & (H - 1), logH));
+      const float2 zk = S(b, Rev(k, logH));
       const float2 zm = Conj(S(b, Rev((H - k) & (H - 1), logH)));
       const float2 e = Cadd(zk, zm), o = Csub(zk, zm);
       const float2 w = __ldg(tw + (k << (d.logG - d.logGX)));
       const float2 wo = Cmul(w, o);   // then times -i: (x, y) -> (y, -x)
-      const float2 X = make_float2(0.5f * (e.x + wo.y), 0.5f * (e.y - wo.x));
-      A[(static_cast<size_t>(z) * d.NK + k) * d.nyv + y0 + b] = X;
+      out[static_cast<size_t>(k) * d.nyv + b] = make_float2(0.5f * (e.x + wo.y), 0.5f * (e.y - wo.x));
+      if (2 * k < H)
+         out[static_cast<size_t>(H - k) * d.nyv + b] = make_float2(0.5f * (e.x - wo.y), -0.5f * (e.y + wo.x));
    }
 }
 
@@ -855,14 +859,16 @@ __global__ void __launch_bounds__(kThreads, kMinCtas) XInverseKernel(const float
    __syncthreads();
    InverseRest<true>(P, twg, S, nb, BY, logBY, P.groups - 2, 0);
    float* out = image + (static_cast<size_t>(z) * d.nyv + y0) * d.nxv;
-   for (int t = threadIdx.x; t < nb * d.nxv; t += blockDim.x)
-   {
-      const int b = t / d.nxv, x = t % d.nxv;
-      const int m = x + ox;
-      const float2 c = S(b, m >> 1);
-      const float v = (m & 1 ? c.y : c.x) * scale;
-      out[t] = (clamp && !(v > 0.f) ? 0.f : v) + background;
-   }
+   // a warp per row: 64 planes of 512 x 512 px 64 us, 84 with a division per pixel. (Packing both bins of a pair in
+   // one task of XLoad, each value read once, was slower: 78.)
+   for (int b = threadIdx.x >> 5; b < nb; b += kThreads / 32)
+      for (int x = threadIdx.x & 31; x < d.nxv; x += 32)
+      {
+         const int m = x + ox;
+         const float2 c = S(b, m >> 1);
+         const float v = (m & 1 ? c.y : c.x) * scale;
+         out[b * d.nxv + x] = (clamp && !(v > 0.f) ? 0.f : v) + background;
+      }
 }
 
 // The noise chain of every pixel of the photon frames (frame frame0 + plane) -> ADU. A kernel of its own: the
