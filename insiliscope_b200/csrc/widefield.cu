@@ -508,6 +508,7 @@ __global__ void __launch_bounds__(kThreads, kMinCtas) XForwardKernel(const float
    // same two values: (e, o, W) there are (conj e, -conj o, -conj W). 64 planes of 512 x 512 px: 73 us, 91 with each
    // bin by itself (the pass is bound by instructions and latency: 31 us of bytes).
    float2* out = A + static_cast<size_t>(z) * d.NK * d.nyv + y0;
+#pragma unroll 2
    for (int t = threadIdx.x; t < (H / 2 + 1) << logBY; t += blockDim.x)
    {
       const int k = t >> logBY, b = t & (BY - 1);
@@ -1227,6 +1228,17 @@ int YLines(const LinePlan& P)
    const int N = 1 << P.logN;
    return std::max<int>(1, std::min<int>(std::max(1, 8192 / N), static_cast<int>(kSmemBudget / RowBytes(P))));
 }
+// Fewer lines per CTA where a volume's CTAs would leave SMs idle: `lines` halved, to no fewer than `least`, while
+// `planes` planes of `total` lines make fewer than `want` CTAs. A convolution of 186 x 151 x 11 cells on a 256 x 256 x
+// 16 grid (110 CTAs in x, 55 in y; 32 of 256 threads busy in z with 32 columns a block) takes 50.0 us with full CTAs,
+// 45.3 with 4 lines in y, 47.5 with 256 columns in z, 41.8 with all three rules; 4 lines in x cost its 128-byte stores
+// (52.8).
+int FewerLines(int lines, int least, int total, int planes, int want)
+{
+   while (lines / 2 >= least && static_cast<int64_t>((total + lines - 1) / lines) * planes < want)
+      lines /= 2;
+   return lines;
+}
 // The z pass's column blocks: BZ columns per block (a power of two).
 struct ZLaunch
 {
@@ -1240,18 +1252,31 @@ size_t ZSmem(const Dims& d, int BZ, bool convolve)
 }
 
 // Codelets: the transform lengths each pass is compiled for (log2 of X's half length H, of GY, of GZ); any other
-// length runs the runtime-plan kernel (K = 0).
-#define ISCU_WF_CODELETS(logN, a, b, c, ...)                                                                            \
+// length runs the runtime-plan kernel (K = 0), whose switches and index arithmetic take about half as long again
+// (186 x 151 x 11 cells: 61.7 us a convolution, 50.0 with the codelets of its lengths).
+#define ISCU_WF_CODELET(k, ...) case k: { constexpr int K = k; __VA_ARGS__; } break;
+#define ISCU_WF_RUNTIME_PLAN(...) default: { constexpr int K = 0; __VA_ARGS__; } break;
+#define ISCU_WF_X_CODELETS(logN, ...)                                                                                   \
    switch (logN)                                                                                                       \
    {                                                                                                                   \
-   case a: { constexpr int K = a; __VA_ARGS__; } break;                                                                \
-   case b: { constexpr int K = b; __VA_ARGS__; } break;                                                                \
-   case c: { constexpr int K = c; __VA_ARGS__; } break;                                                                \
-   default: { constexpr int K = 0; __VA_ARGS__; } break;                                                               \
+      ISCU_WF_CODELET(5, __VA_ARGS__) ISCU_WF_CODELET(6, __VA_ARGS__) ISCU_WF_CODELET(7, __VA_ARGS__)                  \
+      ISCU_WF_CODELET(8, __VA_ARGS__) ISCU_WF_CODELET(9, __VA_ARGS__) ISCU_WF_CODELET(10, __VA_ARGS__)                 \
+      ISCU_WF_RUNTIME_PLAN(__VA_ARGS__)                                                                                \
    }
-#define ISCU_WF_X_CODELETS(logN, ...) ISCU_WF_CODELETS(logN, 8, 9, 10, __VA_ARGS__)
-#define ISCU_WF_Y_CODELETS(logN, ...) ISCU_WF_CODELETS(logN, 9, 10, 11, __VA_ARGS__)
-#define ISCU_WF_Z_CODELETS(logN, ...) ISCU_WF_CODELETS(logN, 6, 7, 8, __VA_ARGS__)
+#define ISCU_WF_Y_CODELETS(logN, ...)                                                                                   \
+   switch (logN)                                                                                                       \
+   {                                                                                                                   \
+      ISCU_WF_CODELET(6, __VA_ARGS__) ISCU_WF_CODELET(7, __VA_ARGS__) ISCU_WF_CODELET(8, __VA_ARGS__)                  \
+      ISCU_WF_CODELET(9, __VA_ARGS__) ISCU_WF_CODELET(10, __VA_ARGS__) ISCU_WF_CODELET(11, __VA_ARGS__)                \
+      ISCU_WF_RUNTIME_PLAN(__VA_ARGS__)                                                                                \
+   }
+#define ISCU_WF_Z_CODELETS(logN, ...)                                                                                   \
+   switch (logN)                                                                                                       \
+   {                                                                                                                   \
+      ISCU_WF_CODELET(2, __VA_ARGS__) ISCU_WF_CODELET(3, __VA_ARGS__) ISCU_WF_CODELET(4, __VA_ARGS__)                  \
+      ISCU_WF_CODELET(5, __VA_ARGS__) ISCU_WF_CODELET(6, __VA_ARGS__) ISCU_WF_CODELET(7, __VA_ARGS__)                  \
+      ISCU_WF_CODELET(8, __VA_ARGS__) ISCU_WF_RUNTIME_PLAN(__VA_ARGS__)                                                \
+   }
 
 // The forward x and y passes of a (kzv x kyv x kxv) volume into A, B.
 int ForwardXY(iscu_wf_plan* p, const float* in, const Dims& d, float2* A, float2* B, bool mark = false)
@@ -1259,13 +1284,13 @@ int ForwardXY(iscu_wf_plan* p, const float* in, const Dims& d, float2* A, float2
    iscu_ctx* ctx = p->ctx;
    const float2* tw = p->tw.as<float2>();
    const float2* twg = p->twg.as<float2>();
-   const int BY = XLines(d.H);
+   const int BY = FewerLines(XLines(d.H), 8, d.nyv, d.nzv, ctx->smCount);
    ISCU_WF_X_CODELETS(d.logH, (XForwardKernel<K><<<dim3((d.nyv + BY - 1) / BY, d.nzv), kThreads, XSmem(d.H, BY),
                                                  ctx->stream>>>(in, d, BY, Log2(BY), tw, twg, A)));
    ISCU_CK_LAUNCH(ctx, "XForwardKernel");
    if (mark)
       p->Mark(1);
-   const int BK = YLines(d.py);
+   const int BK = FewerLines(YLines(d.py), 4, d.NK, d.nzv, 2 * ctx->smCount);
    ISCU_WF_Y_CODELETS(d.logGY, (YForwardKernel<K><<<dim3((d.NK + BK - 1) / BK, d.nzv), kThreads,
                                                     BK * RowBytes(d.py), ctx->stream>>>(A, d, BK, twg, B)));
    ISCU_CK_LAUNCH(ctx, "YForwardKernel");
@@ -1309,10 +1334,11 @@ int SetFftSmem(int logH, int logGY, int logGZ)
    return ISCU_OK;
 }
 
-int ZPlan(const Dims& d, bool convolve, ZLaunch& z)
+int ZPlan(const iscu_ctx* ctx, const Dims& d, bool convolve, ZLaunch& z)
 {
-   // as many columns as leave room for three CTAs an SM
-   z.BZ = ISCU_WF_Z_COLUMNS;
+   // A 16-point task per thread and as many columns as leave room for three CTAs an SM.
+   z.BZ = std::max(ISCU_WF_Z_COLUMNS, std::min(d.GY, 4096 / d.GZ));
+   z.BZ = FewerLines(z.BZ, ISCU_WF_Z_COLUMNS, d.GY, d.NK, ctx->smCount);
    while (z.BZ > 1 && ZSmem(d, z.BZ, convolve) > kSmemThird)
       z.BZ >>= 1;
    z.smem = ZSmem(d, z.BZ, convolve);
@@ -1339,12 +1365,12 @@ static int ConvolveToA(iscu_wf_plan* p, const float* density)
       return rc;
    p->Mark(2);
    int rc2 = ISCU_OK;
-   ISCU_WF_Z_CODELETS(d.logGZ, ZLaunch zl; rc2 = ZPlan(d, true, zl); if (rc2 != ISCU_OK) return rc2;
+   ISCU_WF_Z_CODELETS(d.logGZ, ZLaunch zl; rc2 = ZPlan(ctx, d, true, zl); if (rc2 != ISCU_OK) return rc2;
                       (ZKernel<true, K><<<zl.nBlocks, kThreads, zl.smem, ctx->stream>>>(
                          p->B.as<float2>(), d, zl.BZ, zl.logBZ, zl.blocksPerK, static_cast<int>(p->kz / 2), twg, p->Kh.as<float2>())));
    ISCU_CK_LAUNCH(ctx, "ZKernel<convolve>");
    p->Mark(3);
-   const int BK = YLines(d.py);
+   const int BK = FewerLines(YLines(d.py), 4, d.NK, d.nzv, 2 * ctx->smCount);
    ISCU_WF_Y_CODELETS(d.logGY, (YInverseKernel<K><<<dim3((d.NK + BK - 1) / BK, d.nzv), kThreads,
                                                     BK * RowBytes(d.py), ctx->stream>>>(
                                    p->B.as<float2>(), d, BK, static_cast<int>(p->ky / 2), twg, p->A.as<float2>())));
@@ -1377,7 +1403,7 @@ static int FinishX(iscu_wf_plan* p, double background, const iscu_camera* cam, u
       ISCU_CK(p->cells.Reserve(static_cast<size_t>(p->nx) * p->ny * p->nz * sizeof(float)));
       xout = p->cells.as<float>();
    }
-   const int BY = XLines(d.H);
+   const int BY = FewerLines(XLines(d.H), 8, d.nyv, d.nzv, ctx->smCount);
    ISCU_WF_X_CODELETS(d.logH, (XInverseKernel<K><<<dim3((d.nyv + BY - 1) / BY, d.nzv), kThreads, XSmem(d.H, BY),
                                                    ctx->stream>>>(
                                   p->A.as<float2>(), d, BY, Log2(BY), static_cast<int>(p->kx / 2), scale,
@@ -1593,7 +1619,7 @@ int MakePlan(iscu_ctx* ctx, uint32_t nx, uint32_t ny, uint32_t nz, const float* 
    rc = ForwardXY(p.get(), psf, dk, p->A.as<float2>(), p->B.as<float2>());
    if (rc != ISCU_OK)
       return rc;
-   ISCU_WF_Z_CODELETS(dk.logGZ, ZLaunch zl; rc = ZPlan(dk, false, zl); if (rc != ISCU_OK) return rc;
+   ISCU_WF_Z_CODELETS(dk.logGZ, ZLaunch zl; rc = ZPlan(ctx, dk, false, zl); if (rc != ISCU_OK) return rc;
                       (ZKernel<false, K><<<zl.nBlocks, kThreads, zl.smem, ctx->stream>>>(
                          p->B.as<float2>(), dk, zl.BZ, zl.logBZ, zl.blocksPerK, 0, p->twg.as<float2>(),
                          p->Kh.as<float2>())));

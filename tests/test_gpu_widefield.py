@@ -156,6 +156,26 @@ def test_codelet_lengths_vs_oracle(engine, vol_shape, psf_shape, grid):
     plan.close()
 
 
+@pytest.mark.parametrize("vol_shape,psf_shape,grid", [
+    ((1, 30, 60), (1, 5, 7), (64, 32, 4)), ((3, 50, 100), (1, 9, 9), (128, 64, 4)), ((6, 91, 152), (3, 31, 61), (256, 128, 8)),
+    ((11, 151, 186), (9, 61, 61), (256, 256, 16)), ((20, 64, 62), (9, 1, 2), (64, 64, 32)),
+    ((260, 13, 10), (9, 3, 3), (16, 16, 512))])
+def test_short_and_odd_lengths_vs_oracle(engine, vol_shape, psf_shape, grid):
+    """The codelets of the shorter transforms, with fewer lines per CTA and wider column blocks where the volume is
+    small, and the runtime plans (the last case's x, y and z) against the float64 oracle."""
+    import torch
+    rng = np.random.default_rng(sum(vol_shape))
+    vol = rng.random(vol_shape).astype(np.float32)
+    vol[vol < 0.7] = 0.0
+    psf = rng.random(psf_shape).astype(np.float32) - 0.2
+    plan = WidefieldPlan(engine, vol_shape, psf)
+    assert plan.grid() == grid
+    got = plan.convolve_dev(torch.from_numpy(vol).cuda()).cpu().numpy()
+    want = np.maximum(fft_convolve_same_f64(vol, psf), 0.0)
+    assert _rel(got, want) <= TOL
+    plan.close()
+
+
 def test_codelet_2048_impulse(engine):
     """A 2048 x 2048 grid (x half length 1024, y 2048 codelets): unit dyes image to the PSF shifted there."""
     import torch
