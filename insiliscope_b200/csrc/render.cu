@@ -169,11 +169,17 @@ __device__ __forceinline__ int StageChunk(const iscu_emitter* __restrict__ ems, 
       {
          const int nb2 = kv.nb * kv.nb;
          const double* base = kv.phase + static_cast<size_t>(s.plane) * os * os * nb2;
+         // phase and cell of tap rows R + k and tap columns Cc + k: one division each, then steps
+         int ry = R / os, py = R - ry * os, cx = Cc / os, px = Cc - cx * os;
 #pragma unroll
          for (int k = 0; k < 4; ++k)
          {
-            s.row[k] = base + ((R + k) % os) * os * nb2 + ((R + k) / os) * kv.nb;
-            s.xb[k] = ((Cc + k) % os) * nb2 + (Cc + k) / os;
+            s.row[k] = base + py * os * nb2 + ry * kv.nb;
+            s.xb[k] = px * nb2 + cx;
+            if (++py == os)
+               py = 0, ++ry;
+            if (++px == os)
+               px = 0, ++cx;
          }
       }
    }
@@ -337,7 +343,10 @@ __global__ void __launch_bounds__(kThreads, kStep == 1 ? 4 : 2) RenderTilesKerne
                   for (int u = m; u < min(m + kStep, n); ++u)
                      SplatSingle(sEm[list[u]], a.K, inside, X, Y, acc);
             }
-         __syncthreads();
+         // the staged emitters are rewritten (after a tile's last chunk the next tile's barriers serve, so that a warp
+         // with few emitters is at its noise while another adds)
+         if (e0 + kChunk < emCount)
+            __syncthreads();
       }
       if (inside)
       {

@@ -808,7 +808,8 @@ __global__ void __launch_bounds__(kGT, 6) GatherTilesKernel(GatherArgs a)
                listed = 0;
             }
          }
-         __syncthreads();
+         if (e0 + kGChunk < emCount)   // (a persistent CTA's next tile starts with barriers)
+            __syncthreads();
       }
       GatherFlush<TX, kSub>(list, listed, lane, bit, lx, ly, acc);
       // (one copy of the noise chain, gone through kSub times)
