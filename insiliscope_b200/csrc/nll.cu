@@ -13,7 +13,7 @@
 //
 // One CTA per emitter at a time (a persistent grid): the pupil phase in float64, reduced mod 2 pi, then float32
 // sincos; the four products (forward 32x32 -> 32x64 -> 64x64, adjoint back) folded about the ROI's centre, in float32;
-// the per-emitter sums in float64. The gradient pass recomputes the field instead of storing per-emitter PSFs. The
+// the per-emitter sums in float64. The gradient pass forms the field itself: no per-emitter PSF is stored. The
 // Zernike gradient accumulates per CTA in float64 across its emitters and is added once per CTA.
 
 #include "iscu_internal.h"
@@ -241,10 +241,12 @@ __device__ __forceinline__ void Pixels(const NllArgs& a, uint32_t e, const int (
 // +tau and C - i S at -tau -- real by complex products of a quarter of the size. With the aperture's 29 of the 32
 // samples an emitter's four products take 334 K multiply-adds instead of 1.57 M, exactly the same sums.
 //
-// What bounds it: shared-memory reads and FP32 multiply-adds about equally (each product reads its constants by
-// broadcast -- a warp's t or q group is the same for its lanes -- and its data once per lane, 16 bytes at a time),
-// then the float64 logarithm of each pixel. 128 threads and 55 KB, four CTAs per SM, so that one CTA's products run
-// under another's logarithms and barriers.
+// What bounds it: shared-memory wavefronts (79 % of the data path with gradients, 62 % without; each product reads its
+// constants by broadcast -- a warp's t or q group is the same for its lanes, and such a 16-byte read takes two -- and its
+// data once per lane), then the float64 logarithm of each pixel. 128 threads and 55 KB, four CTAs per SM, so that one
+// CTA's products run under another's logarithms and barriers. 256,000 emitters of 32 x 32 px, os = 2: likelihood and
+// gradients 7.6 ms (unfolded 23.3), the likelihood alone 3.65 (11.6). Constants as kernel parameters were slower (the
+// two passes 14.0 ms against 11.7).
 template <bool kGrad, int OS>
 __global__ void __launch_bounds__(kThreads, kCtasPerSm) NllKernel(NllArgs a)
 {
