@@ -207,7 +207,8 @@ __global__ void __launch_bounds__(kThreads) BinnedRenderKernel(const iscu_emitte
 //
 // What bounds it: issue and the latency of 16 warps per SM (the accumulators are half the registers), the shared loads
 // at 45 %, the float64 pipe at 15 %; 54 % of the multiply-adds lie in an emitter's reach at R = 32. 200 frames of
-// 128 x 128 px, 2,400 emitters a frame, u = 2, R = 32: 1.10 ms against 2.03 ms of the kernel above.
+// 128 x 128 px, 2,400 emitters a frame, u = 2, R = 32: 1.10 ms against 2.03 ms of the kernel above. Slower (with the
+// noise, against 1.18): 512 threads of four rows, 32 warps per SM, 1.34; a 64-bit multiply for the two shifts, 1.26.
 constexpr int kTileX = 128, kTileY = 64, kRows = 8, kCap = 1024, kMaxPlanes = 512;
 constexpr size_t kDenseMaxBytes = 226 * 1024;
 
