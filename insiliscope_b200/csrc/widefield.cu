@@ -1228,6 +1228,10 @@ int YLines(const LinePlan& P)
    const int N = 1 << P.logN;
    return std::max<int>(1, std::min<int>(std::max(1, 8192 / N), static_cast<int>(kSmemBudget / RowBytes(P))));
 }
+// Threads of a y CTA, and its lines by them: 128 with half the lines where those fill it, four CTAs an SM instead of two
+// of 256, so that more of them are at different phases (loads, groups, stores): 64 planes of 512 x 512 px, 1,024-point
+// lines, a series 957 -> 943 us.
+int YThreads(const LinePlan& P) { return P.logN <= 11 ? kThreads / 2 : kThreads; }
 // Fewer lines per CTA where a volume's CTAs would leave SMs idle: `lines` halved, to no fewer than `least`, while
 // `planes` planes of `total` lines make fewer than `want` CTAs. A convolution of 186 x 151 x 11 cells on a 256 x 256 x
 // 16 grid (110 CTAs in x, 55 in y; 32 of 256 threads busy in z with 32 columns a block) takes 50.0 us with full CTAs,
@@ -1290,8 +1294,9 @@ int ForwardXY(iscu_wf_plan* p, const float* in, const Dims& d, float2* A, float2
    ISCU_CK_LAUNCH(ctx, "XForwardKernel");
    if (mark)
       p->Mark(1);
-   const int BK = FewerLines(YLines(d.py), 4, d.NK, d.nzv, 2 * ctx->smCount);
-   ISCU_WF_Y_CODELETS(d.logGY, (YForwardKernel<K><<<dim3((d.NK + BK - 1) / BK, d.nzv), kThreads,
+   const int yThreads = YThreads(d.py);
+   const int BK = FewerLines(std::max(1, YLines(d.py) * yThreads / kThreads), 4, d.NK, d.nzv, 2 * ctx->smCount);
+   ISCU_WF_Y_CODELETS(d.logGY, (YForwardKernel<K><<<dim3((d.NK + BK - 1) / BK, d.nzv), yThreads,
                                                     BK * RowBytes(d.py), ctx->stream>>>(A, d, BK, twg, B)));
    ISCU_CK_LAUNCH(ctx, "YForwardKernel");
    return ISCU_OK;
@@ -1370,8 +1375,9 @@ static int ConvolveToA(iscu_wf_plan* p, const float* density)
                          p->B.as<float2>(), d, zl.BZ, zl.logBZ, zl.blocksPerK, static_cast<int>(p->kz / 2), twg, p->Kh.as<float2>())));
    ISCU_CK_LAUNCH(ctx, "ZKernel<convolve>");
    p->Mark(3);
-   const int BK = FewerLines(YLines(d.py), 4, d.NK, d.nzv, 2 * ctx->smCount);
-   ISCU_WF_Y_CODELETS(d.logGY, (YInverseKernel<K><<<dim3((d.NK + BK - 1) / BK, d.nzv), kThreads,
+   const int yThreads = YThreads(d.py);
+   const int BK = FewerLines(std::max(1, YLines(d.py) * yThreads / kThreads), 4, d.NK, d.nzv, 2 * ctx->smCount);
+   ISCU_WF_Y_CODELETS(d.logGY, (YInverseKernel<K><<<dim3((d.NK + BK - 1) / BK, d.nzv), yThreads,
                                                     BK * RowBytes(d.py), ctx->stream>>>(
                                    p->B.as<float2>(), d, BK, static_cast<int>(p->ky / 2), twg, p->A.as<float2>())));
    ISCU_CK_LAUNCH(ctx, "YInverseKernel");
