@@ -144,12 +144,6 @@ def _poisson_function():
     """The autograd function (made on first use: torch is imported there)."""
     import torch
 
-    def scaled(g, go, like):
-        # go x g in float64, rounded to like's type: one kernel where all are on one device and nothing differentiates it
-        if g.device == like.device == go.device and not (torch.is_grad_enabled() and go.requires_grad):
-            return torch.mul(g, go.reshape(1), out=torch.empty(g.shape, dtype=like.dtype, device=g.device))
-        return (go.to(like.device) * g.to(torch.float64).to(like.device)).to(like.dtype)
-
     class PoissonNll(torch.autograd.Function):
         """Where an input needs its gradient the forward pass runs the adjoint kernel, which evaluates the likelihood on
         its way, and the backward pass scales what it left (a likelihood pass before it recomputes every emitter's field
@@ -165,9 +159,12 @@ def _poisson_function():
 
         @staticmethod
         def backward(ctx, gout):
-            params, bg, zern, gp, gb, gz = ctx.saved_tensors
-            go = gout.to(torch.float64)
-            return scaled(gp, go, params), scaled(gb, go, bg), scaled(gz, go, zern), None
+            # go x g in float64, rounded to the input's type, for the inputs that want it (an integer input has no
+            # gradient; out-of-place products alone, so that a batch of gradients can run through: is_grads_batched)
+            inputs, grads = ctx.saved_tensors[:3], ctx.saved_tensors[3:]
+            go = gout.to(torch.float64).reshape(1)
+            return tuple((g.to(x.device) * go.to(x.device)).to(x.dtype) if wanted else None
+                         for x, g, wanted in zip(inputs, grads, ctx.needs_input_grad)) + (None,)
 
     return PoissonNll
 
@@ -175,7 +172,7 @@ def _poisson_function():
 def poisson_nll(model: NllModel, params, bg, zern, counts, frame):
     """The NLL as a differentiable torch scalar (float64) in params (n, 4), bg (F,) and zern (J,)."""
     import torch
-    grad = torch.is_grad_enabled() and any(t.requires_grad for t in (params, bg, zern))
+    grad = torch.is_grad_enabled() and any(getattr(t, "requires_grad", False) for t in (params, bg, zern))
     return _poisson_function().apply(params, bg, zern, (model, counts, frame, grad))
 
 
