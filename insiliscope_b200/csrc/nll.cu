@@ -245,7 +245,7 @@ __device__ __forceinline__ void Pixels(const NllArgs& a, uint32_t e, const int (
 // constants by broadcast -- a warp's t or q group is the same for its lanes, and such a 16-byte read takes two -- and its
 // data once per lane), then the float64 logarithm of each pixel. 128 threads and 55 KB, four CTAs per SM, so that one
 // CTA's products run under another's logarithms and barriers. 256,000 emitters of 32 x 32 px, os = 2: likelihood and
-// gradients 7.6 ms (unfolded 23.3), the likelihood alone 3.65 (11.6). Constants as kernel parameters were slower (the
+// gradients 7.7 ms (unfolded 23.3), the likelihood alone 3.7 (11.6). Constants as kernel parameters were slower (the
 // two passes 14.0 ms against 11.7).
 template <bool kGrad, int OS>
 __global__ void __launch_bounds__(kThreads, kCtasPerSm) NllKernel(NllArgs a)
@@ -287,9 +287,11 @@ __global__ void __launch_bounds__(kThreads, kCtasPerSm) NllKernel(NllArgs a)
             for (int ix = 0; ix < 2; ++ix)
             {
                const int m = m0 + (iy ? -qy : qy) * kM + (ix ? -qx : qx);
-               const double ph = ReduceTwoPi(zk + a.zphase[m] - ((ix ? -ax : ax) + (iy ? -ay : ay)));
+               // in revolutions, less the whole ones. (The fast sine and cosine, 2^-21 off, were half of the gradients'
+               // error; the folded products' own roundings are the other half.)
+               const double ph = (zk + a.zphase[m] - ((ix ? -ax : ax) + (iy ? -ay : ay))) * 0.15915494309189533577;
                float sn, cs;
-               __sincosf(static_cast<float>(ph), &sn, &cs);
+               sincospif(2.f * static_cast<float>(ph - rint(ph)), &sn, &cs);
                const float am = (iy && qy == 0) || (ix && qx == 0) ? 0.f : amp;   // one sample on an axis, not two
                u[iy][ix] = make_float2(am * cs, am * sn);
             }
