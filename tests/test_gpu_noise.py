@@ -112,3 +112,56 @@ def test_float_decisions_bit_exact(engine, oracle, name):
         if gain is not None:
             diff.reshape(-1)[3] = False              # a zero gain's ADU is not a number
         assert not diff.any(), (k, int(diff.sum()), ph[k][diff][:4], got[k][diff][:4], want[diff][:4])
+
+
+@pytest.mark.parametrize("gain,em_gain,read,depth", [(1.0, 300.0, 50.0, 16), (0.05, 4.0, 30.0, 14), (40.0, 1.0, 200.0, 16),
+                                                     (-3.0, 20.0, 5.0, 12)])
+def test_bright_emccd_bit_exact(engine, oracle, gain, em_gain, read, depth):
+    """EMCCD means from 150 to 3e6 photons, dense around the 512 electrons from which the register is worked out in
+    float64 and around the million from which the whole chain is, clamped and not: every ADU the CPU chain's."""
+    import torch
+    rng = np.random.default_rng(int(abs(gain) * 100) + depth)
+    W, H, n = 203, 101, 8
+    ph = 10.0 ** rng.uniform(np.log10(150.0), np.log10(3e6), (n, H, W))
+    ph[1] = rng.uniform(480.0, 620.0, (H, W))
+    ph[2] = 10.0 ** rng.uniform(5.99, 6.01, (H, W))
+    ph[3:5] = rng.uniform(2000.0, 30000.0, (2, H, W))
+    ph = ph.astype(np.float32)
+    off = rng.uniform(-2000.0, 3000.0, W * H).astype(np.float32)
+    cam = CameraParams(quantum_efficiency=0.93, dark_electrons=0.01, gain=gain, read_noise_e=read, emccd=True,
+                       em_gain=em_gain, cic_electrons=0.005, bit_depth=depth)
+    engine.set_static(W, H, pixel_base=W, offset=off, flat_bg=0.0)
+    frames = [3, 77, 2**31 + 1, 4, 5, 6, 7, 8]
+    got = engine.noise_frames_dev(torch.from_numpy(ph).cuda(), frames, cam, 311).cpu().numpy()
+    for k in range(n):
+        want = oracle.noise_chain(ph[k], cam, off.reshape(H, W), None, None, 311, frames[k], pixel_base=W)
+        assert np.array_equal(got[k], want), (k, int((got[k] != want).sum()))
+
+
+def _noise_us(engine, mean, cam):
+    """The noise of 8 frames of 512 x 512 px at a mean, in us by the device's clock (the best of ten)."""
+    import torch
+    W, n = 512, 8
+    engine.set_static(W, W, flat_bg=0.0)
+    ph = mean * (0.8 + 0.4 * torch.rand((n, W, W), generator=torch.Generator(device="cuda").manual_seed(1), device="cuda"))
+    fr = torch.arange(n, dtype=torch.int32, device="cuda")
+    out = torch.empty((n, W, W), dtype=torch.uint16, device="cuda")
+    best = 1e9
+    with torch.cuda.stream(engine.torch_stream()):
+        for _ in range(10):
+            a, b = (torch.cuda.Event(enable_timing=True) for _ in range(2))
+            a.record()
+            engine.noise_frames_dev(ph, fr, cam, 7, out=out, sync=False)
+            b.record()
+            b.synchronize()
+            best = min(best, a.elapsed_time(b) * 1e3)
+    return best
+
+
+def test_bright_emccd_frames_take_no_longer(engine):
+    """The chain's float32 bounds grow with the electrons; bright frames must not fall through to the float64 chain."""
+    cam = CameraParams(quantum_efficiency=0.95, gain=1.0, read_noise_e=50.0, emccd=True, em_gain=300.0,
+                       cic_electrons=0.002)
+    dim = _noise_us(engine, 300.0, cam)
+    for mean in (1e3, 6e3, 1.9e4, 3e4, 2e5):
+        assert _noise_us(engine, mean, cam) <= 1.6 * dim, mean
