@@ -230,8 +230,9 @@ __device__ __forceinline__ uint16_t NoisePixel(float photonValue, uint32_t i, co
    const uint32_t seed = u.seed, frame = u.frame, pix = i + st.pixelBase;
    const float readF = st.readNoise ? st.readNoise[i] : cam.readF, gainF = st.gain ? st.gain[i] : cam.gainF,
                offF = st.offset ? st.offset[i] : 0.f;
-   // lambda within 3 roundings (1.8e-7 relative) of the float64 mean: its terms are not negative
-   const float lf = fmaxf(photonValue, 0.f) * cam.qeF + cam.addF;
+   // lambda within 3 roundings (1.8e-7 relative) of the float64 mean: its terms are not negative. (A camera without
+   // float32 bounds: NaN, which no float32 branch below takes -- the Knuth loop for nothing had cost it a third.)
+   const float lf = cam.fast ? fmaxf(photonValue, 0.f) * cam.qeF + cam.addF : __int_as_float(0x7fc00000);
    bool ok = cam.fast != 0;
    float ne = 0.f;
    uint32_t pos = 0;          // words of the stream consumed
@@ -275,7 +276,7 @@ __device__ __forceinline__ uint16_t NoisePixel(float photonValue, uint32_t i, co
          g2 = o3 ? x[1] : (o2 ? x[0] : (o1 ? w[3] : w[2]));
       }
    }
-   else
+   else if (ok)
    {
       uint32_t w[4];
       H.At(frame, 0, w);

@@ -165,3 +165,10 @@ def test_bright_emccd_frames_take_no_longer(engine):
     dim = _noise_us(engine, 300.0, cam)
     for mean in (1e3, 6e3, 1.9e4, 3e4, 2e5):
         assert _noise_us(engine, mean, cam) <= 1.6 * dim, mean
+
+
+def test_cameras_without_float_bounds_skip_the_float_chain(engine):
+    """A camera that the float32 bounds do not hold for (here a negative dark current) takes the float64 chain alone: one
+    and a half times the float32 chain's time, twice with both."""
+    fast = _noise_us(engine, 20.0, CameraParams(gain=2.2, read_noise_e=1.5, dark_electrons=0.5))
+    assert _noise_us(engine, 20.0, CameraParams(gain=2.2, read_noise_e=1.5, dark_electrons=-0.5)) <= 1.75 * fast
