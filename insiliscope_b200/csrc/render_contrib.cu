@@ -49,6 +49,15 @@ struct KeyMap
    int lo[ISCU_MAX_KERNELS];
    int n1[ISCU_MAX_KERNELS];
    int side[ISCU_MAX_KERNELS];   // splat square side, 2 camRad + 1
+   int pbs[ISCU_MAX_KERNELS];    // pixel blocks of the square: a chunk's work items
+};
+
+// The contribution pass's work list (the last CTA of the setup writes it): the items' total, the next item, and each
+// slot's first chunk and first item. A slot's keys, so its chunks and items, are consecutive.
+struct Work
+{
+   uint32_t items, next;
+   uint32_t chunk[ISCU_MAX_KERNELS], item[ISCU_MAX_KERNELS];
 };
 
 __device__ __forceinline__ int TapsOf(const KernelView& kv)
@@ -69,7 +78,7 @@ struct SetupArgs
    uint32_t* start;   // the offsets (ScanKeys)
    uint32_t* cursor;
    uint32_t* chunkStart;
-   uint32_t* ctr;
+   Work* work;
 };
 
 // An emitter's slot, SplatSetup and key (false: not splatted).
@@ -91,16 +100,16 @@ __device__ __forceinline__ bool SetupEmitter(const Kernels& K, const KeyMap& km,
 }
 
 // 2. The offsets, by one CTA of kSetupThreads threads, kScanPer consecutive keys a thread and pass: start[k] = cursor[k] =
-// exclusive sum of count, chunkStart[k] = exclusive sum of the keys' chunks (ceil(count / kE)); ctr[0] = the chunks'
-// total; ctr[1] = 0. (The chunks' records are written by the scatter: one thread listing all of a key's work in turn
-// took 14 of 26 us on the two-colour movie.)
+// exclusive sum of count, chunkStart[k] = exclusive sum of the keys' chunks (ceil(count / kE)); the work list. (The
+// chunks' records are written by the scatter: one thread listing all of a key's work in turn took 14 of 26 us on the
+// two-colour movie.)
 constexpr int kSetupThreads = 512, kScanPer = 8;
 __device__ __forceinline__ void ScanKeys(const SetupArgs& a)
 {
    constexpr int kWarps = kSetupThreads / 32;
    const int nKeys = a.km.base[ISCU_MAX_KERNELS];
    const int lane = threadIdx.x & 31, warp = threadIdx.x >> 5;
-   __shared__ uint32_t sw[2][kWarps];
+   __shared__ uint32_t sw[2][kWarps], firstChunk[ISCU_MAX_KERNELS + 1];
    uint32_t carryC = 0, carryI = 0;
    for (int k0 = 0; k0 < nKeys; k0 += kSetupThreads * kScanPer)
    {
@@ -152,15 +161,31 @@ __device__ __forceinline__ void ScanKeys(const SetupArgs& a)
             a.start[k] = ec;
             a.cursor[k] = ec;
             a.chunkStart[k] = ei;
+#pragma unroll
+            for (int t = 0; t < ISCU_MAX_KERNELS; ++t)
+               if (k == a.km.base[t])
+                  firstChunk[t] = ei;
          }
          ec += c[j];
          ei += it[j];
       }
    }
+   __syncthreads();
    if (threadIdx.x == 0)
    {
-      a.ctr[0] = carryI;
-      a.ctr[1] = 0;
+      firstChunk[ISCU_MAX_KERNELS] = carryI;
+      for (int t = ISCU_MAX_KERNELS; t-- > 0;)
+         if (a.km.base[t] == a.km.base[t + 1])
+            firstChunk[t] = firstChunk[t + 1];   // a slot without keys
+      uint32_t items = 0;
+      for (int t = 0; t < ISCU_MAX_KERNELS; ++t)
+      {
+         a.work->chunk[t] = firstChunk[t];
+         a.work->item[t] = items;
+         items += (firstChunk[t + 1] - firstChunk[t]) * static_cast<uint32_t>(a.km.pbs[t]);
+      }
+      a.work->items = items;
+      a.work->next = 0;
    }
 }
 
@@ -323,8 +348,7 @@ struct ContribArgs
    Kernels K;
    const CChunk* chunk;
    const CStage* stage;  // the emitters in group order
-   uint32_t* ctr;        // [0] chunks, [1] the next work item
-   uint32_t blocks;      // pixel blocks of the largest square: work items per chunk
+   Work* work;
    float* contrib;       // emitter g's square at contrib[g S ..]
    uint32_t S;
 };
@@ -470,7 +494,9 @@ __device__ __forceinline__ void GroupContrib(const ContribArgs& a, const KernelV
 // has item i + 1's emitters arriving, issues item i + 2's copy, whose chunk it asked for an item ago, and asks for item
 // i + 3's chunk and number i + 4, so that each of these round trips has an item's time. (Fetched one after the other
 // within an item they took longer than a short item's work.) An item is one block of computing threads' pixels of a
-// chunk.
+// chunk, as many a chunk as its own slot's square has (as many as the largest square of all slots, 120,000 emitters of
+// 7 x 7 squares beside a stack of 81 x 81 took 205 us instead of 46). The two roles have a loop each: in one loop the
+// staging warp's variables made the others spill (118.8 us for the dSTORM movie's 35 M contributions, 114.7 without).
 //
 // What bounds it: the emitter loop, 86 cycles a warp's contribution and scheduler where its 20 float64 operations and
 // the conversion need 56 (a float64 operation issues every 2.35 cycles, a conversion takes 8.5); 54 instructions in all,
@@ -478,32 +504,49 @@ __device__ __forceinline__ void GroupContrib(const ContribArgs& a, const KernelV
 // contributions of the dSTORM movie 136 -> 122 us, 484 M of the two-colour movie 1.55 -> 1.27 ms against unfused sums
 // with each thread's own tap offsets. Building the float from the double's bits instead of converting, and two or four
 // emitters without a branch between them, measured 5 to 40 % slower (more integer instructions; spilled taps).
+// All of the CTA's warps, from either role's loop.
+__device__ __forceinline__ void RoleBarrier() { asm volatile("bar.sync 0;" ::: "memory"); }
+
 __global__ void __launch_bounds__(kMaxCT + 32, kContribPerSm) ContribKernel(ContribArgs a)
 {
    __shared__ CStage sE[3][kE];
    __shared__ CChunk sChunk[3];
-   __shared__ uint32_t sItem[3];
+   __shared__ uint32_t sBlock[3];   // the items' pixel blocks; kNoItem: none is left
+   constexpr uint32_t kNoItem = 0xFFFFFFFFu;
    const int nc = static_cast<int>(blockDim.x) - 32;   // computing threads
    const bool stager = static_cast<int>(threadIdx.x) >= nc;
    const int sl = static_cast<int>(threadIdx.x) - nc;  // lane of the staging warp
-   const uint32_t items = a.ctr[0] * a.blocks;
+   const uint32_t items = a.work->items;
    constexpr int kHead = static_cast<int>(sizeof(CChunk) / 16), kRec = static_cast<int>(sizeof(CStage) / 16);
-   uint32_t ahead = 0, asked = 0;      // lane 0: the number asked for; the item whose chunk is on its way
+   uint32_t ahead = 0, asked = 0, block = 0;   // lane 0: the number asked for; the item whose chunk is on its way
    int4 head = make_int4(0, 0, 0, 0);  // that chunk's 16 bytes of this lane
    // (a CTA's first three items are its own; the counter hands out the rest)
    auto number = [&] {
       if (sl == 0)
-         ahead = 3 * gridDim.x + atomicAdd(&a.ctr[1], 1u);
+         ahead = 3 * gridDim.x + atomicAdd(&a.work->next, 1u);
    };
-   auto chunk = [&](uint32_t i) {
+   // lane t holds slot t's first item, first chunk and items per chunk
+   uint32_t item0 = 0xFFFFFFFFu, chunk0 = 0, per = 1;
+   if (stager && sl < ISCU_MAX_KERNELS)
+   {
+      item0 = a.work->item[sl];
+      chunk0 = a.work->chunk[sl];
+      per = static_cast<uint32_t>(max(1, a.km.pbs[sl]));
+   }
+   auto chunk = [&](uint32_t i, uint32_t& block) {
+      // the last slot whose items start at or before i (those that share its start have none)
+      const int slot = 31 - __clz(static_cast<int>(__ballot_sync(0xffffffffu, i >= item0)));
+      const uint32_t in = i - __shfl_sync(0xffffffffu, item0, slot), n = __shfl_sync(0xffffffffu, per, slot);
+      const uint32_t c = in / n, at = __shfl_sync(0xffffffffu, chunk0, slot) + c;
+      block = in - c * n;
       int4 h = make_int4(0, 0, 0, 0);
       if (i < items && sl < kHead)
-         h = __ldg(reinterpret_cast<const int4*>(a.chunk + i / a.blocks) + sl);
+         h = __ldg(reinterpret_cast<const int4*>(a.chunk + at) + sl);
       return h;
    };
-   auto copy = [&](int buf, uint32_t i, const int4& h) {
+   auto copy = [&](int buf, uint32_t i, uint32_t block, const int4& h) {
       if (sl == 0)
-         sItem[buf] = i;
+         sBlock[buf] = i < items ? block : kNoItem;
       if (i < items)
       {
          if (sl < kHead)
@@ -522,62 +565,63 @@ __global__ void __launch_bounds__(kMaxCT + 32, kContribPerSm) ContribKernel(Cont
       number();
       const uint32_t i0 = blockIdx.x, i1 = i0 + gridDim.x;
       asked = i1 + gridDim.x;
-      const int4 h0 = chunk(i0), h1 = chunk(i1);
-      head = chunk(asked);
-      copy(0, i0, h0);
-      copy(1, i1, h1);
+      uint32_t b0, b1;
+      const int4 h0 = chunk(i0, b0), h1 = chunk(i1, b1);
+      head = chunk(asked, block);
+      copy(0, i0, b0, h0);
+      copy(1, i1, b1, h1);
       asm volatile("cp.async.wait_group 1;" ::: "memory");
-   }
-   __syncthreads();
-   for (int cur = 0;; cur = cur == 2 ? 0 : cur + 1)
-   {
-      const uint32_t item = sItem[cur];
-      if (item >= items)
-         return;
-      if (stager)
+      RoleBarrier();
+      for (int cur = 0; sBlock[cur] != kNoItem; cur = cur == 2 ? 0 : cur + 1)
       {
-         copy(cur == 0 ? 2 : cur - 1, asked, head);   // item i + 2 (the buffer of item i - 1, done)
+         copy(cur == 0 ? 2 : cur - 1, asked, block, head);   // item i + 2 (the buffer of item i - 1, done)
          asked = __shfl_sync(0xffffffffu, ahead, 0);
-         head = chunk(asked);
+         head = chunk(asked, block);
          number();
          asm volatile("cp.async.wait_group 1;" ::: "memory");   // item i + 1 is there
+         RoleBarrier();
       }
-      else
+      return;
+   }
+   RoleBarrier();
+   for (int cur = 0;; cur = cur == 2 ? 0 : cur + 1)
+   {
+      const uint32_t pixels = sBlock[cur];
+      if (pixels == kNoItem)
+         return;
+      const CChunk& it = sChunk[cur];
+      const int slot = it.slot;
+      const KernelView& kv = a.K.k[slot];
+      const int side = a.km.side[slot], cr = kv.camRad;
+      const int p = static_cast<int>(pixels) * nc + static_cast<int>(threadIdx.x);
+      const bool inSquare = p < side * side;
+      // p / side: the quotient's fraction is at least half a 1 / side from a whole number, the float product's error
+      // below that for squares of up to 4 M pixels; larger ones divide
+      int row = static_cast<int>((static_cast<float>(p) + 0.5f) * it.invSide);
+      if (side > 2000)
+         row = p / side;
+      const int dx = inSquare ? p - row * side - cr : 0, dy = inSquare ? row - cr : 0;
+      const int nt = TapsOf(kv);
+      const CStage* E = sE[cur];
+      if (__any_sync(0xffffffffu, inSquare))
       {
-         const CChunk& it = sChunk[cur];
-         const int slot = it.slot;
-         const KernelView& kv = a.K.k[slot];
-         const int side = a.km.side[slot], cr = kv.camRad;
-         const int p = static_cast<int>(item % a.blocks) * nc + static_cast<int>(threadIdx.x);
-         const bool inSquare = p < side * side;
-         // p / side: the quotient's fraction is at least half a 1 / side from a whole number, the float product's error
-         // below that for squares of up to 4 M pixels; larger ones divide
-         int row = static_cast<int>((static_cast<float>(p) + 0.5f) * it.invSide);
-         if (side > 2000)
-            row = p / side;
-         const int dx = inSquare ? p - row * side - cr : 0, dy = inSquare ? row - cr : 0;
-         const int nt = TapsOf(kv);
-         const CStage* E = sE[cur];
-         if (__any_sync(0xffffffffu, inSquare))
+         const bool active = inSquare && (it.kind == 0 || HaloKeeps(kv, it.plane, dx, dy));
+         if (it.kind == 0)
          {
-            const bool active = inSquare && (it.kind == 0 || HaloKeeps(kv, it.plane, dx, dy));
-            if (it.kind == 0)
-            {
-               // the misc group: every emitter with its own plane and tap origin
-               for (int k = 0; k < it.cnt; ++k)
-                  if (inSquare && HaloKeeps(kv, E[k].plane, dx, dy))
-                     a.contrib[static_cast<size_t>(E[k].g) * a.S + p] =
-                        static_cast<float>(E[k].photons * BoundedTaps(kv, E[k], nt, dx, dy));
-            }
-            else if (nt == 4)
-               GroupContrib<4>(a, kv, it, E, p, dx, dy, active);
-            else if (nt == 2)
-               GroupContrib<2>(a, kv, it, E, p, dx, dy, active);
-            else
-               GroupContrib<1>(a, kv, it, E, p, dx, dy, active);
+            // the misc group: every emitter with its own plane and tap origin
+            for (int k = 0; k < it.cnt; ++k)
+               if (inSquare && HaloKeeps(kv, E[k].plane, dx, dy))
+                  a.contrib[static_cast<size_t>(E[k].g) * a.S + p] =
+                     static_cast<float>(E[k].photons * BoundedTaps(kv, E[k], nt, dx, dy));
          }
+         else if (nt == 4)
+            GroupContrib<4>(a, kv, it, E, p, dx, dy, active);
+         else if (nt == 2)
+            GroupContrib<2>(a, kv, it, E, p, dx, dy, active);
+         else
+            GroupContrib<1>(a, kv, it, E, p, dx, dy, active);
       }
-      __syncthreads();
+      RoleBarrier();
    }
 }
 
@@ -860,7 +904,7 @@ namespace {
 struct ContribGeometry
 {
    KeyMap km = {};
-   int nKeys = 0, ct = 32, blocks = 1;   // computing threads of a contribution CTA; its blocks of the largest square
+   int nKeys = 0, ct = 32;   // computing threads of a contribution CTA
    size_t S = 1;
 };
 
@@ -882,8 +926,10 @@ ContribGeometry GeometryOf(const iscu_ctx* ctx)
       maxS2 = std::max(maxS2, side * side);
    }
    G.km.base[ISCU_MAX_KERNELS] = G.nKeys;
-   G.blocks = (maxS2 + kMaxCT - 1) / kMaxCT;
-   G.ct = std::min(kMaxCT, ((maxS2 + G.blocks - 1) / G.blocks + 31) / 32 * 32);
+   const int blocks = (maxS2 + kMaxCT - 1) / kMaxCT;   // of the largest square
+   G.ct = std::min(kMaxCT, ((maxS2 + blocks - 1) / blocks + 31) / 32 * 32);
+   for (int s = 0; s < ISCU_MAX_KERNELS; ++s)
+      G.km.pbs[s] = (G.km.side[s] * G.km.side[s] + G.ct - 1) / G.ct;
    G.S = static_cast<size_t>(maxS2);
    return G;
 }
@@ -916,7 +962,7 @@ int ReserveContrib(iscu_ctx* ctx, uint32_t nEm, ContribScratch& sc)
    ISCU_CK(sc.contrib.Reserve(std::max<size_t>(contribBytes, 16)));
    ISCU_CK(sc.keys.Reserve((4 * static_cast<size_t>(G.nKeys) + 1) * sizeof(uint32_t)));
    ISCU_CK(sc.chunks.Reserve(MaxChunks(G, nEm) * sizeof(CChunk)));
-   ISCU_CK(sc.ctr.Reserve(4 * sizeof(uint32_t)));
+   ISCU_CK(sc.ctr.Reserve(sizeof(Work)));
    return ISCU_OK;
 }
 
@@ -945,7 +991,7 @@ int LaunchContribRender(iscu_ctx* ctx, int tileConfig, const iscu_emitter* ems, 
    {
       ISCU_CK(cudaMemsetAsync(count, 0, (static_cast<size_t>(nKeys) + 1) * sizeof(uint32_t), ctx->stream));
       SetupArgs sa{ems,   nEm,   K,      km,         sc.rec.as<int>(), sc.grec.as<int4>(),
-                   count, start, cursor, chunkStart, sc.ctr.as<uint32_t>()};
+                   count, start, cursor, chunkStart, sc.ctr.as<Work>()};
       ContribSetupKernel<<<(nEm + kSetupThreads - 1) / kSetupThreads, kSetupThreads, 0, ctx->stream>>>(sa);
       ISCU_CK_LAUNCH(ctx, "ContribSetupKernel");
       if (nKeys > 0)
@@ -956,8 +1002,8 @@ int LaunchContribRender(iscu_ctx* ctx, int tileConfig, const iscu_emitter* ems, 
          ISCU_CK_LAUNCH(ctx, "ContribScatterKernel");
          if (marks)
             ISCU_CK(cudaEventRecord(marks[1], ctx->stream));
-         ContribArgs ca{km, K, sc.chunks.as<CChunk>(), sc.list.as<CStage>(), sc.ctr.as<uint32_t>(),
-                        static_cast<uint32_t>(G.blocks), sc.contrib.as<float>(), static_cast<uint32_t>(S)};
+         ContribArgs ca{km, K, sc.chunks.as<CChunk>(), sc.list.as<CStage>(), sc.ctr.as<Work>(),
+                        sc.contrib.as<float>(), static_cast<uint32_t>(S)};
          ContribKernel<<<kContribPerSm * ctx->smCount, G.ct + 32, 0, ctx->stream>>>(ca);
          ISCU_CK_LAUNCH(ctx, "ContribKernel");
       }

@@ -293,3 +293,48 @@ def test_small_batches_equal_the_one_emitter_step(engine, per):
     for got in out[1:]:
         assert np.array_equal(got[0].view(np.uint32), out[0][0].view(np.uint32))
         assert np.array_equal(got[1], out[0][1])
+
+
+def _mixed_squares(engine, big_half, per, frames):
+    """A movie whose emitters are all of a 7 x 7-square stack, beside a stack of squares of big_half (0: alone): device
+    emitters and frames, after the stacks are set."""
+    import torch
+    rng = np.random.default_rng(3)
+    planes = rng.uniform(0.0, 1e-3, (5, 25, 25)).astype(np.float32)
+    if big_half:
+        n = 4 * big_half + 1
+        engine.kernel_set_planes(0, rng.uniform(0.0, 1e-5, (3, n, n)).astype(np.float32), 2, 25.0, INTERP_CUBIC)
+    engine.kernel_set_planes(1 if big_half else 0, planes, 4, 25.0, INTERP_CUBIC)
+    n = per * frames
+    em = np.zeros(n, EMITTER_DTYPE)
+    em["x_px"], em["y_px"] = rng.uniform(-1.0, 100.0, (2, n))
+    em["photons"] = rng.uniform(100.0, 3000.0, n)
+    em["plane"] = rng.integers(0, 5, n) + (65536 if big_half else 0)
+    engine.set_static(100, 100, flat_bg=20.0)
+    return [torch.from_numpy(a.view(np.uint8)).cuda() for a in (em, frames_table(np.full(frames, per)))]
+
+
+def test_small_squares_beside_large_ones():
+    """The contributions of a stack of small squares take no more work for a stack of large squares in another slot that
+    no emitter is of, and are the one-pass form's bits."""
+    import torch
+    from insiliscope_b200 import Engine
+    times = {}
+    for half in (0, 40):
+        with Engine(0) as engine:
+            dem, dfr = _mixed_squares(engine, half, 500, 150)
+            cam, out = CameraParams(gain=2.0, read_noise_e=1.5), {}
+            for config in (0, 12):
+                engine.set_render_config(config)
+                ph = torch.empty((150, 100, 100), dtype=torch.float32, device="cuda")
+                adu = torch.empty((150, 100, 100), dtype=torch.uint16, device="cuda")
+                best = 1e9
+                for _ in range(6):
+                    engine.set_render_timing(True)
+                    engine.render_frames_dev(dem, dfr, 150, cam, 5, ph, adu)
+                    best = min(best, engine.render_pass_times()[0]["contributions"])
+                engine.set_render_timing(False)
+                out[config], times[half] = (ph.cpu().numpy(), adu.cpu().numpy()), best
+            assert np.array_equal(out[0][0].view(np.uint32), out[12][0].view(np.uint32))
+            assert np.array_equal(out[0][1], out[12][1])
+    assert times[40] <= 1.5 * times[0], times
