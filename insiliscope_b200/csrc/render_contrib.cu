@@ -232,7 +232,8 @@ struct __align__(16) CStage
 {
    double wx[4], wp[4];   // the column weights; the row weights times the photons
    uint32_t g;
-   float thr;             // 2^-10 x 1.6 photons: below thr x the taps' largest magnitude a sum cancels too much
+   float thr;             // 2^-10 x 1.6 photons: below thr x the taps' largest magnitude a sum cancels too much;
+                          // infinite (every sum in doubt) where that is no normal float
    int bx, by;
    double photons;
    double wy[4];
@@ -300,6 +301,8 @@ __global__ void ContribScatterKernel(ScatterArgs a)
    }
    c.photons = em.photons;
    c.thr = static_cast<float>(em.photons * (1.6 / 1024.0));
+   if (!(c.thr >= 1.17549435e-38f))
+      c.thr = __int_as_float(0x7f800000);   // (no float bound of so few photons)
    c.g = g;
    c.bx = s.bx;
    c.by = s.by;
