@@ -368,3 +368,40 @@ def test_cancelling_taps_at_extreme_photons():
                 out.append(ph.cpu().numpy().view(np.uint32))
             assert (out[0] != 0).any()
             assert np.array_equal(*out), (photons, int((out[0] != out[1]).sum()))
+
+
+def test_steep_stacks_take_no_second_sum():
+    """A Gaussian stack whose far samples fall by more than the fused sums' bound allows takes about a slowly falling
+    stack's time for its contributions (each sum once, in the reference's order), and gives the one-pass bits."""
+    import torch
+    from insiliscope_b200 import Engine
+    rng = np.random.default_rng(31)
+    half, os_, frames, per = 16, 4, 150, 160
+    n = 2 * half * os_ + 1
+    y, x = np.mgrid[0:n, 0:n] - (n - 1) / 2.0
+    r2 = (x * x + y * y) / (1.2 * os_) ** 2
+    em = np.zeros(frames * per, EMITTER_DTYPE)
+    em["x_px"], em["y_px"] = rng.uniform(-0.5, 127.5, (2, len(em)))
+    em["photons"], em["plane"] = 2000.0 * np.exp(0.5 * rng.standard_normal(len(em))), rng.integers(0, 25, len(em))
+    dem, dfr = (torch.from_numpy(t.view(np.uint8)).cuda() for t in (em, frames_table(np.full(frames, per))))
+    cam, times = CameraParams(gain=2.0, read_noise_e=1.5), {}
+    for name, plane in (("steep", np.exp(-0.5 * r2)), ("slow", (1.0 + r2) ** -1.5)):
+        with Engine(0) as eng:
+            eng.kernel_set_planes(0, np.repeat((plane / plane.sum())[None], 25, 0).astype(np.float32), os_, 25.0,
+                                  INTERP_CUBIC)
+            eng.set_static(128, 128, flat_bg=0.0)
+            out = []
+            for config in (0, 12):
+                eng.set_render_config(config)
+                ph = torch.empty((frames, 128, 128), dtype=torch.float32, device="cuda")
+                adu = torch.empty((frames, 128, 128), dtype=torch.uint16, device="cuda")
+                best = 1e9
+                for _ in range(6):
+                    eng.set_render_timing(True)
+                    eng.render_frames_dev(dem, dfr, frames, cam, 5, ph, adu)
+                    best = min(best, eng.render_pass_times()[0]["contributions"])
+                eng.set_render_timing(False)
+                out.append(ph.cpu().numpy().view(np.uint32))
+                times[name] = best
+            assert np.array_equal(*out), name
+    assert times["steep"] <= 1.45 * times["slow"], times
