@@ -177,11 +177,11 @@ struct StaticView
    uint32_t width = 0, height = 0, pixelBase = 0;
 };
 
-// Device scratch of the two-pass render (render_contrib.cu): per-emitter setup records, the (slot, plane, tap
-// origin) groups, and every emitter's float contribution to each pixel of its square.
+// Device scratch of the two-pass render (render_contrib.cu): per-emitter keys and positions, the (slot, plane, tap
+// origin) groups' lists, and every emitter's float contribution to each pixel of its square.
 struct ContribScratch
 {
-   DevBuf rec, grec, keys, list, chunks, contrib, ctr;
+   DevBuf buf;
 };
 
 // One I/O slot of the event render (iscu_render_events[_async]): the batch's device staging (events, bucket and

@@ -974,6 +974,24 @@ size_t MaxChunks(const ContribGeometry& G, uint32_t nEm)
    return std::min<size_t>(nEm, static_cast<size_t>(nEm) / kE + static_cast<size_t>(G.nKeys)) + 1;
 }
 
+// The scratch of nEm emitters: one buffer's parts, each on 256 bytes.
+struct ContribLayout
+{
+   size_t key = 0, grec, keys, list, chunks, work, contrib, bytes;
+   ContribLayout(const ContribGeometry& G, uint32_t nEm)
+   {
+      const size_t n = std::max<uint32_t>(nEm, 1u);
+      const auto after = [](size_t at, size_t size) { return (at + size + 255) / 256 * 256; };
+      grec = after(key, n * sizeof(int));
+      keys = after(grec, n * sizeof(int4));
+      list = after(keys, (4 * static_cast<size_t>(G.nKeys) + 1) * sizeof(uint32_t));
+      chunks = after(list, n * sizeof(CStage));
+      work = after(chunks, MaxChunks(G, nEm) * sizeof(CChunk));
+      contrib = after(work, sizeof(Work));
+      bytes = after(contrib, n * G.S * sizeof(float));
+   }
+};
+
 } // namespace
 
 int ReserveContrib(iscu_ctx* ctx, uint32_t nEm, ContribScratch& sc)
@@ -989,14 +1007,17 @@ int ReserveContrib(iscu_ctx* ctx, uint32_t nEm, ContribScratch& sc)
    if (contribBytes > ctx->contribLimit)
       return Fail(ISCU_ERR_LIMIT, "two-pass render: contributions of " + std::to_string(nEm) + " emitters need " +
                                      std::to_string(contribBytes >> 20) + " MiB, over the limit");
-   const size_t n = std::max<uint32_t>(nEm, 1u);
-   ISCU_CK(sc.rec.Reserve(n * sizeof(int)));
-   ISCU_CK(sc.grec.Reserve(n * sizeof(int4)));
-   ISCU_CK(sc.list.Reserve(n * sizeof(CStage)));
-   ISCU_CK(sc.contrib.Reserve(std::max<size_t>(contribBytes, 16)));
-   ISCU_CK(sc.keys.Reserve((4 * static_cast<size_t>(G.nKeys) + 1) * sizeof(uint32_t)));
-   ISCU_CK(sc.chunks.Reserve(MaxChunks(G, nEm) * sizeof(CChunk)));
-   ISCU_CK(sc.ctr.Reserve(sizeof(Work)));
+   if (ContribLayout(G, nEm).bytes <= sc.buf.bytes && sc.buf.p)
+      return ISCU_OK;
+   // Room for some more emitters than asked for, so that a movie's batches, a few emitters apart, are not each the first
+   // pass of a larger buffer (an allocation and a free wait for the device: 0.1 to 5 ms): a 32nd at first, an eighth when
+   // it grows, within the limit.
+   const uint64_t most = ctx->contribLimit / (G.S * sizeof(float));
+   const uint64_t more = std::min<uint64_t>(std::min<uint64_t>(most, 0xFFFFFFFFu), nEm + nEm / (sc.buf.p ? 8u : 32u));
+   if (more > nEm && sc.buf.Reserve(ContribLayout(G, static_cast<uint32_t>(more)).bytes) == cudaSuccess)
+      return ISCU_OK;
+   cudaGetLastError();
+   ISCU_CK(sc.buf.Reserve(ContribLayout(G, nEm).bytes));
    return ISCU_OK;
 }
 
@@ -1016,7 +1037,15 @@ int LaunchContribRender(iscu_ctx* ctx, int tileConfig, const iscu_emitter* ems, 
    cudaEvent_t* marks = RenderMarks(ctx);
    if (marks)
       ISCU_CK(cudaEventRecord(marks[0], ctx->stream));
-   uint32_t* count = sc.keys.as<uint32_t>();   // and the CTAs done
+   const ContribLayout L(G, nEm);
+   unsigned char* base = sc.buf.as<unsigned char>();
+   int* key = reinterpret_cast<int*>(base + L.key);
+   int4* grec = reinterpret_cast<int4*>(base + L.grec);
+   CStage* list = reinterpret_cast<CStage*>(base + L.list);
+   CChunk* chunks = reinterpret_cast<CChunk*>(base + L.chunks);
+   Work* work = reinterpret_cast<Work*>(base + L.work);
+   float* contrib = reinterpret_cast<float*>(base + L.contrib);
+   uint32_t* count = reinterpret_cast<uint32_t*>(base + L.keys);   // and the CTAs done
    uint32_t* start = count + nKeys + 1;
    uint32_t* cursor = start + nKeys;
    uint32_t* chunkStart = cursor + nKeys;
@@ -1024,20 +1053,17 @@ int LaunchContribRender(iscu_ctx* ctx, int tileConfig, const iscu_emitter* ems, 
    if (nEm > 0)
    {
       ISCU_CK(cudaMemsetAsync(count, 0, (static_cast<size_t>(nKeys) + 1) * sizeof(uint32_t), ctx->stream));
-      SetupArgs sa{ems,   nEm,   K,      km,         sc.rec.as<int>(), sc.grec.as<int4>(),
-                   count, start, cursor, chunkStart, sc.ctr.as<Work>()};
+      SetupArgs sa{ems, nEm, K, km, key, grec, count, start, cursor, chunkStart, work};
       ContribSetupKernel<<<(nEm + kSetupThreads - 1) / kSetupThreads, kSetupThreads, 0, ctx->stream>>>(sa);
       ISCU_CK_LAUNCH(ctx, "ContribSetupKernel");
       if (nKeys > 0)
       {
-         ScatterArgs xa{ems,    nEm,        K, km, sc.rec.as<int>(), count, start, cursor, chunkStart,
-                        sc.list.as<CStage>(), sc.chunks.as<CChunk>()};
+         ScatterArgs xa{ems, nEm, K, km, key, count, start, cursor, chunkStart, list, chunks};
          ContribScatterKernel<<<(nEm + 255) / 256, 256, 0, ctx->stream>>>(xa);
          ISCU_CK_LAUNCH(ctx, "ContribScatterKernel");
          if (marks)
             ISCU_CK(cudaEventRecord(marks[1], ctx->stream));
-         ContribArgs ca{km, K, sc.chunks.as<CChunk>(), sc.list.as<CStage>(), sc.ctr.as<Work>(),
-                        sc.contrib.as<float>(), static_cast<uint32_t>(S)};
+         ContribArgs ca{km, K, chunks, list, work, contrib, static_cast<uint32_t>(S)};
          ContribKernel<<<kContribPerSm * ctx->smCount, G.ct + 32, 0, ctx->stream>>>(ca);
          ISCU_CK_LAUNCH(ctx, "ContribKernel");
       }
@@ -1052,8 +1078,8 @@ int LaunchContribRender(iscu_ctx* ctx, int tileConfig, const iscu_emitter* ems, 
    ga.frames = frames;
    ga.nFrames = nFrames;
    ga.nEm = nEm;
-   ga.grec = sc.grec.as<int4>();
-   ga.contrib = sc.contrib.as<float>();
+   ga.grec = grec;
+   ga.contrib = contrib;
    ga.S = static_cast<uint32_t>(S);
    ga.K = K;
    ga.st = ctx->Static();

@@ -405,3 +405,30 @@ def test_steep_stacks_take_no_second_sum():
                 times[name] = best
             assert np.array_equal(*out), name
     assert times["steep"] <= 1.45 * times["slow"], times
+
+
+def test_batches_of_about_one_size_share_the_scratch():
+    """Two-pass batches that grow by a few emitters at a time stay in the first one's scratch: no allocation, and so no
+    wait for one, between them."""
+    import torch
+    from insiliscope_b200 import Engine
+    rng = np.random.default_rng(37)
+    half, os_ = 16, 4
+    n = 2 * half * os_ + 1
+    with Engine(0) as eng:
+        eng.kernel_set_planes(0, rng.uniform(0.0, 1e-4, (3, n, n)).astype(np.float32), os_, 25.0, INTERP_CUBIC)
+        eng.set_static(128, 128, flat_bg=5.0)
+        eng.set_render_config(12)
+        free = []
+        for count in (32000, 32001, 32100, 32600, 32900, 20000, 32900):
+            em = np.zeros(count, EMITTER_DTYPE)
+            em["x_px"], em["y_px"] = rng.uniform(0.0, 127.0, (2, count))
+            em["photons"], em["plane"] = 1000.0, rng.integers(0, 3, count)
+            per = np.full(200, count // 200)
+            per[0] += count - int(per.sum())
+            dem, dfr = (torch.from_numpy(t.view(np.uint8)).cuda() for t in (em, frames_table(per)))
+            ph = torch.empty((200, 128, 128), dtype=torch.float32, device="cuda")
+            eng.render_frames_dev(dem, dfr, 200, None, 5, ph)
+            del dem, dfr, ph
+            free.append(torch.cuda.mem_get_info()[0])
+        assert len(set(free[1:])) == 1, free
