@@ -1089,15 +1089,20 @@ int LaunchContribRender(iscu_ctx* ctx, int tileConfig, const iscu_emitter* ems, 
    ga.aduOut = cam ? adu : nullptr;
    const int tile = tileConfig % 3;
    const bool persistent = tileConfig / 3 == 1;
-   // four or two tiles a CTA where that leaves CTAs enough to even out the last round (six run on an SM): four from 48
-   // an SM (two-colour movie, 442: tiles pass 2.19 ms against 2.39 with two and 2.85 with one; dSTORM movie, 22: 122
-   // against 118.5 and 128 us), two from 12
+   // Two tiles a CTA from 12 CTAs an SM on (six run on one): tiles pass of frames of 128 x 128 px, 160 emitters each, at 9
+   // a SM 32 us with one and with two, at 17 55 and 52, at 43 124 and 115; 131 x 97 px, 40 emitters, at 9 and 14 23.5 and
+   // 23.6, 31.6 and 30.7. Four from 8 on where a frame has more emitters than are staged at once, whose staging four tiles
+   // share: frames of 256 x 256 px, 430 emitters, at 4 33.8 us with two and 34.8 with four, at 9 57 and 55, at 87 464 and
+   // 429; with 160 emitters the two are within 2 % of each other from 20 to 100 CTAs an SM. Neither where the tile would
+   // be wider than the frame (900 frames of 64 x 64 px in tiles of 32: 99 us with two, 112 with four, half of them empty).
    const int th = kTileH[tile];
    const auto tilesOf = [&](int tw) { return (ga.st.width + tw - 1) / tw * ((ga.st.height + th - 1) / th); };
    int sub = 1;
    for (int q = persistent ? 1 : 4; q > 1 && sub == 1; q /= 2)
-      if (static_cast<uint64_t>(tilesOf(q * kTileW[tile])) * nFrames >=
-          static_cast<uint64_t>(q == 4 ? 48 : 12) * ctx->smCount)
+      if (static_cast<uint32_t>((q - 1) * kTileW[tile]) < ga.st.width &&
+          (q == 2 || nEm >= static_cast<uint64_t>(kGChunk) * nFrames) &&
+          static_cast<uint64_t>(tilesOf(q * kTileW[tile])) * nFrames >=
+             static_cast<uint64_t>(q == 4 ? 8 : 12) * ctx->smCount)
          sub = q;
    const int tw = kTileW[tile] * sub;
    GatherFn fn = nullptr;

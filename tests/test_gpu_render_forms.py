@@ -432,3 +432,44 @@ def test_batches_of_about_one_size_share_the_scratch():
             del dem, dfr, ph
             free.append(torch.cuda.mem_get_info()[0])
         assert len(set(free[1:])) == 1, free
+
+
+@pytest.mark.parametrize("per", [30, 300])
+@pytest.mark.parametrize("halo", [0.0, 2e-4])
+def test_wide_gather_tiles_at_ragged_edges(engine, per, halo):
+    """Frames enough for two and (with more emitters than are staged at once) four tiles a CTA, three pixels wider than a
+    whole number of either: the one-pass form's bits, with and without a halo cut, some frames empty."""
+    import torch
+    sms = torch.cuda.get_device_properties(0).multi_processor_count
+    rng = np.random.default_rng(per)
+    half, os_, w, h = 5, 3, 131, 61
+    n = 2 * half * os_ + 1
+    y, x = np.mgrid[0:n, 0:n] - (n - 1) / 2.0
+    plane = (1.0 + (x * x + y * y) / 20.0) ** -1.5
+    engine.kernel_set_planes(0, np.repeat((plane / plane.sum())[None], 3, 0).astype(np.float32), os_, 25.0, INTERP_CUBIC)
+    if halo:
+        engine.kernel_set_halo(0, halo)
+    counts = rng.poisson(per, 12 * sms // 10)
+    counts[::7] = 0
+    counts[1::7] *= 2
+    em = np.zeros(int(counts.sum()), EMITTER_DTYPE)
+    em["x_px"] = rng.uniform(-half - 1.0, w + half, len(em))
+    em["y_px"] = rng.uniform(-half - 1.0, h + half, len(em))
+    em["photons"], em["plane"] = rng.uniform(1.0, 3000.0, len(em)), rng.integers(0, 3, len(em))
+    engine.set_static(w, h, flat_bg=7.0)
+    cam = CameraParams(gain=2.0, read_noise_e=1.5)
+    dem, dfr = (torch.from_numpy(t.view(np.uint8)).cuda() for t in (em, frames_table(counts)))
+    out = {}
+    try:
+        for config in (0, 12, 13, 14):
+            engine.set_render_config(config)
+            ph = torch.empty((len(counts), h, w), dtype=torch.float32, device="cuda")
+            adu = torch.empty((len(counts), h, w), dtype=torch.uint16, device="cuda")
+            engine.render_frames_dev(dem, dfr, len(counts), cam, 5, ph, adu)
+            out[config] = ph.cpu().numpy().view(np.uint32), adu.cpu().numpy()
+    finally:
+        engine.set_render_config(0)
+        if halo:
+            engine.kernel_set_halo(0, 0.0)
+    for config in (12, 13, 14):
+        assert np.array_equal(out[config][0], out[0][0]) and np.array_equal(out[config][1], out[0][1]), config
