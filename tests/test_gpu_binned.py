@@ -171,3 +171,37 @@ def test_signed_stacks_and_extreme_photons_take_no_detour(engine):
     assert _rel(img[:2], want) <= 1e-6
     r.close()
     assert extreme <= 1.3 * plain and signed <= 2.4 * plain, (plain, extreme, signed)
+
+
+def _order_movie(frames):
+    """Frames of a 1, a 2^-24 and many 2^-54 photons in one cell, the large ones first and on the last plane: in event
+    order the small ones are lost one after the other and the sum is float32's midpoint (1); by plane they come first and
+    take it past (1 + 2^-23)."""
+    per = 900
+    em = np.zeros(per * frames, EMITTER_DTYPE)
+    em["x_px"], em["y_px"] = 20.0, 20.0
+    em["photons"], em["plane"] = 2.0 ** -54, np.arange(per * frames) % 2
+    em["photons"][::per], em["photons"][1::per] = 1.0, 2.0 ** -24
+    em["plane"][::per] = em["plane"][1::per] = 2
+    return em, frames_table(np.full(frames, per))
+
+
+def test_images_do_not_depend_on_the_batch(engine):
+    """A frame's image is the event-order sum's, to the bit, whether its batch takes the dense kernel or the per-pixel one:
+    frames built so that the order of the sum decides the rounding, and 100 frames of a movie."""
+    planes = np.zeros((3, 5, 5), np.float32)
+    planes[:, 2, 2] = 1.0
+    engine.kernel_set_planes(0, planes, 1, 100.0, INTERP_CUBIC)
+    r = BinnedRenderer(engine, 64, 48, 1, slot=0)
+    em, fr = _order_movie(400)
+    img, _ = _render_ms(engine, r, em, fr)
+    want = np.zeros((48, 64), np.float32)
+    want[20, 20] = 1.0
+    assert np.array_equal(img[0], want) and all(np.array_equal(f, want) for f in img)
+    r.close()
+    r, em, fr = _dense_movie(engine, 8, 4, 2, 96, 80, 9, 700, 300, seed=3)
+    whole, _ = _render_ms(engine, r, em, fr)
+    for k in range(0, 100, 4):     # four frames at a time: too few for the dense kernel
+        part, _ = _render_ms(engine, r, em, fr[k:k + 4])
+        assert np.array_equal(part.view(np.uint32), whole[k:k + 4].view(np.uint32)), k
+    r.close()
