@@ -30,8 +30,9 @@ struct iscu_binned
    uint32_t W = 0, H = 0;
    int u = 1, R = 1, nz = 1;
    bool dense = false;     // the dense kernel's shared memory, plane table and number format hold this renderer
-   iscu::DevBuf kernels;   // nz x (2R + 1)^2 floats
-   iscu::DevBuf denseKernels;   // the same with rows of a multiple of 16 bytes
+   int Pitch();            // sets the pitch from R and nz
+   int pitch = 3;          // floats per kernel row: a multiple of 4 (zeros behind the row) where the dense kernel fits
+   iscu::DevBuf kernels;   // nz x (2R + 1) x pitch floats
 };
 
 namespace iscu {
@@ -42,20 +43,29 @@ constexpr int kSide = 16;
 
 // KernelWidefieldPsf::Kernel: cell (dx, dy) of plane p = the sum, in float64 and row order, of the oversampled plane
 // over [s0 + dy r, +r) x [s0 + dx r, +r) clipped to the plane, rounded to float.
-__global__ void CellKernelsKernel(const float* __restrict__ planes, int n, int nz, int r, int s0, int R,
-                                  float* __restrict__ out)
+// Rows of `pitch` floats, zeros behind the cells. odd (nullable): set to 1 by a cell that is negative or not finite.
+__global__ void CellKernelsKernel(const float* __restrict__ planes, int n, int nz, int r, int s0, int R, int pitch,
+                                  float* __restrict__ out, int* __restrict__ odd)
 {
    const int D = 2 * R + 1, i = blockIdx.x * blockDim.x + threadIdx.x;
-   if (i >= nz * D * D)
+   if (i >= nz * D * pitch)
       return;
-   const int p = i / (D * D), c = i - p * D * D, dy = c / D - R, dx = c % D - R;
+   const int p = i / (D * pitch), c = i - p * D * pitch, dy = c / pitch - R, dx = c % pitch - R;
+   if (dx > R)
+   {
+      out[i] = 0.f;
+      return;
+   }
    const float* P = planes + static_cast<size_t>(p) * n * n;
    const int ya = s0 + dy * r, yb = min(n, ya + r), xa = s0 + dx * r, xb = min(n, xa + r);
    double acc = 0.0;
    for (int y = max(0, ya); y < yb; ++y)
       for (int x = max(0, xa); x < xb; ++x)
          acc += P[static_cast<size_t>(y) * n + x];
-   out[i] = static_cast<float>(acc);
+   const float v = static_cast<float>(acc);
+   out[i] = v;
+   if (odd && __float_as_uint(v) >= 0x7F800000u)
+      *odd = 1;
 }
 
 } // namespace
@@ -63,7 +73,7 @@ __global__ void CellKernelsKernel(const float* __restrict__ planes, int n, int n
 int LaunchCellKernels(iscu_ctx* ctx, const float* planes, int n, int nz, int r, int s0, int R, float* out)
 {
    const int D = 2 * R + 1, total = nz * D * D;
-   CellKernelsKernel<<<(total + 255) / 256, 256, 0, ctx->stream>>>(planes, n, nz, r, s0, R, out);
+   CellKernelsKernel<<<(total + 255) / 256, 256, 0, ctx->stream>>>(planes, n, nz, r, s0, R, D, out, nullptr);
    ISCU_CK_LAUNCH(ctx, "CellKernelsKernel");
    return ISCU_OK;
 }
@@ -82,8 +92,8 @@ struct Staged
 template <int U>
 __global__ void __launch_bounds__(kThreads) BinnedRenderKernel(const iscu_emitter* __restrict__ em, uint32_t nEm,
                                                               const iscu_frame* __restrict__ frames,
-                                                              const float* __restrict__ K, int nz, int R, uint32_t W,
-                                                              uint32_t H, float* __restrict__ img,
+                                                              const float* __restrict__ K, int nz, int R, int pitch,
+                                                              uint32_t W, uint32_t H, float* __restrict__ img,
                                                               float* __restrict__ alone)
 {
    __shared__ Staged st[kThreads];
@@ -143,17 +153,17 @@ __global__ void __launch_bounds__(kThreads) BinnedRenderKernel(const iscu_emitte
          const int dx0 = cx - t.cx, dy0 = cy - t.cy;
          if (dx0 > R || dx0 + U - 1 < -R || dy0 > R || dy0 + U - 1 < -R)
             continue;
-         const float* Kp = K + t.plane * D * D;
+         const float* Kp = K + t.plane * D * pitch;
          const double ph = t.photons;
          if (dx0 >= -R && dx0 + U - 1 <= R && dy0 >= -R && dy0 + U - 1 <= R)
          {
             // every cell of the pixel in reach (the common case): no per-cell test
-            const float* Kc = Kp + (dy0 + R) * D + (dx0 + R);
+            const float* Kc = Kp + (dy0 + R) * pitch + (dx0 + R);
 #pragma unroll
             for (int j = 0; j < U; ++j)
 #pragma unroll
                for (int i = 0; i < U; ++i)
-                  acc[j][i] += ph * static_cast<double>(__ldg(Kc + j * D + i));
+                  acc[j][i] += ph * static_cast<double>(__ldg(Kc + j * pitch + i));
             continue;
          }
 #pragma unroll
@@ -167,7 +177,7 @@ __global__ void __launch_bounds__(kThreads) BinnedRenderKernel(const iscu_emitte
             {
                const int dx = dx0 + i;
                if (dx >= -R && dx <= R)
-                  acc[j][i] += ph * static_cast<double>(__ldg(Kp + (dy + R) * D + (dx + R)));
+                  acc[j][i] += ph * static_cast<double>(__ldg(Kp + (dy + R) * pitch + (dx + R)));
             }
          }
       }
@@ -232,26 +242,6 @@ inline int DenseBuffers(int R) { return DensePitch(R) == 128 ? 2 : 1; }
 inline size_t DenseBytes(int R)
 {
    return kDenseHead + std::max(DenseBuffers(R) * DenseKernelBytes(R), sizeof(float) * kTileX * kTileY);
-}
-
-// The kernels with rows of a multiple of 16 bytes (zeros behind them), and whether any has a negative or non-finite
-// value. A CTA per plane.
-__global__ void DenseKernelsKernel(const float* __restrict__ K, int D, int rowPitch, float* __restrict__ out,
-                                   int* __restrict__ odd)
-{
-   const float* Kp = K + static_cast<size_t>(blockIdx.x) * D * D;
-   float* o = out + static_cast<size_t>(blockIdx.x) * D * rowPitch;
-   int any = 0;
-   for (int i = threadIdx.x; i < D * rowPitch; i += blockDim.x)
-   {
-      const int y = i / rowPitch, x = i % rowPitch;
-      const float v = x < D ? Kp[y * D + x] : 0.f;
-      any |= __float_as_uint(v) >= 0x7F800000u;
-      o[i] = v;
-   }
-   any = __syncthreads_or(any);
-   if (threadIdx.x == 0 && any)
-      atomicExch(odd, 1);
 }
 
 // Cell (gx, gy)'s sum over a frame's emitters [begin, end) in event order, as float (thread 0's). Out of line: it is
@@ -610,6 +600,12 @@ bool DensePays(const iscu_binned* b, int smCount, uint32_t nEmitters, uint32_t n
 
 using namespace iscu;
 
+int iscu_binned::Pitch()
+{
+   const int D = 2 * R + 1;
+   return pitch = DenseFits(R, nz) ? (D + 3) / 4 * 4 : D;
+}
+
 extern "C" {
 
 int iscu_binned_create(iscu_ctx* ctx, int32_t slot, double sigma_px, uint32_t width, uint32_t height, int32_t upscale,
@@ -628,6 +624,7 @@ int iscu_binned_create(iscu_ctx* ctx, int32_t slot, double sigma_px, uint32_t wi
    b->ctx = ctx;
    b->W = width;
    b->H = height;
+   int odd = 0;   // a kernel value is negative or not finite (the Gaussian's are neither)
    if (slot >= 0)
    {
       const KernelSlot& k = ctx->kernels[slot];
@@ -652,12 +649,16 @@ int iscu_binned_create(iscu_ctx* ctx, int32_t slot, double sigma_px, uint32_t wi
       }
       b->R = std::max(1, b->R);
       b->nz = std::max(1, k.nz);
-      const int D = 2 * b->R + 1;
-      ISCU_CK(b->kernels.Reserve(static_cast<size_t>(b->nz) * D * D * sizeof(float)));
-      const int total = b->nz * D * D;
+      const int D = 2 * b->R + 1, total = b->nz * D * b->Pitch();
+      const size_t bytes = static_cast<size_t>(total) * sizeof(float);
+      ISCU_CK(b->kernels.Reserve(bytes + sizeof(int)));   // and the flag
+      int* flag = reinterpret_cast<int*>(b->kernels.as<unsigned char>() + bytes);
+      ISCU_CK(cudaMemsetAsync(flag, 0, sizeof(int), ctx->stream));
       CellKernelsKernel<<<(total + 255) / 256, 256, 0, ctx->stream>>>(k.planes.as<float>(), n, b->nz, r, s0, b->R,
-                                                                        b->kernels.as<float>());
+                                                                        b->pitch, b->kernels.as<float>(), flag);
       ISCU_CK_LAUNCH(ctx, "CellKernelsKernel");
+      ISCU_CK(cudaMemcpyAsync(&odd, flag, sizeof(int), cudaMemcpyDeviceToHost, ctx->stream));
+      ISCU_CK(cudaStreamSynchronize(ctx->stream));
    }
    else
    {
@@ -677,31 +678,20 @@ int iscu_binned_create(iscu_ctx* ctx, int32_t slot, double sigma_px, uint32_t wi
             g[static_cast<size_t>(y + R) * D + (x + R)] = v;
             sum += v;
          }
-      std::vector<float> gf(g.size());
+      std::vector<float> gf(static_cast<size_t>(D) * b->Pitch());
       for (size_t i = 0; i < g.size(); ++i)
-         gf[i] = static_cast<float>(g[i] / sum);
+         gf[i / D * b->pitch + i % D] = static_cast<float>(g[i] / sum);
       ISCU_CK(b->kernels.Reserve(gf.size() * sizeof(float)));
       ISCU_CK(cudaMemcpyAsync(b->kernels.p, gf.data(), gf.size() * sizeof(float), cudaMemcpyHostToDevice,
                               ctx->stream));
    }
    if (b->u > 8)
       return Fail(ISCU_ERR_LIMIT, "binned render: at most 8 cells per pixel");
-   if (DenseFits(b->R, b->nz))
+   if (DenseFits(b->R, b->nz) && !odd)
    {
-      const int D = 2 * b->R + 1, rowPitch = (D + 3) / 4 * 4;
-      ISCU_CK(b->denseKernels.Reserve(static_cast<size_t>(b->nz) * D * rowPitch * sizeof(float)));
-      DevBuf flag;
-      int odd = 0;
-      ISCU_CK(flag.Reserve(sizeof(int)));
-      ISCU_CK(cudaMemsetAsync(flag.p, 0, sizeof(int), ctx->stream));
-      DenseKernelsKernel<<<b->nz, 256, 0, ctx->stream>>>(b->kernels.as<float>(), D, rowPitch,
-                                                         b->denseKernels.as<float>(), flag.as<int>());
-      ISCU_CK_LAUNCH(ctx, "DenseKernelsKernel");
-      ISCU_CK(cudaMemcpyAsync(&odd, flag.p, sizeof(int), cudaMemcpyDeviceToHost, ctx->stream));
-      ISCU_CK(cudaStreamSynchronize(ctx->stream));
       ISCU_CK(cudaFuncSetAttribute(DenseOf(b->R), cudaFuncAttributeMaxDynamicSharedMemorySize,
                                    static_cast<int>(kDenseMaxBytes)));
-      b->dense = !odd;
+      b->dense = true;
    }
    ISCU_CK(cudaStreamSynchronize(ctx->stream));
    *out = b.release();
@@ -728,8 +718,8 @@ int iscu_binned_kernels(iscu_binned* b, float* out)
    std::lock_guard<std::recursive_mutex> lock(b->ctx->mu);
    ClearError();
    const size_t D = 2 * static_cast<size_t>(b->R) + 1;
-   ISCU_CK(cudaMemcpyAsync(out, b->kernels.p, b->nz * D * D * sizeof(float), cudaMemcpyDeviceToHost,
-                           b->ctx->stream));
+   ISCU_CK(cudaMemcpy2DAsync(out, D * sizeof(float), b->kernels.p, b->pitch * sizeof(float), D * sizeof(float),
+                             b->nz * D, cudaMemcpyDeviceToHost, b->ctx->stream));
    ISCU_CK(cudaStreamSynchronize(b->ctx->stream));
    return ISCU_OK;
 }
@@ -760,7 +750,7 @@ int iscu_binned_render_dev(iscu_binned* b, const iscu_emitter* emitters_dev, uin
    if (b->dense && DensePays(b, ctx->smCount, n_emitters, n_frames, tiles))
    {
       DenseOf(b->R)<<<tiles, kThreads, DenseBytes(b->R), ctx->stream>>>(
-         emitters_dev, n_emitters, frames_dev, b->denseKernels.as<float>(), b->nz, b->R, b->u, b->W, b->H, img_dev,
+         emitters_dev, n_emitters, frames_dev, K, b->nz, b->R, b->u, b->W, b->H, img_dev,
          alone_dev);
       ISCU_CK_LAUNCH(ctx, "BinnedDenseKernel");
       return ISCU_OK;
@@ -768,7 +758,7 @@ int iscu_binned_render_dev(iscu_binned* b, const iscu_emitter* emitters_dev, uin
    const dim3 grid((b->W + kSide - 1) / kSide, (b->H + kSide - 1) / kSide, n_frames);
 #define ISCU_BINNED_LAUNCH(UU)                                                                                          \
    BinnedRenderKernel<UU><<<grid, kThreads, 0, ctx->stream>>>(emitters_dev, n_emitters, frames_dev, K, b->nz, b->R,  \
-                                                              b->W, b->H, img_dev, alone_dev)
+                                                              b->pitch, b->W, b->H, img_dev, alone_dev)
    switch (b->u)
    {
    case 1: ISCU_BINNED_LAUNCH(1); break;

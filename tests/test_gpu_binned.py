@@ -205,3 +205,19 @@ def test_images_do_not_depend_on_the_batch(engine):
         part, _ = _render_ms(engine, r, em, fr[k:k + 4])
         assert np.array_equal(part.view(np.uint32), whole[k:k + 4].view(np.uint32)), k
     r.close()
+
+
+@pytest.mark.parametrize("half,os_,nz", [(60, 1, 500), (3, 1, 4), (100, 1, 3)])
+def test_a_renderer_holds_its_kernels_once(engine, half, os_, nz):
+    """The plane kernels, read back as the oracle has them, take the device memory of one copy (rows of whole 16 bytes)."""
+    import torch
+    rng = np.random.default_rng(half)
+    n = 2 * half * os_ + 1
+    planes = rng.random((nz, n, n)).astype(np.float32) / (n * n)
+    engine.kernel_set_planes(0, planes, os_, 100.0, INTERP_CUBIC)
+    before = torch.cuda.mem_get_info()[0]
+    r = BinnedRenderer(engine, 64, 64, 1, slot=0)
+    held = before - torch.cuda.mem_get_info()[0]
+    assert held <= 1.05 * r.kernels().nbytes + (4 << 20), (held, r.kernels().nbytes)
+    assert np.array_equal(r.kernels(), binned_cell_kernels_f64(planes, os_, 1)[0])
+    r.close()
