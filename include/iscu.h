@@ -758,6 +758,9 @@ int iscu_binned_create(iscu_ctx* ctx, int32_t slot, double sigma_px, uint32_t wi
                        int32_t upscale, iscu_binned** out);
 /* The renderer's u (cells per pixel), R (kernel radius in cells) and plane count (any output NULL). */
 int iscu_binned_info(iscu_binned* b, int32_t* upscale, int32_t* radius_cells, int32_t* planes);
+/* The emitters from which a frame of a call of n_emitters over n_frames takes the kernel for dense frames (0: none does).
+ * The image is the same, to the bit, from either kernel. */
+int iscu_binned_dense_from(iscu_binned* b, uint32_t n_emitters, uint32_t n_frames, uint32_t* count);
 /* The plane kernels, nz x (2R + 1)^2 floats (row-major, dy outer), into host memory. */
 int iscu_binned_kernels(iscu_binned* b, float* out);
 void iscu_binned_destroy(iscu_binned* b);

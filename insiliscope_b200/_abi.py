@@ -211,6 +211,7 @@ SIGNATURES = {
     "iscu_tiff_close": (C.c_int, [vp]),
     "iscu_binned_create": (C.c_int, [vp, C.c_int32, C.c_double, C.c_uint32, C.c_uint32, C.c_int32, vp]),
     "iscu_binned_info": (C.c_int, [vp, vp, vp, vp]),
+    "iscu_binned_dense_from": (C.c_int, [vp, C.c_uint32, C.c_uint32, vp]),
     "iscu_binned_kernels": (C.c_int, [vp, vp]),
     "iscu_binned_destroy": (None, [vp]),
     "iscu_binned_render_dev": (C.c_int, [vp, vp, C.c_uint32, vp, C.c_uint32, vp, vp]),

@@ -88,13 +88,13 @@ struct Staged
 };
 
 // grid (ceil(W / 16), ceil(H / 16), frames). Frame k's emitters are emitters[em_start, em_start + em_count) cut at
-// nEm. img / alone: frames x H x W, +=.
+// nEm. img / alone: frames x H x W, +=. denseFrom: frames of that many emitters and more are the dense kernel's (0: none).
 template <int U>
 __global__ void __launch_bounds__(kThreads) BinnedRenderKernel(const iscu_emitter* __restrict__ em, uint32_t nEm,
                                                               const iscu_frame* __restrict__ frames,
-                                                              const float* __restrict__ K, int nz, int R, int pitch,
-                                                              uint32_t W, uint32_t H, float* __restrict__ img,
-                                                              float* __restrict__ alone)
+                                                              uint32_t denseFrom, const float* __restrict__ K, int nz,
+                                                              int R, int pitch, uint32_t W, uint32_t H,
+                                                              float* __restrict__ img, float* __restrict__ alone)
 {
    __shared__ Staged st[kThreads];
    __shared__ int warpKept[kThreads / 32];
@@ -107,6 +107,8 @@ __global__ void __launch_bounds__(kThreads) BinnedRenderKernel(const iscu_emitte
    const int reachY0 = max(-R, ty0 - R), reachY1 = min(gh + R - 1, ty0 + kSide * U - 1 + R);
    const iscu_frame fr = frames[blockIdx.z];
    const uint32_t start = min(fr.em_start, nEm), end = min(start + fr.em_count, nEm);
+   if (denseFrom && end > start && end - start >= denseFrom)
+      return;
    const int cx = px * U, cy = py * U;   // this pixel's first cell
    double acc[U][U];
 #pragma unroll
@@ -290,7 +292,7 @@ __device__ __noinline__ float EventOrderCell(const iscu_emitter* __restrict__ em
 // kPitch: the staged row pitch, a constant so that a block's rows are immediate offsets.
 template <int kPitch, int kBuffers>
 __global__ void __launch_bounds__(kThreads, kBuffers) BinnedDenseKernel(
-   const iscu_emitter* __restrict__ em, uint32_t nEm, const iscu_frame* __restrict__ frames,
+   const iscu_emitter* __restrict__ em, uint32_t nEm, const iscu_frame* __restrict__ frames, uint32_t denseFrom,
    const float* __restrict__ K, int nz, int R, int U, uint32_t W, uint32_t H, float* __restrict__ img,
    float* __restrict__ alone)
 {
@@ -307,6 +309,8 @@ __global__ void __launch_bounds__(kThreads, kBuffers) BinnedDenseKernel(
    const int reachY0 = max(-R, ty0 - R), reachY1 = min(gh + R - 1, ty1 + R);
    const iscu_frame fr = frames[blockIdx.z];
    const uint32_t begin = min(fr.em_start, nEm), end = min(begin + fr.em_count, nEm);
+   if (end <= begin || end - begin < denseFrom)
+      return;   // the per-pixel kernel's
    for (int i = tid; i < kBuffers * kPitch * rows; i += kThreads)
       sK[i] = 0.f;
    int total = 0;   // emitters that reach the tile
@@ -566,8 +570,8 @@ __global__ void __launch_bounds__(kThreads, kBuffers) BinnedDenseKernel(
    }
 }
 
-using DenseFn = void (*)(const iscu_emitter*, uint32_t, const iscu_frame*, const float*, int, int, int, uint32_t,
-                         uint32_t, float*, float*);
+using DenseFn = void (*)(const iscu_emitter*, uint32_t, const iscu_frame*, uint32_t, const float*, int, int, int,
+                         uint32_t, uint32_t, float*, float*);
 DenseFn DenseOf(int R) { return DensePitch(R) == 128 ? BinnedDenseKernel<128, 2> : BinnedDenseKernel<192, 1>; }
 
 // KernelWidefieldPsf::ValidUpscale (WidefieldRender.cpp:262-269).
@@ -580,19 +584,27 @@ int ValidUpscale(int oversampling, int requested)
    return 1;
 }
 
-// Whether the dense kernel is the faster one. A CTA pays for each plane it has an emitter of (the kernel's 17-66 KB
-// staged, a barrier), the kernel above for every emitter and pixel: at two emitters of a plane within a tile's reach
-// the two take the same (200 frames of 128 x 128 px, 49 planes, u = 2: 200, 400 and 2,400 emitters a frame 0.40, 0.32
-// (100 frames) and 2.18 ms against 0.44, 0.32 and 1.19, the camera's noise included); with one buffer and one CTA per
-// SM (R > 32) at five (u = 4, R = 64, 20 frames of 2,400 emitters, 5.9 a plane: 0.80 against 0.73 ms; 50 frames of 400:
-// 0.37 against 0.73). Fewer tiles than two per SM leave it idle (100 frames of 64 x 64 px at u = 1: 88 against 108 us).
-bool DensePays(const iscu_binned* b, int smCount, uint32_t nEmitters, uint32_t nFrames, dim3 tiles)
+// The emitters from which a frame is the dense kernel's in a call of n_emitters over n_frames; 0: no frame. A CTA pays
+// for each plane it has an emitter of (the kernel's 17-66 KB staged, a barrier), the kernel above for every emitter and
+// pixel: at two emitters of a plane within a tile's reach the two take the same (200 frames of 128 x 128 px, 49 planes,
+// u = 2: 200, 400 and 2,400 emitters a frame 0.40, 0.32 (100 frames) and 2.18 ms against 0.44, 0.32 and 1.14, the
+// camera's noise included); with one buffer and one CTA per SM (R > 32) at five (u = 4, R = 64, 20 frames of 2,400
+// emitters, 5.9 a plane: 0.80 against 0.73 ms; 50 frames of 400: 0.37 against 0.73). Fewer tiles than two per SM leave it
+// idle (100 frames of 64 x 64 px at u = 1: 88 against 108 us). The call's average only decides whether the dense kernel is
+// launched: each frame goes by its own count, so that sparse frames of a long emitter array stay with the kernel above
+// (200 frames of 100 emitters, their array a hundred times as long: 238 us when the average decided for all,.
+uint32_t DenseFrom(const iscu_binned* b, uint32_t nEmitters, uint32_t nFrames)
 {
+   if (!b->dense || nFrames == 0)
+      return 0;
+   const uint32_t pw = kTileX / b->u, ph = kTileY / b->u;
+   const uint64_t tiles = static_cast<uint64_t>((b->W + pw - 1) / pw) * ((b->H + ph - 1) / ph) * nFrames;
    const double reach = 2.0 * b->R, gw = static_cast<double>(b->W) * b->u, gh = static_cast<double>(b->H) * b->u;
    const double part = std::min(1.0, (kTileX + reach) / (gw + reach)) * std::min(1.0, (kTileY + reach) / (gh + reach));
-   const double perPlane = static_cast<double>(nEmitters) / nFrames * part / b->nz;
-   return perPlane >= (DenseBuffers(b->R) == 2 ? 2.0 : 5.0) &&
-          static_cast<uint64_t>(tiles.x) * tiles.y * tiles.z >= 2ull * static_cast<uint64_t>(smCount);
+   const double from = (DenseBuffers(b->R) == 2 ? 2.0 : 5.0) * b->nz / part;
+   if (tiles < 2ull * static_cast<uint64_t>(b->ctx->smCount) || static_cast<double>(nEmitters) / nFrames < from)
+      return 0;
+   return static_cast<uint32_t>(std::ceil(from));   // (at least 2, and below nEmitters / nFrames + 1)
 }
 
 } // namespace
@@ -711,6 +723,14 @@ int iscu_binned_info(iscu_binned* b, int32_t* upscale, int32_t* radius_cells, in
    return ISCU_OK;
 }
 
+int iscu_binned_dense_from(iscu_binned* b, uint32_t n_emitters, uint32_t n_frames, uint32_t* count)
+{
+   if (!b || !count)
+      return Fail(ISCU_ERR_ARG, "null argument");
+   *count = DenseFrom(b, n_emitters, n_frames);
+   return ISCU_OK;
+}
+
 int iscu_binned_kernels(iscu_binned* b, float* out)
 {
    if (!b || !out)
@@ -745,20 +765,19 @@ int iscu_binned_render_dev(iscu_binned* b, const iscu_emitter* emitters_dev, uin
    if (!n_frames)
       return ISCU_OK;
    const float* K = b->kernels.as<float>();
-   const uint32_t pw = kTileX / b->u, ph = kTileY / b->u;
-   const dim3 tiles((b->W + pw - 1) / pw, (b->H + ph - 1) / ph, n_frames);
-   if (b->dense && DensePays(b, ctx->smCount, n_emitters, n_frames, tiles))
+   const uint32_t denseFrom = DenseFrom(b, n_emitters, n_frames);
+   if (denseFrom)
    {
-      DenseOf(b->R)<<<tiles, kThreads, DenseBytes(b->R), ctx->stream>>>(
-         emitters_dev, n_emitters, frames_dev, K, b->nz, b->R, b->u, b->W, b->H, img_dev,
-         alone_dev);
+      const uint32_t pw = kTileX / b->u, ph = kTileY / b->u;
+      DenseOf(b->R)<<<dim3((b->W + pw - 1) / pw, (b->H + ph - 1) / ph, n_frames), kThreads, DenseBytes(b->R),
+                      ctx->stream>>>(emitters_dev, n_emitters, frames_dev, denseFrom, K, b->nz, b->R, b->u, b->W, b->H,
+                                     img_dev, alone_dev);
       ISCU_CK_LAUNCH(ctx, "BinnedDenseKernel");
-      return ISCU_OK;
    }
    const dim3 grid((b->W + kSide - 1) / kSide, (b->H + kSide - 1) / kSide, n_frames);
 #define ISCU_BINNED_LAUNCH(UU)                                                                                          \
-   BinnedRenderKernel<UU><<<grid, kThreads, 0, ctx->stream>>>(emitters_dev, n_emitters, frames_dev, K, b->nz, b->R,  \
-                                                              b->pitch, b->W, b->H, img_dev, alone_dev)
+   BinnedRenderKernel<UU><<<grid, kThreads, 0, ctx->stream>>>(emitters_dev, n_emitters, frames_dev, denseFrom, K,    \
+                                                              b->nz, b->R, b->pitch, b->W, b->H, img_dev, alone_dev)
    switch (b->u)
    {
    case 1: ISCU_BINNED_LAUNCH(1); break;

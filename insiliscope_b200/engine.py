@@ -1043,6 +1043,12 @@ class BinnedRenderer:
         self.upscale, self.radius, self.planes = u.value, r.value, nz.value
         engine._plans.add(self)
 
+    def dense_from(self, n_emitters, n_frames):
+        """The emitters from which a frame of a call of these sizes takes the kernel for dense frames (0: none does)."""
+        count = C.c_uint32()
+        check(self.lib.iscu_binned_dense_from(self.h, int(n_emitters), int(n_frames), C.byref(count)))
+        return count.value
+
     def kernels(self):
         """The plane kernels at the cell pitch, (planes, 2R + 1, 2R + 1) float32."""
         D = 2 * self.radius + 1

@@ -221,3 +221,48 @@ def test_a_renderer_holds_its_kernels_once(engine, half, os_, nz):
     assert held <= 1.05 * r.kernels().nbytes + (4 << 20), (held, r.kernels().nbytes)
     assert np.array_equal(r.kernels(), binned_cell_kernels_f64(planes, os_, 1)[0])
     r.close()
+
+
+@pytest.mark.parametrize("half,os_,upscale,nz,w,h", [(8, 4, 4, 49, 70, 33), (9, 4, 4, 3, 33, 18), (16, 4, 4, 5, 40, 20),
+                                                     (16, 4, 2, 49, 130, 40), (5, 2, 2, 300, 65, 33)])
+def test_dense_kernel_geometries(engine, half, os_, upscale, nz, w, h):
+    """The dense kernel (as its own query says) at kernels as wide as its row pitches allow (R = 32 and 64), just beyond
+    the first (one staged kernel instead of two), and more planes than the sort scans at once: the oracle within 1e-6,
+    and the per-pixel kernel's bits, which a few frames alone take."""
+    import torch
+    sms = torch.cuda.get_device_properties(0).multi_processor_count
+    probe, _, _ = _dense_movie(engine, half, os_, upscale, w, h, nz, 1, 1)
+    tiles = -(-w // (128 // probe.upscale)) * -(-h // (64 // probe.upscale))
+    frames = -(-2 * sms // tiles)
+    per = probe.dense_from(1 << 30, frames) + 5
+    probe.close()
+    assert per > 5
+    r, em, fr = _dense_movie(engine, half, os_, upscale, w, h, nz, per, frames, seed=half)
+    assert 0 < r.dense_from(len(em), frames) <= per and r.dense_from(2 * per, 2) == 0
+    whole, _ = _render_ms(engine, r, em, fr)
+    want = binned_render_f64(r.kernels().astype(np.float64), r.upscale, r.radius, em, fr[:2], w, h)
+    assert _rel(whole[:2], want) <= 1e-6
+    for k in (0, frames // 2, frames - 2):
+        part, _ = _render_ms(engine, r, em, fr[k:k + 2])
+        assert np.array_equal(part.view(np.uint32), whole[k:k + 2].view(np.uint32)), k
+    r.close()
+
+
+def test_each_frame_by_its_own_count(engine):
+    """Sparse frames whose emitters are the head of a long array take the time that they take with an array of their own,
+    and the image; dense and sparse frames in one call are each the per-pixel kernel's bits."""
+    r, em, fr = _dense_movie(engine, 16, 4, 2, 128, 128, 49, 100, 20000)
+    assert r.dense_from(len(em), 200) > 0 and r.dense_from(100 * 200, 200) == 0
+    own, short = _render_ms(engine, r, em[:100 * 200], fr[:200])
+    img, long_ = _render_ms(engine, r, em, fr[:200])
+    assert np.array_equal(img.view(np.uint32), own.view(np.uint32))
+    assert long_ <= 1.3 * short, (short, long_)
+    counts = np.where(np.arange(120) % 3 == 0, 3000, 60)
+    mixed = frames_table(counts)
+    least = r.dense_from(int(counts.sum()), 120)
+    assert 60 < least <= 3000
+    whole, _ = _render_ms(engine, r, em[:int(counts.sum())], mixed)
+    for k in range(0, 24, 2):
+        part, _ = _render_ms(engine, r, em[:int(counts.sum())], mixed[k:k + 2])
+        assert np.array_equal(part.view(np.uint32), whole[k:k + 2].view(np.uint32)), k
+    r.close()
