@@ -220,7 +220,7 @@ __global__ void __launch_bounds__(kThreads) BinnedRenderKernel(const iscu_emitte
 //
 // What bounds it: issue and the latency of 16 warps per SM (the accumulators are half the registers), the shared loads
 // at 45 %, the float64 pipe at 15 %; 54 % of the multiply-adds lie in an emitter's reach at R = 32. 200 frames of
-// 128 x 128 px, 2,400 emitters a frame, u = 2, R = 32: 1.10 ms against 2.03 ms of the kernel above. Slower (with the
+// 128 x 128 px, 2,400 emitters a frame, u = 2, R = 32: 1.05 ms against 2.03 ms of the kernel above. Slower (with the
 // noise, against 1.18): 512 threads of four rows, 32 warps per SM, 1.34; a 64-bit multiply for the two shifts, 1.26.
 constexpr int kTileX = 128, kTileY = 64, kRows = 8, kCap = 1024, kMaxPlanes = 512;
 constexpr size_t kDenseMaxBytes = 226 * 1024;
@@ -587,12 +587,14 @@ int ValidUpscale(int oversampling, int requested)
 // The emitters from which a frame is the dense kernel's in a call of n_emitters over n_frames; 0: no frame. A CTA pays
 // for each plane it has an emitter of (the kernel's 17-66 KB staged, a barrier), the kernel above for every emitter and
 // pixel: at two emitters of a plane within a tile's reach the two take the same (200 frames of 128 x 128 px, 49 planes,
-// u = 2: 200, 400 and 2,400 emitters a frame 0.40, 0.32 (100 frames) and 2.18 ms against 0.44, 0.32 and 1.14, the
+// u = 2: 200, 400 and 2,400 emitters a frame 0.40, 0.32 (100 frames) and 2.18 ms against 0.44, 0.32 and 1.17, the
 // camera's noise included); with one buffer and one CTA per SM (R > 32) at five (u = 4, R = 64, 20 frames of 2,400
 // emitters, 5.9 a plane: 0.80 against 0.73 ms; 50 frames of 400: 0.37 against 0.73). Fewer tiles than two per SM leave it
 // idle (100 frames of 64 x 64 px at u = 1: 88 against 108 us). The call's average only decides whether the dense kernel is
 // launched: each frame goes by its own count, so that sparse frames of a long emitter array stay with the kernel above
-// (200 frames of 100 emitters, their array a hundred times as long: 238 us when the average decided for all,.
+// (200 frames of 100 emitters, their array a hundred times as long: 239 us when the average decided for all, 144 so, 138
+// with an array of their own; frames of 2,400 emitters 1.05 and 1.08 ms. With one CTA of the kernel above per row of
+// tiles beside the dense one 166 us and 1.07 ms).
 uint32_t DenseFrom(const iscu_binned* b, uint32_t nEmitters, uint32_t nFrames)
 {
    if (!b->dense || nFrames == 0)
