@@ -196,6 +196,51 @@ __device__ __forceinline__ void Cmac(float2& acc, float2 a, float2 b)
    acc.y = fmaf(a.y, b.x, acc.y);
 }
 
+// A sum in two doubles (hi + lo, lo what hi's roundings left): the same to 2^-100 in any order, so that a plane's
+// normalization does not depend on how many CTAs shared the plane, which the call's number of planes decides.
+struct WideSum
+{
+   double hi = 0.0, lo = 0.0;
+   __device__ __forceinline__ void Add(double v)
+   {
+      const double s = hi + v, b = s - hi;
+      lo += (hi - (s - b)) + (v - b);
+      hi = s;
+   }
+   __device__ __forceinline__ void Add(const WideSum& o)
+   {
+      Add(o.hi);
+      lo += o.lo;
+   }
+   __device__ __forceinline__ double Value() const { return hi + lo; }
+};
+
+// The sum over the CTA's threads (thread 0's). red: blockDim.x / 32 entries.
+__device__ __forceinline__ WideSum BlockWideSum(WideSum v, double2* red)
+{
+#pragma unroll
+   for (int o = 16; o > 0; o >>= 1)
+   {
+      WideSum u;
+      u.hi = __shfl_down_sync(0xffffffffu, v.hi, o);
+      u.lo = __shfl_down_sync(0xffffffffu, v.lo, o);
+      v.Add(u);
+   }
+   if ((threadIdx.x & 31) == 0)
+      red[threadIdx.x >> 5] = make_double2(v.hi, v.lo);
+   __syncthreads();
+   WideSum t;
+   if (threadIdx.x == 0)
+      for (int w = 0; w < static_cast<int>(blockDim.x >> 5); ++w)
+      {
+         WideSum u;
+         u.hi = red[w].x;
+         u.lo = red[w].y;
+         t.Add(u);
+      }
+   return t;
+}
+
 constexpr size_t kPsfScratchKept = 64u << 20;
 constexpr int kFoldThreads = 320, kFoldMaxCluster = 8;
 constexpr size_t kFoldMaxBytes = 224 * 1024;
@@ -223,7 +268,7 @@ __global__ void __launch_bounds__(kFoldThreads, 2) CztFoldKernel(const SetParams
    extern __shared__ __align__(16) unsigned char smem[];
    float4* U = reinterpret_cast<float4*>(smem);         // [q][row]: (P.re, P.im, N.re, N.im) of the column pair q
    float4* T = U + static_cast<size_t>(Q + 1) * R;      // [row][own pair]: the samples at +t and -t
-   __shared__ double sRed[kFoldThreads / 32], sPart[kFoldMaxCluster];
+   __shared__ double2 sRed[kFoldThreads / 32], sPart[kFoldMaxCluster];
    const PsfItem it = items[psf];
    const SetParams& sp = sets[it.set];
    const double3* tab = tables + static_cast<size_t>(it.set) * M * M;
@@ -301,7 +346,7 @@ __global__ void __launch_bounds__(kFoldThreads, 2) CztFoldKernel(const SetParams
    // E = A T, I = |E|^2: a column pair and four row pairs per thread
    float* plane = out + static_cast<size_t>(psf) * P * P;
    const int groups = (nT + 3) / 4, half = P / 2, odd = P & 1;
-   double local = 0.0;
+   WideSum local;
    float I[4][4];   // [row pair][+y +x, +y -x, -y +x, -y -x] of the thread's last item
    const int nItems = own * groups;
    // row y = half + t (+), half - t - 1 + odd (-); columns likewise
@@ -355,6 +400,7 @@ __global__ void __launch_bounds__(kFoldThreads, 2) CztFoldKernel(const SetParams
          }
       }
       const bool centreX = odd && t0 + c == 0;
+      double item = 0.0;   // (an item's samples are the same however the plane is shared)
 #pragma unroll
       for (int k = 0; k < 4; ++k)
       {
@@ -367,22 +413,29 @@ __global__ void __launch_bounds__(kFoldThreads, 2) CztFoldKernel(const SetParams
             I[k][x] = pr * pr + pi * pi;
             I[k][2 + x] = mr * mr + mi * mi;
             if (g + k < nT && !(x && centreX))
-               local += static_cast<double>(I[k][x]) + (centreY ? 0.0 : static_cast<double>(I[k][2 + x]));
+               item += static_cast<double>(I[k][x]) + (centreY ? 0.0 : static_cast<double>(I[k][2 + x]));
          }
       }
+      local.Add(item);
       if (!normalize || i + kFoldThreads < nItems)
          store(i);   // the last item stays in registers for its normalization
    }
    if (!normalize)
       return;
-   const double part = BlockSumDouble(local, sRed);
-   if (tid < C)
-      cluster.map_shared_rank(sPart, tid)[rank] = part;
+   const WideSum part = BlockWideSum(local, sRed);
+   if (tid == 0)
+      for (int c = 0; c < C; ++c)
+         cluster.map_shared_rank(sPart, c)[rank] = make_double2(part.hi, part.lo);
    cluster.sync();
-   double sum = 0.0;
+   WideSum all;
    for (int c = 0; c < C; ++c)
-      sum += sPart[c];
-   const double inv = sum > 0.0 ? 1.0 / sum : 1.0;
+   {
+      WideSum u;
+      u.hi = sPart[c].x;
+      u.lo = sPart[c].y;
+      all.Add(u);
+   }
+   const double sum = all.Value(), inv = sum > 0.0 ? 1.0 / sum : 1.0;
    for (int i = tid; i < nItems; i += kFoldThreads)
    {
       if (i + kFoldThreads < nItems)

@@ -207,3 +207,22 @@ def test_folded_planes_vs_oracle(engine, oracle, M, size, n):
             want = oracle.psf_planes(sets[set_of[i]], dz[i:i + 1] * 1e-9, size=size, normalize=normalize)
             assert _max_rel(got[i:i + 1], want) <= TOL, (i, normalize)
     plan.close()
+
+
+def test_planes_do_not_depend_on_how_many_share_the_call(engine):
+    """A normalized plane's bits are the same from a call of 4 planes (a cluster of CTAs each), of 40 and of 200 (a CTA
+    each): 2e8 samples, of which a normalization one place off would round some differently."""
+    import torch
+    p = PsfParams(wavelength_nm=670.0, na=1.4, sample_index=1.33, sample_depth_nm=300.0, pixel_size_nm=100.0,
+                  zernike=[0.0] * 5 + [0.06] * 7 + [0.0] * 16, oversampling=3, kernel_half_width_px=8, nz=3,
+                  pupil_samples=64)
+    n, size = 200, 1001
+    dz = np.linspace(-500.0, 500.0, n)
+    so = np.zeros(n, np.uint32)
+    whole = engine.psf_library_dev([p], so, dz, size=size)
+    off = 0
+    for step in (4, 40):
+        for k in range(0, n, step):
+            part = engine.psf_library_dev([p], so[k:k + step], dz[k:k + step], size=size)
+            off += int((part != whole[k:k + step]).sum())
+    assert off == 0, off
