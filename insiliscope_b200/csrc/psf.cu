@@ -257,14 +257,15 @@ __global__ void __launch_bounds__(kFoldThreads, 2) CztFoldKernel(const SetParams
                                                                  const double3* __restrict__ tables,
                                                                  const float2* __restrict__ cs,
                                                                  const PsfItem* __restrict__ items, int M, int P,
-                                                                 int normalize, float* __restrict__ out)
+                                                                 int normalize, int split, double2* __restrict__ sums,
+                                                                 float* __restrict__ out)
 {
    namespace cg = cooperative_groups;
    cg::cluster_group cluster = cg::this_cluster();
    const int C = static_cast<int>(cluster.num_blocks()), rank = static_cast<int>(cluster.block_rank());
-   const int psf = blockIdx.x / C, tid = threadIdx.x;
+   const int psf = blockIdx.x / (C * split), part = blockIdx.x / C % split, tid = threadIdx.x;
    const Fold F(M, P);
-   const int Q = F.Q, R = F.R, nT = F.nT, pitch = F.Pitch(), share = F.Share(C), tp = share | 1;
+   const int Q = F.Q, R = F.R, nT = F.nT, pitch = F.Pitch(), share = F.Share(C * split), tp = share | 1;
    extern __shared__ __align__(16) unsigned char smem[];
    float4* U = reinterpret_cast<float4*>(smem);         // [q][row]: (P.re, P.im, N.re, N.im) of the column pair q
    float4* T = U + static_cast<size_t>(Q + 1) * R;      // [row][own pair]: the samples at +t and -t
@@ -273,7 +274,7 @@ __global__ void __launch_bounds__(kFoldThreads, 2) CztFoldKernel(const SetParams
    const SetParams& sp = sets[it.set];
    const double3* tab = tables + static_cast<size_t>(it.set) * M * M;
    const float2* ct = cs + static_cast<size_t>(it.set) * Q * pitch;
-   const int t0 = rank * share, own = max(0, min(share, nT - t0));
+   const int t0 = (part * C + rank) * share, own = max(0, min(share, nT - t0));
    cluster.sync();   // every CTA's shared memory is there to be written
    // the pupil (phase = k0 (opd1 + ni (ti - ti0) opd3F) + zernike + mask, ZernikePsf.cpp:240-248, float64 then reduced),
    // folded on both axes
@@ -380,7 +381,7 @@ __global__ void __launch_bounds__(kFoldThreads, 2) CztFoldKernel(const SetParams
          sr[0][k] = si[0][k] = sr[1][k] = si[1][k] = 0.f;
       }
       const float4* c4 = reinterpret_cast<const float4*>(ct + g);
-#pragma unroll 3
+#pragma unroll 2
       for (int q = 1; q <= Q; ++q, c4 += pitch / 2)
       {
          const float4 p = T[q * tp + c], n = T[(Q + q) * tp + c];
@@ -417,15 +418,22 @@ __global__ void __launch_bounds__(kFoldThreads, 2) CztFoldKernel(const SetParams
          }
       }
       local.Add(item);
-      if (!normalize || i + kFoldThreads < nItems)
+      if (!normalize || split > 1 || i + kFoldThreads < nItems)
          store(i);   // the last item stays in registers for its normalization
    }
    if (!normalize)
       return;
-   const WideSum part = BlockWideSum(local, sRed);
+   const WideSum mine = BlockWideSum(local, sRed);
+   if (split > 1)
+   {
+      // several clusters' plane: NormalizeFoldKernel goes on
+      if (tid == 0)
+         sums[blockIdx.x] = make_double2(mine.hi, mine.lo);
+      return;
+   }
    if (tid == 0)
       for (int c = 0; c < C; ++c)
-         cluster.map_shared_rank(sPart, c)[rank] = make_double2(part.hi, part.lo);
+         cluster.map_shared_rank(sPart, c)[rank] = make_double2(mine.hi, mine.lo);
    cluster.sync();
    WideSum all;
    for (int c = 0; c < C; ++c)
@@ -466,11 +474,30 @@ __global__ void __launch_bounds__(kFoldThreads, 2) CztFoldKernel(const SetParams
    }
 }
 
+// The planes that several clusters shared, by the `parts` sums that their CTAs left. grid (any, nPsf).
+__global__ void __launch_bounds__(256) NormalizeFoldKernel(float* __restrict__ planes, const double2* __restrict__ sums,
+                                                           int parts, int planeElems)
+{
+   WideSum all;
+   for (int c = 0; c < parts; ++c)
+   {
+      const double2 v = sums[blockIdx.y * parts + c];
+      WideSum u;
+      u.hi = v.x;
+      u.lo = v.y;
+      all.Add(u);
+   }
+   const double sum = all.Value(), inv = sum > 0.0 ? 1.0 / sum : 1.0;
+   float* p = planes + static_cast<size_t>(blockIdx.y) * planeElems;
+   for (int i = blockIdx.x * 256 + threadIdx.x; i < planeElems; i += gridDim.x * 256)
+      p[i] = static_cast<float>(p[i] * inv);
+}
+
 // ------------------------------------------------------------------------------------------ large pupils
-// When the pupil and the row pass do not fit shared memory (M beyond ~128: a widefield kernel's 512-sample pupil),
-// the same products go through global memory: the pupil phasors U (nPsf x M x M), then two batched complex GEMMs
-// with 64 x 64 output tiles staged 16 deep in shared memory -- T = A U, E = T A^T -- the second one ending in |E|^2
-// and the plane's float64 sum.
+// When the folded pupil and row pass do not fit a cluster's shared memory (M beyond ~165: a widefield kernel's 512
+// samples), the same products go through global memory: the pupil phasors U (nPsf x M x M), then two batched complex
+// GEMMs with 64 x 64 output tiles staged 16 deep in shared memory -- T = A U, E = T A^T -- the second one ending in
+// |E|^2 and the plane's float64 sum.
 __global__ void PupilKernel(const SetParams* __restrict__ sets, const double3* __restrict__ tables,
                             const PsfItem* __restrict__ items, int M, float2* __restrict__ U)
 {
@@ -591,20 +618,34 @@ static int FoldCluster(const Fold& F, uint32_t nPsf, int smCount)
    return c;
 }
 
+// Clusters of kFoldMaxCluster CTAs that share a plane: as many as leave each CTA eight column pairs and take no more than
+// three quarters of the SMs (16 clusters of CTAs that fill an SM do not all find eight SMs in one GPC at once: eight
+// planes of 513 x 513 from 128 pupil samples 151 us on a cluster each, 174 on two). One plane of 1,001 x 1,001 from 64
+// samples, a plan's call: 211 us on one cluster, 75 on seven (90 through global memory, which small plans took).
+static int FoldSplit(const Fold& F, int cluster, uint32_t nPsf, int smCount)
+{
+   if (cluster < kFoldMaxCluster)
+      return 1;
+   const uint64_t ctas = static_cast<uint64_t>(nPsf) * kFoldMaxCluster;
+   return static_cast<int>(std::max<uint64_t>(
+      1, std::min<uint64_t>(static_cast<uint64_t>(smCount) * 3 / 4 / ctas,
+                            static_cast<uint64_t>(F.nT / (8 * kFoldMaxCluster)))));
+}
+
 bool FoldFits(int M, int P) { return Fold(M, P).Bytes(kFoldMaxCluster) <= kFoldMaxBytes; }
 
 // The folded FP32 chirp-Z over its tables (cs).
 static int LaunchCztFold(iscu_ctx* ctx, const SetParams* dSets, const double3* dTab, const float2* cs,
-                         const PsfItem* dItems, uint32_t nPsf, int M, int P, int normalize, float* out)
+                         const PsfItem* dItems, uint32_t nPsf, int M, int P, int normalize, double2* sums, float* out)
 {
    const Fold F(M, P);
-   const int c = FoldCluster(F, nPsf, ctx->smCount);
+   const int c = FoldCluster(F, nPsf, ctx->smCount), split = FoldSplit(F, c, nPsf, ctx->smCount);
    ISCU_CK(cudaFuncSetAttribute(CztFoldKernel, cudaFuncAttributeMaxDynamicSharedMemorySize,
                                 static_cast<int>(kFoldMaxBytes)));
    cudaLaunchConfig_t cfg = {};
-   cfg.gridDim = dim3(nPsf * static_cast<uint32_t>(c));
+   cfg.gridDim = dim3(nPsf * static_cast<uint32_t>(c * split));
    cfg.blockDim = dim3(kFoldThreads);
-   cfg.dynamicSmemBytes = F.Bytes(c);
+   cfg.dynamicSmemBytes = F.Bytes(c * split);
    cfg.stream = ctx->stream;
    cudaLaunchAttribute attr = {};
    attr.id = cudaLaunchAttributeClusterDimension;
@@ -612,8 +653,14 @@ static int LaunchCztFold(iscu_ctx* ctx, const SetParams* dSets, const double3* d
    attr.val.clusterDim.y = attr.val.clusterDim.z = 1;
    cfg.attrs = &attr;
    cfg.numAttrs = 1;
-   ISCU_CK(cudaLaunchKernelEx(&cfg, CztFoldKernel, dSets, dTab, cs, dItems, M, P, normalize, out));
+   ISCU_CK(cudaLaunchKernelEx(&cfg, CztFoldKernel, dSets, dTab, cs, dItems, M, P, normalize, split, sums, out));
    ISCU_CK_LAUNCH(ctx, "CztFoldKernel");
+   if (split > 1 && normalize)
+   {
+      NormalizeFoldKernel<<<dim3(std::max<uint32_t>(1, 2 * static_cast<uint32_t>(ctx->smCount) / nPsf), nPsf), 256, 0,
+                            ctx->stream>>>(out, sums, c * split, P * P);
+      ISCU_CK_LAUNCH(ctx, "NormalizeFoldKernel");
+   }
    return ISCU_OK;
 }
 
@@ -783,7 +830,7 @@ int BuildPsfLibrary(iscu_ctx* ctx, const iscu_psf_request* sets, uint32_t nSets,
    // One buffer: the sets and the items (one copy), the tables, the matrices. The context keeps it up to kPsfScratchKept
    // bytes (calls hold the context's lock and end synchronized): five allocations and frees a call took 20 to 500 us.
    const size_t inBytes = (setBytes + itemBytes + 255) / 256 * 256, tabEnd = inBytes + (tabBytes + 255) / 256 * 256;
-   const size_t aEnd = tabEnd + (matBytes + 255) / 256 * 256, allBytes = folded ? aEnd : aEnd + matBytes;
+   const size_t aEnd = tabEnd + (matBytes + 255) / 256 * 256, allBytes = aEnd + (folded ? kFoldSumBytes : matBytes);
    DevBuf own;
    DevBuf& buf = allBytes <= kPsfScratchKept ? ctx->psfScratch : own;
    ISCU_CK(buf.Reserve(allBytes));
@@ -800,7 +847,8 @@ int BuildPsfLibrary(iscu_ctx* ctx, const iscu_psf_request* sets, uint32_t nSets,
    int rc = LaunchPsfTables(ctx, dSets, nSets, M, P, dTab, dA, dAt, folded);
    if (rc == ISCU_OK)
       rc = split ? LaunchCztSplit(ctx, method, dSets, dTab, dA, nSets, dItems, nPsf, M, P, normalize, out)
-                 : LaunchCztFp32(ctx, dSets, dTab, dA, dAt, dItems, nPsf, M, P, normalize, out);
+                 : LaunchCztFp32(ctx, dSets, dTab, dA, dAt, reinterpret_cast<double2*>(base + aEnd), dItems, nPsf, M, P,
+                                 normalize, out);
    if (rc != ISCU_OK)
       return rc;
    // The temporaries are another call's, or freed, when this returns; the stream must finish with them first.
@@ -851,10 +899,10 @@ int LaunchPsfTables(iscu_ctx* ctx, const SetParams* dSets, uint32_t nSets, int M
 // The plain FP32 chirp-Z of nPsf items over prepared tables (the folded form where FoldFits, else the global-memory
 // form for pupils beyond shared memory).
 int LaunchCztFp32(iscu_ctx* ctx, const SetParams* dSets, const double3* dTab, const float2* dA, const float2* dAt,
-                  const PsfItem* dItems, uint32_t nPsf, int M, int P, int normalize, float* out)
+                  double2* sums, const PsfItem* dItems, uint32_t nPsf, int M, int P, int normalize, float* out)
 {
    if (FoldFits(M, P))
-      return LaunchCztFold(ctx, dSets, dTab, dA, dItems, nPsf, M, P, normalize, out);
+      return LaunchCztFold(ctx, dSets, dTab, dA, dItems, nPsf, M, P, normalize, sums, out);
    return LaunchCztGlobalFp32(ctx, dSets, dTab, dA, dAt, dItems, nPsf, M, P, normalize, out);
 }
 
@@ -882,7 +930,7 @@ int LaunchPsfPipelineFp32(iscu_ctx* ctx, const SetParams* dSets, const PsfItem* 
    if (rc == ISCU_OK)
       rc = LaunchPsfTables(ctx, dSets, nSets, M, P, dTab, dA, dAt, true);
    if (rc == ISCU_OK)
-      rc = LaunchCztFold(ctx, dSets, dTab, dA, dItems, nPsf, M, P, normalize, out);
+      rc = LaunchCztFold(ctx, dSets, dTab, dA, dItems, nPsf, M, P, normalize, nullptr, out);   // (P <= 129: no split)
    return rc;
 }
 

@@ -91,8 +91,10 @@ int LaunchPsfTables(iscu_ctx* ctx, const SetParams* dSets, uint32_t nSets, int M
                     float2* dAt, bool folded);
 // Whether planes of P samples from M pupil samples run as the folded shared-memory kernel.
 bool FoldFits(int M, int P);
+// sums: kFoldSumBytes for the sums of planes that several clusters share (an entry per CTA, no more than the SMs).
+constexpr size_t kFoldSumBytes = 1024 * 16;
 int LaunchCztFp32(iscu_ctx* ctx, const SetParams* dSets, const double3* dTab, const float2* dA, const float2* dAt,
-                  const PsfItem* dItems, uint32_t nPsf, int M, int P, int normalize, float* out);
+                  double2* sums, const PsfItem* dItems, uint32_t nPsf, int M, int P, int normalize, float* out);
 
 int PrepareSetParams(const iscu_psf_request* sets, uint32_t nSets, int32_t size, uint32_t maxSets, SetParams* out,
                      int* M, int* P);

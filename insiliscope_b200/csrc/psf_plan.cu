@@ -15,7 +15,7 @@ struct iscu_psf_plan
    iscu_ctx* ctx = nullptr;
    int M = 0, P = 0, method = 0;
    uint32_t nSets = 0;
-   iscu::DevBuf sets, tab, A, At, ahat, items, setOf, defocus, out, err;
+   iscu::DevBuf sets, tab, A, At, ahat, items, setOf, defocus, out, err, sums;
 };
 
 namespace iscu {
@@ -62,7 +62,7 @@ int RunDev(iscu_psf_plan* p, const uint32_t* setOf, const double* defocusNm, uin
       return LaunchCztTf32x3Core(ctx, p->sets.as<SetParams>(), p->ahat.as<float>(), static_cast<int>(p->nSets),
                                  p->items.as<PsfItem>(), n, p->M, p->P, normalize, out, p->err.as<int>());
    return LaunchCztFp32(ctx, p->sets.as<SetParams>(), p->tab.as<double3>(), p->A.as<float2>(), p->At.as<float2>(),
-                        p->items.as<PsfItem>(), n, p->M, p->P, normalize, out);
+                        p->sums.as<double2>(), p->items.as<PsfItem>(), n, p->M, p->P, normalize, out);
 }
 
 int Check(iscu_psf_plan* p)
@@ -115,6 +115,7 @@ int iscu_psf_plan_create(iscu_ctx* ctx, const iscu_psf_request* sets, uint32_t n
    ISCU_CK(p->A.Reserve(n_sets * std::max<size_t>(P, 2) * M * sizeof(float2)));
    ISCU_CK(p->At.Reserve(n_sets * P * M * sizeof(float2)));
    ISCU_CK(p->err.Reserve(sizeof(int)));
+   ISCU_CK(p->sums.Reserve(kFoldSumBytes));
    ISCU_CK(cudaMemcpyAsync(p->sets.p, hs.data(), n_sets * sizeof(SetParams), cudaMemcpyHostToDevice, ctx->stream));
    rc = LaunchPsfTables(ctx, p->sets.as<SetParams>(), n_sets, p->M, p->P, p->tab.as<double3>(), p->A.as<float2>(),
                         p->At.as<float2>(), method == ISCU_CZT_FP32 && FoldFits(p->M, p->P));

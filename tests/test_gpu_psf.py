@@ -210,8 +210,8 @@ def test_folded_planes_vs_oracle(engine, oracle, M, size, n):
 
 
 def test_planes_do_not_depend_on_how_many_share_the_call(engine):
-    """A normalized plane's bits are the same from a call of 4 planes (a cluster of CTAs each), of 40 and of 200 (a CTA
-    each): 2e8 samples, of which a normalization one place off would round some differently."""
+    """A normalized plane's bits are the same from a call of one plane (several clusters of CTAs), of 4 and 40 (a cluster
+    each) and of 200 (a CTA each): 2e8 samples, of which a normalization one place off would round some differently."""
     import torch
     p = PsfParams(wavelength_nm=670.0, na=1.4, sample_index=1.33, sample_depth_nm=300.0, pixel_size_nm=100.0,
                   zernike=[0.0] * 5 + [0.06] * 7 + [0.0] * 16, oversampling=3, kernel_half_width_px=8, nz=3,
@@ -221,8 +221,52 @@ def test_planes_do_not_depend_on_how_many_share_the_call(engine):
     so = np.zeros(n, np.uint32)
     whole = engine.psf_library_dev([p], so, dz, size=size)
     off = 0
-    for step in (4, 40):
-        for k in range(0, n, step):
+    for step in (1, 4, 40):
+        for k in range(0, n if step > 1 else 40, step):
             part = engine.psf_library_dev([p], so[k:k + step], dz[k:k + step], size=size)
             off += int((part != whole[k:k + step]).sum())
     assert off == 0, off
+
+
+def test_one_large_plane_is_shared_by_more_than_a_cluster(engine):
+    """A plan's call for one plane of 1,001 x 1,001 takes at most two and a half times that for one of 129 x 129 (four
+    and a half when one cluster of CTAs worked it out)."""
+    import time
+    import torch
+    from insiliscope_b200.engine import PsfPlan
+    p = PsfParams(wavelength_nm=670.0, na=1.4, pixel_size_nm=100.0, oversampling=3, kernel_half_width_px=8, nz=3,
+                  pupil_samples=64)
+    times = []
+    for size in (129, 1001):
+        plan = PsfPlan(engine, [p], size=size)
+        so, dz = torch.zeros(1, dtype=torch.int32, device="cuda"), torch.zeros(1, dtype=torch.float64, device="cuda")
+        out = torch.empty((1, size, size), dtype=torch.float32, device="cuda")
+        best = 1e9
+        for _ in range(30):
+            t = time.perf_counter()
+            plan.run_dev(so, dz, out)
+            best = min(best, time.perf_counter() - t)
+        times.append(best)
+        plan.close()
+    assert times[1] <= 2.5 * times[0], times
+
+
+@pytest.mark.parametrize("M,size,n", [(150, 200, 2), (160, 175, 3), (164, 111, 20), (166, 79, 1), (64, 1001, 1),
+                                      (32, 700, 2), (100, 513, 1)])
+def test_large_pupils_and_planes_vs_oracle(engine, oracle, M, size, n):
+    """The folded form at pupils of 129 samples and more, up to where its shared memory ends on a cluster of eight, and
+    at planes that several clusters share: the oracle within the files' tolerance, library and plan alike."""
+    from insiliscope_b200.engine import PsfPlan
+    rng = np.random.default_rng(M + size)
+    p = PsfParams(wavelength_nm=670.0, na=1.4, sample_index=1.33, sample_depth_nm=300.0, pixel_size_nm=100.0,
+                  zernike=[0.0] * 3 + list(rng.normal(0.0, 0.08, 25)), oversampling=3, kernel_half_width_px=8, nz=3,
+                  pupil_samples=M)
+    dz, so = rng.uniform(-500.0, 500.0, n), np.zeros(n, np.uint32)
+    plan = PsfPlan(engine, [p], size=size)
+    for normalize in (True, False):
+        got = engine.psf_library_dev([p], so, dz, size=size, normalize=normalize).cpu().numpy()
+        assert np.array_equal(plan.run(so, dz, normalize=normalize), got)
+        for i in {0, n - 1}:
+            want = oracle.psf_planes(p, dz[i:i + 1] * 1e-9, size=size, normalize=normalize)
+            assert _max_rel(got[i:i + 1], want) <= TOL, (i, normalize)
+    plan.close()
