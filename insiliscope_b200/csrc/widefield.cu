@@ -1230,8 +1230,10 @@ int YLines(const LinePlan& P)
 }
 // Threads of a y CTA, and its lines by them: 128 with half the lines where those fill it, four CTAs an SM instead of two
 // of 256, so that more of them are at different phases (loads, groups, stores): 64 planes of 512 x 512 px, 1,024-point
-// lines, a series 957 -> 943 us.
-int YThreads(const LinePlan& P) { return P.logN <= 11 ? kThreads / 2 : kThreads; }
+// lines, a series 957 -> 943 us. Both y passes, 256 threads and 128: 256-point lines (64 planes of 200 columns) 27.5 and
+// 23.3 us, 512 (40 planes of 400) 49.1 and 45.0, 1,024 86 and 84, 2,048 (24 planes of 250) 149 and 145, 4,096 (16 planes
+// of 250) 190 and 186; 8,192, one line a CTA either way, 41 and 45.
+int YThreads(const LinePlan& P) { return P.logN <= 12 ? kThreads / 2 : kThreads; }
 // Fewer lines per CTA where a volume's CTAs would leave SMs idle: `lines` halved, to no fewer than `least`, while
 // `planes` planes of `total` lines make fewer than `want` CTAs. A convolution of 186 x 151 x 11 cells on a 256 x 256 x
 // 16 grid (110 CTAs in x, 55 in y; 32 of 256 threads busy in z with 32 columns a block) takes 50.0 us with full CTAs,

@@ -249,3 +249,18 @@ def test_scene_plan_full_size_against_reference(engine, reference):
     errs = [_rel(got[f], want[i]) for i, f in enumerate(foci)]
     print("widefield 512x512x64 vs the reference scene, foci", foci, "max rel error", errs)
     assert max(errs) <= TOL
+
+
+@pytest.mark.parametrize("vol_shape,grid", [((2, 3500, 20), (32, 4096, 4)), ((1, 5000, 12), (16, 8192, 4))])
+def test_long_lines_vs_oracle(engine, vol_shape, grid):
+    """y lines of 4,096 and 8,192 points (a y CTA of 128 and of 256 threads) against the float64 oracle."""
+    import torch
+    rng = np.random.default_rng(vol_shape[1])
+    vol = rng.random(vol_shape).astype(np.float32)
+    vol[vol < 0.7] = 0.0
+    psf = rng.random((1, 9, 5)).astype(np.float32) - 0.2
+    plan = WidefieldPlan(engine, vol_shape, psf)
+    assert plan.grid() == grid
+    got = plan.convolve_dev(torch.from_numpy(vol).cuda()).cpu().numpy()
+    assert _rel(got, np.maximum(fft_convolve_same_f64(vol, psf), 0.0)) <= TOL
+    plan.close()
