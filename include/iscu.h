@@ -508,7 +508,7 @@ int iscu_nll_model_create(iscu_ctx* ctx, const iscu_nll_spec* spec, iscu_nll_mod
 void iscu_nll_model_destroy(iscu_nll_model* model);
 int iscu_nll_model_info(iscu_nll_model* model, double* kappa, int32_t* n_zern);
 /* NLL of n_emitters ROIs (params_dev: n x (x, y, z, N) float; frame_dev: each ROI's frame < n_frames; bg_dev:
- * n_frames float; zern: n_zern float64, host or device; counts_dev: n x roi x roi float) into *nll_dev (float64, device);
+ * n_frames float; zern: n_zern float64, host or this device; counts_dev: n x roi x roi float) into *nll_dev (float64, device);
  * mu_dev (nullable): the expected counts. With grad_params_dev (n x 4 float: dNLL/dx, /dy, /dz, /dN) the adjoint
  * runs too (the field recomputed, no per-emitter PSF stored): grad_bg_dev (n_frames float64) and grad_zern_dev
  * (n_zern float64) receive the rest. *err_dev (int32, device) = 1 when an emitter names a frame outside the batch.

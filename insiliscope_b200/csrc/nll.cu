@@ -147,7 +147,7 @@ struct NllArgs
    const double* basis;
    const float* cs;          // the folded transform's cosines and sines (NllTables)
    const double* zphase;
-   int J, R, os;
+   int J, R;
    double kappa;
    uint32_t n;
    const float4* params;     // x, y (ROI px), z (nm), N
@@ -852,7 +852,11 @@ int iscu_nll_eval_dev(iscu_nll_model* model, uint32_t n_emitters, const float* p
       if (cudaPointerGetAttributes(&where, zern) != cudaSuccess)
          cudaGetLastError();   // not a pointer that CUDA knows: the host's
       if (where.type == cudaMemoryTypeDevice)
+      {
+         if (where.device != ctx->device)   // (refused by the copy that this was)
+            return Fail(ISCU_ERR_ARG, "the Zernike coefficients are on another device");
          pa.zernDev = zern;
+      }
       else
          std::copy(zern, zern + model->J, pa.zern);
    }
@@ -874,7 +878,6 @@ int iscu_nll_eval_dev(iscu_nll_model* model, uint32_t n_emitters, const float* p
    a.zphase = model->zphase.as<double>();
    a.J = model->J;
    a.R = model->spec.roi;
-   a.os = model->spec.os;
    a.kappa = model->kappa;
    a.n = n_emitters;
    a.params = reinterpret_cast<const float4*>(params_dev);
