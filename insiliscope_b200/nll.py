@@ -144,6 +144,14 @@ def _poisson_function():
     """The autograd function (made on first use: torch is imported there)."""
     import torch
 
+    def scaled(g, go, x, plain):
+        if plain and g.device == x.device == go.device:
+            try:   # one launch; a batch of output gradients (is_grads_batched) does not write into a plain tensor
+                return torch.mul(g, go, out=torch.empty(g.shape, dtype=x.dtype, device=g.device))
+            except RuntimeError:
+                pass
+        return (g.to(x.device) * go.to(x.device)).to(x.dtype)
+
     class PoissonNll(torch.autograd.Function):
         """Where an input needs its gradient the forward pass runs the adjoint kernel, which evaluates the likelihood on
         its way, and the backward pass scales what it left (a likelihood pass before it recomputes every emitter's field
@@ -159,11 +167,11 @@ def _poisson_function():
 
         @staticmethod
         def backward(ctx, gout):
-            # go x g in float64, rounded to the input's type, for the inputs that want it (an integer input has no
-            # gradient; out-of-place products alone, so that a batch of gradients can run through: is_grads_batched)
+            # go x g in float64, rounded to the input's type, for the inputs that want it (an integer input has none)
             inputs, grads = ctx.saved_tensors[:3], ctx.saved_tensors[3:]
             go = gout.to(torch.float64).reshape(1)
-            return tuple((g.to(x.device) * go.to(x.device)).to(x.dtype) if wanted else None
+            plain = not (torch.is_grad_enabled() and go.requires_grad)
+            return tuple(scaled(g, go, x, plain) if wanted else None
                          for x, g, wanted in zip(inputs, grads, ctx.needs_input_grad)) + (None,)
 
     return PoissonNll
