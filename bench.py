@@ -1437,7 +1437,8 @@ class BinnedWorkload:
         return self.h_em.numel() + self.h_fr.numel(), self.h_adu.numel() * 2
 
     def kernel_name(self):
-        return "BinnedRenderKernel+noise"
+        dense = self.binned.dense_from(len(self.mv.emitters), self.mv.n_frames) > 0
+        return "BinnedDenseKernel+BinnedRenderKernel+noise" if dense else "BinnedRenderKernel+noise"
 
     def alg_bytes_per_launch(self):
         # the emitter records (32 B) and frame table, the photon frames written by the fill, read and written by the

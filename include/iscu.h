@@ -272,8 +272,9 @@ int iscu_render_frames(iscu_ctx* ctx, const iscu_emitter* emitters, uint32_t n_e
 /* The render kernel's form (no reference counterpart: the reference renders a frame per CPU task, ParallelFor over
  * frames, ScopeMovie.cpp:7059-7110). config % 3: the CTA's tile, 16x16, 32x8 or 8x32 pixels; (config / 3) % 2: one
  * CTA per (frame, tile), or a persistent grid that takes (frame, tile) items heaviest frame first (for batches whose
- * frames carry very different emitter counts). Configs 0..11 render in one pass, config / 6 emitters per step of a
- * pixel's loop (*paired 0 or 1); configs 12..17 in two passes (*paired 2): every emitter's float contribution to
+ * frames carry very different emitter counts). Configs 0..11 render in one pass, one or two emitters per step of a
+ * pixel's loop (*paired 0 or 1; a batch whose CTAs are all resident even so takes two in every grid form, whatever
+ * *paired says); configs 12..17 in two passes (*paired 2): every emitter's float contribution to
  * each pixel of its square first, computed by groups of emitters that read the same block sums (kernel slot, plane,
  * tap origin), then the tiles add them in emitter order. The two-pass forms keep up to a quarter of the device's
  * memory for contributions (n_emitters x square pixels floats); a batch beyond that renders in the one-pass form of
