@@ -524,23 +524,23 @@ __device__ __forceinline__ void GroupContrib(const ContribArgs& a, const KernelV
    }
 }
 
+// All of the CTA's warps, from either role's loop.
+__device__ __forceinline__ void RoleBarrier() { asm volatile("bar.sync 0;" ::: "memory"); }
+
 // blockDim.x = computing threads + one staging warp, three buffers: while the others compute item i, the staging warp
 // has item i + 1's emitters arriving, issues item i + 2's copy, whose chunk it asked for an item ago, and asks for item
 // i + 3's chunk and number i + 4, so that each of these round trips has an item's time. (Fetched one after the other
 // within an item they took longer than a short item's work.) An item is one block of computing threads' pixels of a
 // chunk, as many a chunk as its own slot's square has (as many as the largest square of all slots, 120,000 emitters of
 // 7 x 7 squares beside a stack of 81 x 81 took 205 us instead of 46). The two roles have a loop each: in one loop the
-// staging warp's variables made the others spill (118.8 us for the dSTORM movie's 35 M contributions, 114.7 without).
+// staging warp's variables made the others spill (35 M contributions 118.8 us, 114.7 without).
 //
-// What bounds it: the emitter loop, 86 cycles a warp's contribution and scheduler where its 20 float64 operations and
-// the conversion need 56 (a float64 operation issues every 2.35 cycles, a conversion takes 8.5); 54 instructions in all,
-// the FP64 pipe at 39 %. Taps, chunk and barriers are 20 % on the dSTORM movie, 9 % on the two-colour one. 35 M
-// contributions of the dSTORM movie 136 -> 122 us, 484 M of the two-colour movie 1.55 -> 1.27 ms against unfused sums
+// What bounds it: the emitter loop, some 84 cycles a warp's contribution and scheduler where its 20 float64 operations
+// and the conversion need 56 (a float64 operation issues every 2.35 cycles, a conversion takes 8.5); 54 instructions in
+// all, the FP64 pipe at 40 %. Taps, chunk and barriers are 20 % on the dSTORM movie, 9 % on the two-colour one. 35 M
+// contributions of the dSTORM movie 133 -> 115 us, 525 M of the two-colour movie 1.44 -> 1.24 ms against unfused sums
 // with each thread's own tap offsets. Building the float from the double's bits instead of converting, and two or four
 // emitters without a branch between them, measured 5 to 40 % slower (more integer instructions; spilled taps).
-// All of the CTA's warps, from either role's loop.
-__device__ __forceinline__ void RoleBarrier() { asm volatile("bar.sync 0;" ::: "memory"); }
-
 __global__ void __launch_bounds__(kMaxCT + 32, kContribPerSm) ContribKernel(ContribArgs a)
 {
    __shared__ CStage sE[3][kE];
