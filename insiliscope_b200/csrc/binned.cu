@@ -88,8 +88,10 @@ struct Staged
 };
 
 // grid (ceil(W / 16), ceil(H / 16), frames). Frame k's emitters are emitters[em_start, em_start + em_count) cut at
-// nEm. img / alone: frames x H x W, +=. denseFrom: frames of that many emitters and more are the dense kernel's (0: none).
-template <int U>
+// nEm. img / alone: frames x H x W, +=. kSparse: frames of denseFrom emitters and more are the dense kernel's (the test in
+// every call's kernel made the compiler hold it to 32 registers: 20 frames of 93 x 58 px, 2,010 emitters each, 228 -> 239
+// us).
+template <int U, bool kSparse>
 __global__ void __launch_bounds__(kThreads) BinnedRenderKernel(const iscu_emitter* __restrict__ em, uint32_t nEm,
                                                               const iscu_frame* __restrict__ frames,
                                                               uint32_t denseFrom, const float* __restrict__ K, int nz,
@@ -107,7 +109,7 @@ __global__ void __launch_bounds__(kThreads) BinnedRenderKernel(const iscu_emitte
    const int reachY0 = max(-R, ty0 - R), reachY1 = min(gh + R - 1, ty0 + kSide * U - 1 + R);
    const iscu_frame fr = frames[blockIdx.z];
    const uint32_t start = min(fr.em_start, nEm), end = min(start + fr.em_count, nEm);
-   if (denseFrom && end > start && end - start >= denseFrom)
+   if (kSparse && end > start && end - start >= denseFrom)
       return;
    const int cx = px * U, cy = py * U;   // this pixel's first cell
    double acc[U][U];
@@ -570,6 +572,24 @@ __global__ void __launch_bounds__(kThreads, kBuffers) BinnedDenseKernel(
    }
 }
 
+using PixelFn = void (*)(const iscu_emitter*, uint32_t, const iscu_frame*, uint32_t, const float*, int, int, int,
+                         uint32_t, uint32_t, float*, float*);
+template <bool kSparse>
+PixelFn PixelOf(int u)
+{
+   switch (u)
+   {
+   case 1: return BinnedRenderKernel<1, kSparse>;
+   case 2: return BinnedRenderKernel<2, kSparse>;
+   case 3: return BinnedRenderKernel<3, kSparse>;
+   case 4: return BinnedRenderKernel<4, kSparse>;
+   case 5: return BinnedRenderKernel<5, kSparse>;
+   case 6: return BinnedRenderKernel<6, kSparse>;
+   case 7: return BinnedRenderKernel<7, kSparse>;
+   default: return BinnedRenderKernel<8, kSparse>;
+   }
+}
+
 using DenseFn = void (*)(const iscu_emitter*, uint32_t, const iscu_frame*, uint32_t, const float*, int, int, int,
                          uint32_t, uint32_t, float*, float*);
 DenseFn DenseOf(int R) { return DensePitch(R) == 128 ? BinnedDenseKernel<128, 2> : BinnedDenseKernel<192, 1>; }
@@ -777,21 +797,9 @@ int iscu_binned_render_dev(iscu_binned* b, const iscu_emitter* emitters_dev, uin
       ISCU_CK_LAUNCH(ctx, "BinnedDenseKernel");
    }
    const dim3 grid((b->W + kSide - 1) / kSide, (b->H + kSide - 1) / kSide, n_frames);
-#define ISCU_BINNED_LAUNCH(UU)                                                                                          \
-   BinnedRenderKernel<UU><<<grid, kThreads, 0, ctx->stream>>>(emitters_dev, n_emitters, frames_dev, denseFrom, K,    \
-                                                              b->nz, b->R, b->pitch, b->W, b->H, img_dev, alone_dev)
-   switch (b->u)
-   {
-   case 1: ISCU_BINNED_LAUNCH(1); break;
-   case 2: ISCU_BINNED_LAUNCH(2); break;
-   case 3: ISCU_BINNED_LAUNCH(3); break;
-   case 4: ISCU_BINNED_LAUNCH(4); break;
-   case 5: ISCU_BINNED_LAUNCH(5); break;
-   case 6: ISCU_BINNED_LAUNCH(6); break;
-   case 7: ISCU_BINNED_LAUNCH(7); break;
-   default: ISCU_BINNED_LAUNCH(8); break;
-   }
-#undef ISCU_BINNED_LAUNCH
+   const PixelFn fn = denseFrom ? PixelOf<true>(b->u) : PixelOf<false>(b->u);
+   fn<<<grid, kThreads, 0, ctx->stream>>>(emitters_dev, n_emitters, frames_dev, denseFrom, K, b->nz, b->R, b->pitch,
+                                          b->W, b->H, img_dev, alone_dev);
    ISCU_CK_LAUNCH(ctx, "BinnedRenderKernel");
    return ISCU_OK;
 }
