@@ -14,8 +14,8 @@
 // planes; R = KernelWidefieldPsf::Radius (:288-298) capped by the halo cut; or, without a kernel, the normalized
 // Gaussian of sigma_px u (BinnedBlinks.cpp:190-212), made on the host with the same std::exp calls.
 //
-// Render (BinnedBlinks.cpp:216-246), one CTA per 16 x 16 pixels of one frame, one thread per pixel holding its u x u
-// cells: the frame's emitters are examined 256 at a time, those whose cell lies in the padded grid and within R of
+// Render (BinnedBlinks.cpp:216-246; dense frames further down), one CTA per 16 x 16 pixels of one frame, one thread per
+// pixel holding its u x u cells: the frame's emitters are examined 256 at a time, those whose cell lies in the padded grid and within R of
 // the tile staged in shared memory in event order, and every thread adds each staged emitter to its cells.
 
 #include "iscu_internal.h"
