@@ -1014,9 +1014,12 @@ int ReserveContrib(iscu_ctx* ctx, uint32_t nEm, ContribScratch& sc)
    // it grows, within the limit.
    const uint64_t most = ctx->contribLimit / (G.S * sizeof(float));
    const uint64_t more = std::min<uint64_t>(std::min<uint64_t>(most, 0xFFFFFFFFu), nEm + nEm / (sc.buf.p ? 8u : 32u));
-   if (more > nEm && sc.buf.Reserve(ContribLayout(G, static_cast<uint32_t>(more)).bytes) == cudaSuccess)
-      return ISCU_OK;
-   cudaGetLastError();
+   if (more > nEm)
+   {
+      if (sc.buf.Reserve(ContribLayout(G, static_cast<uint32_t>(more)).bytes) == cudaSuccess)
+         return ISCU_OK;
+      cudaGetLastError();   // no room for more than asked for
+   }
    ISCU_CK(sc.buf.Reserve(ContribLayout(G, nEm).bytes));
    return ISCU_OK;
 }
